@@ -11,6 +11,7 @@ from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libasrq_b200.so")
+NATIVE_PATH = os.path.join(_PKG, "_native.so")
 
 F16, BF16 = 0, 1
 WS_A16_GEMV, WS_A16_GEMM, WS_W4A4_GEMM, WS_LINEARQ = 1, 2, 3, 4
@@ -94,9 +95,9 @@ def load() -> ctypes.CDLL:
     global _lib
     if _lib is not None:
         return _lib
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(NATIVE_PATH):
         raise ImportError(
-            f"{LIB_PATH} is missing: build it with `python -m asrq_b200.build` (needs nvcc). "
+            f"{LIB_PATH} or {NATIVE_PATH} is missing: build it with `python -m asrq_b200.build` (needs nvcc). "
             "asrq_b200 has no CPU or PyTorch fallback.")
     lib = ctypes.CDLL(LIB_PATH)
     for name, (res, args) in SIGNATURES.items():
@@ -116,12 +117,21 @@ def check(fn_name: str, code: int) -> None:
         raise AsrqError(fn_name, code, last_error())
 
 
-CALLS = 0  # C-ABI calls made through call() in this process (benchmarks count a step's launches with it)
+_calls = 0
+
+
+def __getattr__(name: str):
+    """``CALLS``: C-ABI calls made in this process, through :func:`call` or by the native module calls (benchmarks count a
+    step's launches with it)."""
+    if name == "CALLS":
+        from .linear import _native
+        return _calls + (0 if _native is None else _native.calls())
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def call(fn_name: str, *args) -> None:
-    global CALLS
-    CALLS += 1
+    global _calls
+    _calls += 1
     check(fn_name, getattr(load(), fn_name)(*args))
 
 

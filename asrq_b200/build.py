@@ -18,6 +18,7 @@ import sys
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libasrq_b200.so")
+NATIVE = os.path.join(PKG, "_native.so")  # the module calls' host path (csrc/host.cpp), a CPython extension on torch's C++ API
 OBJ_DIR = os.path.join(PKG, "build")
 
 SOURCES = ["api.cu", "gemv_a16.cu", "gemv_a16_splitk.cu", "gemv_a16_staged.cu", "gemm_a16_tc.cu", "gemm_a16_tc2.cu", "gemm_a16_skinny.cu", "act_quant.cu", "glue.cu", "offline.cu", "dense_head.cu", "w4a4_mma.cu", "w4a4_tc.cu"]
@@ -75,7 +76,27 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> st
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}")
+    _build_native(force or bool(procs))
     return LIB
+
+
+def _build_native(force: bool) -> None:
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    src = os.path.join(CSRC, "host.cpp")
+    if not force and _newer(NATIVE, [src, LIB, os.path.normpath(os.path.join(CSRC, "..", "..", "include", "asrq_b200.h"))]):
+        return
+    cuda = os.path.dirname(os.path.dirname(find_nvcc()))
+    tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [a for d in inc for a in ("-isystem", d)]
+    cmd += [src, "-o", NATIVE, "-L", PKG, "-lasrq_b200", "-L", tlib, "-ltorch_python", "-ltorch_cuda", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+            "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on host.cpp:\n{r.stdout}")
 
 
 if __name__ == "__main__":

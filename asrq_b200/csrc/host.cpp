@@ -1,0 +1,264 @@
+// The module calls' host path in native code.
+//
+// One eager LinearQ call spent 19 us in Python (attribute lookups through nn.Module, argument checks, an allocation, a
+// fifteen-argument ctypes call) around a launch of 2 us and, for decode sizes, a kernel of 4 us: a program calling layer
+// after layer was bound by the interpreter up to about 1500 tokens.  The functions here do the same work -- the same
+// checks, the same allocation, the same C-ABI call -- for the ordinary case, and return None for everything else (wrong
+// types, CPU tensors, other devices, non-contiguous operands, empty inputs, tensor subclasses, dispatch modes), which the
+// Python code then handles and reports exactly as before.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <atomic>
+
+#include "../../include/asrq_b200.h"
+
+namespace {
+
+std::atomic<long long> g_calls{0};   // C-ABI calls made here
+PyObject* g_workspaces = nullptr;    // linear._workspaces: (device index, stream) -> uint8 tensor
+PyObject* g_check = nullptr;         // _lib.check(function name, status): raises AsrqError
+
+struct Names {
+  PyObject *buffers, *weight, *scales, *zeros, *bias, *in_features, *out_features, *bits, *group_size, *hadamard, *operand, *w8, *w8_key;
+} N;
+
+bool intern_names() {
+  auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
+  N = {s("_buffers"), s("weight"), s("scales"), s("zeros"), s("bias"), s("in_features"), s("out_features"), s("bits"), s("group_size"),
+       s("hadamard"), s("operand"), s("_w8"), s("_w8_key")};
+  return !PyErr_Occurred();
+}
+
+// Plain strided tensors outside any tensor-subclass or dispatch mode; everything else takes the Python path.
+inline const at::Tensor* plain(PyObject* o) { return o && THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+inline bool modes_active() {
+  return at::impl::PythonTorchFunctionTLS::stack_len() != 0 || c10::impl::TorchDispatchModeTLS::any_modes_set();
+}
+inline bool int_of(PyObject* dict, PyObject* name, long long* out) {
+  PyObject* v = PyDict_GetItemWithError(dict, name);
+  if (!v || !PyLong_Check(v)) return false;
+  *out = PyLong_AsLongLong(v);
+  return true;
+}
+
+struct Layer {
+  const at::Tensor *weight, *scales, *zeros, *bias;  // bias NULL: none
+  PyObject* dict;
+  long long k, n, bits, group;
+};
+
+// The layer's operands as module attributes hold them (registered buffers, or plain attributes).  False: not the ordinary case.
+bool layer_of(PyObject* self, const c10::Device& dev, Layer* L) {
+  PyObject** dp = _PyObject_GetDictPtr(self);
+  if (!dp || !*dp) return false;
+  PyObject* d = L->dict = *dp;
+  PyObject* buf = PyDict_GetItemWithError(d, N.buffers);
+  if (!buf || !PyDict_Check(buf)) return false;
+  auto operand = [&](PyObject* name, PyObject** obj) {
+    *obj = PyDict_GetItemWithError(buf, name);
+    if (!*obj) *obj = PyDict_GetItemWithError(d, name);
+    return *obj != nullptr;
+  };
+  PyObject *w, *s, *z, *b;
+  if (!operand(N.weight, &w) || !operand(N.scales, &s) || !operand(N.zeros, &z) || !operand(N.bias, &b)) return false;
+  L->weight = plain(w);
+  L->scales = plain(s);
+  L->zeros = plain(z);
+  L->bias = b == Py_None ? nullptr : plain(b);
+  if (!L->weight || !L->scales || !L->zeros || (b != Py_None && !L->bias)) return false;
+  if (L->weight->scalar_type() != at::kByte || L->scales->scalar_type() != at::kHalf || L->zeros->scalar_type() != at::kHalf) return false;
+  for (const at::Tensor* t : {L->weight, L->scales, L->zeros})
+    if (t->device() != dev || !t->is_contiguous()) return false;
+  if (L->bias && (L->bias->scalar_type() != at::kHalf || L->bias->device() != dev)) return false;
+  return int_of(d, N.in_features, &L->k) && int_of(d, N.out_features, &L->n) && int_of(d, N.bits, &L->bits) && int_of(d, N.group_size, &L->group);
+}
+
+// fp16 / bf16 activations on the current CUDA device, contiguous, at least one row
+bool activations(PyObject* o, const at::Tensor** x, int* dtype) {
+  *x = plain(o);
+  if (!*x || !(*x)->is_cuda() || (*x)->dim() < 1 || !(*x)->is_contiguous() || (*x)->numel() == 0) return false;
+  const auto st = (*x)->scalar_type();
+  if (st != at::kHalf && st != at::kBFloat16) return false;
+  *dtype = st == at::kHalf ? ASRQ_F16 : ASRQ_BF16;
+  return (*x)->device().index() == c10::cuda::current_device() && !modes_active();
+}
+
+// The stream's workspace if it is there and large enough.
+bool workspace(int dev, cudaStream_t stream, size_t need, void** ptr, size_t* bytes) {
+  PyObject* key = PyTuple_New(2);
+  if (!key) return false;
+  PyTuple_SET_ITEM(key, 0, PyLong_FromLong(dev));
+  PyTuple_SET_ITEM(key, 1, PyLong_FromVoidPtr(stream));
+  PyObject* v = PyDict_GetItemWithError(g_workspaces, key);
+  Py_DECREF(key);
+  const at::Tensor* t = plain(v);
+  if (!t || size_t(t->numel()) < need) return false;
+  *ptr = t->data_ptr();
+  *bytes = size_t(t->numel());
+  return true;
+}
+
+at::Tensor output_like(const at::Tensor& x, int64_t n) {
+  c10::SmallVector<int64_t, 5> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = n;
+  return at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt);
+}
+
+PyObject* failed(const char* fn, int rc) {
+  PyObject* r = PyObject_CallFunction(g_check, "si", fn, rc);
+  Py_XDECREF(r);
+  if (r) PyErr_Format(PyExc_RuntimeError, "%s failed with status %d", fn, rc);
+  return nullptr;
+}
+
+// linearq_forward(layer, input, residual or None, gelu) -> output, or None: not the ordinary case
+PyObject* linearq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 4) {
+    PyErr_SetString(PyExc_TypeError, "linearq_forward(layer, input, residual, gelu)");
+    return nullptr;
+  }
+  const at::Tensor* x;
+  int dtype;
+  Layer L;
+  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x->device(), &L) || (L.bits != 2 && L.bits != 4) || x->size(-1) != L.k) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  const int64_t m = x->numel() / L.k;
+  const at::Tensor* res = nullptr;
+  if (a[2] != Py_None) {
+    res = plain(a[2]);
+    if (!res || res->scalar_type() != x->scalar_type() || res->device() != x->device() || res->numel() != m * L.n || !res->is_contiguous()) Py_RETURN_NONE;
+  }
+  const bool gelu = a[3] == Py_True;
+  const int dev = x->device().index();
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  void* ws;
+  size_t ws_bytes;
+  if (!workspace(dev, stream, asrq_workspace_bytes(ASRQ_WS_LINEARQ, m, L.n, L.k), &ws, &ws_bytes)) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;  // the Python path makes it
+  }
+  at::Tensor y = output_like(*x, L.n);
+  g_calls.fetch_add(1, std::memory_order_relaxed);
+  const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
+  int rc;
+  if (!res && !gelu)
+    rc = asrq_linearq_a16(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(), bias,
+                          y.data_ptr(), m, L.n, L.k, int(L.group), dtype, ws, ws_bytes, stream);
+  else
+    rc = asrq_linearq_a16_fused(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(),
+                                bias, res ? res->data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype, gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE, ws,
+                                ws_bytes, stream);
+  if (rc) return failed(!res && !gelu ? "asrq_linearq_a16" : "asrq_linearq_a16_fused", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// linearqq_forward(layer, input) -> output, or None
+PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 2) {
+    PyErr_SetString(PyExc_TypeError, "linearqq_forward(layer, input)");
+    return nullptr;
+  }
+  const at::Tensor* x;
+  int dtype;
+  Layer L;
+  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x->device(), &L) || x->size(-1) != L.k || L.group <= 0) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  PyObject* had_o = PyDict_GetItemWithError(L.dict, N.hadamard);
+  if (had_o != Py_True && had_o != Py_False) Py_RETURN_NONE;
+  const int had = had_o == Py_True;
+  const int64_t m = x->numel() / L.k;
+  const int dev = x->device().index();
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
+  void* ws;
+  size_t ws_bytes;
+  // the activation codes and their scales: one scratch allocation (codes first, the scales at the next multiple of 256 bytes)
+  auto scratch = [&](int64_t code_bytes) {
+    return at::detail::empty_cuda({(code_bytes + 255) / 256 * 256 + m * 4}, at::kByte, x->device(), std::nullopt);
+  };
+  if (m >= 64 && L.n % 128 == 0 && L.k % 128 == 0 && L.group % 128 == 0 && L.k % L.group == 0) {
+    PyObject* op = PyObject_GetAttr(a[0], N.operand);
+    if (!op) return nullptr;
+    const bool f8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "f8") == 0;
+    const bool i8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "int8") == 0;
+    // the prepared weight, if it was derived from this very buffer in this state
+    PyObject *w8_o = PyDict_GetItemWithError(L.dict, N.w8), *key = PyDict_GetItemWithError(L.dict, N.w8_key);
+    const at::Tensor* w8 = plain(w8_o);
+    const bool fresh = (f8 || i8) && w8 && w8->device() == x->device() && key && PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 4 &&
+                       PyLong_AsVoidPtr(PyTuple_GET_ITEM(key, 0)) == L.weight->data_ptr() &&
+                       PyLong_AsLongLong(PyTuple_GET_ITEM(key, 1)) == (long long)L.weight->_version() && PyUnicode_Compare(PyTuple_GET_ITEM(key, 3), op) == 0;
+    Py_DECREF(op);
+    if (PyErr_Occurred()) return nullptr;
+    if (!fresh || !workspace(dev, stream, 256, &ws, &ws_bytes)) Py_RETURN_NONE;
+    at::Tensor sc = scratch(m * L.k), y = output_like(*x, L.n);
+    uint8_t* a8 = static_cast<uint8_t*>(sc.data_ptr());
+    float* sa = reinterpret_cast<float*>(a8 + (m * L.k + 255) / 256 * 256);
+    g_calls.fetch_add(2, std::memory_order_relaxed);
+    int rc = (f8 ? asrq_hadamard_quant_f8 : asrq_hadamard_quant_int8)(x->data_ptr(), a8, sa, m, L.k, had, dtype, stream);
+    if (rc) return failed(f8 ? "asrq_hadamard_quant_f8" : "asrq_hadamard_quant_int8", rc);
+    rc = (f8 ? asrq_w4a4_gemm_f8 : asrq_w4a4_gemm_int8)(a8, sa, static_cast<const uint8_t*>(w8->data_ptr()), L.scales->data_ptr(), bias, y.data_ptr(), nullptr, m,
+                                                        L.n, L.k, int(L.group), dtype, ws, ws_bytes, stream);
+    if (rc) return failed(f8 ? "asrq_w4a4_gemm_f8" : "asrq_w4a4_gemm_int8", rc);
+    return THPVariable_Wrap(std::move(y));
+  }
+  if (!workspace(dev, stream, asrq_workspace_bytes(ASRQ_WS_W4A4_GEMM, m, L.n, L.k), &ws, &ws_bytes)) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  at::Tensor sc = scratch(m * (L.k / 2)), y = output_like(*x, L.n);
+  uint8_t* qa = static_cast<uint8_t*>(sc.data_ptr());
+  float* sa = reinterpret_cast<float*>(qa + (m * (L.k / 2) + 255) / 256 * 256);
+  g_calls.fetch_add(2, std::memory_order_relaxed);
+  int rc = asrq_hadamard_quant_int4(x->data_ptr(), qa, sa, m, L.k, had, dtype, stream);
+  if (rc) return failed("asrq_hadamard_quant_int4", rc);
+  rc = asrq_w4a4_gemm(qa, sa, static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), bias, y.data_ptr(), nullptr, m, L.n, L.k, int(L.group),
+                      dtype, ws, ws_bytes, stream);
+  if (rc) return failed("asrq_w4a4_gemm", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* calls(PyObject*, PyObject*) { return PyLong_FromLongLong(g_calls.load(std::memory_order_relaxed)); }
+
+// bind(workspaces dict, check function)
+PyObject* bind(PyObject*, PyObject* args) {
+  PyObject *ws, *check;
+  if (!PyArg_ParseTuple(args, "O!O", &PyDict_Type, &ws, &check)) return nullptr;
+  Py_INCREF(ws);
+  Py_INCREF(check);
+  Py_XDECREF(g_workspaces);
+  Py_XDECREF(g_check);
+  g_workspaces = ws;
+  g_check = check;
+  Py_RETURN_NONE;
+}
+
+PyMethodDef kMethods[] = {
+    {"linearq_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linearq_forward)), METH_FASTCALL, nullptr},
+    {"linearqq_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linearqq_forward)), METH_FASTCALL, nullptr},
+    {"calls", calls, METH_NOARGS, nullptr},
+    {"bind", bind, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return intern_names() ? PyModule_Create(&kModule) : nullptr; }

@@ -21,6 +21,12 @@ _CHECK = os.environ.get("ASRQ_B200_CHECK_STATUS", "0") == "1"
 # one scratch buffer per (device, stream): kernels on one stream run in order, so they can share it
 _workspaces: dict = {}
 
+try:  # the ordinary case of a module call in native code (csrc/host.cpp); built together with the library
+    from . import _native
+    _native.bind(_workspaces, _lib.check)
+except ImportError:  # not built: the first call raises (see _lib.load)
+    _native = None
+
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
@@ -247,12 +253,20 @@ class LinearQ(nn.Module):
             raise TypeError("LinearQ.bias must be float16 on the input's device")
 
     def forward(self, input):
+        if _native is not None and not _CHECK:
+            y = _native.linearq_forward(self, input, None, False)
+            if y is not None:
+                return y
         return self.forward_fused(input)
 
     def forward_fused(self, input, residual=None, gelu=False):
         """``forward`` with the step that follows the layer in a transformer block done in the kernel's
         epilogue: ``gelu(layer(input))`` or ``residual + layer(input)`` (``residual``: the output's shape and
         dtype).  Same bits as the unfused module sequence."""
+        if _native is not None and not _CHECK:
+            y = _native.linearq_forward(self, input, residual, bool(gelu))
+            if y is not None:
+                return y
         # fp16 / bf16 only (the reference computes in whatever dtype the input has, asrq/core/linear.py:58-59;
         # an fp32 input raises here rather than silently running a slower path)
         dt = _require_cuda_16bit(input, "LinearQ.forward")
@@ -369,6 +383,10 @@ class LinearQQ(LinearQ):
         return m >= 64 and n % 128 == 0 and k % 128 == 0 and g % 128 == 0 and k % g == 0
 
     def forward(self, input, acc_dump=None, two_call=False):
+        if acc_dump is None and not two_call and _native is not None and not _CHECK:
+            y = _native.linearqq_forward(self, input)
+            if y is not None:
+                return y
         _require_cuda_16bit(input, "LinearQQ")
         with _on_device(input.device):
             return self._forward(input, acc_dump, two_call)
