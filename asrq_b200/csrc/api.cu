@@ -16,7 +16,7 @@ namespace asrq {
 // kernels (one translation unit each)
 int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
              void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
-             size_t workspace_bytes, int sm_count, cudaStream_t stream, int max_split);
+             size_t workspace_bytes, int sm_count, cudaStream_t stream, int max_split, const Epilogue& ep, bool* fused);
 size_t gemv_workspace_bytes(int64_t N);
 size_t gemm_tc_workspace_bytes(int64_t M, int64_t N);
 int gemm_a16_tc(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
@@ -35,7 +35,12 @@ int qk_norm_rope(const void* qkv, const void* qw, const void* kw, const void* co
                  long long pos_host, void* q_out, void* k_cache, void* v_cache, int64_t B, int64_t T, int nq, int nkv, int hd,
                  int64_t max_len, float eps, int dtype, cudaStream_t stream);
 int decode_self_attention(const void* qkv, void* kv, const long long* pos_dev, void* out, int64_t B, int H, int hd, int64_t max_len,
-                          float scale, int dtype, cudaStream_t stream);
+                          float scale, int dtype, int sm_count, cudaStream_t stream);
+int decode_cross_attention(const void* q, const void* k, const void* v, void* out, int64_t B, int H, int hd, int64_t keys, int64_t row_stride,
+                           float scale, bool settled, int dtype, int sm_count, cudaStream_t stream);
+int decode_grouped_attention(const void* qkv, const void* qw, const void* kw, const void* cos_t, const void* sin_t, const long long* pos_dev,
+                             void* k_cache, void* v_cache, void* out, int64_t B, int nkv, int64_t max_len, float eps, float scale, int dtype,
+                             int sm_count, cudaStream_t stream);
 int dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, int dtype, int sm_count, cudaStream_t stream);
 int hadamard_quant_int4(const void* x, uint8_t* qa, float* sa, int64_t M, int64_t K, int hadamard, int dtype,
                         int out_int8, cudaStream_t stream);
@@ -295,7 +300,9 @@ size_t asrq_workspace_bytes(int kind, int64_t M, int64_t N, int64_t K) {
 
 static int a16_gemv(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                     void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
-                    size_t workspace_bytes, void* stream) {
+                    size_t workspace_bytes, void* stream, const Epilogue& ep = Epilogue(), bool* fused = nullptr) {
+  bool fused_here = false;
+  if (!fused) fused = &fused_here;
   last_error().clear();
   int rc = check_a16_common(bits == 4 ? "asrq_w4a16_gemv" : "asrq_w2a16_gemv", x, w, scales, zeros, y, M, N, K, dtype,
                             workspace);
@@ -304,7 +311,7 @@ static int a16_gemv(int bits, const void* x, const uint8_t* w, const void* scale
   if ((rc = device_facts(&f))) return rc;
   if (M == 0) return ASRQ_OK;
   return gemv_a16(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes,
-                  f->sm_count, static_cast<cudaStream_t>(stream), kGemvMaxSplit);
+                  f->sm_count, static_cast<cudaStream_t>(stream), kGemvMaxSplit, ep, fused);
 }
 
 static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
@@ -377,7 +384,7 @@ static int linearq_a16(int bits, const void* x, const uint8_t* w, const void* sc
     rc = a16_gemm(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream,
                   ep, &fused);
   else
-    rc = a16_gemv(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream);
+    rc = a16_gemv(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream, ep, &fused);
   if (rc || !want_ep || fused || M == 0) return rc;
   // the kernel that ran does not fuse the epilogue: one more pass over the output
   const DeviceFacts* f;
@@ -479,7 +486,44 @@ int asrq_decode_self_attention(const void* qkv, void* kv_cache, const int64_t* p
   if ((rc = device_facts(&f))) return rc;
   if (B == 0) return ASRQ_OK;
   return decode_self_attention(qkv, kv_cache, reinterpret_cast<const long long*>(pos_device), out, B, n_heads, head_dim, max_len, scale,
-                               dtype, static_cast<cudaStream_t>(stream));
+                               dtype, f->sm_count, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_decode_cross_attention(const void* q, const void* k, const void* v, void* out, int64_t B, int n_heads, int head_dim, int64_t keys,
+                                int64_t row_stride, float scale, int kv_settled, int dtype, void* stream) {
+  last_error().clear();
+  if (!q || !k || !v || !out) return fail(ASRQ_ERR_NULL, "asrq_decode_cross_attention: no pointer may be NULL");
+  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_decode_cross_attention: dtype %d", dtype);
+  if (B < 0 || n_heads <= 0 || (head_dim != 64 && head_dim != 128) || keys <= 0 || keys > (1 << 24) || row_stride % 8 || row_stride < head_dim ||
+      B * n_heads > (int64_t(1) << 28))
+    return fail(ASRQ_ERR_SHAPE, "asrq_decode_cross_attention: B=%lld heads=%d head_dim=%d (64 or 128) keys=%lld row_stride=%lld (a multiple of 8)",
+                (long long)B, n_heads, head_dim, (long long)keys, (long long)row_stride);
+  if (!aligned16(k) || !aligned16(v)) return fail(ASRQ_ERR_ALIGN, "asrq_decode_cross_attention: k and v must be 16-byte aligned");
+  const DeviceFacts* f;
+  int rc;
+  if ((rc = device_facts(&f))) return rc;
+  if (B == 0) return ASRQ_OK;
+  return decode_cross_attention(q, k, v, out, B, n_heads, head_dim, keys, row_stride, scale, kv_settled != 0, dtype, f->sm_count, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_decode_grouped_attention(const void* qkv, const void* q_weight, const void* k_weight, const void* cos_table, const void* sin_table,
+                                  const int64_t* pos_device, void* k_cache, void* v_cache, void* out, int64_t B, int n_q_heads, int n_kv_heads,
+                                  int head_dim, int64_t max_len, float eps, float scale, int dtype, void* stream) {
+  last_error().clear();
+  if (!qkv || !q_weight || !k_weight || !cos_table || !sin_table || !pos_device || !k_cache || !v_cache || !out)
+    return fail(ASRQ_ERR_NULL, "asrq_decode_grouped_attention: no pointer may be NULL");
+  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_decode_grouped_attention: dtype %d", dtype);
+  if (B < 0 || n_kv_heads <= 0 || n_q_heads != 2 * n_kv_heads || head_dim != 128 || max_len <= 0 || B * n_kv_heads > (int64_t(1) << 28))
+    return fail(ASRQ_ERR_SHAPE, "asrq_decode_grouped_attention: B=%lld heads=%d/%d (two query heads per key head) head_dim=%d (128) max_len=%lld",
+                (long long)B, n_q_heads, n_kv_heads, head_dim, (long long)max_len);
+  for (const void* q : {q_weight, k_weight, cos_table, sin_table, static_cast<const void*>(k_cache), static_cast<const void*>(v_cache)})
+    if (!aligned16(q)) return fail(ASRQ_ERR_ALIGN, "asrq_decode_grouped_attention: norm weights, tables and caches must be 16-byte aligned");
+  const DeviceFacts* f;
+  int rc;
+  if ((rc = device_facts(&f))) return rc;
+  if (B == 0) return ASRQ_OK;
+  return decode_grouped_attention(qkv, q_weight, k_weight, cos_table, sin_table, reinterpret_cast<const long long*>(pos_device), k_cache, v_cache, out, B,
+                                  n_kv_heads, max_len, eps, scale, dtype, f->sm_count, static_cast<cudaStream_t>(stream));
 }
 
 int asrq_dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, int dtype, void* stream) {

@@ -81,6 +81,12 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
   return v;
 }
 
+// A constant half through the read-only path.  cuda_fp16.h's __ldg(const __half*) is a non-volatile asm statement, which the
+// compiler may run ahead of the null check that guards an optional bias (seen: an illegal access); this is a load to it.
+__device__ __forceinline__ float ldg_half(const __half* p) {
+  return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short*>(p))));
+}
+
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 

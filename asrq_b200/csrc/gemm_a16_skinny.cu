@@ -208,7 +208,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
       // ------------------------------ epilogue (warps 2-5: lane quadrants 2, 3, 0, 1) ------------------------------
       const int qd = warp & 3;
       const int f = ft * 128 + qd * 32 + lane;
-      const float bias = p.bias ? __half2float(__ldg(p.bias + f)) : 0.f;
+      const float bias = p.bias ? ldg_half(p.bias + f) : 0.f;
       // one decision for the warp, and the lanes together again after the polling loop: the tensor-memory loads
       // below are warp-wide instructions
       if (__all_sync(0xffffffffu, tc::mbar_wait(accf_bar, 0u, p.status, 35))) {

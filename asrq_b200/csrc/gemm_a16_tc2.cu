@@ -203,7 +203,7 @@ gemm_a16_tc2_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_consta
     const int fp = unit % p.n_fpairs, tt = unit / p.n_fpairs;
     const int f = (2 * fp + int(rank)) * 128 + (warp & 3) * 32 + lane;
     t2_drain<BF16>(p.y + size_t(tt) * p.bt * p.N + f, p.N, p.M - tt * p.bt, p.bt / 32,
-                   p.bias ? __half2float(__ldg(p.bias + f)) : 0.f,
+                   p.bias ? ldg_half(p.bias + f) : 0.f,
                    tmem_base + (uint32_t((warp & 3) * 32) << 16) + buf * 256u, ch0, step);
   };
   // a helper that is not an epilogue warp: wait for the last unit's accumulator, drain its share

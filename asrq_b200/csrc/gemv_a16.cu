@@ -45,6 +45,9 @@ struct GemvParams {
   const __half* bias;
   uint16_t* y;
   int M, N, K, groups_per_row, KQ, CPW, bf16;  // CPW repeats the kernel's template argument
+  // fused steps either side of the layer (see Epilogue): residual addition or activation
+  const uint16_t* residual;
+  int act;
   int R;                                       // rounds (LOOP variants): a warp takes R runs of CPW steps, KQ * CPW steps apart
   unsigned long long* trace;  // builds with -DASRQ_TRACE: per-warp clock marks (8 words per warp), NULL otherwise
 };
@@ -189,6 +192,8 @@ gemv_a16_kernel(const GemvParams p) {
     load_group_table<NG>(p.scales + o1, s1);
     load_group_table<NG>(p.zeros + o1, z1);
   };
+  uint16_t res_first = 0;
+  float bias_first = 0.f;
   uint32_t qa[CPW][4], qb[CPW][4], ts0[4], tz0[4], ts1[4], tz1[4];
 #pragma unroll 1
   for (int rd = 0; rd < rounds; ++rd) {
@@ -206,7 +211,15 @@ gemv_a16_kernel(const GemvParams p) {
     }
     load_tables(step0, ts0, tz0, ts1, tz1);
   }
-  if (rd == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (rd == 0) {
+    // the bias and the residual of this warp's first output register, fetched under the arithmetic
+    if (p.bias && p.KQ > 1 && warp < FR) bias_first = ldg_half(p.bias + n_base + g + ((warp >> 1) & 1) * 8);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.residual && p.KQ > 1 && warp < FR) {
+      const int n = n_base + g + ((warp >> 1) & 1) * 8, m = 8 * (warp >> 2) + 2 * c + (warp & 1);
+      if (m < p.M) res_first = p.residual[size_t(m) * p.N + n];
+    }
+  }
   if (TRACE && lane == 0) tr[2] = gemv_clock();
 
   // XC: sum of x over each of the warp's groups for tokens 0 and 1, the same in every lane.  The
@@ -346,6 +359,20 @@ gemv_a16_kernel(const GemvParams p) {
 
   // ---- add the KQ partial tiles through shared memory (fixed order) and write the strip ---------
   // yv[mh][r] of lane (g, c): weight row n_base + g + 8*(r>>1), token 8*mh + 2c + (r&1).
+  auto put = [&](float v, int n, int m, bool first) {
+    if (m >= p.M) return;
+    const size_t idx = size_t(m) * p.N + n;
+    if (p.bias) {
+      if (!first) bias_first = ldg_half(p.bias + n);
+      v += bias_first;
+    }
+    uint16_t y16 = float_to_out16(v, p.bf16);
+    if (p.act != kActNone || p.residual) {
+      if (p.residual && !first) res_first = p.residual[idx];
+      y16 = epilogue16(y16, p.act, p.residual != nullptr, res_first, p.bf16);
+    }
+    p.y[idx] = y16;
+  };
   if (p.KQ > 1) {
 #pragma unroll
     for (int mh = 0; mh < MH; ++mh)
@@ -353,27 +380,18 @@ gemv_a16_kernel(const GemvParams p) {
       for (int r = 0; r < 4; ++r) red[(warp * FR + mh * 4 + r) * 32 + lane] = yv[mh][r];
     __syncthreads();
     if (TRACE && lane == 0) tr[6] = gemv_clock();
-    for (int f = warp; f < FR; f += p.KQ) {  // warp f adds register f of every warp, in warp order
+    auto total = [&](int f) {  // register f of every warp, in warp order
       float v = 0.f;
       for (int q = 0; q < p.KQ; ++q) v += red[(q * FR + f) * 32 + lane];
-      const int n = n_base + g + ((f >> 1) & 1) * 8, m = 8 * (f >> 2) + 2 * c + (f & 1);
-      if (m < p.M) {
-        if (p.bias) v += __half2float(__ldg(p.bias + n));
-        p.y[size_t(m) * p.N + n] = float_to_out16(v, p.bf16);
-      }
-    }
+      return v;
+    };
+    for (int f = warp; f < FR; f += p.KQ)
+      put(total(f), n_base + g + ((f >> 1) & 1) * 8, 8 * (f >> 2) + 2 * c + (f & 1), f == warp);
   } else {
 #pragma unroll
     for (int mh = 0; mh < MH; ++mh)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int n = n_base + g + (r >> 1) * 8, m = 8 * mh + 2 * c + (r & 1);
-        if (m < p.M) {
-          float v = yv[mh][r];
-          if (p.bias) v += __half2float(__ldg(p.bias + n));
-          p.y[size_t(m) * p.N + n] = float_to_out16(v, p.bf16);
-        }
-      }
+      for (int r = 0; r < 4; ++r) put(yv[mh][r], n_base + g + (r >> 1) * 8, 8 * mh + 2 * c + (r & 1), false);
   }
   if (TRACE && lane == 0) tr[7] = gemv_globaltimer();
 }
@@ -547,9 +565,19 @@ int launch_gemv(const GemvSplit& sp, const GemvParams& p, cudaStream_t stream) {
 
 }  // namespace
 
+namespace {
+int groups_per_step(int bits, int group_size) {  // 1, 2 or 4; 0: not in this kernel's menu
+  const int chunk = (128 / bits) * 4;
+  const int gps = group_size > 0 && chunk % group_size == 0 ? chunk / group_size : 0;
+  return gps == 1 || gps == 2 || gps == 4 ? gps : 0;
+}
+}  // namespace
+
+// *fused: whether `ep` was applied.
 int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros,
              const void* bias, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype,
-             void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, int max_split) {
+             void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, int max_split, const Epilogue& ep, bool* fused) {
+  *fused = false;
   const int chunk = (128 / bits) * 4;
   if (N % 16 || K % chunk || group_size <= 0 || K % group_size || group_size % (128 / bits))
     return fail(ASRQ_ERR_SHAPE,
@@ -561,7 +589,7 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
   if (workspace_bytes < gemv_workspace_bytes(N, max_split))
     return fail(ASRQ_ERR_WORKSPACE, "w%da16 gemv: workspace %zu < %zu bytes", bits, workspace_bytes,
                 gemv_workspace_bytes(N, max_split));
-  const int gps = chunk % group_size == 0 ? chunk / group_size : 0;  // groups per step: 1, 2 or 4
+  const int gps = groups_per_step(bits, group_size);
   // Staged variant (gemv_a16_staged.cu): weights prefetched into shared memory ahead of the stream dependency,
   // up to 32 tokens per launch.  Measured no faster than the kernel below, so it runs only on request.
   const int which = option(kOptGemvKernel);
@@ -582,7 +610,7 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
 #else
   const bool trace = false;
 #endif
-  if (force_splitk || (gps != 1 && gps != 2 && gps != 4) || !aligned16(scales) || !aligned16(zeros))
+  if (force_splitk || !gps || !aligned16(scales) || !aligned16(zeros))
     return gemv_a16_splitk(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace,
                            workspace_bytes, sm_count, stream, max_split);
   // one split per token-count class (the kernel variant, hence its occupancy, depends on it):
@@ -605,14 +633,17 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
   p.K = int(K);
   p.groups_per_row = int(K / group_size);
   p.bf16 = dtype == ASRQ_BF16;
+  p.act = ep.act;
+  *fused = true;
   // diagnostic marks go to the (otherwise unused) partial-sum area of the workspace
   p.trace = trace ? reinterpret_cast<unsigned long long*>(static_cast<char*>(workspace) + kPartialOffset) : nullptr;
   for (int64_t m0 = 0; m0 < M; m0 += 16) {
     const int mb = int(std::min<int64_t>(16, M - m0));
     p.x = static_cast<const uint16_t*>(x) + m0 * K;
     p.y = static_cast<uint16_t*>(y) + m0 * N;
+    p.residual = ep.residual ? static_cast<const uint16_t*>(ep.residual) + m0 * N : nullptr;
     p.M = mb;
-    const GemvSplit& sp = split[mb <= 2 ? 0 : (mb <= 8 ? 1 : 2)];
+    const GemvSplit& sp = split[mb <= 8 ? (mb <= 2 ? 0 : 1) : 2];
     p.KQ = sp.KQ;
     p.CPW = sp.CPW;
     p.R = sp.R;

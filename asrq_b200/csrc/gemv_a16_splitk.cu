@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_a16_kernel(const GemvPar
     const int m = 8 * (fi >> 2) + 2 * (l & 3) + (fi & 1);
     if (n < p.N && m < p.M) {
       if (p.S == 1) {
-        if (p.bias) v += __half2float(__ldg(p.bias + n));
+        if (p.bias) v += ldg_half(p.bias + n);
         p.y[size_t(m) * p.N + n] = float_to_out16(v, p.bf16);
       } else {
         __stcg(p.partials + (size_t(blockIdx.y) * MR + m) * p.N + n, v);
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_a16_kernel(const GemvPar
         v += a0; v += a1; v += a2; v += a3;
       }
       for (; s < p.S; ++s) v += __ldcg(src + s * sstride);
-      if (p.bias) v += __half2float(__ldg(p.bias + n));
+      if (p.bias) v += ldg_half(p.bias + n);
       p.y[size_t(m) * p.N + n] = float_to_out16(v, p.bf16);
     }
   }

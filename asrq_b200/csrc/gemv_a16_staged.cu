@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * st_warps(MH), 2) gemv_a16_staged_kernel(c
     const int n = (tile0 + tl) * 16 + (ln >> 2) + ((f >> 1) & 1) * 8;
     const int m = tg * 8 * MH + 8 * (f >> 2) + 2 * (ln & 3) + (f & 1);
     if (m < p.M) {
-      if (p.bias) v += __half2float(__ldg(p.bias + n));
+      if (p.bias) v += ldg_half(p.bias + n);
       p.y[size_t(m) * p.N + n] = float_to_out16(v, p.bf16);
     }
   }

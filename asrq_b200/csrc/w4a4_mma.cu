@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(128) w4a4_mma_kernel(const W4A4Params p) {
         const int n0 = n_base + 8 * fn + 2 * c;
         float v0 = accf[fm][fn][2 * h] * s, v1 = accf[fm][fn][2 * h + 1] * s;
         if (p.bias) {
-          v0 += __half2float(__ldg(p.bias + n0));
-          v1 += __half2float(__ldg(p.bias + n0 + 1));
+          v0 += ldg_half(p.bias + n0);
+          v1 += ldg_half(p.bias + n0 + 1);
         }
         const uint32_t o = uint32_t(float_to_out16(v0, p.bf16)) | (uint32_t(float_to_out16(v1, p.bf16)) << 16);
         *reinterpret_cast<uint32_t*>(p.y + size_t(m) * p.N + n0) = o;

@@ -360,7 +360,7 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
         if (++buf == uint32_t(p.nbuf)) { buf = 0; aph ^= 1u; }
       }
       if (!ok) break;
-      const float bias = p.bias ? __half2float(__ldg(p.bias + f)) : 0.f;
+      const float bias = p.bias ? ldg_half(p.bias + f) : 0.f;
 #pragma unroll
       for (int ch = 0; ch < NCH; ++ch) {
         if (ch < nch) {

@@ -154,6 +154,36 @@ def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.
     return out
 
 
+def decode_cross_attention(q: torch.Tensor, kv: torch.Tensor, heads: int, scale: float = 1.0, settled: bool = False) -> torch.Tensor:
+    """Cross-attention of one decoding step: ``q`` (B, d), ``kv`` (B, T, 2 d) with keys and values side by side (a fused
+    projection's output).  Returns (B, d).  ``settled``: ``kv`` is older than the kernels just ahead on the stream (a step's cross
+    keys are), so it may be fetched while these still run."""
+    dt = _require_cuda_16bit(q, "decode_cross_attention")
+    B, T, d2 = kv.shape
+    d = d2 // 2
+    q2 = q.reshape(B, d)
+    q2 = q2 if q2.is_contiguous() else q2.contiguous()
+    out = torch.empty((B, d), dtype=q.dtype, device=q.device)
+    with _on_device(q.device):
+        _lib.call("asrq_decode_cross_attention", q2.data_ptr(), kv.data_ptr(), kv.data_ptr() + 2 * d, out.data_ptr(), B, heads, d // heads, T,
+                  2 * d, float(scale), int(settled), dt, torch.cuda.current_stream(q.device).cuda_stream)
+    return out
+
+
+def decode_grouped_attention(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
+                             k_cache: torch.Tensor, v_cache: torch.Tensor, pos: torch.Tensor, n_q: int, eps: float, scale: float) -> torch.Tensor:
+    """:func:`qk_norm_rope` for one new position and the attention over the cache in one kernel: ``qkv`` (B, (n_q + 2 n_kv) * 128),
+    caches (B, n_kv, max_len, 128), ``pos`` a one-element int64 CUDA tensor; two query heads per key head.  Returns (B, n_q * 128)."""
+    dt = _require_cuda_16bit(qkv, "decode_grouped_attention")
+    B, nkv, max_len, hd = k_cache.shape
+    out = torch.empty((B, n_q * hd), dtype=qkv.dtype, device=qkv.device)
+    with _on_device(qkv.device):
+        _lib.call("asrq_decode_grouped_attention", qkv.data_ptr(), q_weight.data_ptr(), k_weight.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                  pos.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), B, n_q, nkv, hd, max_len, float(eps), float(scale), dt,
+                  torch.cuda.current_stream(qkv.device).cuda_stream)
+    return out
+
+
 def dense_head(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
     """``x @ weight.T`` for the floating-point output head of a decoding step (``weight`` is (vocabulary, K) in the
     activations' 16-bit type): this library's kernel for up to 32 rows of ``x`` and K a multiple of 32 up to 3200,

@@ -23,7 +23,7 @@ import torch.nn.functional as F
 
 from . import packing
 from .convert import linearq_from_linear
-from .linear import LinearQ, add_rmsnorm, dense_head, qk_norm_rope, silu_mul
+from .linear import LinearQ, add_rmsnorm, decode_grouped_attention, dense_head, qk_norm_rope, silu_mul
 from .whisper import _cat_linearq
 
 try:
@@ -212,24 +212,34 @@ class Qwen3Engine:
         return [L[k] for L in self.layers for k in ("qkv", "o", "gu", "down")]
 
     # ---- one block ------------------------------------------------------------------------------
-    def _block(self, L, x, delta, kc, vc, pos0: int, pos_t, T: int, mask):
+    def _block(self, L, x, delta, kc, vc, pos0: int, T: int):
         """x: (B*T, H) residual stream, delta: pending residual contribution or None.  Writes keys and values of the
-        T new positions into the caches (at pos0.., or at the device-side position pos_t when decoding under a
-        graph) and returns (x', delta') with delta' = the block's MLP output, still to be added."""
+        T new positions into the caches from pos0 on and returns (x', delta') with delta' = the block's MLP output, still
+        to be added."""
         B = x.shape[0] // T
         x, h = add_rmsnorm(x, delta, L["ln1"], self.eps)
         # per-head q/k norms, rotary embedding and the cache write of the new positions: one kernel
-        q = qk_norm_rope(L["qkv"](h), L["qn"], L["kn"], self.cos, self.sin, kc, vc, pos0 if pos_t is None else pos_t, B, T,
-                         self.nq, self.nkv, self.eps)
-        if pos_t is None:
-            keys, vals = kc[:, :, :pos0 + T], vc[:, :, :pos0 + T]
-        else:  # one new position whose index lives on the device: attend over the whole cache under a mask
-            keys, vals = kc, vc
-        a = F.scaled_dot_product_attention(q, keys, vals, attn_mask=mask, is_causal=(mask is None and T > 1),
+        q = qk_norm_rope(L["qkv"](h), L["qn"], L["kn"], self.cos, self.sin, kc, vc, pos0, B, T, self.nq, self.nkv, self.eps)
+        a = F.scaled_dot_product_attention(q, kc[:, :, :pos0 + T], vc[:, :, :pos0 + T], is_causal=T > 1,
                                            enable_gqa=self.nq != self.nkv)
         a = a.transpose(1, 2).reshape(B * T, self.nq * self.hd)
         att = L["o"](a)
         x, h = add_rmsnorm(x, att, L["ln2"], self.eps)
+        return x, L["down"](silu_mul(L["gu"](h)))
+
+    def _block_step(self, L, x, delta, kc, vc, mask):
+        """:meth:`_block` for one new position per sequence, which lives on the device: q/k norm, rotary embedding, cache write
+        and attention are one kernel for heads of 128 in pairs (Qwen3's), else the prompt's kernel and a masked attention."""
+        B = x.shape[0]
+        x, h = add_rmsnorm(x, delta, L["ln1"], self.eps)
+        qkv = L["qkv"](h)
+        if self.hd == 128 and self.nq == 2 * self.nkv:
+            a = decode_grouped_attention(qkv, L["qn"], L["kn"], self.cos, self.sin, kc, vc, self.pos, self.nq, self.eps, self.hd ** -0.5)
+        else:
+            q = qk_norm_rope(qkv, L["qn"], L["kn"], self.cos, self.sin, kc, vc, self.pos, B, 1, self.nq, self.nkv, self.eps)
+            a = F.scaled_dot_product_attention(q, kc, vc, attn_mask=mask, enable_gqa=self.nq != self.nkv)
+            a = a.transpose(1, 2).reshape(B, self.nq * self.hd)
+        x, h = add_rmsnorm(x, L["o"](a), L["ln2"], self.eps)
         return x, L["down"](silu_mul(L["gu"](h)))
 
     def _final(self, x, delta):
@@ -262,7 +272,7 @@ class Qwen3Engine:
         x = inputs_embeds.to(device=dev, dtype=dt).reshape(B * T, H).contiguous()
         delta = None
         for i, L in enumerate(self.layers):
-            x, delta = self._block(L, x, delta, self.kc[i], self.vc[i], 0, None, T, None)
+            x, delta = self._block(L, x, delta, self.kc[i], self.vc[i], 0, T)
         h = self._final(x, delta).view(B, T, H)[:, -1]
         logits = dense_head(h.contiguous(), self.head)
         self.pos.fill_(T)
@@ -278,7 +288,7 @@ class Qwen3Engine:
         mask = (torch.arange(self.max_len, device=self.device) <= self.pos).view(1, 1, 1, self.max_len)
         delta = None
         for i, L in enumerate(self.layers):
-            x, delta = self._block(L, x, delta, self.kc[i], self.vc[i], 0, self.pos, 1, mask)
+            x, delta = self._block_step(L, x, delta, self.kc[i], self.vc[i], mask)
         h = self._final(x, delta)
         logits = dense_head(h, self.head)
         self.last_logits.copy_(logits)

@@ -30,7 +30,7 @@ import torch.nn.functional as F
 
 from . import packing
 from .convert import linearq_from_linear
-from .linear import LinearQ, add_layernorm, decode_self_attention, dense_head
+from .linear import LinearQ, add_layernorm, decode_cross_attention, decode_self_attention, dense_head
 
 try:  # the model classes need transformers; the engine does not
     from transformers.models.whisper.modeling_whisper import (WhisperAttention, WhisperConfig, WhisperDecoder,
@@ -214,6 +214,8 @@ class WhisperEngine:
     """
 
     fused_self_attention = os.environ.get("ASRQ_B200_WHISPER_FUSED_SELF_ATTENTION", "1") == "1"
+    # Cross-attention of a step: this library's kernel up to this many (sequence, head) pairs, the vendor library's above.
+    own_cross_attention_items = int(os.environ.get("ASRQ_B200_WHISPER_OWN_CROSS_ITEMS", "296"))
     cross_kv_views = os.environ.get("ASRQ_B200_WHISPER_CROSS_KV_VIEWS", "1") == "1"
 
     def __init__(self, config, device, dtype=torch.float16):
@@ -435,9 +437,12 @@ class WhisperEngine:
             x = L["out"].forward_fused(a, residual=x)
             h = L["lnx"](x)
             q = L["xq"](h)
-            if not L["xq_folded"]:
-                q = q * scaling
-            a = self._attend(q, self.k_cross[i], self.v_cross[i], self.heads_d)
+            if self.cross_kv_views and hd in (64, 128) and b * self.heads_d <= self.own_cross_attention_items:
+                a = decode_cross_attention(q, self.xkv[i], self.heads_d, 1.0 if L["xq_folded"] else scaling, settled=True).unsqueeze(1)
+            else:
+                if not L["xq_folded"]:
+                    q = q * scaling
+                a = self._attend(q, self.k_cross[i], self.v_cross[i], self.heads_d)
             x = L["xout"].forward_fused(a, residual=x)
             h = L["ln2"](x)
             x = L["fc2"].forward_fused(L["fc1"].forward_fused(h, gelu=True), residual=x)

@@ -215,6 +215,28 @@ int asrq_decode_self_attention(const void* qkv, void* kv_cache, const int64_t* p
                                int head_dim, int64_t max_len, float scale, int dtype, void* stream);
 
 /*
+ * The cross-attention of one decoding step: one query per sequence and head against `keys` given keys and values.  q, out:
+ * B x (n_heads * head_dim); key t of sequence b and head h at k + (b * keys + t) * row_stride + h * head_dim values, the value
+ * likewise at v: what a fused key/value projection of the encoder states leaves ([k | v] rows: row_stride 2 * n_heads *
+ * head_dim, v = k + n_heads * head_dim).  kv_settled: 1 allows k and v to be read ahead of the stream
+ * dependency -- no kernel of this library that the stream may still be running writes them; 0 is always right.
+ * head_dim 64 or 128; k and v 16-byte aligned.
+ */
+int asrq_decode_cross_attention(const void* q, const void* k, const void* v, void* out, int64_t B, int n_heads, int head_dim, int64_t keys,
+                                int64_t row_stride, float scale, int kv_settled, int dtype, void* stream);
+
+/*
+ * The self-attention of one decoding step of a grouped-query decoder with what surrounds it: per-head RMS norm of queries and
+ * keys, rotary embedding, the cache write at *pos_device, and the attention over positions 0..pos.  qkv, the tables and the
+ * caches as for asrq_qk_norm_rope with T = 1; out: B x (n_q_heads * head_dim).  n_q_heads = 2 n_kv_heads, head_dim 128.
+ * The cache below the position is read ahead of the stream dependency: calls of this function may follow each other at once,
+ * other kernels of this library that write the cache (asrq_qk_norm_rope) need an ordinary kernel or copy in between.
+ */
+int asrq_decode_grouped_attention(const void* qkv, const void* q_weight, const void* k_weight, const void* cos_table, const void* sin_table,
+                                  const int64_t* pos_device, void* k_cache, void* v_cache, void* out, int64_t B, int n_q_heads, int n_kv_heads,
+                                  int head_dim, int64_t max_len, float eps, float scale, int dtype, void* stream);
+
+/*
  * The floating-point output head of a decoding step: y[M, N] = x[M, K] . w[N, K]^T, all of the 16-bit type `dtype`,
  * fp32 accumulation, for M <= 32 tokens and a vocabulary-sized N (any N >= 1).  The reference keeps these layers as
  * nn.Linear (proj_out, asrq/models/transformers/whisper.py:268; lm_head, asrq/models/nemo/canary_qwen.py:179); after
