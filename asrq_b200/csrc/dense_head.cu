@@ -6,8 +6,12 @@
 // activations and logits).  The decode kernel's skeleton without the unpacking: a warp owns 16 weight rows, every
 // lane reads 16 bytes of rows g and g + 8 per 32-wide K step straight from global memory (its own fragment of
 // mma.sync.m16n8k16 under a fixed permutation of k inside the step, which the activation fragments follow), the
-// activations sit in shared memory for the whole block, accumulation in fp32.  Four steps of loads are in flight
-// per warp before the first is used.
+// activations sit in shared memory for the whole block, accumulation in fp32.
+//
+// Shared memory, MMAs and the loads in flight follow the number of token tiles (NT: 8, 16 or 32 tokens).  With one form for
+// 32 tokens a single token paid for four tiles of MMAs, and at K = 2048 its 133 KB allowed one block of 12 warps with four
+// steps ahead: 49 KB in flight on an SM, about what the memory's latency takes at full rate -- 213 us for 622 MB.  Two blocks of
+// six steps, or one of eight where the activations fill the shared memory, hold 98-147 KB in flight.
 #include <algorithm>
 
 #include "common.cuh"
@@ -19,8 +23,6 @@ int ensure_dynamic_smem(const void* kernel, size_t bytes);
 namespace {
 
 constexpr int kHeadWarps = 12;
-constexpr int kHeadTokens = 32;  // per launch: four token tiles of eight
-constexpr int kHeadAhead = 4;    // K steps of weight loads in flight per warp
 
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, bool bf16) {
   if (bf16) {
@@ -40,10 +42,12 @@ __device__ __forceinline__ uint4 ldg_stream16(const void* p) {
   return v;
 }
 
-// x: M x K, w: N x K, y: M x N, all 16-bit of one type; K a multiple of 32; shared memory: dense_head_smem(K) bytes
-template <bool BF16>
-__global__ void __launch_bounds__(32 * kHeadWarps, 2)
+// x: M x K, w: N x K, y: M x N, all 16-bit of one type; K a multiple of 32; shared memory: head_smem(NT, K) bytes.
+// PER_SM: blocks that share an SM; AHEAD: K steps of weight loads in flight per warp.
+template <bool BF16, int NT, int PER_SM>
+__global__ void __launch_bounds__(32 * kHeadWarps, PER_SM)
 dense_head_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, uint16_t* __restrict__ y, int M, int N, int K) {
+  constexpr int kHeadTokens = 8 * NT, kHeadAhead = PER_SM == 1 ? 8 : (NT == 4 ? 4 : 6);
   extern __shared__ __align__(16) uint16_t xs[];
   // row pitch = 64 bytes modulo 128: the eight lanes of a quarter warp (two token rows x four 16-byte pieces) then
   // read eight distinct 16-byte bank groups
@@ -85,9 +89,9 @@ dense_head_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w
   __syncthreads();
 
   for (; tile < n_tiles; tile += tile_stride) {
-    float acc[4][4];
+    float acc[NT][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
     for (int s0 = 0; s0 < steps; s0 += kHeadAhead) {
@@ -96,14 +100,14 @@ dense_head_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w
         const int s = s0 + i;
         if (s < steps) {
           const uint4 a = wa[i], b = wb[i];
-          if (s + kHeadAhead < steps) {  // refill this slot with the step four ahead
+          if (s + kHeadAhead < steps) {  // refill this slot
             wa[i] = ldg_stream16(ra + 32 * (s + kHeadAhead));
             wb[i] = ldg_stream16(rb + 32 * (s + kHeadAhead));
           }
           // k slots (2t, 2t+1 | 2t+8, 2t+9) of the two MMAs of this step hold actual k = 8t + (0,1 | 2,3) and 8t + (4,5 | 6,7)
           const uint32_t a0[4] = {a.x, b.x, a.y, b.y}, a1[4] = {a.z, b.z, a.w, b.w};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < NT; ++j) {
             const uint4 xv = *reinterpret_cast<const uint4*>(xs + (8 * j + g) * pitch + 32 * s + 8 * t);
             mma16816(acc[j], a0, xv.x, xv.y, BF16);
             mma16816(acc[j], a1, xv.z, xv.w, BF16);
@@ -125,7 +129,7 @@ dense_head_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w
     }
     const int r0 = tile * 16 + g, r1 = r0 + 8;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < NT; ++j) {
       const int m0 = 8 * j + 2 * t, m1 = m0 + 1;
       if (m0 < M) {
         if (r0 < N) y[size_t(m0) * N + r0] = float_to_out16(acc[j][0], BF16);
@@ -139,16 +143,24 @@ dense_head_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w
   }
 }
 
+size_t head_smem(int tiles, int64_t K) { return size_t(8 * tiles) * size_t(K + ((K & 63) ? 0 : 32)) * 2; }
+
+using HeadKernel = void (*)(const uint16_t*, const uint16_t*, uint16_t*, int, int, int);
+template <bool BF16>
+HeadKernel head_kernel(int tiles, int per_sm) {
+  if (tiles == 1) return dense_head_kernel<BF16, 1, 2>;
+  if (tiles == 2) return per_sm == 2 ? dense_head_kernel<BF16, 2, 2> : dense_head_kernel<BF16, 2, 1>;
+  return per_sm == 2 ? dense_head_kernel<BF16, 4, 2> : dense_head_kernel<BF16, 4, 1>;
+}
+
 }  // namespace
 
-size_t dense_head_smem(int64_t K) { return size_t(kHeadTokens) * size_t(K + ((K & 63) ? 0 : 32)) * 2; }
-
 int dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, int dtype, int sm_count, cudaStream_t stream) {
-  const size_t smem = dense_head_smem(K);
-  const bool bf16 = dtype == ASRQ_BF16;
-  auto kern = bf16 ? dense_head_kernel<true> : dense_head_kernel<false>;
+  const int tiles = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
+  const size_t smem = head_smem(tiles, K);
+  const int blocks_per_sm = smem <= 100 * 1024 ? 2 : 1;  // (K <= 3200: always 2 for one tile)
+  const HeadKernel kern = dtype == ASRQ_BF16 ? head_kernel<true>(tiles, blocks_per_sm) : head_kernel<false>(tiles, blocks_per_sm);
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
-  const int blocks_per_sm = smem <= 100 * 1024 ? 2 : 1;
   const int64_t n_tiles = (N + 15) / 16;
   const int grid = int(std::min<int64_t>(int64_t(sm_count) * blocks_per_sm, (n_tiles + kHeadWarps - 1) / kHeadWarps));
   cudaLaunchConfig_t cfg = {};
