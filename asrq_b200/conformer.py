@@ -23,7 +23,7 @@ import torch
 import torch.nn.functional as F
 
 from . import packing
-from .linear import LinearQQ
+from .linear import LinearQQ, glu_dwconv, residual_norms
 
 
 class FastConformerStandIn:
@@ -66,7 +66,26 @@ class FastConformerStandIn:
                 pw2=(rnd(d_model, d_model, 1), rnd(d_model)),
                 ln_ff2=ln(), ff2_a=qq(ffn, d_model), ff2_b=qq(d_model, ffn), ln_out=ln()))
         self.conv_kernel = conv_kernel
+        self._shared: list = []  # (layer, buffer name, the rows of the joined buffer it was given)
+        self._parts, self._pos_parts = [[L["q"], L["k"], L["v"]] for L in self.layers], [L["pos"] for L in self.layers]
+        self._qkv, self._pos = [self._joined(p) for p in self._parts], self._joined(self._pos_parts)
         torch.cuda.current_stream(self.device).synchronize()
+
+    def _joined(self, parts: List[LinearQQ]) -> LinearQQ:
+        """Layers of one input as one layer over all their output features, whose buffers the parts then share."""
+        m = LinearQQ(parts[0].in_features, sum(p.out_features for p in parts), 4, 4, parts[0].group_size, bias=parts[0].bias is not None,
+                     hadamard=parts[0].hadamard).to(parts[0].weight.device)
+        cat = lambda name: torch.cat([getattr(p, name) for p in parts])  # noqa: E731
+        m.load_quantized_params(cat("scales"), cat("zeros"), cat("weight"))
+        if parts[0].bias is not None:
+            m.bias = cat("bias")
+        n = 0
+        for p in parts:
+            for name in ("weight", "scales", "zeros") + (("bias",) if p.bias is not None else ()):
+                setattr(p, name, getattr(m, name)[n:n + p.out_features])
+                self._shared.append((p, name, getattr(p, name)))
+            n += p.out_features
+        return m
 
     def linear_layers(self) -> List[LinearQQ]:
         return [L[k] for L in self.layers for k in ("ff1_a", "ff1_b", "q", "k", "v", "out", "pos", "ff2_a", "ff2_b")]
@@ -111,11 +130,42 @@ class FastConformerStandIn:
         x = x + 0.5 * lin("ff2_b", F.silu(lin("ff2_a", h)))
         return F.layer_norm(x, (d,), *L["ln_out"])
 
+    def _blocks(self, x: torch.Tensor, pe: torch.Tensor) -> torch.Tensor:
+        """All blocks with what lies between their layers in this library's kernels: the same steps and roundings as
+        :meth:`block`, channels last throughout, q/k/v as one layer over one quantised input, and the positional keys of all
+        blocks (whose input is the same) as one layer ahead of them."""
+        b, t, d = x.shape
+        hd = d // self.heads
+        sp = lambda z: z.view(b, t, self.heads, hd).transpose(1, 2)  # noqa: E731
+        pos = self._pos(pe)
+        x, h = residual_norms(x, None, 1.0, self.layers[0]["ln_ff1"])
+        for i, L in enumerate(self.layers):
+            x, h = residual_norms(x, L["ff1_b"](F.silu(L["ff1_a"](h), inplace=True)), 0.5, L["ln_att"])
+            qkv = self._qkv[i](h)
+            k = qkv[..., d:2 * d] + pos[:, i * d:(i + 1) * d]
+            a = F.scaled_dot_product_attention(sp(qkv[..., :d]), sp(k), sp(qkv[..., 2 * d:])).transpose(1, 2).reshape(b, t, d)
+            x, h = residual_norms(x, L["out"](a), 1.0, L["ln_conv"])
+            h = glu_dwconv(F.linear(h, L["pw1"][0].view(2 * d, d), L["pw1"][1]), *L["dw"], *L["bn"])
+            x, h = residual_norms(x, F.linear(h, L["pw2"][0].view(d, d), L["pw2"][1]), 1.0, L["ln_ff2"])
+            y = L["ff2_b"](F.silu(L["ff2_a"](h), inplace=True))
+            more = i + 1 < len(self.layers)
+            x, h = residual_norms(x, y, 0.5, L["ln_out"], self.layers[i + 1]["ln_ff1"] if more else None, write_h=more)
+        return x
+
+    def _blocks_covered(self) -> bool:
+        # the joined layers stand for their parts only while these hold the shared buffers and are the blocks' layers
+        return (self.d % 256 == 0 and self.d <= 2048 and self.conv_kernel == 9 and len(self.layers) == len(self._qkv) > 0 and
+                all(p._buffers.get(name) is t for p, name, t in self._shared) and
+                all(L[name] is p for L, parts in zip(self.layers, self._parts) for name, p in zip("qkv", parts)) and
+                all(L["pos"] is p for L, p in zip(self.layers, self._pos_parts)))
+
     @torch.no_grad()
     def encode(self, feats: torch.Tensor, hook=None) -> torch.Tensor:
         with torch.cuda.device(self.device):
             x = self.subsample(feats)
             pe = self._pos_emb(x.shape[1])
+            if hook is None and x.numel() and self._blocks_covered():
+                return self._blocks(x.contiguous(), pe)
             for L in self.layers:
                 x = self.block(L, x, pe, hook)
             return x
