@@ -320,7 +320,7 @@ static int a16_gemv(int bits, const void* x, const uint8_t* w, const void* scale
 
 static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                     void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
-                    size_t workspace_bytes, void* stream, const Epilogue& ep = Epilogue(), bool* fused = nullptr) {
+                    size_t workspace_bytes, void* stream, const Epilogue& ep = Epilogue(), bool* fused = nullptr, bool any_m = false) {
   last_error().clear();
   bool fused_here = false;
   if (!fused) fused = &fused_here;
@@ -338,6 +338,8 @@ static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scale
     return gemm_a16_skinny(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes,
                            f->sm_count, static_cast<cudaStream_t>(stream), ep);
   }
+  if (M < 32 && !any_m && N % 128 == 0 && K % 64 == 0 && group_size > 0 && group_size % 64 == 0 && K % group_size == 0)
+    return fail(ASRQ_ERR_SHAPE, "w%da16 gemm: M=%lld < 32 (use the gemv entry point)", bits, (long long)M);
   return gemm_a16_tc(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes,
                      f->sm_count, static_cast<cudaStream_t>(stream), ep, fused);
 }
@@ -377,16 +379,12 @@ static int linearq_a16(int bits, const void* x, const uint8_t* w, const void* sc
   const bool tc_ok = N % 128 == 0 && K % 64 == 0 && group_size > 0 && group_size % 64 == 0 && K % group_size == 0;
   bool fused = false;
   int rc;
-  // 17..32 tokens: the tensor cores (gemm_a16_skinny.cu) unless switched off; the mma.sync decode kernel is bound
-  // by the legacy MMA pipe there
-  bool mid = false;
-  if (M > 16 && M <= kGemvMaxM && tc_ok && option(kOptMidKernel) != 1 && workspace) {
-    int sms = 0;
-    mid = current_device_sm_count(&sms) == ASRQ_OK && gemm_a16_skinny_supports(M, N, K, group_size, sms, workspace_bytes);
-  }
-  if (mid || (M > kGemvMaxM && tc_ok))
+  // From 17 tokens the tensor cores, unless switched off for 17..32: the mma.sync decode kernel takes sixteen tokens per
+  // launch and is bound by the legacy MMA pipe (12288 x 2048, which the one-wave skinny kernel does not cover, us: 15 for 16
+  // tokens, 22-30 for 17-32; the persistent kernel 16).
+  if (tc_ok && (M > kGemvMaxM || (M > 16 && option(kOptMidKernel) != 1)))
     rc = a16_gemm(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream,
-                  ep, &fused);
+                  ep, &fused, true);
   else
     rc = a16_gemv(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream, ep, &fused);
   if (rc || !want_ep || fused || M == 0) return rc;

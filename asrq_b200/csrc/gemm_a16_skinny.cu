@@ -5,25 +5,26 @@
 // costs (set-up, first TMA and first dequantisation pass before the first MMA, an epilogue nothing
 // overlaps): 10-15 us for a 1-3 MB layer either way.  This kernel is built for a CHAIN of such layers:
 //
-//   * a block owns ONE work item -- a 128-feature tile and a part of K of at most 12 blocks of 64 -- so all
-//     of its packed weights (<= 48 KB) and all of its activation tiles fit shared memory at once;
+//   * a block owns ONE work item -- a 128-feature tile and a part of K of at most 14 blocks of 64 -- so all
+//     of its packed weights (<= 56 KB) and all of its activation tiles fit shared memory at once;
 //   * it triggers its dependents as its first instruction and is small enough (448 threads, <= 73
 //     registers, < 113 KB) for two launches to share an SM.  Packed weights are fetched by TMA and the
 //     first three K blocks are dequantised BEFORE griddepcontrol.wait: weights do not depend on the
 //     kernel before, so the next launch's weight traffic and unpacking run under this launch's tail;
 //   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32 or 64 TMEM columns)
 //     are fetched, all at once; tcgen05.mma kind::f16 128 x BT x 16, fp32 accumulator in tensor memory;
-//   * K parts of a tile meet through the workspace: fp32 partial tiles and one arrival counter per tile.
-//     The last BLOCK to arrive adds the parts in part order (results do not depend on timing) with all
-//     of its threads, every thread's loads of all parts in flight together, adds the bias, converts,
-//     stores, and leaves the counter at zero.  (With one warp per lane quadrant doing this, one L2 round
-//     trip per part in turn, the reduction took 8 of a launch's 9.6 us.)
+//   * the K parts of a tile are a thread-block cluster and meet in distributed shared memory: every block leaves its
+//     fp32 part in its own shared memory (over the A slots, whose MMAs are done), and after one cluster barrier each
+//     adds its share of the tokens over all parts in part order, with all of its threads, adds the bias, converts
+//     and stores.  Through the workspace (partial tiles, a counter per tile, the last block adding) the same step
+//     cost a release to memory, an atomic and two to four L2 round trips of one block while the others were done.
 //
 // Roles (14 warps): warp 0 TMA producer, warp 1 MMA issuer (owns the tensor-memory allocation), warps
 // 2-13 three dequant groups of 128 threads (one weight row per thread, group d takes K blocks d, d+3, ...
 // and owns A slot d); the first group (warps 2-5, one per TMEM lane quadrant) then runs the epilogue.
 // No TMA multicast.  Every wait is bounded.
 #include <algorithm>
+#include <atomic>
 
 #include "dequant.cuh"
 #include "tcgen05.cuh"
@@ -36,9 +37,11 @@ namespace {
 
 constexpr int kSkWarps = 14;
 constexpr int kSkThreads = 32 * kSkWarps;
-constexpr int kSkMaxKb = 12;                    // K blocks of 64 per work item
+constexpr int kSkMaxKb = 14;                    // K blocks of 64 per work item
 constexpr int kSkMaxSplit = 8;
 constexpr uint32_t kSkATile = 128 * 128;        // one dequantised A slot: 128 rows x 64 16-bit elements
+constexpr size_t kSkMaxSmem = 220 * 1024;
+constexpr size_t kSkTwoPerSm = 112 * 1024;      // two blocks share an SM
 constexpr uint32_t kSkWSlot = 4096;             // packed weights of one K block (<= 128 x 32 B)
 
 struct SkinnyParams {
@@ -49,8 +52,6 @@ struct SkinnyParams {
   int act;                   // fused epilogue: activation on the layer output (kActNone / kActGelu)
   uint16_t* y;
   unsigned* status;
-  float* partials;     // [tile][part][bt tokens][128 features]
-  unsigned* counters;  // one per tile, zero between launches
   int M, N, K, group_size, groups_per_row, bt, ksplit, nkb, kbmax;
   unsigned long long* trace;  // builds with -DASRQ_TRACE: 8 globaltimer marks per block, NULL otherwise
 };
@@ -74,7 +75,6 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
                        const SkinnyParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[kSkMaxKb + 8];
-  __shared__ int is_last;
   __shared__ uint32_t tmem_slot;
   // the next launch on the stream may start its own set-up, weight fetch and first dequantisation now
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -229,14 +229,14 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
               }
           }
         } else {
-          // this block's part of the tile, fp32 [token][128 features]: a warp writes 128 contiguous bytes per token
-          float* part = p.partials + (size_t(ft) * p.ksplit + ks) * size_t(p.bt) * 128 + qd * 32 + lane;
+          // this block's part of the tile, fp32 [token][128 features], over the A slots
+          float* part = reinterpret_cast<float*>(smem) + qd * 32 + lane;
           for (int ch = 0; ch < p.bt / 32; ++ch) {
             uint32_t r[32];
             tc::tmem_ld_32x32(taddr + ch * 32, r);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) __stcg(part + size_t(ch * 32 + j) * 128, __uint_as_float(r[j]));
+            for (int j = 0; j < 32; ++j) part[(ch * 32 + j) * 128] = __uint_as_float(r[j]);
           }
         }
       }
@@ -245,50 +245,45 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
 
   __syncwarp();
   tc::fence_before_sync();
-  __syncthreads();
-  if (p.ksplit > 1) {
-    // the block that arrives last for its tile adds the parts; which block that is depends on timing, the
-    // order of the additions does not.  Ordering as in a grid-wide barrier: the block's stores are ordered before
-    // thread 0's fence by the block barrier above, the fence is cumulative, and the last block's loads follow
-    // thread 0's second fence through the barrier below -- one thread fences, not 448 (1.5 % of a decode step).
-    if (threadIdx.x == 0) {
-      __threadfence();
-      is_last = atomicAdd(p.counters + ft, 1u) == unsigned(p.ksplit - 1);
-      __threadfence();
-    }
+  if (p.ksplit == 1) {
     __syncthreads();
-    if (is_last) {
-      const int total = p.bt * 128;
-      const float* part0 = p.partials + size_t(ft) * p.ksplit * total;
-      // four features per thread and step, all parts' loads of a step in flight together: the reduction costs
-      // three L2 round trips (one load at a time per part it cost nine, 6 us)
-      for (int o4 = threadIdx.x; o4 < total / 4; o4 += kSkThreads) {
-        float4 a[kSkMaxSplit];
+  } else {
+    tc::cluster_sync();  // every part is in its block's shared memory
+    const int m0 = ks * p.M / p.ksplit, count = ((ks + 1) * p.M / p.ksplit - m0) * 32;  // four features of a token per step
+    uint32_t part[kSkMaxSplit];
 #pragma unroll
-        for (int s = 0; s < kSkMaxSplit; ++s)
-          if (s < p.ksplit) a[s] = __ldcg(reinterpret_cast<const float4*>(part0 + size_t(s) * total) + o4);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < kSkMaxSplit; ++s) part[s] = s < p.ksplit ? tc::mapa(base, s) : 0u;
+    for (int o4 = threadIdx.x; o4 < count; o4 += kSkThreads) {
+      const int tok = m0 + (o4 >> 5), f = ft * 128 + (o4 & 31) * 4;
+      const size_t idx = size_t(tok) * p.N + f;
+      uint2 res = make_uint2(0u, 0u);
+      if (p.residual) res = *reinterpret_cast<const uint2*>(p.residual + idx);
+      float4 a[kSkMaxSplit];
 #pragma unroll
-        for (int s = 0; s < kSkMaxSplit; ++s)
-          if (s < p.ksplit) {
-            v.x += a[s].x; v.y += a[s].y; v.z += a[s].z; v.w += a[s].w;
-          }
-        const int tok = o4 >> 5, f = ft * 128 + (o4 & 31) * 4;
-        if (tok < p.M) {
-          if (p.bias) {
-            const uint2 b = __ldg(reinterpret_cast<const uint2*>(p.bias + f));
-            const float2 b01 = __half22float2(u32_as_h2(b.x)), b23 = __half22float2(u32_as_h2(b.y));
-            v.x += b01.x; v.y += b01.y; v.z += b23.x; v.w += b23.y;
-          }
-          const size_t idx = size_t(tok) * p.N + f;
-          uint2 out;
-          out.x = uint32_t(finish16(v.x, p.act, p.residual, idx, BF16)) | (uint32_t(finish16(v.y, p.act, p.residual, idx + 1, BF16)) << 16);
-          out.y = uint32_t(finish16(v.z, p.act, p.residual, idx + 2, BF16)) | (uint32_t(finish16(v.w, p.act, p.residual, idx + 3, BF16)) << 16);
-          *reinterpret_cast<uint2*>(p.y + idx) = out;
+      for (int s = 0; s < kSkMaxSplit; ++s)
+        if (s < p.ksplit) a[s] = tc::ld_dsmem_v4(part[s] + uint32_t(tok * 128 + (o4 & 31) * 4) * 4u);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int s = 0; s < kSkMaxSplit; ++s)
+        if (s < p.ksplit) {
+          v.x += a[s].x; v.y += a[s].y; v.z += a[s].z; v.w += a[s].w;
         }
+      if (p.bias) {
+        const uint2 b = __ldg(reinterpret_cast<const uint2*>(p.bias + f));
+        const float2 b01 = __half22float2(u32_as_h2(b.x)), b23 = __half22float2(u32_as_h2(b.y));
+        v.x += b01.x; v.y += b01.y; v.z += b23.x; v.w += b23.y;
       }
-      if (threadIdx.x == 0) p.counters[ft] = 0u;
+      const float vv[4] = {v.x, v.y, v.z, v.w};
+      const uint16_t rr[4] = {uint16_t(res.x & 0xffffu), uint16_t(res.x >> 16), uint16_t(res.y & 0xffffu), uint16_t(res.y >> 16)};
+      uint16_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        o[e] = float_to_out16(vv[e], BF16);
+        if (p.act != kActNone || p.residual) o[e] = epilogue16(o[e], p.act, p.residual != nullptr, rr[e], BF16);
+      }
+      *reinterpret_cast<uint2*>(p.y + idx) = make_uint2(uint32_t(o[0]) | (uint32_t(o[1]) << 16), uint32_t(o[2]) | (uint32_t(o[3]) << 16));
     }
+    tc::cluster_sync_relaxed();  // no block leaves while another reads its part
   }
   if (threadIdx.x == 0) SK_MARK(7);
   if (warp == 1) {
@@ -302,24 +297,57 @@ struct SkinnyPlan {
   size_t smem;
 };
 
+// Blocks of one launch that run at once as clusters of `split` (the size leaves some SMs without a whole cluster): the
+// answer of the driver for the kernel's block at one block per SM, or two where its shared memory allows.
+int skinny_capacity(int split, size_t smem) {
+  static std::atomic<int> known[kSkMaxSplit + 1][2];  // one kind of device: asked once per process
+  const bool two = smem <= kSkTwoPerSm;
+  std::atomic<int>& k = known[split][two];
+  int n = k.load(std::memory_order_relaxed);
+  if (n) return n;
+  auto kern = gemm_a16_skinny_kernel<4, false>;
+  const size_t ask = two ? kSkTwoPerSm : kSkMaxSmem;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), ask)) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(split));
+  cfg.blockDim = dim3(kSkThreads);
+  cfg.dynamicSmemBytes = ask;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  k.store(n * split, std::memory_order_relaxed);
+  return n * split;
+}
+
 bool skinny_plan(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes, SkinnyPlan* pl) {
   if (M < 1 || M > 64 || N % 128 || K % 64 || group_size <= 0 || group_size % 64 || K % group_size) return false;
   if (workspace_bytes < kStatusBytes) return false;
   const int64_t tiles = N / 128, nkb = K / 64;
   const int bt = M <= 32 ? 32 : 64;
-  // parts of K: as many as fill the machine in one wave, at most 8, at least enough for kSkMaxKb K blocks per part
-  int64_t split = std::max<int64_t>((nkb + kSkMaxKb - 1) / kSkMaxKb, std::min<int64_t>(sm_count / tiles, kSkMaxSplit));
-  split = std::max<int64_t>(1, std::min<int64_t>(split, nkb));
-  if (split > kSkMaxSplit || tiles * split > sm_count) return false;
-  if (tiles > int64_t(kCounterBytes / sizeof(unsigned))) return false;
-  if (split > 1 && workspace_bytes < kPartialOffset + size_t(4) * N * bt * split) return false;
+  auto smem_of = [&](int64_t sp) { return 1024 + 3 * kSkATile + size_t((nkb + sp - 1) / sp) * (size_t(bt) * 128 + kSkWSlot); };
+  // Parts of K: the most that run in one wave with a block per SM, at least enough for kSkMaxKb K blocks per part.  Where
+  // clusters of that many leave too few SMs, fewer; where none fits (the last clusters then run in a second wave), the most.
+  int64_t least = (nkb + kSkMaxKb - 1) / kSkMaxKb, split = std::min<int64_t>({std::max<int64_t>(least, sm_count / tiles), kSkMaxSplit, nkb});
+  if (split < least || tiles * split > sm_count) return false;
+  for (int64_t sp = split; sp >= least; --sp)
+    if (sp == 1 || skinny_capacity(int(sp), smem_of(sp)) >= tiles * sp) {
+      split = sp;
+      break;
+    }
   pl->bt = bt;
   pl->ksplit = int(split);
   pl->nkb = int(nkb);
   pl->kbmax = int((nkb + split - 1) / split);
   pl->grid = int(tiles * split);
-  pl->smem = 1024 + 3 * kSkATile + size_t(pl->kbmax) * (size_t(bt) * 128 + kSkWSlot);
-  return pl->smem <= 200 * 1024;
+  pl->smem = smem_of(split);
+  return pl->smem <= kSkMaxSmem;
 }
 
 template <int BITS, bool BF16>
@@ -332,11 +360,14 @@ int launch_skinny(const CUtensorMap& tmx, const CUtensorMap& tmw, const SkinnyPa
   cfg.blockDim = dim3(kSkThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.ksplit;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = option(kOptNoPdl) ? 0 : 1;
+  cfg.numAttrs = option(kOptNoPdl) ? 1 : 2;
   ASRQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmx, tmw, p));
   return ASRQ_OK;
 }
@@ -364,8 +395,6 @@ int gemm_a16_skinny(int bits, const void* x, const uint8_t* w, const void* scale
   p.act = ep.act;
   p.y = static_cast<uint16_t*>(y);
   p.status = static_cast<unsigned*>(workspace);
-  p.partials = reinterpret_cast<float*>(static_cast<char*>(workspace) + kPartialOffset);
-  p.counters = reinterpret_cast<unsigned*>(static_cast<char*>(workspace) + kStatusBytes);
   p.M = int(M);
   p.N = int(N);
   p.K = int(K);
