@@ -331,8 +331,8 @@ static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scale
   const DeviceFacts* f;
   if ((rc = device_facts(&f))) return rc;
   if (M == 0) return ASRQ_OK;
-  // decode batches (17..64 tokens): the chain-oriented tensor-core kernel where its one-wave grid fits
-  if (M <= 64 && option(kOptMidKernel) != 1 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0 &&
+  // decode batches (17..128 tokens): the chain-oriented tensor-core kernel where its one-wave grid fits
+  if (M <= 128 && option(kOptMidKernel) != 1 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0 &&
       gemm_a16_skinny_supports(M, N, K, group_size, f->sm_count, workspace_bytes)) {
     *fused = true;
     return gemm_a16_skinny(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes,

@@ -1,17 +1,17 @@
-// Decode batches on the tensor cores: y[M,N] = x[M,K] . dequant(W)[N,K]^T (+ bias) for 17 <= M <= 64.
+// Decode batches on the tensor cores: y[M,N] = x[M,K] . dequant(W)[N,K]^T (+ bias) for 17 <= M <= 128.
 //
 // At these token counts the mma.sync decode kernel is bound by the legacy MMA pipe (one m16n8k16 per ~13
 // clocks per scheduler, one per 8 tokens per 256 codes), and the persistent prefill kernel by its fixed
 // costs (set-up, first TMA and first dequantisation pass before the first MMA, an epilogue nothing
 // overlaps): 10-15 us for a 1-3 MB layer either way.  This kernel is built for a CHAIN of such layers:
 //
-//   * a block owns ONE work item -- a 128-feature tile and a part of K of at most 14 blocks of 64 -- so all
-//     of its packed weights (<= 56 KB) and all of its activation tiles fit shared memory at once;
+//   * a block owns ONE work item -- a 128-feature tile and a part of K of at most 16 blocks of 64 -- so that
+//     its packed weights (twelve blocks at a time) and all of its activation tiles fit shared memory at once;
 //   * it triggers its dependents as its first instruction and is small enough (448 threads, <= 73
 //     registers, < 113 KB) for two launches to share an SM.  Packed weights are fetched by TMA and the
 //     first three K blocks are dequantised BEFORE griddepcontrol.wait: weights do not depend on the
 //     kernel before, so the next launch's weight traffic and unpacking run under this launch's tail;
-//   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32 or 64 TMEM columns)
+//   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32, 64, 96 or 128 TMEM columns)
 //     are fetched, all at once; tcgen05.mma kind::f16 128 x BT x 16, fp32 accumulator in tensor memory;
 //   * the K parts of a tile are a thread-block cluster and meet in distributed shared memory: every block leaves its
 //     fp32 part in its own shared memory (over the A slots, whose MMAs are done), and after one cluster barrier each
@@ -37,10 +37,13 @@ namespace {
 
 constexpr int kSkWarps = 14;
 constexpr int kSkThreads = 32 * kSkWarps;
-constexpr int kSkMaxKb = 14;                    // K blocks of 64 per work item
+constexpr int kSkMaxKb = 16;                    // K blocks of 64 per work item
 constexpr int kSkMaxSplit = 8;
+constexpr int kSkMaxM = 128;
 constexpr uint32_t kSkATile = 128 * 128;        // one dequantised A slot: 128 rows x 64 16-bit elements
-constexpr size_t kSkMaxSmem = 220 * 1024;
+constexpr int kSkWSlots = 12;                   // packed K blocks held at once; the rest follow into the first slots
+constexpr int kSkWAgain = kSkMaxKb - kSkWSlots; // ... of which so many are filled twice
+constexpr size_t kSkMaxSmem = 226 * 1024;
 constexpr size_t kSkTwoPerSm = 112 * 1024;      // two blocks share an SM
 constexpr uint32_t kSkWSlot = 4096;             // packed weights of one K block (<= 128 x 32 B)
 
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(kSkThreads, 2)
 gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
                        const SkinnyParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[kSkMaxKb + 8];
+  __shared__ __align__(8) uint64_t bars[kSkMaxKb + 8 + kSkWAgain];
   __shared__ uint32_t tmem_slot;
   // the next launch on the stream may start its own set-up, weight fetch and first dequantisation now
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -88,7 +91,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   const int ks = blockIdx.x % p.ksplit, ft = blockIdx.x / p.ksplit;
   const int kb0 = ks * p.nkb / p.ksplit, kb1 = (ks + 1) * p.nkb / p.ksplit, kbn = kb1 - kb0;
   const uint32_t xbytes = uint32_t(p.bt) * 128u;
-  // [A slot x 3] [activation tile x kbmax] [packed weights x kbmax]
+  // [A slot x 3] [activation tile x kbmax] [packed weights x min(kbmax, kSkWSlots)]
   const uint32_t x_base = 3 * kSkATile, w_base = x_base + uint32_t(p.kbmax) * xbytes;
   constexpr uint32_t wbytes = 128u * 8u * BITS;
   const uint32_t bar0 = tc::smem_u32(bars);
@@ -96,7 +99,8 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   const uint32_t x_bar = bar0 + 8u * kSkMaxKb, accf_bar = x_bar + 8u;
   auto deq_bar = [&](int a) { return x_bar + 16u + 8u * a; };
   auto afree_bar = [&](int a) { return x_bar + 40u + 8u * a; };
-  const uint32_t tmem_cols = p.bt <= 32 ? 32u : 64u;
+  auto wfree_bar = [&](int i) { return x_bar + 64u + 8u * i; };
+  const uint32_t tmem_cols = p.bt <= 32 ? 32u : (p.bt <= 64 ? 64u : 128u);
 
   if (threadIdx.x == 0) {
     for (int kb = 0; kb < kSkMaxKb; ++kb) tc::mbar_init(w_bar(kb), 1);
@@ -106,6 +110,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
       tc::mbar_init(deq_bar(a), 128);
       tc::mbar_init(afree_bar(a), 1);
     }
+    for (int i = 0; i < kSkWAgain; ++i) tc::mbar_init(wfree_bar(i), 128);
     tc::fence_barrier_init();
     tc::fence_proxy_async_smem();
     tc::prefetch_tmap(&tmx);
@@ -124,16 +129,21 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
-      for (int kb = 0; kb < kbn; ++kb) {  // weights: constants, fetched ahead of the stream dependency
+      auto fetch_w = [&](int kb) {
         tc::mbar_arrive_expect_tx(w_bar(kb), wbytes);
-        tc::tma_load_2d(base + w_base + kb * kSkWSlot, &tmw, (kb0 + kb) * 8 * BITS, ft * 128, w_bar(kb));
-      }
+        tc::tma_load_2d(base + w_base + (kb % kSkWSlots) * kSkWSlot, &tmw, (kb0 + kb) * 8 * BITS, ft * 128, w_bar(kb));
+      };
+      for (int kb = 0; kb < kbn && kb < kSkWSlots; ++kb) fetch_w(kb);  // constants: ahead of the stream dependency
       SK_MARK(2);
       // activations belong to this kernel only once its predecessor on the stream is complete
       asm volatile("griddepcontrol.wait;" ::: "memory");
       SK_MARK(3);
       tc::mbar_arrive_expect_tx(x_bar, uint32_t(kbn) * xbytes);
       for (int kb = 0; kb < kbn; ++kb) tc::tma_load_2d(base + x_base + kb * xbytes, &tmx, (kb0 + kb) * 64, 0, x_bar);
+      for (int kb = kSkWSlots; kb < kbn; ++kb) {
+        if (!tc::mbar_wait(wfree_bar(kb - kSkWSlots), 0u, p.status, 36)) break;
+        fetch_w(kb);
+      }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
@@ -180,7 +190,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
       if (kb >= 3) ok = tc::mbar_wait(afree_bar(dgroup), uint32_t(kb / 3 - 1) & 1u, p.status, 33);
       ok = ok && tc::mbar_wait(w_bar(kb), 0u, p.status, 34);
       if (!ok) break;
-      const uint4* wp = reinterpret_cast<const uint4*>(smem + w_base + kb * kSkWSlot + t * (8 * BITS));
+      const uint4* wp = reinterpret_cast<const uint4*>(smem + w_base + (kb % kSkWSlots) * kSkWSlot + t * (8 * BITS));
       uint8_t* arow = smem + dgroup * kSkATile + t * 128;
       constexpr int NV = BITS / 2;  // 16-byte vectors of packed weights per row per K block
 #pragma unroll
@@ -201,6 +211,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
         }
       }
       tc::fence_proxy_async_smem();
+      if (kb + kSkWSlots < kbn) tc::mbar_arrive(wfree_bar(kb));
       tc::mbar_arrive(deq_bar(dgroup));
     }
     ok = __all_sync(0xffffffffu, ok);  // a wait that gave up in any lane ends the warp's work
@@ -327,15 +338,19 @@ int skinny_capacity(int split, size_t smem) {
 }
 
 bool skinny_plan(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes, SkinnyPlan* pl) {
-  if (M < 1 || M > 64 || N % 128 || K % 64 || group_size <= 0 || group_size % 64 || K % group_size) return false;
+  if (M < 1 || M > kSkMaxM || N % 128 || K % 64 || group_size <= 0 || group_size % 64 || K % group_size) return false;
   if (workspace_bytes < kStatusBytes) return false;
   const int64_t tiles = N / 128, nkb = K / 64;
-  const int bt = M <= 32 ? 32 : 64;
-  auto smem_of = [&](int64_t sp) { return 1024 + 3 * kSkATile + size_t((nkb + sp - 1) / sp) * (size_t(bt) * 128 + kSkWSlot); };
+  const int bt = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128));
+  auto smem_of = [&](int64_t sp) {
+    const int64_t kb = (nkb + sp - 1) / sp;
+    return 1024 + 3 * kSkATile + size_t(kb) * (size_t(bt) * 128) + size_t(std::min<int64_t>(kb, kSkWSlots)) * kSkWSlot;
+  };
   // Parts of K: the most that run in one wave with a block per SM, at least enough for kSkMaxKb K blocks per part.  Where
   // clusters of that many leave too few SMs, fewer; where none fits (the last clusters then run in a second wave), the most.
   int64_t least = (nkb + kSkMaxKb - 1) / kSkMaxKb, split = std::min<int64_t>({std::max<int64_t>(least, sm_count / tiles), kSkMaxSplit, nkb});
   if (split < least || tiles * split > sm_count) return false;
+  while (least < split && smem_of(least) > kSkMaxSmem) ++least;
   for (int64_t sp = split; sp >= least; --sp)
     if (sp == 1 || skinny_capacity(int(sp), smem_of(sp)) >= tiles * sp) {
       split = sp;

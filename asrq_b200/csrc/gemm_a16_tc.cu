@@ -429,20 +429,32 @@ gemm_a16_tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   }
 }
 
-// Token-tile width: the multiple of 32 (<= 256, M rounded up at most) that minimises rounds over the SMs x the time of a tile.
-// Up to 128 columns that is the dequantisation of its weights, which the MMAs hide behind (12288 x 2048: 16.1 us for 64 columns
-// in one round, 16.6 for 128, 27.7 for two rounds of 32).
-int gemm_tc_pick_bt(int64_t M, int64_t N, int sm_count) {
+// Split K (mid-size M): with few output tiles most SMs would idle while each busy one walks the
+// whole K range, so the K blocks of a tile are divided among `split` blocks.  Bounded by the SM
+// count, by two K blocks per part, and by the partial-sum area the workspace contract provides
+// (split x padded M <= 512: 2048 bytes per output feature).
+int gemm_tc_pick_split(int64_t M, int64_t N, int64_t K, int bt, int sm_count) {
+  if (option(kOptTcSplit) == 1) return 1;  // tuning knob: 1 disables
+  const int64_t n_tt = (M + bt - 1) / bt, tiles = (N / 128) * n_tt, nkb = K / 64;
+  int64_t split = std::min<int64_t>({int64_t(sm_count) / tiles, nkb / 2, 512 / (n_tt * bt), kTcMaxSplit});
+  return int(std::max<int64_t>(split, 1));
+}
+// Token-tile width: the multiple of 32 (<= 256, M rounded up at most) with the least rounds over the SMs x K blocks of an item x
+// time of a K block -- up to 128 columns that is the dequantisation of its weights (0.37 us), which the MMAs hide behind -- plus
+// the addition of the parts where K is split (0.017 us per column and part).  Measured: 12288 x 2048, us: 16.1 for 64 columns
+// in one round, 16.6 for 128, 27.7 for two rounds of 32; 1280 x 1280 at 96 tokens: 8.7 for 32 columns in 4 parts, 13.5 for 96 in 5.
+int gemm_tc_pick_bt(int64_t M, int64_t N, int64_t K, int sm_count) {
   const int forced = option(kOptTcBt);  // tuning knob: force the token-tile width
   if (forced >= 32 && forced <= 256 && forced % 32 == 0) return forced;
   int best = 32;
   double best_cost = 1e30;
-  const int64_t nft = N / 128;
+  const int64_t nft = N / 128, nkb = K / 64;
   for (int bt = 32; bt <= 256; bt += 32) {
     if (bt - 32 >= M) break;
+    const int split = gemm_tc_pick_split(M, N, K, bt, sm_count);
     const int64_t tiles = nft * ((M + bt - 1) / bt);
-    const int64_t rounds = (tiles + sm_count - 1) / sm_count;
-    const double cost = double(rounds) * (std::max(bt, 128) + 24);
+    const int64_t rounds = (tiles * split + sm_count - 1) / sm_count;
+    const double cost = double(rounds) * double((nkb + split - 1) / split) * 0.37 * (std::max(bt, 128) + 24) / 152 + (split > 1 ? 0.017 * bt * split : 0.0);
     if (cost <= best_cost) {
       best_cost = cost;
       best = bt;
@@ -451,16 +463,6 @@ int gemm_tc_pick_bt(int64_t M, int64_t N, int sm_count) {
   return best;
 }
 
-// Split K (mid-size M): with few output tiles most SMs would idle while each busy one walks the
-// whole K range, so the K blocks of a tile are divided among `split` blocks.  Bounded by the SM
-// count, by two K blocks per part, and by the partial-sum area the workspace contract provides
-// (split x padded M <= 512, the skinny kernel's 2048 bytes per output feature).
-int gemm_tc_pick_split(int64_t M, int64_t N, int64_t K, int bt, int sm_count) {
-  if (option(kOptTcSplit) == 1) return 1;  // tuning knob: 1 disables
-  const int64_t n_tt = (M + bt - 1) / bt, tiles = (N / 128) * n_tt, nkb = K / 64;
-  int64_t split = std::min<int64_t>({int64_t(sm_count) / tiles, nkb / 2, 512 / (n_tt * bt), kTcMaxSplit});
-  return int(std::max<int64_t>(split, 1));
-}
 size_t gemm_tc_workspace_bytes(int64_t M, int64_t N) {
   return M <= 256 ? kPartialOffset + size_t(2048) * size_t(N) : kStatusBytes;
 }
@@ -531,7 +533,7 @@ int gemm_a16_tc(int bits, const void* x, const uint8_t* w, const void* scales, c
   p.K = int(K);
   p.group_size = group_size;
   p.groups_per_row = int(K / group_size);
-  p.bt = gemm_tc_pick_bt(M, N, sm_count);
+  p.bt = gemm_tc_pick_bt(M, N, K, sm_count);
   p.n_ftiles = int(N / 128);
   p.n_ttiles = int((M + p.bt - 1) / p.bt);
   const size_t stage_bytes = size_t(p.bt) * 128 + kWSlotBytes;

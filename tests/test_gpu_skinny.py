@@ -1,0 +1,31 @@
+"""The tensor-core decode-batch kernel at its edges: token tiles of 32, 64, 96 and 128 columns, one to eight K parts, parts longer
+than the packed weights it holds at once (more than twelve K blocks), and tokens that do not divide among the parts."""
+import pytest
+import torch
+
+from oracle import linearq_oracle as O
+from tests.gpu_util import assert_close_rows, make_layer
+from tests.test_gpu_a16 import _ref32
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,k,n,bits", [
+    (17, 1280, 1280, 4),   # eight parts of two or three K blocks
+    (33, 2048, 4096, 4),   # four parts
+    (64, 1280, 5120, 2),   # three parts
+    (65, 1280, 1280, 4), (96, 2048, 2048, 4), (97, 1280, 3840, 2), (128, 1280, 5120, 4), (128, 64, 128, 4),
+    (20, 6144, 2048, 4), (64, 6144, 2048, 4),   # six parts of sixteen: the weight slots are filled twice
+    (31, 8192, 128, 4),    # eight parts of sixteen
+    (24, 2048, 12288, 4),  # more tiles than one wave takes: the persistent kernel
+    (65, 2048, 12288, 4),
+])
+def test_decode_batches(m, k, n, bits):
+    case = O.make_c3(seed=m + k, m=m, k=k, n=n, bits=bits, group_size=64 if k == 64 else 128)
+    layer = make_layer(case)
+    x = case["x"].cuda()
+    y = layer(x)
+    assert_close_rows(y.cpu(), _ref32(case), what=f"w{bits} m{m} {k}x{n}")
+    assert torch.equal(y, layer(x))
+    res = torch.randn_like(y)
+    assert torch.equal(layer.forward_fused(x, residual=res), res + y)
