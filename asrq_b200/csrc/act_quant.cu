@@ -207,33 +207,28 @@ quant_int4_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, floa
   }
 }
 
-// K = 4096 specialisation.  The five butterfly strides that cross lanes in the generic kernel
-// (640 shuffles per lane) are replaced by one transpose through shared memory:
-//   phase A  lane L owns elements L*128 .. L*128+127 (index bits 0-6 private): strides 1..64;
-//   phase B  lane L owns elements o*128 + L*4 + c, o = 0..31, c = 0..3 (bits 0-1 and 7-11 private):
-//            strides 128..2048, and the four consecutive elements pack into one store.
-// A lane's 128 values live in registers as 64 pairs of neighbouring elements (e_2j, e_2j+1), in
-// both phases, so every butterfly except stride 1 is one packed fp32 add and one packed fp32
-// subtract (add.f32x2 / fma.f32x2) on two pairs.  The transpose goes through a per-warp
-// shared-memory array of 16-byte slots, slot(owner, g) = g*32 + (owner ^ g) for the four elements
-// 4g..4g+3: conflict-free both when every lane writes its own groups and when lane L reads group L
-// of every owner.
-// The division by sqrt(4096) = 64 is exact and is applied to the scale only: rint((v/64) / (s/64))
-// is rint(v/s) bit for bit.
+// K = 1024 and 4096: 32 and 64 threads per token, each with 32 and 64 values, and ONE transpose through shared memory where the
+// kernel above has five levels of shuffles:
+//   phase A  thread t holds the pairs (e, e + 1), e = i * 2T + 2t, i = 0..NI-1, as it loads them (a warp 128 contiguous bytes per
+//            i): strides 1 and 2T .. K/2 are private;
+//   phase B  thread u = 2i + c holds the elements i * 2T + 2j + c, j = 0..T-1: strides 2 .. T.  The two threads of an i hold every
+//            other element; they swap halves of their packed codes so that each stores T consecutive ones.
+// Values live as pairs, so every butterfly but the one inside the pair is a packed fp32 add and a packed subtract (add.f32x2 /
+// fma.f32x2) on two pairs.  Rows of the transpose are padded by four floats: its 4-byte writes and 16-byte reads are free of bank
+// conflicts.
+// Bound: instruction issue (about 500 clocks per token of 4096 and SM, 110 per token of 1024) as long as enough warps hide the
+// latencies.  One warp per token of 4096 (128 values a lane, nine warps per SM, 41 KB of straight-line code) took 24.5 us for 6000
+// tokens; shuffles for 1024 took 1100 instructions per token.
+// The division by sqrt(K) = 32 or 64 is exact and is applied to the scale only: rint((v/64) / (s/64)) is rint(v/s) bit for bit.
 // Quantisation without a division per element: t_lo = fma(v, inv_lo, magic), t_hi = fma(v, inv_hi,
 // magic) with inv_lo < 1/s < inv_hi (2^-22 apart) bracket the exact quotient, and adding 1.5*2^23
 // rounds to nearest-even and leaves the two's-complement code in the low mantissa bits; where the
 // two agree (all but a few elements in a million) that is rint(v/s); where they differ the true
 // quotient is computed.
-constexpr int kHad4096Warps = 3;
-constexpr int kHad4096WarpBytes = 16384;  // fp32 transpose array; the fp16 staging area is overlaid on its first half
-
 __device__ __forceinline__ float2 sub2(float2 a, float2 c) { return __ffma2_rn(c, make_float2(-1.f, -1.f), a); }
 
-// The rare path of quant4_bytes, out of line so that its 32 call sites do not double the size of the
-// kernel (inlined, the kernel was 66 KB of code against 41 KB and took 31 us against 24.5 us for 6000
-// tokens: its hot path is ~2000 instructions of straight-line code per token, fetched once per warp):
-// IEEE division and round-half-even, as magic + code.
+// The rare path of quant4_bytes, out of line so that its call sites do not swell the kernel: IEEE division and round-half-even,
+// as magic + code.
 __device__ __noinline__ float4 quant4_exact(float2 v01, float2 v23, float s) {
   return make_float4(__fadd_rn(rintf(__fdiv_rn(v01.x, s)), 12582912.f), __fadd_rn(rintf(__fdiv_rn(v01.y, s)), 12582912.f),
                      __fadd_rn(rintf(__fdiv_rn(v23.x, s)), 12582912.f), __fadd_rn(rintf(__fdiv_rn(v23.y, s)), 12582912.f));
@@ -263,102 +258,142 @@ __device__ __forceinline__ uint32_t quant4_bytes(float2 v01, float2 v23, float2 
   return prmt(p01, p23, 0x5410u);
 }
 
-template <int OUT, bool BF16>
-__global__ void __launch_bounds__(kHad4096Warps * 32, 3)
-hadamard4096_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {
-  extern __shared__ uint4 smem4[];
+// log2 levels over an array of pairs: strides of 1 .. N / 2 pairs
+template <int N>
+__device__ __forceinline__ void butterflies(float2 (&P)[N]) {
+#pragma unroll
+  for (int h = 1; h < N; h <<= 1)
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if ((j & h) == 0) {
+        const float2 a = P[j], c = P[j + h];
+        P[j] = __fadd2_rn(a, c);
+        P[j + h] = sub2(a, c);
+      }
+}
+template <int N>
+__device__ __forceinline__ void inside_pairs(float2 (&P)[N]) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) P[j] = make_float2(P[j].x + P[j].y, P[j].x - P[j].y);
+}
+
+template <int K, int T>
+constexpr int kHadTokens = T == 64 ? 1 : 4;  // per block
+
+template <int K, int T, int OUT, bool BF16>
+__global__ void __launch_bounds__(T * kHadTokens<K, T>, T == 64 ? 8 : 5)
+hadamard_transpose_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {
+  constexpr int NI = K / (2 * T), PITCH = T + 4, TOKENS = kHadTokens<K, T>;
+  static_assert(2 * NI == T, "one row of the transpose per thread");
+  __shared__ __align__(16) float rows_all[TOKENS][T * PITCH];
+  __shared__ float part[2];
   // A GEMM launched behind this kernel with programmatic stream serialisation may be scheduled once
   // every block of this grid has started, and set itself up on SMs the last wave leaves idle; it
   // orders itself with griddepcontrol.wait before it touches this kernel's output.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int token = blockIdx.x * kHad4096Warps + warp;
-  if (token >= M) return;  // warp-uniform; only warp-level synchronisation below
-  uint4* stg = smem4 + warp * (kHad4096WarpBytes / 16);  // 512 slots of 8 fp16, dead once phase A has loaded them
-  float4* pv = reinterpret_cast<float4*>(stg);           // 1024 slots of 4 fp32
-  // coalesced global load, each 16-byte unit handed to the lane that owns it in phase A
-  const uint4* src = reinterpret_cast<const uint4*>(x + size_t(token) * 4096);
+  const int t = threadIdx.x % T, token = blockIdx.x * TOKENS + threadIdx.x / T;
+  float* rows = rows_all[threadIdx.x / T];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (token >= M) return;  // a whole warp, which meets no other (T = 32), or nobody (T = 64)
+  auto meet = [&]() {
+    if (T == 64) {
+      __syncthreads();
+    } else {
+      __syncwarp();
+    }
+  };
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(x + size_t(token) * K) + t;
+  uint32_t raw[NI];
 #pragma unroll
-  for (int jj = 0; jj < 16; ++jj) {
-    const int u = jj * 32 + lane;
-    const int owner = u >> 4, j = u & 15;
-    stg[owner * 16 + (j ^ (owner & 15))] = __ldg(src + u);
+  for (int i = 0; i < NI; ++i) raw[i] = __ldg(src + i * T);
+  {
+    float2 P[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      P[i] = BF16 ? make_float2(__uint_as_float(raw[i] << 16), __uint_as_float(raw[i] & 0xffff0000u)) : __half22float2(u32_as_h2(raw[i]));
+    inside_pairs(P);
+    butterflies(P);
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      rows[(2 * i) * PITCH + t] = P[i].x;
+      rows[(2 * i + 1) * PITCH + t] = P[i].y;
+    }
   }
-  __syncwarp();
-  // phase A: 64 pairs (e_2j, e_2j+1) of this lane's 128 consecutive elements
-  float2 P[64];
+  meet();
+  float2 Q[T / 2];
 #pragma unroll
-  for (int u = 0; u < 16; ++u) {
-    const uint4 q = stg[lane * 16 + (u ^ (lane & 15))];
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      P[4 * u + e] = BF16 ? make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u))
-                          : __half22float2(u32_as_h2(w[e]));
+  for (int k = 0; k < T / 4; ++k) {
+    const float4 z = *reinterpret_cast<const float4*>(rows + t * PITCH + 4 * k);
+    Q[2 * k] = make_float2(z.x, z.y);
+    Q[2 * k + 1] = make_float2(z.z, z.w);
   }
-  __syncwarp();  // every lane has read its staging row: pv may overwrite the area
-#pragma unroll
-  for (int j = 0; j < 64; ++j) {  // stride 1: inside the pair
-    const float a = P[j].x, c = P[j].y;
-    P[j] = make_float2(a + c, a - c);
-  }
-#pragma unroll
-  for (int h = 1; h < 64; h <<= 1)  // strides 2..64: pair j with pair j + h
-#pragma unroll
-    for (int j = 0; j < 64; ++j)
-      if ((j & h) == 0) {
-        const float2 a = P[j], c = P[j + h];
-        P[j] = __fadd2_rn(a, c);
-        P[j + h] = sub2(a, c);
-      }
-#pragma unroll
-  for (int g = 0; g < 32; ++g) pv[g * 32 + (lane ^ g)] = make_float4(P[2 * g].x, P[2 * g].y, P[2 * g + 1].x, P[2 * g + 1].y);
-  __syncwarp();
-  // phase B: transpose (lane L takes group L of every owner o), strides 128..2048 over o
-#pragma unroll
-  for (int o = 0; o < 32; ++o) {
-    const float4 z = pv[lane * 32 + (o ^ lane)];
-    P[2 * o] = make_float2(z.x, z.y);
-    P[2 * o + 1] = make_float2(z.z, z.w);
-  }
-#pragma unroll
-  for (int h = 2; h < 64; h <<= 1)
-#pragma unroll
-    for (int j = 0; j < 64; ++j)
-      if ((j & h) == 0) {
-        const float2 a = P[j], c = P[j + h];
-        P[j] = __fadd2_rn(a, c);
-        P[j + h] = sub2(a, c);
-      }
+  inside_pairs(Q);
+  butterflies(Q);
   float amax = 0.f;
 #pragma unroll
-  for (int j = 0; j < 64; ++j) amax = fmaxf(amax, fmaxf(fabsf(P[j].x), fabsf(P[j].y)));
+  for (int j = 0; j < T / 2; ++j) amax = fmaxf(amax, fmaxf(fabsf(Q[j].x), fabsf(Q[j].y)));
 #pragma unroll
   for (int mask = 16; mask > 0; mask >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, mask));
-  // scale of the unnormalised values; the token's scale is that / 64 (exact)
+  if (T == 64) {
+    if ((t & 31) == 0) part[t >> 5] = amax;
+    meet();
+    amax = fmaxf(part[0], part[1]);
+  }
+  // scale of the unnormalised values; the token's scale is that / sqrt(K) (exact)
   float s = __fdiv_rn(amax, 7.f);
   const bool zero = s == 0.f;
-  if (lane == 0) sa[token] = zero ? 1e-3f : s * 0.015625f;
+  if (t == 0) sa[token] = zero ? 1e-3f : s * (K == 4096 ? 0.015625f : 0.03125f);
   if (zero) s = 1.f;  // every value is 0: any scale gives code 0
   const float inv = __fdiv_rn(1.f, s);
   const float il = inv * (1.f - 2.384185791015625e-07f), ih = inv * (1.f + 2.384185791015625e-07f);  // 2^-22
   const float2 inv_lo = make_float2(il, il), inv_hi = make_float2(ih, ih);
-  // element index of (o, lane, c) is o*128 + lane*4 + c: one 32-bit (int8) or 16-bit (packed) store per o
-  uint32_t* d8 = reinterpret_cast<uint32_t*>(qa + size_t(token) * 4096);
-  uint16_t* d4 = reinterpret_cast<uint16_t*>(qa + size_t(token) * 2048);
+  uint32_t W[T / 4];  // the codes of elements 2j + c, four j per word
 #pragma unroll
-  for (int o = 0; o < 32; ++o) {
-    const uint32_t b = quant4_bytes<OUT>(P[2 * o], P[2 * o + 1], inv_lo, inv_hi, s);
-    if (OUT == 2) {
-      d8[o * 32 + lane] = b;
-    } else if (OUT == 1) {
-      d8[o * 32 + lane] = (b << 4) & 0xf0f0f0f0u;
-    } else {
-      const uint32_t n = b & 0x0f0f0f0fu;  // four nibbles in four bytes -> 16 bits, element 0 lowest
-      const uint32_t m = n | (n >> 4);     // bytes 0 and 2 now hold two nibbles each
-      d4[o * 32 + lane] = uint16_t((m & 0xffu) | ((m >> 8) & 0xff00u));
-    }
+  for (int k = 0; k < T / 4; ++k) W[k] = quant4_bytes<OUT>(Q[2 * k], Q[2 * k + 1], inv_lo, inv_hi, s);
+  const bool odd = t & 1;
+  uint32_t o[T / 4];  // T consecutive codes: the first or second half of this i
+#pragma unroll
+  for (int k = 0; k < T / 8; ++k) {
+    const uint32_t give = odd ? W[k] : W[k + T / 8], keep = odd ? W[k + T / 8] : W[k];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, give, 1);
+    const uint32_t ev = odd ? got : keep, od = odd ? keep : got;
+    o[2 * k] = prmt(ev, od, 0x5140u);
+    o[2 * k + 1] = prmt(ev, od, 0x7362u);
   }
+  if (OUT >= 1) {
+    uint4* d = reinterpret_cast<uint4*>(qa + size_t(token) * K + t * T);
+#pragma unroll
+    for (int k = 0; k < T / 4; ++k)
+      if (OUT == 1) o[k] = (o[k] << 4) & 0xf0f0f0f0u;
+#pragma unroll
+    for (int k = 0; k < T / 16; ++k) d[k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+  } else {
+    uint32_t n[T / 8];  // four nibbles in four bytes -> 16 bits, element 0 lowest; two words -> one
+#pragma unroll
+    for (int k = 0; k < T / 8; ++k) {
+      const uint32_t a = o[2 * k] & 0x0f0f0f0fu, b = o[2 * k + 1] & 0x0f0f0f0fu;
+      n[k] = prmt(a | (a >> 4), b | (b >> 4), 0x6420u);
+    }
+    uint4* d = reinterpret_cast<uint4*>(qa + size_t(token) * (K / 2) + t * (T / 2));
+#pragma unroll
+    for (int k = 0; k < T / 32; ++k) d[k] = make_uint4(n[4 * k], n[4 * k + 1], n[4 * k + 2], n[4 * k + 3]);
+  }
+}
+
+template <int K, int T, int OUT, bool BF16>
+static int launch_transpose_quant(const uint16_t* xp, uint8_t* qa, float* sa, int64_t M, cudaStream_t stream) {
+  constexpr int TOKENS = kHadTokens<K, T>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned((M + TOKENS - 1) / TOKENS));
+  cfg.blockDim = dim3(T * TOKENS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = option(kOptNoPdl) ? 0 : 1;
+  ASRQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, hadamard_transpose_quant_kernel<K, T, OUT, BF16>, xp, qa, sa, int(M)));
+  return ASRQ_OK;
 }
 
 template <int OUT>
@@ -373,15 +408,11 @@ static int launch_quant(const uint16_t* xp, uint8_t* qa, float* sa, int64_t M, i
     switch (K) {
       case 256: hadamard_quant_kernel<8, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
       case 512: hadamard_quant_kernel<16, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
-      case 1024: hadamard_quant_kernel<32, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
+      case 1024:
+        return bf16 ? launch_transpose_quant<1024, 32, OUT, true>(xp, qa, sa, M, stream) : launch_transpose_quant<1024, 32, OUT, false>(xp, qa, sa, M, stream);
       case 2048: hadamard_quant_kernel<64, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
-      case 4096: {
-        const int smem = kHad4096Warps * kHad4096WarpBytes;
-        auto kern = bf16 ? hadamard4096_quant_kernel<OUT, true> : hadamard4096_quant_kernel<OUT, false>;
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), size_t(smem))) return rc;
-        kern<<<int((M + kHad4096Warps - 1) / kHad4096Warps), kHad4096Warps * 32, smem, stream>>>(xp, qa, sa, int(M));
-        break;
-      }
+      case 4096:
+        return bf16 ? launch_transpose_quant<4096, 64, OUT, true>(xp, qa, sa, M, stream) : launch_transpose_quant<4096, 64, OUT, false>(xp, qa, sa, M, stream);
       default:
         return fail(ASRQ_ERR_SHAPE, "hadamard_quant_int4: K must be 256, 512, 1024, 2048 or 4096 (K=%lld)",
                     (long long)K);
