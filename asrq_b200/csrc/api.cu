@@ -462,8 +462,8 @@ int asrq_glu_dwconv(const void* in, const void* weight, const void* bias, const 
   if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_glu_dwconv: dtype %d", dtype);
   if (B < 0 || B > 65535 || T < 0 || T > (1 << 20) - 16 || channels <= 0 || channels % 2 || channels > (1 << 20) || taps != 9)
     return fail(ASRQ_ERR_SHAPE, "asrq_glu_dwconv: B=%lld T=%lld channels=%lld (even) taps=%d (9)", (long long)B, (long long)T, (long long)channels, taps);
-  if (reinterpret_cast<uintptr_t>(in) % 4 || reinterpret_cast<uintptr_t>(out) % 4)
-    return fail(ASRQ_ERR_ALIGN, "asrq_glu_dwconv: in and out must be 4-byte aligned");
+  for (const void* q : {in, weight, bias, scale, shift, static_cast<const void*>(out)})
+    if (reinterpret_cast<uintptr_t>(q) % 4) return fail(ASRQ_ERR_ALIGN, "asrq_glu_dwconv: pointers must be 4-byte aligned");
   const DeviceFacts* f;
   int rc;
   if ((rc = device_facts(&f))) return rc;

@@ -50,17 +50,16 @@ struct NormsParams {
   const uint16_t *x, *delta, *g1, *b1, *g2, *b2;
   uint16_t *x_out, *h_out;  // x_out: the residual stream that goes on (s, or y when there is a second norm); may be NULL
   float scale, eps1, eps2;
-  int rows, bf16;
+  int rows;
 };
 
-template <int VEC>
+template <int VEC, bool bf16>
 __global__ void __launch_bounds__(32 * kRowWarps)
 residual_norms_kernel(const NormsParams p) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31, r = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
   if (r >= p.rows) return;
-  const bool bf16 = p.bf16 != 0;
   const size_t off = size_t(r) * (256 * VEC) + lane * 8;
   uint4 row[VEC];
 #pragma unroll
@@ -97,24 +96,26 @@ residual_norms_kernel(const NormsParams p) {
 // A thread takes two channels (a warp 128 contiguous bytes of a row) and TL positions: all TL + KW - 1 gated inputs go into
 // registers first, so every load of the thread is in flight at once and the taps are fully unrolled.  TL = 16: the halo costs
 // half as many loads again (from L2); longer runs leave a single sequence with too few threads.
-template <int KW, int TL>
+template <int KW, int TL, bool bf16>
 __global__ void __launch_bounds__(128)
 glu_dwconv_kernel(const uint16_t* __restrict__ in, const uint16_t* __restrict__ w, const uint16_t* __restrict__ bias, const uint16_t* __restrict__ scale,
-                  const uint16_t* __restrict__ shift, uint16_t* __restrict__ out, int T, int d, int bf) {
+                  const uint16_t* __restrict__ shift, uint16_t* __restrict__ out, int T, int d) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const bool bf16 = bf != 0;
   const int c = (blockIdx.x * 128 + threadIdx.x) * 2, t0 = blockIdx.y * TL;
   const bool on = c < d;
   float wt[2][KW], bs[2], sc[2], sh[2];
   if (on) {
+    auto two = [&](const uint16_t* q) { return __ldg(reinterpret_cast<const unsigned int*>(q)); };
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-#pragma unroll
-      for (int i = 0; i < KW; ++i) wt[k][i] = out16_to_float(__ldg(w + size_t(c + k) * KW + i), bf16);
-      bs[k] = out16_to_float(__ldg(bias + c + k), bf16);
-      sc[k] = out16_to_float(__ldg(scale + c + k), bf16);
-      sh[k] = out16_to_float(__ldg(shift + c + k), bf16);
+    for (int i = 0; i < KW; ++i) {  // 2 KW consecutive taps
+      const uint32_t v = two(w + size_t(c) * KW + 2 * i);
+      wt[(2 * i) / KW][(2 * i) % KW] = lo16(v, bf16);
+      wt[(2 * i + 1) / KW][(2 * i + 1) % KW] = hi16(v, bf16);
     }
+    const uint32_t vb = two(bias + c), vs = two(scale + c), vh = two(shift + c);
+    bs[0] = lo16(vb, bf16), bs[1] = hi16(vb, bf16);
+    sc[0] = lo16(vs, bf16), sc[1] = hi16(vs, bf16);
+    sh[0] = lo16(vh, bf16), sh[1] = hi16(vh, bf16);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (!on) return;
@@ -128,11 +129,13 @@ glu_dwconv_kernel(const uint16_t* __restrict__ in, const uint16_t* __restrict__ 
     g[i] = in_range ? __ldg(reinterpret_cast<const unsigned int*>(base + size_t(t) * 2 * d + d)) : 0u;
   }
   auto r16 = [&](float v) { return out16_to_float(float_to_out16(v, bf16), bf16); };
+  // a few fp32 ulps (exponential and quotient) under a rounding to 16 bits; a denominator past 2^126 gives 0, its limit
+  auto sigmoid_of = [](float v, float g) { return __fdividef(v, 1.f + __expf(-g)); };
   float u[2][TL + KW - 1];
 #pragma unroll
   for (int i = 0; i < TL + KW - 1; ++i) {  // outside the sequence a = 0: the padding of the convolution
-    u[0][i] = r16(lo16(a[i], bf16) / (1.f + expf(-lo16(g[i], bf16))));
-    u[1][i] = r16(hi16(a[i], bf16) / (1.f + expf(-hi16(g[i], bf16))));
+    u[0][i] = r16(sigmoid_of(lo16(a[i], bf16), lo16(g[i], bf16)));
+    u[1][i] = r16(sigmoid_of(hi16(a[i], bf16), hi16(g[i], bf16)));
   }
   uint16_t* o = out + (size_t(blockIdx.z) * T + t0) * d + c;
 #pragma unroll
@@ -145,7 +148,7 @@ glu_dwconv_kernel(const uint16_t* __restrict__ in, const uint16_t* __restrict__ 
 #pragma unroll
       for (int i = 0; i < KW; ++i) acc = fmaf(u[k][t + i], wt[k][i], acc);
       const float v = r16(r16(r16(acc + bs[k]) * sc[k]) + sh[k]);
-      y[k] = v / (1.f + expf(-v));
+      y[k] = sigmoid_of(v, v);
     }
     *reinterpret_cast<unsigned int*>(o + size_t(t) * d) = pack16(y[0], y[1], bf16);
   }
@@ -172,17 +175,22 @@ int residual_norms(const void* x, const void* delta, float scale, const void* g1
                    void* x_out, void* h_out, int64_t rows, int64_t dim, int dtype, cudaStream_t stream) {
   auto in = [](const void* q) { return static_cast<const uint16_t*>(q); };
   const NormsParams p = {in(x), in(delta), in(g1), in(b1), in(g2), in(b2), static_cast<uint16_t*>(x_out), static_cast<uint16_t*>(h_out),
-                         scale, eps1, eps2, int(rows), dtype == ASRQ_BF16};
+                         scale, eps1, eps2, int(rows)};
   const dim3 grid(unsigned((rows + kRowWarps - 1) / kRowWarps)), block(32 * kRowWarps);
+  const bool bf16 = dtype == ASRQ_BF16;
   switch (dim / 256) {
-    case 1: return launch(residual_norms_kernel<1>, grid, block, stream, p);
-    case 2: return launch(residual_norms_kernel<2>, grid, block, stream, p);
-    case 3: return launch(residual_norms_kernel<3>, grid, block, stream, p);
-    case 4: return launch(residual_norms_kernel<4>, grid, block, stream, p);
-    case 5: return launch(residual_norms_kernel<5>, grid, block, stream, p);
-    case 6: return launch(residual_norms_kernel<6>, grid, block, stream, p);
-    case 7: return launch(residual_norms_kernel<7>, grid, block, stream, p);
-    default: return launch(residual_norms_kernel<8>, grid, block, stream, p);
+#define ASRQ_NORMS(V) \
+  case V: return bf16 ? launch(residual_norms_kernel<V, true>, grid, block, stream, p) : launch(residual_norms_kernel<V, false>, grid, block, stream, p)
+    ASRQ_NORMS(1);
+    ASRQ_NORMS(2);
+    ASRQ_NORMS(3);
+    ASRQ_NORMS(4);
+    ASRQ_NORMS(5);
+    ASRQ_NORMS(6);
+    ASRQ_NORMS(7);
+    ASRQ_NORMS(8);
+#undef ASRQ_NORMS
+    default: return fail(ASRQ_ERR_SHAPE, "residual_norms: dim=%lld", (long long)dim);
   }
 }
 
@@ -191,8 +199,8 @@ int glu_dwconv(const void* in, const void* w, const void* bias, const void* scal
   constexpr int TL = 16;
   auto q = [](const void* v) { return static_cast<const uint16_t*>(v); };
   const dim3 grid(unsigned((d / 2 + 127) / 128), unsigned((T + TL - 1) / TL), unsigned(B));
-  return launch(glu_dwconv_kernel<9, TL>, grid, dim3(128), stream, q(in), q(w), q(bias), q(scale), q(shift), static_cast<uint16_t*>(out), int(T), int(d),
-                int(dtype == ASRQ_BF16));
+  return launch(dtype == ASRQ_BF16 ? glu_dwconv_kernel<9, TL, true> : glu_dwconv_kernel<9, TL, false>, grid, dim3(128), stream, q(in), q(w), q(bias), q(scale),
+                q(shift), static_cast<uint16_t*>(out), int(T), int(d));
 }
 
 }  // namespace asrq

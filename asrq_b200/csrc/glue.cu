@@ -33,11 +33,11 @@ __device__ __forceinline__ float in16(uint16_t b, bool bf16) {
 constexpr int kLnWarps = 8;
 
 // VEC: 16-byte vectors per lane (dim = 256 * VEC); generic dims take the strided loop with VEC = 0
-template <int VEC>
+template <int VEC, bool bf16>
 __global__ void __launch_bounds__(32 * kLnWarps)
 add_layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ delta, const uint16_t* __restrict__ gamma,
                      const uint16_t* __restrict__ beta, float eps, uint16_t* __restrict__ x_out, uint16_t* __restrict__ h_out,
-                     int rows, int dim, int bf16) {
+                     int rows, int dim) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * kLnWarps + (threadIdx.x >> 5);
@@ -78,7 +78,7 @@ add_layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
       if (x_out) *reinterpret_cast<uint4*>(x_out + off + e) = xr[i];
     }
     float mean, rstd;
-    ln_row_stats<(VEC > 0 ? VEC : 1)>(xr, dim, eps, bf16 != 0, mean, rstd);
+    ln_row_stats<(VEC > 0 ? VEC : 1)>(xr, dim, eps, bf16, mean, rstd);
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int e = (i * 32 + lane) * 8;
@@ -128,11 +128,12 @@ add_layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
   }
 }
 
-// One warp per row; VEC 16-byte vectors per lane when dim == 256 * VEC, else (VEC = 0) a strided loop.
-template <int VEC>
+// One warp per row; VEC 16-byte vectors per lane when dim == 256 * VEC, else (VEC = 0) a strided loop.  All of a row's loads go
+// out before the first is used.
+template <int VEC, bool bf16>
 __global__ void __launch_bounds__(32 * kLnWarps)
 add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ delta, const uint16_t* __restrict__ gamma,
-                   float eps, uint16_t* __restrict__ x_out, uint16_t* __restrict__ h_out, int rows, int dim, int bf16) {
+                   float eps, uint16_t* __restrict__ x_out, uint16_t* __restrict__ h_out, int rows, int dim) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31;
@@ -142,16 +143,17 @@ add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
   if constexpr (VEC > 0) {
     float v[VEC > 0 ? VEC * 8 : 1];
     float sq = 0.f;
+    uint4 a8[VEC > 0 ? VEC : 1], d8[VEC > 0 ? VEC : 1];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) a8[i] = *reinterpret_cast<const uint4*>(x + off + (i * 32 + lane) * 8);
+    if (delta) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) d8[i] = *reinterpret_cast<const uint4*>(delta + off + (i * 32 + lane) * 8);
+    }
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int e = (i * 32 + lane) * 8;
-      const uint4 a = *reinterpret_cast<const uint4*>(x + off + e);
-      const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-      uint32_t dw[4] = {0, 0, 0, 0};
-      if (delta) {
-        const uint4 d = *reinterpret_cast<const uint4*>(delta + off + e);
-        dw[0] = d.x; dw[1] = d.y; dw[2] = d.z; dw[3] = d.w;
-      }
+      const uint32_t aw[4] = {a8[i].x, a8[i].y, a8[i].z, a8[i].w}, dw[4] = {d8[i].x, d8[i].y, d8[i].z, d8[i].w};
       uint32_t ow[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -209,118 +211,163 @@ add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
   }
 }
 
-// gu: rows x 2*inter (gate columns first, then up), out: rows x inter; eight elements per thread
+// gu: rows x 2*inter (gate columns first, then up), out: rows x inter; eight elements per thread and row, kSiluRows rows in
+// flight.  Bound: memory; with one row at a time, a division to find it and exact quotients it took 2.2x the time of its bytes.
+// The exponential and the quotient are a few fp32 ulps off, under a rounding to 16 bits.
+constexpr int kSiluRows = 2;
+template <bool bf16>
 __global__ void __launch_bounds__(256)
-silu_mul_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int rows, int inter, int bf16) {
+silu_mul_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int rows, int inter) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int vpr = inter / 8;  // vectors per output row
-  const size_t n_vec = size_t(rows) * vpr;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n_vec; i += size_t(gridDim.x) * blockDim.x) {
-    const size_t r = i / vpr, c = (i - r * vpr) * 8;
-    const uint4 g = *reinterpret_cast<const uint4*>(gu + r * 2 * inter + c);
-    const uint4 u = *reinterpret_cast<const uint4*>(gu + r * 2 * inter + inter + c);
-    const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
-    uint32_t ow[4];
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+  if (c >= inter) return;
+  for (int r0 = blockIdx.y * kSiluRows; r0 < rows; r0 += gridDim.y * kSiluRows) {
+    uint4 g[kSiluRows], u[kSiluRows];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint16_t o2[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float gv = in16(uint16_t(gw[j] >> (16 * h)), bf16), uv = in16(uint16_t(uw[j] >> (16 * h)), bf16);
-        const float sv = in16(float_to_out16(gv / (1.f + expf(-gv)), bf16), bf16);  // silu, rounded as the module rounds it
-        o2[h] = float_to_out16(sv * uv, bf16);
-      }
-      ow[j] = uint32_t(o2[0]) | (uint32_t(o2[1]) << 16);
+    for (int k = 0; k < kSiluRows; ++k) {
+      const uint16_t* src = gu + size_t(min(r0 + k, rows - 1)) * 2 * inter + c;
+      g[k] = *reinterpret_cast<const uint4*>(src);
+      u[k] = *reinterpret_cast<const uint4*>(src + inter);
     }
-    *reinterpret_cast<uint4*>(out + r * inter + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+#pragma unroll
+    for (int k = 0; k < kSiluRows; ++k) {
+      const uint32_t gw[4] = {g[k].x, g[k].y, g[k].z, g[k].w}, uw[4] = {u[k].x, u[k].y, u[k].z, u[k].w};
+      uint32_t ow[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint16_t o2[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float gv = in16(uint16_t(gw[j] >> (16 * h)), bf16), uv = in16(uint16_t(uw[j] >> (16 * h)), bf16);
+          const float sv = in16(float_to_out16(__fdividef(gv, 1.f + __expf(-gv)), bf16), bf16);  // silu, rounded as the module rounds it
+          o2[h] = float_to_out16(sv * uv, bf16);
+        }
+        ow[j] = uint32_t(o2[0]) | (uint32_t(o2[1]) << 16);
+      }
+      if (r0 + k < rows) *reinterpret_cast<uint4*>(out + size_t(r0 + k) * inter + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    }
   }
 }
 
-// qkv: rows x (nq + 2 nkv) x hd, a row = sequence b, step t (rows = B * T).  One warp per (row, head); E = hd / 32
-// elements per lane; the rotary partner of element i is i +- hd / 2, i.e. the same slot of lane ^ 16.
-// q_out: B x nq x T x hd; caches: B x nkv x max_len x hd, written at position pos0 + t.
-template <int E>
+// qkv: rows x (nq + 2 nkv) x HD, a row = sequence b, step t (rows = B * T).  A warp takes up to kRopeHeads heads of one row, so
+// that the row's cosines and sines are read once for them and all its loads are in flight together; HD / 8 lanes share a head,
+// 8 elements each; the rotary partner of an element is the same slot of the lane HD / 16 away.  VEC: 16-byte accesses (else 8-byte
+// aligned tensors).  q_out: B x nq x T x HD; caches: B x nkv x max_len x HD, written at position pos0 + t.
+// Bound: memory.  With a warp per head, 4 elements a lane and the tables read by element it took four times its bytes.
+constexpr int kRopeHeads = 8;
+template <int HD, bool bf16, bool VEC>
 __global__ void __launch_bounds__(256)
 qk_norm_rope_kernel(const uint16_t* __restrict__ qkv, const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
                     const uint16_t* __restrict__ cos_t, const uint16_t* __restrict__ sin_t, const long long* __restrict__ pos_dev,
                     long long pos_host, uint16_t* __restrict__ q_out, uint16_t* __restrict__ k_cache, uint16_t* __restrict__ v_cache,
-                    int rows, int T, int nq, int nkv, int max_len, float eps, int bf16) {
+                    int rows, int T, int nq, int nkv, int max_len, float eps) {
+  constexpr int LPH = HD / 8, PER = 32 / LPH, PASSES = kRopeHeads / PER;  // lanes per head, heads per pass
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  constexpr int hd = 32 * E;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, sub = lane % LPH, hg = lane / LPH;
   const int heads = nq + 2 * nkv;
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= (long long)rows * heads) return;
-  const int row = int(item / heads), head = int(item - (long long)row * heads);
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), head0 = blockIdx.y * kRopeHeads;
+  if (row >= rows) return;  // whole warps
+  auto load8 = [&](const uint16_t* p, uint32_t (&w)[4]) {
+    if (VEC) {
+      const uint4 u = *reinterpret_cast<const uint4*>(p);
+      w[0] = u.x, w[1] = u.y, w[2] = u.z, w[3] = u.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = uint32_t(p[2 * i]) | (uint32_t(p[2 * i + 1]) << 16);
+    }
+  };
+  auto value = [&](const uint32_t (&w)[4], int i) { return in16(uint16_t(w[i >> 1] >> (16 * (i & 1))), bf16); };
   const int b = row / T, t = row - b * T;
   const long long pos = (pos_dev ? *pos_dev : pos_host) + t;
-  const uint16_t* src = qkv + (size_t(row) * heads + head) * hd + lane * E;
-  uint16_t v16[E];
-  if (E == 4) {
-    const uint2 u = *reinterpret_cast<const uint2*>(src);
-    v16[0] = uint16_t(u.x & 0xffffu); v16[1] = uint16_t(u.x >> 16); v16[2 % E] = uint16_t(u.y & 0xffffu); v16[3 % E] = uint16_t(u.y >> 16);
-  } else {
-    const uint32_t u = *reinterpret_cast<const uint32_t*>(src);
-    v16[0] = uint16_t(u & 0xffffu); v16[1] = uint16_t(u >> 16);
-  }
-  uint16_t* dst;
-  if (head < nq) {
-    dst = q_out + ((size_t(b) * nq + head) * T + t) * hd + lane * E;
-  } else if (head < nq + nkv) {
-    dst = k_cache + ((size_t(b) * nkv + (head - nq)) * max_len + size_t(pos)) * hd + lane * E;
-  } else {
-    dst = v_cache + ((size_t(b) * nkv + (head - nq - nkv)) * max_len + size_t(pos)) * hd + lane * E;
-  }
-  if (head < nq + nkv) {  // queries and keys: norm over the head, weight, rotary embedding
-    const uint16_t* w = (head < nq ? qw : kw) + lane * E;
-    float f[E], sq = 0.f;
+  uint32_t v[PASSES][4], cw[4], sw[4], wq[4], wk[4];
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      f[i] = in16(v16[i], bf16);
-      sq = fmaf(f[i], f[i], sq);
+  for (int i = 0; i < PASSES; ++i) {
+    const int head = head0 + i * PER + hg;
+    if (head < heads) load8(qkv + (size_t(row) * heads + head) * HD + sub * 8, v[i]);
+  }
+  load8(cos_t + size_t(pos) * HD + sub * 8, cw);
+  load8(sin_t + size_t(pos) * HD + sub * 8, sw);
+  load8(qw + sub * 8, wq);
+  load8(kw + sub * 8, wk);
+#pragma unroll
+  for (int i = 0; i < PASSES; ++i) {
+    const int head = head0 + i * PER + hg;
+    const bool is_q = head < nq, is_k = !is_q && head < nq + nkv, on = head < heads;
+    // queries and keys: norm over the head, weight, rotary embedding (every lane takes part in the shuffles)
+    float f[8], sq = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      f[e] = on ? value(v[i], e) : 0.f;
+      sq = fmaf(f[e], f[e], sq);
     }
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    const float rs = rsqrtf(sq / float(hd) + eps);
+    for (int o = 1; o < LPH; o *= 2) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    const float rs = rsqrtf(sq / float(HD) + eps);
+    uint32_t out[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const float n = in16(float_to_out16(f[i] * rs, bf16), bf16);
-      const float y = in16(float_to_out16(in16(w[i], bf16) * n, bf16), bf16);
-      const float partner = __shfl_xor_sync(0xffffffffu, y, 16);
-      const float rot = lane < 16 ? -partner : partner;
-      const size_t ci = size_t(pos) * hd + lane * E + i;
-      const float a = in16(float_to_out16(y * in16(cos_t[ci], bf16), bf16), bf16);
-      const float c = in16(float_to_out16(rot * in16(sin_t[ci], bf16), bf16), bf16);
-      v16[i] = float_to_out16(a + c, bf16);
+    for (int e = 0; e < 8; ++e) {
+      const float n = in16(float_to_out16(f[e] * rs, bf16), bf16);
+      const float y = in16(float_to_out16((is_q ? value(wq, e) : value(wk, e)) * n, bf16), bf16);
+      const float partner = __shfl_xor_sync(0xffffffffu, y, LPH / 2);
+      const float rot = sub < LPH / 2 ? -partner : partner;
+      const float a = in16(float_to_out16(y * value(cw, e), bf16), bf16);
+      const float c = in16(float_to_out16(rot * value(sw, e), bf16), bf16);
+      out[e >> 1] |= uint32_t(float_to_out16(a + c, bf16)) << (16 * (e & 1));
     }
-  }
-  if (E == 4) {
-    *reinterpret_cast<uint2*>(dst) = make_uint2(uint32_t(v16[0]) | (uint32_t(v16[1]) << 16), uint32_t(v16[2 % E]) | (uint32_t(v16[3 % E]) << 16));
-  } else {
-    *reinterpret_cast<uint32_t*>(dst) = uint32_t(v16[0]) | (uint32_t(v16[1]) << 16);
+    if (!on) continue;
+    uint16_t* dst;
+    if (is_q) {
+      dst = q_out + ((size_t(b) * nq + head) * T + t) * HD + sub * 8;
+    } else if (is_k) {
+      dst = k_cache + ((size_t(b) * nkv + (head - nq)) * max_len + size_t(pos)) * HD + sub * 8;
+    } else {
+      dst = v_cache + ((size_t(b) * nkv + (head - nq - nkv)) * max_len + size_t(pos)) * HD + sub * 8;
+    }
+    const bool rotated = is_q || is_k;
+    const uint4 o = make_uint4(rotated ? out[0] : v[i][0], rotated ? out[1] : v[i][1], rotated ? out[2] : v[i][2], rotated ? out[3] : v[i][3]);
+    if (VEC) {
+      *reinterpret_cast<uint4*>(dst) = o;
+    } else {
+      reinterpret_cast<uint2*>(dst)[0] = make_uint2(o.x, o.y);
+      reinterpret_cast<uint2*>(dst)[1] = make_uint2(o.z, o.w);
+    }
   }
 }
 
+// kEpiVecs 16-byte vectors per thread in flight.  Bound: memory (with one vector at a time and the type, the activation and the
+// residual tested per element it ran at half of that).
+constexpr int kEpiVecs = 4;
+template <bool bf16, bool GELU, bool RES>
 __global__ void __launch_bounds__(256)
-epilogue16_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ residual, size_t n_vec, int act, int bf16) {
+epilogue16_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ residual, size_t n_vec) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n_vec; i += size_t(gridDim.x) * blockDim.x) {
-    uint4 a = reinterpret_cast<uint4*>(y)[i];
-    uint32_t aw[4] = {a.x, a.y, a.z, a.w}, rw[4] = {0, 0, 0, 0};
-    if (residual) {
-      const uint4 r = reinterpret_cast<const uint4*>(residual)[i];
-      rw[0] = r.x; rw[1] = r.y; rw[2] = r.z; rw[3] = r.w;
+  for (size_t i0 = size_t(blockIdx.x) * (256 * kEpiVecs) + threadIdx.x; i0 < n_vec; i0 += size_t(gridDim.x) * (256 * kEpiVecs)) {
+    uint4 a[kEpiVecs], r[kEpiVecs];
+#pragma unroll
+    for (int k = 0; k < kEpiVecs; ++k) {
+      const size_t i = i0 + k * 256;
+      if (i < n_vec) {
+        a[k] = reinterpret_cast<const uint4*>(y)[i];
+        if (RES) r[k] = __ldcs(reinterpret_cast<const uint4*>(residual) + i);
+      }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint16_t lo = epilogue16(uint16_t(aw[j] & 0xffffu), act, residual != nullptr, uint16_t(rw[j] & 0xffffu), bf16 != 0);
-      const uint16_t hi = epilogue16(uint16_t(aw[j] >> 16), act, residual != nullptr, uint16_t(rw[j] >> 16), bf16 != 0);
-      aw[j] = uint32_t(lo) | (uint32_t(hi) << 16);
+    for (int k = 0; k < kEpiVecs; ++k) {
+      const size_t i = i0 + k * 256;
+      if (i >= n_vec) break;
+      uint32_t aw[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
+      const uint32_t rw[4] = {RES ? r[k].x : 0u, RES ? r[k].y : 0u, RES ? r[k].z : 0u, RES ? r[k].w : 0u};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint16_t lo = epilogue16(uint16_t(aw[j] & 0xffffu), GELU ? kActGelu : kActNone, RES, uint16_t(rw[j] & 0xffffu), bf16);
+        const uint16_t hi = epilogue16(uint16_t(aw[j] >> 16), GELU ? kActGelu : kActNone, RES, uint16_t(rw[j] >> 16), bf16);
+        aw[j] = uint32_t(lo) | (uint32_t(hi) << 16);
+      }
+      reinterpret_cast<uint4*>(y)[i] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
     }
-    reinterpret_cast<uint4*>(y)[i] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
   }
 }
 
@@ -342,64 +389,87 @@ int launch_pdl(K kern, dim3 grid, dim3 block, cudaStream_t stream, Args... args)
 
 }  // namespace
 
-int add_layernorm(const void* x, const void* delta, const void* gamma, const void* beta, float eps, void* x_out, void* h_out,
-                  int64_t rows, int64_t dim, int dtype, cudaStream_t stream) {
-  const int bf16 = dtype == ASRQ_BF16;
+namespace {
+template <bool bf16>
+int add_layernorm_as(const uint16_t* x, const uint16_t* delta, const uint16_t* gamma, const uint16_t* beta, float eps, uint16_t* x_out, uint16_t* h_out,
+                     int rows, int dim, cudaStream_t stream) {
   const dim3 grid(unsigned((rows + kLnWarps - 1) / kLnWarps)), block(32 * kLnWarps);
-  auto xp = static_cast<const uint16_t*>(x), dp = static_cast<const uint16_t*>(delta);
-  auto gp = static_cast<const uint16_t*>(gamma), bp = static_cast<const uint16_t*>(beta);
-  auto xo = static_cast<uint16_t*>(x_out), ho = static_cast<uint16_t*>(h_out);
   const bool vec_ok = aligned16(x) && aligned16(h_out) && aligned16(gamma) && aligned16(beta) && (!delta || aligned16(delta)) &&
                       (!x_out || aligned16(x_out));
-  if (vec_ok && dim == 1280) return launch_pdl(add_layernorm_kernel<5>, grid, block, stream, xp, dp, gp, bp, eps, xo, ho, int(rows), int(dim), bf16);
-  if (vec_ok && dim == 1024) return launch_pdl(add_layernorm_kernel<4>, grid, block, stream, xp, dp, gp, bp, eps, xo, ho, int(rows), int(dim), bf16);
-  if (vec_ok && dim == 2048) return launch_pdl(add_layernorm_kernel<8>, grid, block, stream, xp, dp, gp, bp, eps, xo, ho, int(rows), int(dim), bf16);
-  if (vec_ok && dim == 256) return launch_pdl(add_layernorm_kernel<1>, grid, block, stream, xp, dp, gp, bp, eps, xo, ho, int(rows), int(dim), bf16);
-  return launch_pdl(add_layernorm_kernel<0>, grid, block, stream, xp, dp, gp, bp, eps, xo, ho, int(rows), int(dim), bf16);
+  auto run = [&](auto kern) { return launch_pdl(kern, grid, block, stream, x, delta, gamma, beta, eps, x_out, h_out, rows, dim); };
+  if (vec_ok && dim == 1280) return run(add_layernorm_kernel<5, bf16>);
+  if (vec_ok && dim == 1024) return run(add_layernorm_kernel<4, bf16>);
+  if (vec_ok && dim == 2048) return run(add_layernorm_kernel<8, bf16>);
+  if (vec_ok && dim == 256) return run(add_layernorm_kernel<1, bf16>);
+  return run(add_layernorm_kernel<0, bf16>);
+}
+template <bool bf16>
+int add_rmsnorm_as(const uint16_t* x, const uint16_t* delta, const uint16_t* gamma, float eps, uint16_t* x_out, uint16_t* h_out, int rows, int dim,
+                   cudaStream_t stream) {
+  const dim3 grid(unsigned((rows + kLnWarps - 1) / kLnWarps)), block(32 * kLnWarps);
+  const bool vec_ok = aligned16(x) && aligned16(h_out) && aligned16(gamma) && (!delta || aligned16(delta)) && (!x_out || aligned16(x_out));
+  auto run = [&](auto kern) { return launch_pdl(kern, grid, block, stream, x, delta, gamma, eps, x_out, h_out, rows, dim); };
+  if (vec_ok && dim == 2048) return run(add_rmsnorm_kernel<8, bf16>);
+  if (vec_ok && dim == 1024) return run(add_rmsnorm_kernel<4, bf16>);
+  if (vec_ok && dim == 256) return run(add_rmsnorm_kernel<1, bf16>);
+  return run(add_rmsnorm_kernel<0, bf16>);
+}
+const uint16_t* in_ptr(const void* v) { return static_cast<const uint16_t*>(v); }
+uint16_t* out_ptr(void* v) { return static_cast<uint16_t*>(v); }
+}  // namespace
+
+int add_layernorm(const void* x, const void* delta, const void* gamma, const void* beta, float eps, void* x_out, void* h_out,
+                  int64_t rows, int64_t dim, int dtype, cudaStream_t stream) {
+  auto run = dtype == ASRQ_BF16 ? add_layernorm_as<true> : add_layernorm_as<false>;
+  return run(in_ptr(x), in_ptr(delta), in_ptr(gamma), in_ptr(beta), eps, out_ptr(x_out), out_ptr(h_out), int(rows), int(dim), stream);
 }
 
 int add_rmsnorm(const void* x, const void* delta, const void* gamma, float eps, void* x_out, void* h_out, int64_t rows,
                 int64_t dim, int dtype, cudaStream_t stream) {
-  const int bf16 = dtype == ASRQ_BF16;
-  const dim3 grid(unsigned((rows + kLnWarps - 1) / kLnWarps)), block(32 * kLnWarps);
-  auto xp = static_cast<const uint16_t*>(x), dp = static_cast<const uint16_t*>(delta);
-  auto gp = static_cast<const uint16_t*>(gamma);
-  auto xo = static_cast<uint16_t*>(x_out), ho = static_cast<uint16_t*>(h_out);
-  const bool vec_ok = aligned16(x) && aligned16(h_out) && aligned16(gamma) && (!delta || aligned16(delta)) && (!x_out || aligned16(x_out));
-  if (vec_ok && dim == 2048) return launch_pdl(add_rmsnorm_kernel<8>, grid, block, stream, xp, dp, gp, eps, xo, ho, int(rows), int(dim), bf16);
-  if (vec_ok && dim == 1024) return launch_pdl(add_rmsnorm_kernel<4>, grid, block, stream, xp, dp, gp, eps, xo, ho, int(rows), int(dim), bf16);
-  if (vec_ok && dim == 256) return launch_pdl(add_rmsnorm_kernel<1>, grid, block, stream, xp, dp, gp, eps, xo, ho, int(rows), int(dim), bf16);
-  return launch_pdl(add_rmsnorm_kernel<0>, grid, block, stream, xp, dp, gp, eps, xo, ho, int(rows), int(dim), bf16);
+  auto run = dtype == ASRQ_BF16 ? add_rmsnorm_as<true> : add_rmsnorm_as<false>;
+  return run(in_ptr(x), in_ptr(delta), in_ptr(gamma), eps, out_ptr(x_out), out_ptr(h_out), int(rows), int(dim), stream);
 }
 
 int silu_mul(const void* gu, void* out, int64_t rows, int64_t inter, int dtype, int sm_count, cudaStream_t stream) {
-  const size_t n_vec = size_t(rows) * size_t(inter) / 8;
-  const unsigned blocks = unsigned(std::max<size_t>(1, std::min<size_t>(size_t(sm_count) * 8, (n_vec + 255) / 256)));
-  return launch_pdl(silu_mul_kernel, dim3(blocks), dim3(256), stream, static_cast<const uint16_t*>(gu), static_cast<uint16_t*>(out),
-                    int(rows), int(inter), int(dtype == ASRQ_BF16));
+  const unsigned gx = unsigned((inter / 8 + 255) / 256);
+  const int64_t passes = (rows + kSiluRows - 1) / kSiluRows;
+  const unsigned gy = unsigned(std::max<int64_t>(1, std::min<int64_t>({passes, int64_t(sm_count) * 16 / gx + 1, 65535})));
+  return launch_pdl(dtype == ASRQ_BF16 ? silu_mul_kernel<true> : silu_mul_kernel<false>, dim3(gx, gy), dim3(256), stream, in_ptr(gu), out_ptr(out),
+                    int(rows), int(inter));
 }
 
 int qk_norm_rope(const void* qkv, const void* qw, const void* kw, const void* cos_t, const void* sin_t, const long long* pos_dev,
                  long long pos_host, void* q_out, void* k_cache, void* v_cache, int64_t B, int64_t T, int nq, int nkv, int hd,
                  int64_t max_len, float eps, int dtype, cudaStream_t stream) {
-  const int64_t items = B * T * (nq + 2 * nkv);
-  const dim3 grid(unsigned((items + 7) / 8)), block(256);
-  auto p = [](const void* v) { return static_cast<const uint16_t*>(v); };
-  auto o = [](void* v) { return static_cast<uint16_t*>(v); };
-  const int bf16 = dtype == ASRQ_BF16;
-  if (hd == 128)
-    return launch_pdl(qk_norm_rope_kernel<4>, grid, block, stream, p(qkv), p(qw), p(kw), p(cos_t), p(sin_t), pos_dev, pos_host, o(q_out),
-                      o(k_cache), o(v_cache), int(B * T), int(T), nq, nkv, int(max_len), eps, bf16);
-  return launch_pdl(qk_norm_rope_kernel<2>, grid, block, stream, p(qkv), p(qw), p(kw), p(cos_t), p(sin_t), pos_dev, pos_host, o(q_out),
-                    o(k_cache), o(v_cache), int(B * T), int(T), nq, nkv, int(max_len), eps, bf16);
+  const dim3 grid(unsigned((B * T + 7) / 8), unsigned((nq + 2 * nkv + kRopeHeads - 1) / kRopeHeads)), block(256);
+  bool vec = true;
+  for (const void* q : {qkv, qw, kw, cos_t, sin_t, static_cast<const void*>(q_out), static_cast<const void*>(k_cache), static_cast<const void*>(v_cache)})
+    vec = vec && aligned16(q);
+  auto run = [&](auto kern) {
+    return launch_pdl(kern, grid, block, stream, in_ptr(qkv), in_ptr(qw), in_ptr(kw), in_ptr(cos_t), in_ptr(sin_t), pos_dev, pos_host, out_ptr(q_out),
+                      out_ptr(k_cache), out_ptr(v_cache), int(B * T), int(T), nq, nkv, int(max_len), eps);
+  };
+  const bool bf16 = dtype == ASRQ_BF16;
+  if (hd == 128) {
+    if (vec) return bf16 ? run(qk_norm_rope_kernel<128, true, true>) : run(qk_norm_rope_kernel<128, false, true>);
+    return bf16 ? run(qk_norm_rope_kernel<128, true, false>) : run(qk_norm_rope_kernel<128, false, false>);
+  }
+  if (vec) return bf16 ? run(qk_norm_rope_kernel<64, true, true>) : run(qk_norm_rope_kernel<64, false, true>);
+  return bf16 ? run(qk_norm_rope_kernel<64, true, false>) : run(qk_norm_rope_kernel<64, false, false>);
 }
 
 // y = act(y) / y = residual + y over M x N 16-bit elements (M*N a multiple of 8, pointers 16-byte aligned)
 int epilogue16_apply(void* y, const void* residual, int64_t M, int64_t N, int act, int dtype, int sm_count, cudaStream_t stream) {
   const size_t n_vec = size_t(M) * size_t(N) / 8;
-  const unsigned blocks = unsigned(std::max<size_t>(1, std::min<size_t>(size_t(sm_count) * 8, (n_vec + 255) / 256)));
-  return launch_pdl(epilogue16_kernel, dim3(blocks), dim3(256), stream, static_cast<uint16_t*>(y),
-                    static_cast<const uint16_t*>(residual), n_vec, act, int(dtype == ASRQ_BF16));
+  const unsigned blocks = unsigned(std::max<size_t>(1, std::min<size_t>(size_t(sm_count) * 8, (n_vec + 256 * kEpiVecs - 1) / (256 * kEpiVecs))));
+  auto run = [&](auto kern) { return launch_pdl(kern, dim3(blocks), dim3(256), stream, out_ptr(y), in_ptr(residual), n_vec); };
+  const bool gelu = act == kActGelu;
+  if (dtype == ASRQ_BF16) {
+    if (residual) return gelu ? run(epilogue16_kernel<true, true, true>) : run(epilogue16_kernel<true, false, true>);
+    return gelu ? run(epilogue16_kernel<true, true, false>) : run(epilogue16_kernel<true, false, false>);
+  }
+  if (residual) return gelu ? run(epilogue16_kernel<false, true, true>) : run(epilogue16_kernel<false, false, true>);
+  return gelu ? run(epilogue16_kernel<false, true, false>) : run(epilogue16_kernel<false, false, false>);
 }
 
 }  // namespace asrq

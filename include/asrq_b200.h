@@ -188,7 +188,8 @@ int asrq_residual_norms(const void* x, const void* delta, float scale, const voi
 /*
  * A Conformer block's convolution module between its pointwise projections, channels last: u = in[.., :C] * sigmoid(in[.., C:]),
  * depthwise convolution of `taps` (9) over time with zero padding and bias, * scale + shift per channel, SiLU; rounded to `dtype`
- * after each of these.  in: B x T x 2 C; weight: C x taps; out: B x T x C; C even.
+ * after each of these.  in: B x T x 2 C; weight: C x taps; out: B x T x C; C even; 4-byte
+ * aligned.
  */
 int asrq_glu_dwconv(const void* in, const void* weight, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t T,
                     int64_t channels, int taps, int dtype, void* stream);
