@@ -158,10 +158,15 @@ def residual_norms(x: torch.Tensor, delta, scale: float, norm, norm2=None, write
     """``s = x + scale * delta``, ``h = layer_norm(s)`` -> ``(s, h)``; with a second norm ``y = layer_norm(s)``, ``h = layer_norm2(y)``
     -> ``(y, h)``.  ``norm`` / ``norm2``: (weight, bias).  ``write_h=False`` (two norms: not needed after the last) -> ``(y, None)``.
     Contiguous 16-bit tensors; the last dimension a multiple of 256 up to 2048."""
+    if _native is not None:
+        w2, b2 = (None, None) if norm2 is None else norm2
+        r = _native.residual_norms(x, delta, scale, norm[0], norm[1], w2, b2, write_h, eps)
+        if r is not None:
+            return r
     dt = _require_cuda_16bit(x, "residual_norms")
     dim = x.shape[-1]
     last = norm2 is None and not write_h  # the block's closing norm alone: its output is the residual stream
-    out = torch.empty_like(x) if delta is not None or norm2 is not None else None
+    out = torch.empty_like(x) if last or delta is not None or norm2 is not None else None
     h = None if last else torch.empty_like(x)
     ho, xo = (out, None) if last else (h, out)
     g2, b2 = (None, None) if norm2 is None else (norm2[0].data_ptr(), norm2[1].data_ptr())
