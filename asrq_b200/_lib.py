@@ -59,9 +59,6 @@ SIGNATURES = {
                                    c_int64, c_int, c_void_p]),
     "asrq_add_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, ctypes.c_float, c_void_p, c_void_p, c_int64, c_int64, c_int,
                                  c_void_p]),
-    "asrq_residual_norms": (c_int, [c_void_p, c_void_p, ctypes.c_float, c_void_p, c_void_p, ctypes.c_float, c_void_p, c_void_p, ctypes.c_float,
-                                    c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p]),
-    "asrq_glu_dwconv": (c_int, [c_void_p] * 6 + [c_int64, c_int64, c_int64, c_int, c_int, c_void_p]),
     "asrq_silu_mul": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p]),
     "asrq_qk_norm_rope": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                   c_int64, c_int64, c_int, c_int, c_int, c_int64, ctypes.c_float, c_int, c_void_p]),

@@ -17,13 +17,14 @@ and against this same model evaluated with the CPU oracle's layers.
 from __future__ import annotations
 
 import math
+import threading
 from typing import List, Optional
 
 import torch
 import torch.nn.functional as F
 
 from . import packing
-from .linear import LinearQQ, glu_dwconv, residual_norms
+from .linear import LinearQQ
 
 
 class FastConformerStandIn:
@@ -66,6 +67,7 @@ class FastConformerStandIn:
                 pw2=(rnd(d_model, d_model, 1), rnd(d_model)),
                 ln_ff2=ln(), ff2_a=qq(ffn, d_model), ff2_b=qq(d_model, ffn), ln_out=ln()))
         self.conv_kernel = conv_kernel
+        self._graph_lock, self._graphs, self._seen = threading.Lock(), {}, set()  # captured shapes, least recently used first
         self._shared: list = []  # (layer, buffer name, the rows of the joined buffer it was given)
         self._parts, self._pos_parts = [[L["q"], L["k"], L["v"]] for L in self.layers], [L["pos"] for L in self.layers]
         self._qkv, self._pos = [self._joined(p) for p in self._parts], self._joined(self._pos_parts)
@@ -131,41 +133,106 @@ class FastConformerStandIn:
         return F.layer_norm(x, (d,), *L["ln_out"])
 
     def _blocks(self, x: torch.Tensor, pe: torch.Tensor) -> torch.Tensor:
-        """All blocks with what lies between their layers in this library's kernels: the same steps and roundings as
-        :meth:`block`, channels last throughout, q/k/v as one layer over one quantised input, and the positional keys of all
-        blocks (whose input is the same) as one layer ahead of them."""
+        """All blocks, bit for bit :meth:`block` one after another (behind 4-bit activations a last-place difference moves a
+        code, and thirty-two blocks make a percent of it): q/k/v as one layer over one quantised input, the positional keys of
+        all blocks, whose input is the same, as one layer ahead of them, and a half-step residual in one pass."""
         b, t, d = x.shape
         hd = d // self.heads
         sp = lambda z: z.view(b, t, self.heads, hd).transpose(1, 2)  # noqa: E731
         pos = self._pos(pe)
-        x, h = residual_norms(x, None, 1.0, self.layers[0]["ln_ff1"])
         for i, L in enumerate(self.layers):
-            x, h = residual_norms(x, L["ff1_b"](F.silu(L["ff1_a"](h), inplace=True)), 0.5, L["ln_att"])
-            qkv = self._qkv[i](h)
+            h = F.layer_norm(x, (d,), *L["ln_ff1"])
+            x = torch.add(x, L["ff1_b"](F.silu(L["ff1_a"](h), inplace=True)), alpha=0.5)
+            qkv = self._qkv[i](F.layer_norm(x, (d,), *L["ln_att"]))
             k = qkv[..., d:2 * d] + pos[:, i * d:(i + 1) * d]
             a = F.scaled_dot_product_attention(sp(qkv[..., :d]), sp(k), sp(qkv[..., 2 * d:])).transpose(1, 2).reshape(b, t, d)
-            x, h = residual_norms(x, L["out"](a), 1.0, L["ln_conv"])
-            h = glu_dwconv(F.linear(h, L["pw1"][0].view(2 * d, d), L["pw1"][1]), *L["dw"], *L["bn"])
-            x, h = residual_norms(x, F.linear(h, L["pw2"][0].view(d, d), L["pw2"][1]), 1.0, L["ln_ff2"])
-            y = L["ff2_b"](F.silu(L["ff2_a"](h), inplace=True))
-            more = i + 1 < len(self.layers)
-            x, h = residual_norms(x, y, 0.5, L["ln_out"], self.layers[i + 1]["ln_ff1"] if more else None, write_h=more)
+            x = x + L["out"](a)
+            h = F.layer_norm(x, (d,), *L["ln_conv"]).transpose(1, 2)
+            h = F.glu(F.conv1d(h, *L["pw1"]), dim=1)
+            h = F.conv1d(h, *L["dw"], padding=self.conv_kernel // 2, groups=d)
+            h = F.silu(h * L["bn"][0].view(1, -1, 1) + L["bn"][1].view(1, -1, 1), inplace=True)
+            x = x + F.conv1d(h, *L["pw2"]).transpose(1, 2)
+            h = F.layer_norm(x, (d,), *L["ln_ff2"])
+            x = torch.add(x, L["ff2_b"](F.silu(L["ff2_a"](h), inplace=True)), alpha=0.5)
+            x = F.layer_norm(x, (d,), *L["ln_out"])
         return x
 
-    def _blocks_covered(self) -> bool:
+    def _joined_ok(self) -> bool:
         # the joined layers stand for their parts only while these hold the shared buffers and are the blocks' layers
-        return (self.d % 256 == 0 and self.d <= 2048 and self.conv_kernel == 9 and len(self.layers) == len(self._qkv) > 0 and
-                all(p._buffers.get(name) is t for p, name, t in self._shared) and
+        return (len(self.layers) == len(self._qkv) > 0 and all(p._buffers.get(name) is t for p, name, t in self._shared) and
                 all(L[name] is p for L, parts in zip(self.layers, self._parts) for name, p in zip("qkv", parts)) and
                 all(L["pos"] is p for L, p in zip(self.layers, self._pos_parts)))
+
+    # A few hundred rows keep the device busy for a third of the time that their launches take the host: such a shape is replayed
+    # as a CUDA graph from its second call on (one that comes once would pay for a capture that it never replays).
+    graph_rows = 4096   # (batch x time) rows up to which a shape is captured: 16 utterances of 20 s take the device as long as the host
+    graph_shapes = 4    # graphs kept, the least recently used given back first
+
+    def _operands(self):
+        """Everything a captured encode has baked in: a graph is replayed only while all of it is what it was."""
+        ops = [LinearQQ.operand, self.heads, self.conv_kernel, len(self.layers)]
+        for L in self.layers:
+            for v in L.values():
+                if isinstance(v, tuple):
+                    ops.extend(v)
+                else:
+                    bufs = v._buffers
+                    ops.extend((bufs.get("weight"), bufs.get("scales"), bufs.get("bias"), bufs["weight"]._version))
+        ops.extend(self.sub_out)
+        return ops
+
+    def _encode_graph(self, x: torch.Tensor):
+        """Subsampled frames through the blocks by a graph, or None where there is none (yet)."""
+        key = tuple(x.shape)
+        with self._graph_lock:
+            ops = self._operands()
+            hit = self._graphs.pop(key, None)
+            if hit is not None and not (len(hit["ops"]) == len(ops) and all(a is b or (type(a) in (int, str) and a == b) for a, b in zip(hit["ops"], ops))):
+                hit = None
+            if hit is None:  # seen once: the next call of this shape captures
+                if len(self._seen) > 64:
+                    self._seen.clear()
+                if key not in self._seen:
+                    self._seen.add(key)
+                    return None
+                hit = self._capture(x, ops)
+                while len(self._graphs) >= self.graph_shapes:
+                    self._graphs.pop(next(iter(self._graphs)))["done"].synchronize()  # not while it runs
+            self._graphs[key] = hit  # most recently used last
+            stream = torch.cuda.current_stream(self.device)
+            stream.wait_event(hit["done"])  # another stream may still be in this graph's buffers
+            hit["x"].copy_(x)
+            hit["graph"].replay()
+            out = hit["out"].clone()
+            hit["done"].record(stream)
+            return out
+
+    def _capture(self, x: torch.Tensor, ops) -> dict:
+        xs = x.clone()
+        cur, side = torch.cuda.current_stream(self.device), torch.cuda.Stream(self.device)
+        side.wait_stream(cur)
+        with torch.cuda.stream(side):
+            self._blocks(xs, self._pos_emb(x.shape[1]))  # prepared weights and workspaces exist before the capture
+            pe = self._pos_emb(x.shape[1])
+        side.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side, capture_error_mode="thread_local"):
+            out = self._blocks(xs, pe)
+        done = torch.cuda.Event()
+        done.record(cur)
+        return {"graph": g, "x": xs, "pe": pe, "out": out, "ops": ops, "done": done}
 
     @torch.no_grad()
     def encode(self, feats: torch.Tensor, hook=None) -> torch.Tensor:
         with torch.cuda.device(self.device):
             x = self.subsample(feats)
+            if hook is None and x.numel() and self._joined_ok():
+                if x.shape[0] * x.shape[1] <= self.graph_rows and not torch.cuda.is_current_stream_capturing():
+                    y = self._encode_graph(x)
+                    if y is not None:
+                        return y
+                return self._blocks(x, self._pos_emb(x.shape[1]))
             pe = self._pos_emb(x.shape[1])
-            if hook is None and x.numel() and self._blocks_covered():
-                return self._blocks(x.contiguous(), pe)
             for L in self.layers:
                 x = self.block(L, x, pe, hook)
             return x

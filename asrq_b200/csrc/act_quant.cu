@@ -209,10 +209,12 @@ quant_int4_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, floa
 
 // K = 1024 and 4096: 32 and 64 threads per token, each with 32 and 64 values, and ONE transpose through shared memory where the
 // kernel above has five levels of shuffles:
-//   phase A  thread t holds the pairs (e, e + 1), e = i * 2T + 2t, i = 0..NI-1, as it loads them (a warp 128 contiguous bytes per
-//            i): strides 1 and 2T .. K/2 are private;
-//   phase B  thread u = 2i + c holds the elements i * 2T + 2j + c, j = 0..T-1: strides 2 .. T.  The two threads of an i hold every
-//            other element; they swap halves of their packed codes so that each stores T consecutive ones.
+//   phase A  thread t holds the T consecutive elements t * T + e (staged through shared memory, so that the loads are whole
+//            lines): strides 1 .. T / 2;
+//   phase B  thread u holds the elements o * T + u, o = 0..T-1: strides T .. K / 2.  Four neighbouring threads transpose their
+//            4 x 4 bytes of codes by two shuffles per word, so that a warp stores whole 32-byte sectors.
+// The strides are taken in ascending order, as everywhere in this file: another order rounds differently, and behind four bits a
+// difference in the last place can move a code.
 // Values live as pairs, so every butterfly but the one inside the pair is a packed fp32 add and a packed subtract (add.f32x2 /
 // fma.f32x2) on two pairs.  Rows of the transpose are padded by four floats: its 4-byte writes and 16-byte reads are free of bank
 // conflicts.
@@ -283,9 +285,9 @@ constexpr int kHadTokens = T == 64 ? 1 : 4;  // per block
 template <int K, int T, int OUT, bool BF16>
 __global__ void __launch_bounds__(T * kHadTokens<K, T>, T == 64 ? 8 : 5)
 hadamard_transpose_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {
-  constexpr int NI = K / (2 * T), PITCH = T + 4, TOKENS = kHadTokens<K, T>;
-  static_assert(2 * NI == T, "one row of the transpose per thread");
-  __shared__ __align__(16) float rows_all[TOKENS][T * PITCH];
+  constexpr int PITCH = T + 4, TOKENS = kHadTokens<K, T>, UNITS = T / 8;  // 16-byte units per thread
+  static_assert(K == T * T, "one row of the transpose per thread");
+  __shared__ __align__(16) float rows_all[TOKENS][T * PITCH];  // the 16-bit input is staged in its first half
   __shared__ float part[2];
   // A GEMM launched behind this kernel with programmatic stream serialisation may be scheduled once
   // every block of this grid has started, and set itself up on SMs the last wave leaves idle; it
@@ -302,19 +304,30 @@ hadamard_transpose_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restr
       __syncwarp();
     }
   };
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(x + size_t(token) * K) + t;
-  uint32_t raw[NI];
+  const uint4* src = reinterpret_cast<const uint4*>(x + size_t(token) * K) + t;
+  uint4* stage = reinterpret_cast<uint4*>(rows);
+  auto slot = [](int owner, int j) { return owner * UNITS + (T == 64 ? (j ^ (owner & 7)) : (j ^ ((owner >> 1) & 3))); };  // conflict-free both ways
+  uint4 raw[UNITS];
 #pragma unroll
-  for (int i = 0; i < NI; ++i) raw[i] = __ldg(src + i * T);
+  for (int i = 0; i < UNITS; ++i) raw[i] = __ldg(src + i * T);
+#pragma unroll
+  for (int i = 0; i < UNITS; ++i) stage[slot((i * T + t) / UNITS, (i * T + t) % UNITS)] = raw[i];
+  meet();
   {
-    float2 P[NI];
+    float2 P[T / 2];
 #pragma unroll
-    for (int i = 0; i < NI; ++i)
-      P[i] = BF16 ? make_float2(__uint_as_float(raw[i] << 16), __uint_as_float(raw[i] & 0xffff0000u)) : __half22float2(u32_as_h2(raw[i]));
+    for (int i = 0; i < UNITS; ++i) {
+      const uint4 q = stage[slot(t, i)];
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        P[4 * i + e] = BF16 ? make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u)) : __half22float2(u32_as_h2(w[e]));
+    }
     inside_pairs(P);
     butterflies(P);
+    meet();  // the staged rows have been read
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
+    for (int i = 0; i < T / 2; ++i) {
       rows[(2 * i) * PITCH + t] = P[i].x;
       rows[(2 * i + 1) * PITCH + t] = P[i].y;
     }
@@ -347,36 +360,20 @@ hadamard_transpose_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restr
   const float inv = __fdiv_rn(1.f, s);
   const float il = inv * (1.f - 2.384185791015625e-07f), ih = inv * (1.f + 2.384185791015625e-07f);  // 2^-22
   const float2 inv_lo = make_float2(il, il), inv_hi = make_float2(ih, ih);
-  uint32_t W[T / 4];  // the codes of elements 2j + c, four j per word
+  const uint32_t sel1 = (t & 2) ? 0x3276u : 0x5410u, sel2 = (t & 1) ? 0x3715u : 0x6240u;
+  const size_t first = size_t(t & 3) * T + (t & ~3);  // this thread's four elements of o = 4 k + (t & 3)
 #pragma unroll
-  for (int k = 0; k < T / 4; ++k) W[k] = quant4_bytes<OUT>(Q[2 * k], Q[2 * k + 1], inv_lo, inv_hi, s);
-  const bool odd = t & 1;
-  uint32_t o[T / 4];  // T consecutive codes: the first or second half of this i
-#pragma unroll
-  for (int k = 0; k < T / 8; ++k) {
-    const uint32_t give = odd ? W[k] : W[k + T / 8], keep = odd ? W[k + T / 8] : W[k];
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, give, 1);
-    const uint32_t ev = odd ? got : keep, od = odd ? keep : got;
-    o[2 * k] = prmt(ev, od, 0x5140u);
-    o[2 * k + 1] = prmt(ev, od, 0x7362u);
-  }
-  if (OUT >= 1) {
-    uint4* d = reinterpret_cast<uint4*>(qa + size_t(token) * K + t * T);
-#pragma unroll
-    for (int k = 0; k < T / 4; ++k)
-      if (OUT == 1) o[k] = (o[k] << 4) & 0xf0f0f0f0u;
-#pragma unroll
-    for (int k = 0; k < T / 16; ++k) d[k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-  } else {
-    uint32_t n[T / 8];  // four nibbles in four bytes -> 16 bits, element 0 lowest; two words -> one
-#pragma unroll
-    for (int k = 0; k < T / 8; ++k) {
-      const uint32_t a = o[2 * k] & 0x0f0f0f0fu, b = o[2 * k + 1] & 0x0f0f0f0fu;
-      n[k] = prmt(a | (a >> 4), b | (b >> 4), 0x6420u);
+  for (int k = 0; k < T / 4; ++k) {
+    uint32_t w = quant4_bytes<OUT>(Q[2 * k], Q[2 * k + 1], inv_lo, inv_hi, s);  // element u of o = 4 k .. 4 k + 3
+    w = prmt(w, __shfl_xor_sync(0xffffffffu, w, 2), sel1);
+    w = prmt(w, __shfl_xor_sync(0xffffffffu, w, 1), sel2);  // elements u & ~3 .. of o = 4 k + (t & 3)
+    const size_t at = first + size_t(4 * k) * T;
+    if (OUT >= 1) {
+      *reinterpret_cast<uint32_t*>(qa + size_t(token) * K + at) = OUT == 1 ? (w << 4) & 0xf0f0f0f0u : w;
+    } else {
+      const uint32_t n = w & 0x0f0f0f0fu, m = n | (n >> 4);  // bytes 0 and 2 hold two nibbles each, element 0 lowest
+      *reinterpret_cast<uint16_t*>(qa + size_t(token) * (K / 2) + at / 2) = uint16_t((m & 0xffu) | ((m >> 8) & 0xff00u));
     }
-    uint4* d = reinterpret_cast<uint4*>(qa + size_t(token) * (K / 2) + t * (T / 2));
-#pragma unroll
-    for (int k = 0; k < T / 32; ++k) d[k] = make_uint4(n[4 * k], n[4 * k + 1], n[4 * k + 2], n[4 * k + 3]);
   }
 }
 

@@ -41,10 +41,6 @@ int decode_cross_attention(const void* q, const void* k, const void* v, void* ou
 int decode_grouped_attention(const void* qkv, const void* qw, const void* kw, const void* cos_t, const void* sin_t, const long long* pos_dev,
                              void* k_cache, void* v_cache, void* out, int64_t B, int nkv, int64_t max_len, float eps, float scale, int dtype,
                              int sm_count, cudaStream_t stream);
-int residual_norms(const void* x, const void* delta, float scale, const void* g1, const void* b1, float eps1, const void* g2, const void* b2, float eps2,
-                   void* x_out, void* h_out, int64_t rows, int64_t dim, int dtype, cudaStream_t stream);
-int glu_dwconv(const void* in, const void* w, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t T, int64_t d,
-               int dtype, cudaStream_t stream);
 int dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, int dtype, int sm_count, cudaStream_t stream);
 int hadamard_quant_int4(const void* x, uint8_t* qa, float* sa, int64_t M, int64_t K, int hadamard, int dtype,
                         int out_int8, cudaStream_t stream);
@@ -436,39 +432,6 @@ int asrq_add_rmsnorm(const void* x, const void* delta, const void* gamma, float 
   if ((rc = device_facts(&f))) return rc;
   if (rows == 0) return ASRQ_OK;
   return add_rmsnorm(x, delta, gamma, eps, x_out, h_out, rows, dim, dtype, static_cast<cudaStream_t>(stream));
-}
-
-int asrq_residual_norms(const void* x, const void* delta, float scale, const void* gamma, const void* beta, float eps, const void* gamma2,
-                        const void* beta2, float eps2, void* x_out, void* h_out, int64_t rows, int64_t dim, int dtype, void* stream) {
-  last_error().clear();
-  if (!x || !gamma || !beta || (!x_out && !h_out) || (!gamma2 != !beta2) || (gamma2 && !h_out))
-    return fail(ASRQ_ERR_NULL, "asrq_residual_norms: x, gamma, beta and an output must not be NULL; gamma2 and beta2 go together");
-  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_residual_norms: dtype %d", dtype);
-  if (rows < 0 || rows > (int64_t(1) << 31) - 64 || dim <= 0 || dim % 256 || dim > 2048)
-    return fail(ASRQ_ERR_SHAPE, "asrq_residual_norms: rows=%lld dim=%lld (a multiple of 256 up to 2048)", (long long)rows, (long long)dim);
-  for (const void* q : {x, delta, gamma, beta, gamma2, beta2, static_cast<const void*>(x_out), static_cast<const void*>(h_out)})
-    if (q && !aligned16(q)) return fail(ASRQ_ERR_ALIGN, "asrq_residual_norms: pointers must be 16-byte aligned");
-  const DeviceFacts* f;
-  int rc;
-  if ((rc = device_facts(&f))) return rc;
-  if (rows == 0) return ASRQ_OK;
-  return residual_norms(x, delta, scale, gamma, beta, eps, gamma2, beta2, eps2, x_out, h_out, rows, dim, dtype, static_cast<cudaStream_t>(stream));
-}
-
-int asrq_glu_dwconv(const void* in, const void* weight, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t T,
-                    int64_t channels, int taps, int dtype, void* stream) {
-  last_error().clear();
-  if (!in || !weight || !bias || !scale || !shift || !out) return fail(ASRQ_ERR_NULL, "asrq_glu_dwconv: no pointer may be NULL");
-  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_glu_dwconv: dtype %d", dtype);
-  if (B < 0 || B > 65535 || T < 0 || T > (1 << 20) - 16 || channels <= 0 || channels % 2 || channels > (1 << 20) || taps != 9)
-    return fail(ASRQ_ERR_SHAPE, "asrq_glu_dwconv: B=%lld T=%lld channels=%lld (even) taps=%d (9)", (long long)B, (long long)T, (long long)channels, taps);
-  for (const void* q : {in, weight, bias, scale, shift, static_cast<const void*>(out)})
-    if (reinterpret_cast<uintptr_t>(q) % 4) return fail(ASRQ_ERR_ALIGN, "asrq_glu_dwconv: pointers must be 4-byte aligned");
-  const DeviceFacts* f;
-  int rc;
-  if ((rc = device_facts(&f))) return rc;
-  if (B == 0 || T == 0) return ASRQ_OK;
-  return glu_dwconv(in, weight, bias, scale, shift, out, B, T, channels, dtype, static_cast<cudaStream_t>(stream));
 }
 
 int asrq_silu_mul(const void* gate_up, void* out, int64_t rows, int64_t inter, int dtype, void* stream) {

@@ -235,56 +235,6 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   END_HANDLE_TH_ERRORS
 }
 
-// residual_norms(x, delta or None, scale, weight, bias, weight2 or None, bias2 or None, write_h, eps) -> (stream, normed or None), or None
-PyObject* residual_norms(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
-  HANDLE_TH_ERRORS
-  if (n_args != 9) {
-    PyErr_SetString(PyExc_TypeError, "residual_norms: nine arguments");
-    return nullptr;
-  }
-  const at::Tensor* x;
-  int dtype;
-  if (!activations(a[0], &x, &dtype)) Py_RETURN_NONE;
-  const at::Tensor* t[5] = {};  // delta, weight, bias, weight2, bias2
-  PyObject* const given[5] = {a[1], a[3], a[4], a[5], a[6]};
-  for (int i = 0; i < 5; ++i) {
-    if (given[i] == Py_None) continue;
-    t[i] = plain(given[i]);
-    if (!t[i] || t[i]->scalar_type() != x->scalar_type() || t[i]->device() != x->device() || !t[i]->is_contiguous() ||
-        t[i]->numel() != (i ? x->size(-1) : x->numel()))
-      Py_RETURN_NONE;
-  }
-  const double scale = PyFloat_AsDouble(a[2]), eps = PyFloat_AsDouble(a[8]);
-  if (PyErr_Occurred()) return nullptr;
-  if (!t[1] || !t[2] || !t[3] != !t[4]) Py_RETURN_NONE;
-  const bool last = !t[3] && a[7] != Py_True;  // the only norm's output is the residual stream
-  at::Tensor out, h;
-  if (last || t[0] || t[3]) out = output_like(*x, x->size(-1));
-  if (!last) h = output_like(*x, x->size(-1));
-  auto ptr = [](const at::Tensor* v) { return v ? v->data_ptr() : nullptr; };
-  void *xo = out.defined() && !last ? out.data_ptr() : nullptr, *ho = last ? out.data_ptr() : h.data_ptr();
-  g_calls.fetch_add(1, std::memory_order_relaxed);
-  const int rc = asrq_residual_norms(x->data_ptr(), ptr(t[0]), float(scale), ptr(t[1]), ptr(t[2]), float(eps), ptr(t[3]), ptr(t[4]), float(eps), xo, ho,
-                                     x->numel() / x->size(-1), x->size(-1), dtype, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
-  if (rc) return failed("asrq_residual_norms", rc);
-  PyObject* r = PyTuple_New(2);
-  if (!r) return nullptr;
-  if (out.defined()) {
-    PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(out)));
-  } else {
-    Py_INCREF(a[0]);
-    PyTuple_SET_ITEM(r, 0, a[0]);
-  }
-  if (h.defined()) {
-    PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(std::move(h)));
-  } else {
-    Py_INCREF(Py_None);
-    PyTuple_SET_ITEM(r, 1, Py_None);
-  }
-  return r;
-  END_HANDLE_TH_ERRORS
-}
-
 PyObject* calls(PyObject*, PyObject*) { return PyLong_FromLongLong(g_calls.load(std::memory_order_relaxed)); }
 
 // bind(workspaces dict, check function)
@@ -303,7 +253,6 @@ PyObject* bind(PyObject*, PyObject* args) {
 PyMethodDef kMethods[] = {
     {"linearq_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linearq_forward)), METH_FASTCALL, nullptr},
     {"linearqq_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linearqq_forward)), METH_FASTCALL, nullptr},
-    {"residual_norms", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(residual_norms)), METH_FASTCALL, nullptr},
     {"calls", calls, METH_NOARGS, nullptr},
     {"bind", bind, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},

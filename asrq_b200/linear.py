@@ -154,41 +154,6 @@ def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.
     return out
 
 
-def residual_norms(x: torch.Tensor, delta, scale: float, norm, norm2=None, write_h: bool = True, eps: float = 1e-5):
-    """``s = x + scale * delta``, ``h = layer_norm(s)`` -> ``(s, h)``; with a second norm ``y = layer_norm(s)``, ``h = layer_norm2(y)``
-    -> ``(y, h)``.  ``norm`` / ``norm2``: (weight, bias).  ``write_h=False`` (two norms: not needed after the last) -> ``(y, None)``.
-    Contiguous 16-bit tensors; the last dimension a multiple of 256 up to 2048."""
-    if _native is not None:
-        w2, b2 = (None, None) if norm2 is None else norm2
-        r = _native.residual_norms(x, delta, scale, norm[0], norm[1], w2, b2, write_h, eps)
-        if r is not None:
-            return r
-    dt = _require_cuda_16bit(x, "residual_norms")
-    dim = x.shape[-1]
-    last = norm2 is None and not write_h  # the block's closing norm alone: its output is the residual stream
-    out = torch.empty_like(x) if last or delta is not None or norm2 is not None else None
-    h = None if last else torch.empty_like(x)
-    ho, xo = (out, None) if last else (h, out)
-    g2, b2 = (None, None) if norm2 is None else (norm2[0].data_ptr(), norm2[1].data_ptr())
-    with _on_device(x.device):
-        _lib.call("asrq_residual_norms", x.data_ptr(), None if delta is None else delta.data_ptr(), float(scale), norm[0].data_ptr(), norm[1].data_ptr(),
-                  float(eps), g2, b2, float(eps), None if xo is None else xo.data_ptr(), ho.data_ptr(), x.numel() // dim, dim, dt,
-                  torch.cuda.current_stream(x.device).cuda_stream)
-    return (x if out is None else out), h
-
-
-def glu_dwconv(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor) -> torch.Tensor:
-    """``silu(depthwise_conv(x[..., :C] * sigmoid(x[..., C:])) * scale + shift)`` over time, channels last: x (B, T, 2 C),
-    weight (C, 1, 9), the rest (C,).  Returns (B, T, C)."""
-    dt = _require_cuda_16bit(x, "glu_dwconv")
-    B, T, c2 = x.shape
-    out = torch.empty((B, T, c2 // 2), dtype=x.dtype, device=x.device)
-    with _on_device(x.device):
-        _lib.call("asrq_glu_dwconv", x.data_ptr(), weight.data_ptr(), bias.data_ptr(), scale.data_ptr(), shift.data_ptr(), out.data_ptr(), B, T,
-                  c2 // 2, weight.shape[-1], dt, torch.cuda.current_stream(x.device).cuda_stream)
-    return out
-
-
 def decode_cross_attention(q: torch.Tensor, kv: torch.Tensor, heads: int, scale: float = 1.0, settled: bool = False) -> torch.Tensor:
     """Cross-attention of one decoding step: ``q`` (B, d), ``kv`` (B, T, 2 d) with keys and values side by side (a fused
     projection's output).  Returns (B, d).  ``settled``: ``kv`` is older than the kernels just ahead on the stream (a step's cross

@@ -176,25 +176,6 @@ int asrq_add_rmsnorm(const void* x, const void* delta, const void* gamma, float 
                      int64_t rows, int64_t dim, int dtype, void* stream);
 
 /*
- * s = x + scale * delta (delta may be NULL), y = LayerNorm(s) * gamma + beta; with gamma2 and beta2 also z = LayerNorm(y) * gamma2 +
- * beta2.  x_out (optional) is the residual stream that goes on: s, or y when there is a second norm; h_out the last norm's output
- * (optional without a second norm).  scale * delta and every sum and norm are rounded to `dtype`, as the sequence of modules
- * rounds them: the half-step residuals and the end of a Conformer block (asrq/models/nemo/conformerq.py replaces the linear
- * layers of that block only).  rows x dim, dim a multiple of 256 up to 2048; 16-byte aligned; x_out may alias x.
- */
-int asrq_residual_norms(const void* x, const void* delta, float scale, const void* gamma, const void* beta, float eps, const void* gamma2,
-                        const void* beta2, float eps2, void* x_out, void* h_out, int64_t rows, int64_t dim, int dtype, void* stream);
-
-/*
- * A Conformer block's convolution module between its pointwise projections, channels last: u = in[.., :C] * sigmoid(in[.., C:]),
- * depthwise convolution of `taps` (9) over time with zero padding and bias, * scale + shift per channel, SiLU; rounded to `dtype`
- * after each of these.  in: B x T x 2 C; weight: C x taps; out: B x T x C; C even; 4-byte
- * aligned.
- */
-int asrq_glu_dwconv(const void* in, const void* weight, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t T,
-                    int64_t channels, int taps, int dtype, void* stream);
-
-/*
  * out[m, i] = silu(gate_up[m, i]) * gate_up[m, inter + i]: the gated activation between a fused gate/up
  * projection (one LinearQ call over 2*inter output features) and the down projection
  * (act_fn(gate_proj(x)) * up_proj(x) of Qwen3MLPQ, asrq/models/nemo/canary_qwen.py:70-86).  silu is rounded to
