@@ -59,6 +59,10 @@ SIGNATURES = {
                                    c_int64, c_int, c_void_p]),
     "asrq_add_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, ctypes.c_float, c_void_p, c_void_p, c_int64, c_int64, c_int,
                                  c_void_p]),
+    "asrq_bias_glu": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "asrq_bias_affine_silu": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "asrq_half_step": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p]),
+    "asrq_bias_add_transposed": (c_int, [c_void_p] * 4 + [c_int64, c_int64, c_int64, c_int, c_void_p]),
     "asrq_silu_mul": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p]),
     "asrq_qk_norm_rope": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                   c_int64, c_int64, c_int, c_int, c_int, c_int64, ctypes.c_float, c_int, c_void_p]),

@@ -24,7 +24,7 @@ import torch
 import torch.nn.functional as F
 
 from . import packing
-from .linear import LinearQQ
+from .linear import LinearQQ, bias_add_transposed, bias_affine_silu, bias_glu, half_step
 
 
 class FastConformerStandIn:
@@ -135,31 +135,31 @@ class FastConformerStandIn:
     def _blocks(self, x: torch.Tensor, pe: torch.Tensor) -> torch.Tensor:
         """All blocks, bit for bit :meth:`block` one after another (behind 4-bit activations a last-place difference moves a
         code, and thirty-two blocks make a percent of it): q/k/v as one layer over one quantised input, the positional keys of
-        all blocks, whose input is the same, as one layer ahead of them, and a half-step residual in one pass."""
+        all blocks, whose input is the same, as one layer ahead of them, a half-step residual in one pass, and the elementwise steps
+        around each convolution in one (its bias, which the library adds in a pass of its own, among them)."""
         b, t, d = x.shape
         hd = d // self.heads
         sp = lambda z: z.view(b, t, self.heads, hd).transpose(1, 2)  # noqa: E731
         pos = self._pos(pe)
         for i, L in enumerate(self.layers):
             h = F.layer_norm(x, (d,), *L["ln_ff1"])
-            x = torch.add(x, L["ff1_b"](F.silu(L["ff1_a"](h), inplace=True)), alpha=0.5)
+            x = half_step(x, L["ff1_b"](F.silu(L["ff1_a"](h), inplace=True)))
             qkv = self._qkv[i](F.layer_norm(x, (d,), *L["ln_att"]))
             k = qkv[..., d:2 * d] + pos[:, i * d:(i + 1) * d]
             a = F.scaled_dot_product_attention(sp(qkv[..., :d]), sp(k), sp(qkv[..., 2 * d:])).transpose(1, 2).reshape(b, t, d)
             x = x + L["out"](a)
             h = F.layer_norm(x, (d,), *L["ln_conv"]).transpose(1, 2)
-            h = F.glu(F.conv1d(h, *L["pw1"]), dim=1)
-            h = F.conv1d(h, *L["dw"], padding=self.conv_kernel // 2, groups=d)
-            h = F.silu(h * L["bn"][0].view(1, -1, 1) + L["bn"][1].view(1, -1, 1), inplace=True)
-            x = x + F.conv1d(h, *L["pw2"]).transpose(1, 2)
+            h = bias_glu(F.conv1d(h, L["pw1"][0]), L["pw1"][1])
+            h = bias_affine_silu(F.conv1d(h, L["dw"][0], padding=self.conv_kernel // 2, groups=d), L["dw"][1], *L["bn"])
+            x = bias_add_transposed(x, F.conv1d(h, L["pw2"][0]), L["pw2"][1])
             h = F.layer_norm(x, (d,), *L["ln_ff2"])
-            x = torch.add(x, L["ff2_b"](F.silu(L["ff2_a"](h), inplace=True)), alpha=0.5)
+            x = half_step(x, L["ff2_b"](F.silu(L["ff2_a"](h), inplace=True)))
             x = F.layer_norm(x, (d,), *L["ln_out"])
         return x
 
     def _joined_ok(self) -> bool:
         # the joined layers stand for their parts only while these hold the shared buffers and are the blocks' layers
-        return (len(self.layers) == len(self._qkv) > 0 and all(p._buffers.get(name) is t for p, name, t in self._shared) and
+        return (len(self.layers) == len(self._qkv) > 0 and self.d % 8 == 0 and all(p._buffers.get(name) is t for p, name, t in self._shared) and
                 all(L[name] is p for L, parts in zip(self.layers, self._parts) for name, p in zip("qkv", parts)) and
                 all(L["pos"] is p for L, p in zip(self.layers, self._pos_parts)))
 

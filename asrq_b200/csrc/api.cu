@@ -41,6 +41,10 @@ int decode_cross_attention(const void* q, const void* k, const void* v, void* ou
 int decode_grouped_attention(const void* qkv, const void* qw, const void* kw, const void* cos_t, const void* sin_t, const long long* pos_dev,
                              void* k_cache, void* v_cache, void* out, int64_t B, int nkv, int64_t max_len, float eps, float scale, int dtype,
                              int sm_count, cudaStream_t stream);
+int conv_elementwise(const void* in, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t C, int64_t T, int dtype,
+                     cudaStream_t stream);
+int bias_add_transposed(const void* x, const void* conv, const void* bias, void* out, int64_t B, int64_t T, int64_t C, int dtype, cudaStream_t stream);
+int half_step(const void* x, const void* y, void* out, int64_t n, int dtype, cudaStream_t stream);
 int dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, int dtype, int sm_count, cudaStream_t stream);
 int hadamard_quant_int4(const void* x, uint8_t* qa, float* sa, int64_t M, int64_t K, int hadamard, int dtype,
                         int out_int8, cudaStream_t stream);
@@ -432,6 +436,50 @@ int asrq_add_rmsnorm(const void* x, const void* delta, const void* gamma, float 
   if ((rc = device_facts(&f))) return rc;
   if (rows == 0) return ASRQ_OK;
   return add_rmsnorm(x, delta, gamma, eps, x_out, h_out, rows, dim, dtype, static_cast<cudaStream_t>(stream));
+}
+
+static int check_conv(const char* who, const void* a, const void* b, const void* c, int64_t B, int64_t C, int64_t T, int dtype) {
+  last_error().clear();
+  if (!a || !b || !c) return fail(ASRQ_ERR_NULL, "%s: NULL pointer", who);
+  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "%s: dtype %d", who, dtype);
+  if (B < 0 || B > 65535 || C <= 0 || T < 0 || C > (1 << 20) || T > (1 << 24) || C * T > (int64_t(1) << 30))
+    return fail(ASRQ_ERR_SHAPE, "%s: B=%lld C=%lld T=%lld", who, (long long)B, (long long)C, (long long)T);
+  const DeviceFacts* f;
+  return device_facts(&f);
+}
+
+int asrq_bias_glu(const void* in, const void* bias, void* out, int64_t B, int64_t C, int64_t T, int dtype, void* stream) {
+  const int rc = check_conv("asrq_bias_glu", in, bias, out, B, C, T, dtype);
+  if (rc || B == 0 || T == 0) return rc;
+  return conv_elementwise(in, bias, nullptr, nullptr, out, B, C, T, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_bias_affine_silu(const void* in, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t C, int64_t T,
+                          int dtype, void* stream) {
+  const int rc = check_conv("asrq_bias_affine_silu", in, bias, out, B, C, T, dtype);
+  if (rc) return rc;
+  if (!scale || !shift) return fail(ASRQ_ERR_NULL, "asrq_bias_affine_silu: NULL pointer");
+  if (B == 0 || T == 0) return ASRQ_OK;
+  return conv_elementwise(in, bias, scale, shift, out, B, C, T, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_half_step(const void* x, const void* y, void* out, int64_t n, int dtype, void* stream) {
+  const int rc = check_conv("asrq_half_step", x, y, out, 0, 1, 0, dtype);
+  if (rc) return rc;
+  if (n < 0 || n % 8 || n > (int64_t(1) << 38)) return fail(ASRQ_ERR_SHAPE, "asrq_half_step: n=%lld (a multiple of 8)", (long long)n);
+  if (!aligned16(x) || !aligned16(y) || !aligned16(out)) return fail(ASRQ_ERR_ALIGN, "asrq_half_step: pointers must be 16-byte aligned");
+  if (n == 0) return ASRQ_OK;
+  return half_step(x, y, out, n, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_bias_add_transposed(const void* x, const void* conv, const void* bias, void* out, int64_t B, int64_t T, int64_t C, int dtype, void* stream) {
+  const int rc = check_conv("asrq_bias_add_transposed", x, conv, out, B, C, T, dtype);
+  if (rc) return rc;
+  if (!bias) return fail(ASRQ_ERR_NULL, "asrq_bias_add_transposed: NULL pointer");
+  if (C % 2 || reinterpret_cast<uintptr_t>(x) % 4 || reinterpret_cast<uintptr_t>(bias) % 4 || reinterpret_cast<uintptr_t>(out) % 4)
+    return fail(ASRQ_ERR_ALIGN, "asrq_bias_add_transposed: C must be even, x, bias and out 4-byte aligned");
+  if (B == 0 || T == 0) return ASRQ_OK;
+  return bias_add_transposed(x, conv, bias, out, B, T, C, dtype, static_cast<cudaStream_t>(stream));
 }
 
 int asrq_silu_mul(const void* gate_up, void* out, int64_t rows, int64_t inter, int dtype, void* stream) {

@@ -135,8 +135,13 @@ __global__ void __launch_bounds__(32 * kLnWarps)
 add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ delta, const uint16_t* __restrict__ gamma,
                    float eps, uint16_t* __restrict__ x_out, uint16_t* __restrict__ h_out, int rows, int dim) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31;
+  uint4 gpre[VEC > 0 ? VEC : 1];  // the weight is a constant: fetched ahead of the stream dependency
+  if constexpr (VEC > 0) {
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) gpre[i] = __ldg(reinterpret_cast<const uint4*>(gamma + (i * 32 + lane) * 8));
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int row = blockIdx.x * kLnWarps + (threadIdx.x >> 5);
   if (row >= rows) return;
   const size_t off = size_t(row) * dim;
@@ -178,7 +183,7 @@ add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int e = (i * 32 + lane) * 8;
-      const uint4 g = __ldg(reinterpret_cast<const uint4*>(gamma + e));
+      const uint4 g = gpre[i];
       const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
       uint32_t ow[4];
 #pragma unroll

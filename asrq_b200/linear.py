@@ -154,6 +154,34 @@ def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.
     return out
 
 
+def _conv_step(fn: str, tensors, out: torch.Tensor, sizes) -> torch.Tensor:
+    dt = _require_cuda_16bit(tensors[0], fn)
+    with _on_device(out.device):
+        _lib.call(fn, *(t.data_ptr() for t in tensors), out.data_ptr(), *sizes, dt, torch.cuda.current_stream(out.device).cuda_stream)
+    return out
+
+
+def bias_glu(x: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+    """``glu(x + bias)`` over the channels of a contiguous (B, 2C, T) convolution output, in one pass."""
+    B, c2, T = x.shape
+    return _conv_step("asrq_bias_glu", (x, bias), x.new_empty(B, c2 // 2, T), (B, c2 // 2, T))
+
+
+def bias_affine_silu(x: torch.Tensor, bias: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor) -> torch.Tensor:
+    """``silu((x + bias) * scale + shift)`` per channel of a contiguous (B, C, T) convolution output, in one pass."""
+    return _conv_step("asrq_bias_affine_silu", (x, bias, scale, shift), torch.empty_like(x), x.shape)
+
+
+def half_step(x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+    """``x + 0.5 * y``, contiguous tensors of a multiple of 8 values, in one pass."""
+    return _conv_step("asrq_half_step", (x, y), torch.empty_like(x), (x.numel(),))
+
+
+def bias_add_transposed(x: torch.Tensor, conv: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+    """``x + (conv + bias).transpose(1, 2)``: x (B, T, C), conv (B, C, T), both contiguous, in one pass."""
+    return _conv_step("asrq_bias_add_transposed", (x, conv, bias), torch.empty_like(x), x.shape)
+
+
 def decode_cross_attention(q: torch.Tensor, kv: torch.Tensor, heads: int, scale: float = 1.0, settled: bool = False) -> torch.Tensor:
     """Cross-attention of one decoding step: ``q`` (B, d), ``kv`` (B, T, 2 d) with keys and values side by side (a fused
     projection's output).  Returns (B, d).  ``settled``: ``kv`` is older than the kernels just ahead on the stream (a step's cross

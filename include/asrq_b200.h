@@ -176,6 +176,20 @@ int asrq_add_rmsnorm(const void* x, const void* delta, const void* gamma, float 
                      int64_t rows, int64_t dim, int dtype, void* stream);
 
 /*
+ * The elementwise steps of a Conformer block's convolution module around its convolutions, contiguous tensors of `dtype`, every
+ * step rounded to it as the sequence of modules rounds:
+ *   asrq_bias_glu             in B x 2C x T -> out B x C x T: u = in + bias (2C), u[:, :C] * sigmoid(u[:, C:]);
+ *   asrq_bias_affine_silu     in, out B x C x T: silu((in + bias) * scale + shift), all of C values;
+ *   asrq_half_step            out = x + 0.5 * y, n values, a multiple of 8, 16-byte aligned;
+ *   asrq_bias_add_transposed  out = x + (conv + bias)^T: x, out B x T x C, conv B x C x T; C even, x, bias, out 4-byte aligned.
+ */
+int asrq_bias_glu(const void* in, const void* bias, void* out, int64_t B, int64_t C, int64_t T, int dtype, void* stream);
+int asrq_bias_affine_silu(const void* in, const void* bias, const void* scale, const void* shift, void* out, int64_t B, int64_t C, int64_t T,
+                          int dtype, void* stream);
+int asrq_half_step(const void* x, const void* y, void* out, int64_t n, int dtype, void* stream);
+int asrq_bias_add_transposed(const void* x, const void* conv, const void* bias, void* out, int64_t B, int64_t T, int64_t C, int dtype, void* stream);
+
+/*
  * out[m, i] = silu(gate_up[m, i]) * gate_up[m, inter + i]: the gated activation between a fused gate/up
  * projection (one LinearQ call over 2*inter output features) and the down projection
  * (act_fn(gate_proj(x)) * up_proj(x) of Qwen3MLPQ, asrq/models/nemo/canary_qwen.py:70-86).  silu is rounded to
