@@ -216,6 +216,66 @@ add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
   }
 }
 
+// A few rows (a decoding step's): one block per row, eight elements per thread, so that a row's loads leave from all of its warps
+// at once and the norm's weights are there before the stream dependency resolves.  A warp per row took 3.2 us (RMS, 2048) between
+// two kernels of a step of one sequence and 4.8 us for 64, most of it the warp's own chain.
+constexpr int kRowBlockMax = 256;  // threads: dim up to 2048
+template <bool bf16, bool LAYER>
+__global__ void __launch_bounds__(kRowBlockMax)
+row_norm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ delta, const uint16_t* __restrict__ gamma, const uint16_t* __restrict__ beta,
+                float eps, uint16_t* __restrict__ x_out, uint16_t* __restrict__ h_out, int dim) {
+  __shared__ float part[2][kRowBlockMax / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int e = threadIdx.x * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const uint4 gq = __ldg(reinterpret_cast<const uint4*>(gamma + e)), bq = LAYER ? __ldg(reinterpret_cast<const uint4*>(beta + e)) : make_uint4(0, 0, 0, 0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const size_t off = size_t(blockIdx.x) * dim + e;
+  const uint4 a = *reinterpret_cast<const uint4*>(x + off);
+  uint32_t w[4] = {a.x, a.y, a.z, a.w};
+  if (delta) {
+    const uint4 d = *reinterpret_cast<const uint4*>(delta + off);
+    const uint32_t dw[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      w[j] = uint32_t(float_to_out16(in16(uint16_t(w[j] & 0xffffu), bf16) + in16(uint16_t(dw[j] & 0xffffu), bf16), bf16)) |
+             (uint32_t(float_to_out16(in16(uint16_t(w[j] >> 16), bf16) + in16(uint16_t(dw[j] >> 16), bf16), bf16)) << 16);
+  }
+  if (x_out) *reinterpret_cast<uint4*>(x_out + off) = make_uint4(w[0], w[1], w[2], w[3]);
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = in16(uint16_t(w[i >> 1] >> (16 * (i & 1))), bf16);
+  auto total = [&](float s, int which) {  // over the block, the same in every thread
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) part[which][warp] = s;
+    __syncthreads();
+    float t = 0.f;
+    for (int i = 0; i < nw; ++i) t += part[which][i];
+    return t;
+  };
+  float mean = 0.f;
+  if (LAYER) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += v[i];
+    mean = total(s, 0) / float(dim);
+  }
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sq = fmaf(v[i] - mean, v[i] - mean, sq);
+  const float rs = rsqrtf(total(sq, 1) / float(dim) + eps);
+  const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w}, bw[4] = {bq.x, bq.y, bq.z, bq.w};
+  uint32_t o[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float g = in16(uint16_t(gw[i >> 1] >> (16 * (i & 1))), bf16);
+    const float y = LAYER ? ln_apply(v[i], mean, rs, g, in16(uint16_t(bw[i >> 1] >> (16 * (i & 1))), bf16))
+                          : in16(float_to_out16(v[i] * rs, bf16), bf16) * g;
+    o[i >> 1] |= uint32_t(float_to_out16(y, bf16)) << (16 * (i & 1));
+  }
+  *reinterpret_cast<uint4*>(h_out + off) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // gu: rows x 2*inter (gate columns first, then up), out: rows x inter; eight elements per thread and row, kSiluRows rows in
 // flight.  Bound: memory; with one row at a time, a division to find it and exact quotients it took 2.2x the time of its bytes.
 // The exponential and the quotient are a few fp32 ulps off, under a rounding to 16 bits.
@@ -395,12 +455,16 @@ int launch_pdl(K kern, dim3 grid, dim3 block, cudaStream_t stream, Args... args)
 }  // namespace
 
 namespace {
+// Rows up to which a block takes one: with more, warps of different rows hide each other's latencies and need no block barrier.
+constexpr int kRowBlockRows = 296;
 template <bool bf16>
 int add_layernorm_as(const uint16_t* x, const uint16_t* delta, const uint16_t* gamma, const uint16_t* beta, float eps, uint16_t* x_out, uint16_t* h_out,
                      int rows, int dim, cudaStream_t stream) {
   const dim3 grid(unsigned((rows + kLnWarps - 1) / kLnWarps)), block(32 * kLnWarps);
   const bool vec_ok = aligned16(x) && aligned16(h_out) && aligned16(gamma) && aligned16(beta) && (!delta || aligned16(delta)) &&
                       (!x_out || aligned16(x_out));
+  if (vec_ok && rows <= kRowBlockRows && dim % 256 == 0 && dim <= 8 * kRowBlockMax)
+    return launch_pdl(row_norm_kernel<bf16, true>, dim3(unsigned(rows)), dim3(unsigned(dim / 8)), stream, x, delta, gamma, beta, eps, x_out, h_out, dim);
   auto run = [&](auto kern) { return launch_pdl(kern, grid, block, stream, x, delta, gamma, beta, eps, x_out, h_out, rows, dim); };
   if (vec_ok && dim == 1280) return run(add_layernorm_kernel<5, bf16>);
   if (vec_ok && dim == 1024) return run(add_layernorm_kernel<4, bf16>);
@@ -413,6 +477,9 @@ int add_rmsnorm_as(const uint16_t* x, const uint16_t* delta, const uint16_t* gam
                    cudaStream_t stream) {
   const dim3 grid(unsigned((rows + kLnWarps - 1) / kLnWarps)), block(32 * kLnWarps);
   const bool vec_ok = aligned16(x) && aligned16(h_out) && aligned16(gamma) && (!delta || aligned16(delta)) && (!x_out || aligned16(x_out));
+  if (vec_ok && rows <= kRowBlockRows && dim % 256 == 0 && dim <= 8 * kRowBlockMax)
+    return launch_pdl(row_norm_kernel<bf16, false>, dim3(unsigned(rows)), dim3(unsigned(dim / 8)), stream, x, delta, gamma,
+                      static_cast<const uint16_t*>(nullptr), eps, x_out, h_out, dim);
   auto run = [&](auto kern) { return launch_pdl(kern, grid, block, stream, x, delta, gamma, eps, x_out, h_out, rows, dim); };
   if (vec_ok && dim == 2048) return run(add_rmsnorm_kernel<8, bf16>);
   if (vec_ok && dim == 1024) return run(add_rmsnorm_kernel<4, bf16>);
