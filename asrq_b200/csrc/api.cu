@@ -63,7 +63,8 @@ int w4a4_gemm_int8(const uint8_t* w8, const uint8_t* a8, const float* sa, const 
                    int32_t* acc_dump, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int fmt,
                    void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream);
 size_t w4a4_tc_workspace_bytes(int64_t M, int64_t N, int64_t K);
-bool gemm_a16_skinny_supports(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes);
+double gemm_a16_skinny_estimate(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes);
+double gemm_a16_tc_estimate(int64_t M, int64_t N, int64_t K, int group_size, int sm_count);
 int gemm_a16_skinny(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                     void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
                     size_t workspace_bytes, int sm_count, cudaStream_t stream, const Epilogue& ep);
@@ -331,9 +332,11 @@ static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scale
   const DeviceFacts* f;
   if ((rc = device_facts(&f))) return rc;
   if (M == 0) return ASRQ_OK;
-  // decode batches (17..128 tokens): the chain-oriented tensor-core kernel where its one-wave grid fits
-  if (M <= 128 && option(kOptMidKernel) != 1 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0 &&
-      gemm_a16_skinny_supports(M, N, K, group_size, f->sm_count, workspace_bytes)) {
+  // Decode batches (17..128 tokens): the one-wave kernel, where it covers the layer.  Above, while a tile with all of K leaves SMs
+  // idle: where its estimate, which the fused epilogue is not even counted in, is the lower one.
+  const double one_wave = option(kOptMidKernel) != 1 && option(kOptTcPair) < 0 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0
+                              ? gemm_a16_skinny_estimate(M, N, K, group_size, f->sm_count, workspace_bytes) : -1.0;
+  if (one_wave > 0 && (M <= 128 || one_wave < gemm_a16_tc_estimate(M, N, K, group_size, f->sm_count))) {
     *fused = true;
     return gemm_a16_skinny(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes,
                            f->sm_count, static_cast<cudaStream_t>(stream), ep);

@@ -1,20 +1,20 @@
-// Decode batches on the tensor cores: y[M,N] = x[M,K] . dequant(W)[N,K]^T (+ bias) for 17 <= M <= 128.
+// Decode batches and short prompts on the tensor cores: y[M,N] = x[M,K] . dequant(W)[N,K]^T (+ bias), 17 <= M <= 2048, in one wave.
 //
 // At these token counts the mma.sync decode kernel is bound by the legacy MMA pipe (one m16n8k16 per ~13
 // clocks per scheduler, one per 8 tokens per 256 codes), and the persistent prefill kernel by its fixed
 // costs (set-up, first TMA and first dequantisation pass before the first MMA, an epilogue nothing
 // overlaps): 10-15 us for a 1-3 MB layer either way.  This kernel is built for a CHAIN of such layers:
 //
-//   * a block owns ONE work item -- a 128-feature tile and a part of K of at most 16 blocks of 64 -- so that
-//     its packed weights (twelve blocks at a time) and all of its activation tiles fit shared memory at once;
+//   * a block owns ONE work item -- a tile of 128 features x BT tokens and a part of K.  Its activation tiles and packed
+//     weights pass through a ring of stages in shared memory, which for decode batches holds all of them at once;
 //   * it triggers its dependents as its first instruction and is small enough (448 threads, <= 73
 //     registers, < 113 KB) for two launches to share an SM.  Packed weights are fetched by TMA and the
 //     first three K blocks are dequantised BEFORE griddepcontrol.wait: weights do not depend on the
 //     kernel before, so the next launch's weight traffic and unpacking run under this launch's tail;
-//   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32, 64, 96 or 128 TMEM columns)
-//     are fetched, all at once; tcgen05.mma kind::f16 128 x BT x 16, fp32 accumulator in tensor memory;
+//   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32 to 256 TMEM columns)
+//     are fetched, as many as there are stages at once; tcgen05.mma kind::f16 128 x BT x 16, fp32 accumulator in tensor memory;
 //   * the K parts of a tile are a thread-block cluster and meet in distributed shared memory: every block leaves its
-//     fp32 part in its own shared memory (over the A slots, whose MMAs are done), and after one cluster barrier each
+//     fp32 part in its own shared memory (over A slots and stages, whose MMAs are done), and after one cluster barrier each
 //     adds its share of the tokens over all parts in part order, with all of its threads, adds the bias, converts
 //     and stores.  Through the workspace (partial tiles, a counter per tile, the last block adding) the same step
 //     cost a release to memory, an atomic and two to four L2 round trips of one block while the others were done.
@@ -23,6 +23,9 @@
 // 2-13 three dequant groups of 128 threads (one weight row per thread, group d takes K blocks d, d+3, ...
 // and owns A slot d); the first group (warps 2-5, one per TMEM lane quadrant) then runs the epilogue.
 // No TMA multicast.  Every wait is bounded.
+//
+// Prompts of some hundred tokens: the persistent kernels give a tile the whole of K, and with few tiles most SMs idle (1280 x 5120
+// at 260 to 1500 tokens: 31 us on 20 to 60 of them).  Here K is cut so that one wave fills the chip.
 #include <algorithm>
 #include <atomic>
 
@@ -37,12 +40,10 @@ namespace {
 
 constexpr int kSkWarps = 14;
 constexpr int kSkThreads = 32 * kSkWarps;
-constexpr int kSkMaxKb = 16;                    // K blocks of 64 per work item
+constexpr int kSkMaxStages = 16;                // K blocks of 64 in shared memory at once
 constexpr int kSkMaxSplit = 8;
-constexpr int kSkMaxM = 128;
+constexpr int kSkMaxM = 2048;
 constexpr uint32_t kSkATile = 128 * 128;        // one dequantised A slot: 128 rows x 64 16-bit elements
-constexpr int kSkWSlots = 12;                   // packed K blocks held at once; the rest follow into the first slots
-constexpr int kSkWAgain = kSkMaxKb - kSkWSlots; // ... of which so many are filled twice
 constexpr size_t kSkMaxSmem = 226 * 1024;
 constexpr size_t kSkTwoPerSm = 112 * 1024;      // two blocks share an SM
 constexpr uint32_t kSkWSlot = 4096;             // packed weights of one K block (<= 128 x 32 B)
@@ -55,7 +56,7 @@ struct SkinnyParams {
   int act;                   // fused epilogue: activation on the layer output (kActNone / kActGelu)
   uint16_t* y;
   unsigned* status;
-  int M, N, K, group_size, groups_per_row, bt, ksplit, nkb, kbmax;
+  int M, N, K, group_size, groups_per_row, bt, n_tt, ksplit, nkb, stages;
   unsigned long long* trace;  // builds with -DASRQ_TRACE: 8 globaltimer marks per block, NULL otherwise
 };
 
@@ -72,12 +73,14 @@ struct SkinnyParams {
 #define SK_MARK(i) do { } while (0)
 #endif
 
-template <int BITS, bool BF16>
+// RING: parts longer than the ring of stages.  Without it every K block has a stage of its own: one barrier for all activation
+// tiles and nothing to count (with both forms in one kernel a launch of 32 tokens took 0.5 to 1 us more).
+template <int BITS, bool BF16, bool RING>
 __global__ void __launch_bounds__(kSkThreads, 2)
 gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
                        const SkinnyParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[kSkMaxKb + 8 + kSkWAgain];
+  __shared__ __align__(8) uint64_t bars[3 * kSkMaxStages + 7];
   __shared__ uint32_t tmem_slot;
   // the next launch on the stream may start its own set-up, weight fetch and first dequantisation now
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -87,30 +90,39 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw_addr);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // work item: feature tile ft, K part ks (parts of a tile on neighbouring blocks)
-  const int ks = blockIdx.x % p.ksplit, ft = blockIdx.x / p.ksplit;
-  const int kb0 = ks * p.nkb / p.ksplit, kb1 = (ks + 1) * p.nkb / p.ksplit, kbn = kb1 - kb0;
+  // work item: feature tile ft, token tile tt, K part ks (parts of a tile on neighbouring blocks: a cluster)
+  const int ks = blockIdx.x % p.ksplit, tile = blockIdx.x / p.ksplit, tt = tile % p.n_tt, ft = tile / p.n_tt;
+  const int kb0 = ks * p.nkb / p.ksplit, kb1 = (ks + 1) * p.nkb / p.ksplit, kbn = kb1 - kb0, nst = p.stages;
   const uint32_t xbytes = uint32_t(p.bt) * 128u;
-  // [A slot x 3] [activation tile x kbmax] [packed weights x min(kbmax, kSkWSlots)]
-  const uint32_t x_base = 3 * kSkATile, w_base = x_base + uint32_t(p.kbmax) * xbytes;
+  // [A slot x 3] [activation tile x stages] [packed weights x stages]
+  const uint32_t x_base = 3 * kSkATile, w_base = x_base + uint32_t(nst) * xbytes;
   constexpr uint32_t wbytes = 128u * 8u * BITS;
   const uint32_t bar0 = tc::smem_u32(bars);
-  auto w_bar = [&](int kb) { return bar0 + 8u * kb; };
-  const uint32_t x_bar = bar0 + 8u * kSkMaxKb, accf_bar = x_bar + 8u;
-  auto deq_bar = [&](int a) { return x_bar + 16u + 8u * a; };
-  auto afree_bar = [&](int a) { return x_bar + 40u + 8u * a; };
-  auto wfree_bar = [&](int i) { return x_bar + 64u + 8u * i; };
-  const uint32_t tmem_cols = p.bt <= 32 ? 32u : (p.bt <= 64 ? 64u : 128u);
+  auto w_bar = [&](int st) { return bar0 + 8u * st; };
+  auto x_bar = [&](int st) { return bar0 + 8u * (kSkMaxStages + st); };
+  auto sfree_bar = [&](int st) { return bar0 + 8u * (2 * kSkMaxStages + st); };  // the stage's MMAs are done
+  const uint32_t accf_bar = bar0 + 8u * (3 * kSkMaxStages);
+  auto deq_bar = [&](int a) { return accf_bar + 8u + 8u * a; };
+  auto afree_bar = [&](int a) { return accf_bar + 32u + 8u * a; };
+  const uint32_t tmem_cols = p.bt <= 32 ? 32u : (p.bt <= 64 ? 64u : (p.bt <= 128 ? 128u : 256u));
+
+  // The bias of the four features this thread stores (the same in each of its steps): a constant, and fetched here a first touch
+  // of memory that the last step would otherwise wait for.
+  uint2 bias4 = make_uint2(0u, 0u);
+  if (p.bias) bias4 = __ldg(reinterpret_cast<const uint2*>(p.bias + ft * 128 + lane * 4));
 
   if (threadIdx.x == 0) {
-    for (int kb = 0; kb < kSkMaxKb; ++kb) tc::mbar_init(w_bar(kb), 1);
-    tc::mbar_init(x_bar, 1);
+    for (int st = 0; st < nst; ++st) {
+      tc::mbar_init(w_bar(st), 1);
+      if (st && !RING) continue;
+      tc::mbar_init(x_bar(st), 1);
+      tc::mbar_init(sfree_bar(st), 1);
+    }
     tc::mbar_init(accf_bar, 1);
     for (int a = 0; a < 3; ++a) {
       tc::mbar_init(deq_bar(a), 128);
       tc::mbar_init(afree_bar(a), 1);
     }
-    for (int i = 0; i < kSkWAgain; ++i) tc::mbar_init(wfree_bar(i), 128);
     tc::fence_barrier_init();
     tc::fence_proxy_async_smem();
     tc::prefetch_tmap(&tmx);
@@ -129,43 +141,58 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
-      auto fetch_w = [&](int kb) {
-        tc::mbar_arrive_expect_tx(w_bar(kb), wbytes);
-        tc::tma_load_2d(base + w_base + (kb % kSkWSlots) * kSkWSlot, &tmw, (kb0 + kb) * 8 * BITS, ft * 128, w_bar(kb));
+      auto fetch_w = [&](int kb, int st) {
+        tc::mbar_arrive_expect_tx(w_bar(st), wbytes);
+        tc::tma_load_2d(base + w_base + st * kSkWSlot, &tmw, (kb0 + kb) * 8 * BITS, ft * 128, w_bar(st));
       };
-      for (int kb = 0; kb < kbn && kb < kSkWSlots; ++kb) fetch_w(kb);  // constants: ahead of the stream dependency
+      auto fetch_x = [&](int kb, int st) {
+        if (RING) tc::mbar_arrive_expect_tx(x_bar(st), xbytes);
+        tc::tma_load_2d(base + x_base + st * xbytes, &tmx, (kb0 + kb) * 64, tt * p.bt, x_bar(RING ? st : 0));
+      };
+      for (int kb = 0; kb < kbn && kb < nst; ++kb) fetch_w(kb, kb);  // constants: ahead of the stream dependency
       SK_MARK(2);
       // activations belong to this kernel only once its predecessor on the stream is complete
       asm volatile("griddepcontrol.wait;" ::: "memory");
       SK_MARK(3);
-      tc::mbar_arrive_expect_tx(x_bar, uint32_t(kbn) * xbytes);
-      for (int kb = 0; kb < kbn; ++kb) tc::tma_load_2d(base + x_base + kb * xbytes, &tmx, (kb0 + kb) * 64, 0, x_bar);
-      for (int kb = kSkWSlots; kb < kbn; ++kb) {
-        if (!tc::mbar_wait(wfree_bar(kb - kSkWSlots), 0u, p.status, 36)) break;
-        fetch_w(kb);
+      if (!RING) tc::mbar_arrive_expect_tx(x_bar(0), uint32_t(kbn) * xbytes);
+      for (int kb = 0; kb < kbn && kb < nst; ++kb) fetch_x(kb, kb);
+      if constexpr (RING) {
+        int st = 0;
+        uint32_t ph = 0;
+        for (int kb = nst; kb < kbn; ++kb) {
+          if (!tc::mbar_wait(sfree_bar(st), ph, p.status, 36)) break;
+          fetch_w(kb, st);
+          fetch_x(kb, st);
+          if (++st == nst) { st = 0; ph ^= 1u; }
+        }
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     const bool el = tc::elect_one();
     const uint32_t idesc = tc::instr_desc(1u, BF16 ? 1u : 0u, 128u, uint32_t(p.bt));
-    bool ok = tc::mbar_wait_spin(x_bar, 0u, p.status, 31);
+    int st = 0;
+    uint32_t ph = 0;
+    bool ok = tc::mbar_wait_spin(x_bar(0), 0u, p.status, 31);
     if (lane == 0) SK_MARK(4);
     for (int kb = 0; kb < kbn && ok; ++kb) {
       const int a = kb % 3;
-      ok = tc::mbar_wait_spin(deq_bar(a), uint32_t(kb / 3) & 1u, p.status, 32);
+      if (RING && kb) ok = tc::mbar_wait_spin(x_bar(st), ph, p.status, 31);
+      ok = ok && tc::mbar_wait_spin(deq_bar(a), uint32_t(kb / 3) & 1u, p.status, 32);
       if (!ok) break;
       tc::fence_after_sync();
       const uint64_t da = tc::smem_desc_sw128(base + a * kSkATile);
-      const uint64_t db = tc::smem_desc_sw128(base + x_base + kb * xbytes);
+      const uint64_t db = tc::smem_desc_sw128(base + x_base + st * xbytes);
       if (el) {
         tc::mma_f16(tmem_base, da, db, idesc, uint32_t(kb != 0));
         tc::mma_f16(tmem_base, da + 2, db + 2, idesc, 1u);
         tc::mma_f16(tmem_base, da + 4, db + 4, idesc, 1u);
         tc::mma_f16(tmem_base, da + 6, db + 6, idesc, 1u);
         tc::mma_commit(afree_bar(a));
+        if (RING && kb + nst < kbn) tc::mma_commit(sfree_bar(st));
         if (kb + 1 == kbn) tc::mma_commit(accf_bar);
       }
+      if (++st == nst && RING) { st = 0; ph ^= 1u; }
     }
     if (lane == 0) SK_MARK(5);
   } else {
@@ -174,10 +201,17 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
     const int t = ((warp - 2) & 3) * 32 + lane;  // weight row inside the tile
     const int kbpg = p.group_size / 64;
     bool ok = true;
+    auto load_sz = [&](int kb) {
+      const size_t idx = (size_t(ft) * 128 + t) * p.groups_per_row + (kb0 + kb) / kbpg;
+      return uint32_t(__half_as_ushort(__ldg(p.scales + idx))) | (uint32_t(__half_as_ushort(__ldg(p.zeros + idx))) << 16);
+    };
+    uint32_t sz_next = RING && dgroup < kbn ? load_sz(dgroup) : 0u;
+    int st = dgroup;  // a ring that goes round has at least four stages
+    uint32_t ph = 0;
     for (int kb = dgroup; kb < kbn && ok; kb += 3) {
-      const int gi = (kb0 + kb) / kbpg;
-      const size_t idx = (size_t(ft) * 128 + t) * p.groups_per_row + gi;
-      const __half sh = __ldg(p.scales + idx), zh = __ldg(p.zeros + idx);
+      const uint32_t sz = RING ? sz_next : load_sz(kb);
+      if (RING && kb + 3 < kbn) sz_next = load_sz(kb + 3);
+      const __half sh = __ushort_as_half(uint16_t(sz & 0xffffu)), zh = __ushort_as_half(uint16_t(sz >> 16));
       uint32_t s2, z2;
       if (BF16) {
         s2 = __float_as_uint(__half2float(sh));
@@ -188,9 +222,9 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
       }
       // the slot's previous K block (three back) must have been consumed by its MMAs
       if (kb >= 3) ok = tc::mbar_wait(afree_bar(dgroup), uint32_t(kb / 3 - 1) & 1u, p.status, 33);
-      ok = ok && tc::mbar_wait(w_bar(kb), 0u, p.status, 34);
+      ok = ok && tc::mbar_wait(w_bar(st), ph, p.status, 34);
       if (!ok) break;
-      const uint4* wp = reinterpret_cast<const uint4*>(smem + w_base + (kb % kSkWSlots) * kSkWSlot + t * (8 * BITS));
+      const uint4* wp = reinterpret_cast<const uint4*>(smem + w_base + st * kSkWSlot + t * (8 * BITS));
       uint8_t* arow = smem + dgroup * kSkATile + t * 128;
       constexpr int NV = BITS / 2;  // 16-byte vectors of packed weights per row per K block
 #pragma unroll
@@ -211,15 +245,14 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
         }
       }
       tc::fence_proxy_async_smem();
-      if (kb + kSkWSlots < kbn) tc::mbar_arrive(wfree_bar(kb));
       tc::mbar_arrive(deq_bar(dgroup));
+      st += 3;
+      if (RING && st >= nst) { st -= nst; ph ^= 1u; }
     }
     ok = __all_sync(0xffffffffu, ok);  // a wait that gave up in any lane ends the warp's work
     if (dgroup == 0 && ok) {
       // ------------------------------ epilogue (warps 2-5: lane quadrants 2, 3, 0, 1) ------------------------------
       const int qd = warp & 3;
-      const int f = ft * 128 + qd * 32 + lane;
-      const float bias = p.bias ? ldg_half(p.bias + f) : 0.f;
       // one decision for the warp, and the lanes together again after the polling loop: the tensor-memory loads
       // below are warp-wide instructions
       if (__all_sync(0xffffffffu, tc::mbar_wait(accf_bar, 0u, p.status, 35))) {
@@ -227,28 +260,14 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
         tc::fence_after_sync();
         if (warp == 2 && lane == 0) SK_MARK(6);
         const uint32_t taddr = tmem_base + (uint32_t(qd * 32) << 16);
-        if (p.ksplit == 1) {
-          for (int ch = 0; ch < p.bt / 32; ++ch) {
-            uint32_t r[32];
-            tc::tmem_ld_32x32(taddr + ch * 32, r);
-            tc::tmem_ld_wait();
+        // this block's part of the tile, fp32 [token][128 features], over A slots and stages
+        float* part = reinterpret_cast<float*>(smem) + qd * 32 + lane;
+        for (int ch = 0; ch < p.bt / 32; ++ch) {
+          uint32_t r[32];
+          tc::tmem_ld_32x32(taddr + ch * 32, r);
+          tc::tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (ch * 32 + j < p.M) {
-                const size_t idx = size_t(ch * 32 + j) * p.N + f;
-                p.y[idx] = finish16(__uint_as_float(r[j]) + bias, p.act, p.residual, idx, BF16);
-              }
-          }
-        } else {
-          // this block's part of the tile, fp32 [token][128 features], over the A slots
-          float* part = reinterpret_cast<float*>(smem) + qd * 32 + lane;
-          for (int ch = 0; ch < p.bt / 32; ++ch) {
-            uint32_t r[32];
-            tc::tmem_ld_32x32(taddr + ch * 32, r);
-            tc::tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) part[(ch * 32 + j) * 128] = __uint_as_float(r[j]);
-          }
+          for (int j = 0; j < 32; ++j) part[(ch * 32 + j) * 128] = __uint_as_float(r[j]);
         }
       }
     }
@@ -256,17 +275,21 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
 
   __syncwarp();
   tc::fence_before_sync();
+  // every part is in its block's shared memory
   if (p.ksplit == 1) {
     __syncthreads();
   } else {
-    tc::cluster_sync();  // every part is in its block's shared memory
-    const int m0 = ks * p.M / p.ksplit, count = ((ks + 1) * p.M / p.ksplit - m0) * 32;  // four features of a token per step
+    tc::cluster_sync();
+  }
+  {
+    const int rows = min(p.bt, p.M - tt * p.bt);  // tokens of this tile
+    const int m0 = ks * rows / p.ksplit, count = ((ks + 1) * rows / p.ksplit - m0) * 32;  // four features of a token per step
     uint32_t part[kSkMaxSplit];
 #pragma unroll
     for (int s = 0; s < kSkMaxSplit; ++s) part[s] = s < p.ksplit ? tc::mapa(base, s) : 0u;
     for (int o4 = threadIdx.x; o4 < count; o4 += kSkThreads) {
       const int tok = m0 + (o4 >> 5), f = ft * 128 + (o4 & 31) * 4;
-      const size_t idx = size_t(tok) * p.N + f;
+      const size_t idx = size_t(tt * p.bt + tok) * p.N + f;
       uint2 res = make_uint2(0u, 0u);
       if (p.residual) res = *reinterpret_cast<const uint2*>(p.residual + idx);
       float4 a[kSkMaxSplit];
@@ -279,11 +302,8 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
         if (s < p.ksplit) {
           v.x += a[s].x; v.y += a[s].y; v.z += a[s].z; v.w += a[s].w;
         }
-      if (p.bias) {
-        const uint2 b = __ldg(reinterpret_cast<const uint2*>(p.bias + f));
-        const float2 b01 = __half22float2(u32_as_h2(b.x)), b23 = __half22float2(u32_as_h2(b.y));
-        v.x += b01.x; v.y += b01.y; v.z += b23.x; v.w += b23.y;
-      }
+      const float2 b01 = __half22float2(u32_as_h2(bias4.x)), b23 = __half22float2(u32_as_h2(bias4.y));
+      v.x += b01.x; v.y += b01.y; v.z += b23.x; v.w += b23.y;
       const float vv[4] = {v.x, v.y, v.z, v.w};
       const uint16_t rr[4] = {uint16_t(res.x & 0xffffu), uint16_t(res.x >> 16), uint16_t(res.y & 0xffffu), uint16_t(res.y >> 16)};
       uint16_t o[4];
@@ -294,7 +314,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
       }
       *reinterpret_cast<uint2*>(p.y + idx) = make_uint2(uint32_t(o[0]) | (uint32_t(o[1]) << 16), uint32_t(o[2]) | (uint32_t(o[3]) << 16));
     }
-    tc::cluster_sync_relaxed();  // no block leaves while another reads its part
+    if (p.ksplit > 1) tc::cluster_sync_relaxed();  // no block leaves while another reads its part
   }
   if (threadIdx.x == 0) SK_MARK(7);
   if (warp == 1) {
@@ -304,8 +324,9 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
 }
 
 struct SkinnyPlan {
-  int bt, ksplit, nkb, kbmax, grid;
+  int bt, n_tt, ksplit, nkb, stages, grid;
   size_t smem;
+  double us;  // estimate
 };
 
 // Blocks of one launch that run at once as clusters of `split` (the size leaves some SMs without a whole cluster): the
@@ -316,7 +337,7 @@ int skinny_capacity(int split, size_t smem) {
   std::atomic<int>& k = known[split][two];
   int n = k.load(std::memory_order_relaxed);
   if (n) return n;
-  auto kern = gemm_a16_skinny_kernel<4, false>;
+  auto kern = gemm_a16_skinny_kernel<4, false, false>;
   const size_t ask = two ? kSkTwoPerSm : kSkMaxSmem;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), ask)) return 0;
   cudaLaunchConfig_t cfg = {};
@@ -337,38 +358,57 @@ int skinny_capacity(int split, size_t smem) {
   return n * split;
 }
 
+// Token tile and K parts: the pair with the least estimated time among those whose blocks run in one wave.  The estimate (us)
+// follows the measurements of 17 to 1500 tokens on eight layer shapes: 4 for launch, first fetches and stores, 0.34 per K block
+// (dequantisation and its hand-over; the MMAs of 256 columns hide behind it), 0.011 per column of the tile for its way out of
+// tensor memory, 0.6 for the clusters' two barriers.
+bool skinny_search(int64_t M, int64_t N, int64_t K, int sm_count, SkinnyPlan* pl) {
+  const int64_t nft = N / 128, nkb = K / 64;
+  pl->us = 1e30;
+  for (int bt : {32, 64, 96, 128, 192, 256}) {
+    if (bt - 32 >= M && bt != 32) break;
+    const int64_t n_tt = (M + bt - 1) / bt, tiles = nft * n_tt;
+    if (tiles > sm_count) continue;
+    const size_t stage = size_t(bt) * 128 + kSkWSlot;
+    const int64_t fit = std::min<int64_t>(kSkMaxStages, int64_t((kSkMaxSmem - 1024 - 3 * kSkATile) / stage));
+    for (int64_t sp = 1; sp <= kSkMaxSplit && sp <= nkb && tiles * sp <= sm_count; ++sp) {
+      const int64_t kb = (nkb + sp - 1) / sp, stages = std::min(kb, fit);
+      const size_t smem = 1024 + std::max(3 * kSkATile + size_t(stages) * stage, size_t(bt) * 512);
+      const double us = 4.0 + 0.34 * double(kb) + 0.011 * bt + (sp > 1 ? 0.6 : 0.0);
+      if (us >= pl->us || (sp > 1 && skinny_capacity(int(sp), smem) < tiles * sp)) continue;
+      *pl = {bt, int(n_tt), int(sp), int(nkb), int(stages), int(tiles * sp), smem, us};
+    }
+  }
+  return pl->us < 1e30;
+}
+
 bool skinny_plan(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes, SkinnyPlan* pl) {
   if (M < 1 || M > kSkMaxM || N % 128 || K % 64 || group_size <= 0 || group_size % 64 || K % group_size) return false;
   if (workspace_bytes < kStatusBytes) return false;
-  const int64_t tiles = N / 128, nkb = K / 64;
-  const int bt = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128));
-  auto smem_of = [&](int64_t sp) {
-    const int64_t kb = (nkb + sp - 1) / sp;
-    return 1024 + 3 * kSkATile + size_t(kb) * (size_t(bt) * 128) + size_t(std::min<int64_t>(kb, kSkWSlots)) * kSkWSlot;
+  struct Entry {
+    int64_t M, N, K;
+    int sms;
+    bool ok;
+    SkinnyPlan plan;
   };
-  // Parts of K: the most that run in one wave with a block per SM, at least enough for kSkMaxKb K blocks per part.  Where
-  // clusters of that many leave too few SMs, fewer; where none fits (the last clusters then run in a second wave), the most.
-  int64_t least = (nkb + kSkMaxKb - 1) / kSkMaxKb, split = std::min<int64_t>({std::max<int64_t>(least, sm_count / tiles), kSkMaxSplit, nkb});
-  if (split < least || tiles * split > sm_count) return false;
-  while (least < split && smem_of(least) > kSkMaxSmem) ++least;
-  for (int64_t sp = split; sp >= least; --sp)
-    if (sp == 1 || skinny_capacity(int(sp), smem_of(sp)) >= tiles * sp) {
-      split = sp;
-      break;
+  thread_local Entry known[16];  // a program's layers come round again; a few thousand candidates' arithmetic does not have to
+  thread_local unsigned next = 0;
+  for (const Entry& e : known)
+    if (e.M == M && e.N == N && e.K == K && e.sms == sm_count) {
+      *pl = e.plan;
+      return e.ok;
     }
-  pl->bt = bt;
-  pl->ksplit = int(split);
-  pl->nkb = int(nkb);
-  pl->kbmax = int((nkb + split - 1) / split);
-  pl->grid = int(tiles * split);
-  pl->smem = smem_of(split);
-  return pl->smem <= kSkMaxSmem;
+  Entry& e = known[next++ % 16];
+  e = {M, N, K, sm_count, false, {}};
+  e.ok = skinny_search(M, N, K, sm_count, &e.plan);
+  *pl = e.plan;
+  return e.ok;
 }
 
 template <int BITS, bool BF16>
 int launch_skinny(const CUtensorMap& tmx, const CUtensorMap& tmw, const SkinnyParams& p, int grid, size_t smem,
                   cudaStream_t stream) {
-  auto kern = gemm_a16_skinny_kernel<BITS, BF16>;
+  auto kern = int64_t(p.nkb + p.ksplit - 1) / p.ksplit > p.stages ? gemm_a16_skinny_kernel<BITS, BF16, true> : gemm_a16_skinny_kernel<BITS, BF16, false>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
@@ -389,9 +429,10 @@ int launch_skinny(const CUtensorMap& tmx, const CUtensorMap& tmw, const SkinnyPa
 
 }  // namespace
 
-bool gemm_a16_skinny_supports(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes) {
+// Estimated time in us, or a negative number where the kernel does not cover the call (in one wave).
+double gemm_a16_skinny_estimate(int64_t M, int64_t N, int64_t K, int group_size, int sm_count, size_t workspace_bytes) {
   SkinnyPlan pl;
-  return skinny_plan(M, N, K, group_size, sm_count, workspace_bytes, &pl);
+  return skinny_plan(M, N, K, group_size, sm_count, workspace_bytes, &pl) ? pl.us : -1.0;
 }
 
 int gemm_a16_skinny(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
@@ -418,7 +459,8 @@ int gemm_a16_skinny(int bits, const void* x, const uint8_t* w, const void* scale
   p.bt = pl.bt;
   p.ksplit = pl.ksplit;
   p.nkb = pl.nkb;
-  p.kbmax = pl.kbmax;
+  p.n_tt = pl.n_tt;
+  p.stages = pl.stages;
   p.trace = nullptr;
 #ifdef ASRQ_TRACE
   if (option(kOptTrace) && workspace_bytes >= (8u << 20)) {  // marks of the launches since the option last changed

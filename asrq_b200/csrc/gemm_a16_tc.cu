@@ -443,7 +443,7 @@ int gemm_tc_pick_split(int64_t M, int64_t N, int64_t K, int bt, int sm_count) {
 // time of a K block -- up to 128 columns that is the dequantisation of its weights (0.37 us), which the MMAs hide behind -- plus
 // the addition of the parts where K is split (0.017 us per column and part).  Measured: 12288 x 2048, us: 16.1 for 64 columns
 // in one round, 16.6 for 128, 27.7 for two rounds of 32; 1280 x 1280 at 96 tokens: 8.7 for 32 columns in 4 parts, 13.5 for 96 in 5.
-int gemm_tc_pick_bt(int64_t M, int64_t N, int64_t K, int sm_count) {
+int gemm_tc_pick_bt(int64_t M, int64_t N, int64_t K, int sm_count, double* us = nullptr) {
   const int forced = option(kOptTcBt);  // tuning knob: force the token-tile width
   if (forced >= 32 && forced <= 256 && forced % 32 == 0) return forced;
   int best = 32;
@@ -460,6 +460,7 @@ int gemm_tc_pick_bt(int64_t M, int64_t N, int64_t K, int sm_count) {
       best = bt;
     }
   }
+  if (us) *us = best_cost + 4.0;  // and the launch, first fetches and stores
   return best;
 }
 
@@ -487,9 +488,18 @@ static int launch_tc(const CUtensorMap& tmx, const CUtensorMap& tmw, const GemmT
 }
 
 bool gemm_a16_tc2_supports(int64_t M, int64_t N, int64_t K, int group_size);
+double gemm_a16_tc2_estimate(int64_t M, int64_t N, int64_t K, int sm_count);
 int gemm_a16_tc2(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                  void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
                  size_t workspace_bytes, int sm_count, cudaStream_t stream);
+
+// Estimated time in us of whichever of the two kernels gemm_a16_tc takes
+double gemm_a16_tc_estimate(int64_t M, int64_t N, int64_t K, int group_size, int sm_count) {
+  if (M > 256 && gemm_a16_tc2_supports(M, N, K, group_size)) return gemm_a16_tc2_estimate(M, N, K, sm_count);
+  double us = 0.0;
+  gemm_tc_pick_bt(M, N, K, sm_count, &us);
+  return us;
+}
 
 // `ep`: an epilogue the caller would like fused; *fused says whether the kernel that ran applied it.  Neither
 // persistent kernel does: their four epilogue warps run under the next tile's main loop and have no slack for an

@@ -506,6 +506,14 @@ int launch_tc2(const CUtensorMap& tmx, const CUtensorMap& tmw, const GemmTc2Para
 
 }  // namespace
 
+// Estimated time in us: 5.5 for set-up and the last epilogue, and the rounds' K blocks (see pick_bt; a tenth on top of the clocks)
+double gemm_a16_tc2_estimate(int64_t M, int64_t N, int64_t K, int sm_count) {
+  const int64_t pairs = N / 256, clusters = sm_count / 2;
+  const int bt = pick_bt(M, pairs, int(clusters));
+  const int64_t rounds = (pairs * ((M + bt - 1) / bt) + clusters - 1) / clusters;
+  return 5.5 + double(rounds) * double(K / 64) * std::max(2.0 * bt, 540.0) * 1.1 / 1900.0;
+}
+
 // The pair kernel needs an even number of feature tiles and enough work for the CTA pairs.
 bool gemm_a16_tc2_supports(int64_t M, int64_t N, int64_t K, int group_size) {
   return M >= 64 && N % 256 == 0 && K % 64 == 0 && group_size > 0 && group_size % 64 == 0 && K % group_size == 0;

@@ -1,5 +1,5 @@
-"""The tensor-core decode-batch kernel at its edges: token tiles of 32, 64, 96 and 128 columns, one to eight K parts, parts longer
-than the packed weights it holds at once (more than twelve K blocks), and tokens that do not divide among the parts."""
+"""The one-wave tensor-core kernel at its edges: token tiles of 32 to 256 columns, one to eight K parts, parts longer than its ring
+of stages, and tokens that divide neither among the parts nor into tiles."""
 import pytest
 import torch
 
@@ -15,12 +15,14 @@ pytestmark = pytest.mark.gpu
     (33, 2048, 4096, 4),   # four parts
     (64, 1280, 5120, 2),   # three parts
     (65, 1280, 1280, 4), (96, 2048, 2048, 4), (97, 1280, 3840, 2), (128, 1280, 5120, 4), (128, 64, 128, 4),
-    (20, 6144, 2048, 4), (64, 6144, 2048, 4),   # six parts of sixteen: the weight slots are filled twice
+    (20, 6144, 2048, 4), (64, 6144, 2048, 4),   # six parts of sixteen
     (31, 8192, 128, 4),    # eight parts of sixteen
     (24, 2048, 12288, 4),  # more tiles than one wave takes: the persistent kernel
     (65, 2048, 12288, 4),
+    (129, 1280, 1280, 4), (257, 5120, 1280, 4), (300, 6144, 2048, 2),   # several token tiles; stages used many times
+    (511, 2048, 2048, 4), (1000, 5120, 1280, 4), (1300, 6144, 256, 4), (2048, 5120, 256, 2),
 ])
-def test_decode_batches(m, k, n, bits):
+def test_one_wave_kernel(m, k, n, bits):
     case = O.make_c3(seed=m + k, m=m, k=k, n=n, bits=bits, group_size=64 if k == 64 else 128)
     layer = make_layer(case)
     x = case["x"].cuda()
