@@ -214,7 +214,8 @@ class WhisperEngine:
     """
 
     fused_self_attention = os.environ.get("ASRQ_B200_WHISPER_FUSED_SELF_ATTENTION", "1") == "1"
-    # Cross-attention of a step: this library's kernel up to this many (sequence, head) pairs, the vendor library's above.
+    # Cross-attention of a step: this library's kernel up to this many (sequence, head) pairs, the vendor library's above, which
+    # runs at the copy rate once there is a wave of them (a step of 160 pairs 1.53 against 1.64 ms, of 320 2.15 against 2.11).
     own_cross_attention_items = int(os.environ.get("ASRQ_B200_WHISPER_OWN_CROSS_ITEMS", "296"))
     cross_kv_views = os.environ.get("ASRQ_B200_WHISPER_CROSS_KV_VIEWS", "1") == "1"
 

@@ -293,7 +293,7 @@ class W4A4Layer(Workload):
                "frac_of_2x_bf16_measured": ach / (2 * peaks["bf16_tflops"]),
                "traffic": tr["dram_bytes_per_launch"] if tr else None, "traffic_algorithmic": self.gemm_bytes()}
         pro = self.prologue_bytes() / (kernel_ms["hadamard_quant"] * 1e-3) / 1e9
-        out["prologue"] = {"kernel": "hadamard4096_quant_kernel", "bound": "hbm", "achieved": pro, "unit": "GB/s",
+        out["prologue"] = {"kernel": "hadamard_transpose_quant_kernel", "bound": "hbm", "achieved": pro, "unit": "GB/s",
                            "peak": peaks["hbm_gbs"], "frac": pro / peaks["hbm_gbs"], "of": peaks["source"]}
         out["library_gemm_same_shape"] = library_gemm_same_shape(self.dev, self.M, self.K, self.N, "int8")
         out["library_f16_gemm_same_shape"] = library_gemm_same_shape(self.dev, self.M, self.K, self.N, "f16")
