@@ -88,6 +88,7 @@ struct W4A4TcParams {
   unsigned* status;
   long long* trace;  // builds with -DASRQ_TRACE: when not NULL, block `trace_block` records clock64() at pipeline milestones
   int M, N, K, groups, blocks_per_group, bt, nbuf, nstages, n_ftiles, n_ttiles, bf16, trace_block;
+  int resident;  // the feature tile's weights stay in shared memory over consecutive token tiles
 };
 
 constexpr int kW4A4MaxBufs = 4;
@@ -100,6 +101,7 @@ constexpr int kW4A4MaxStages = 8;
 constexpr bool kW4A4PairDefault = false;
 constexpr int w4a4_threads(int cg) { return 32 * (4 + 4 * cg); }  // producer, two MMA issuers, one idle, drain
 constexpr uint32_t kW8TileBytes = 128 * 128;
+constexpr int kW4A4MaxResident = 8;  // K blocks of resident weights (128 KB)
 
 // F8 = false: operands are int8 holding 16x the code, kind::i8, int32 sums in TMEM (256x the true sum).
 // F8 = true: operands are e4m3 bytes holding the code, kind::f8f6f4, fp32 sums in TMEM: a group sum is
@@ -114,13 +116,14 @@ constexpr uint32_t kW8TileBytes = 128 * 128;
 template <bool DUMP, bool F8, int CG, int NCH, bool PAIR>
 __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUtensorMap* tma_p, const W4A4TcParams& p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * kW4A4MaxStages + 2 * kW4A4MaxBufs];
+  __shared__ __align__(8) uint64_t bars[3 * kW4A4MaxStages + 2 * kW4A4MaxBufs + kW4A4MaxResident];
   __shared__ uint32_t tmem_slot;
 
   const uint32_t raw_addr = tc::smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   const uint32_t bbytes = uint32_t(PAIR ? p.bt / 2 : p.bt) * 128u;  // this CTA's activation rows of a K block
-  const uint32_t stage_bytes = kW8TileBytes + bbytes;
+  const bool resident = !PAIR && p.resident != 0;
+  const uint32_t stage_bytes = (resident ? 0u : kW8TileBytes) + bbytes;
   const uint32_t rank = PAIR ? tc::cluster_ctarank() : 0u;
   const int worker = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x);     // tile-loop start and stride:
   const int nworkers = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);     // CTAs, or CTA pairs
@@ -133,6 +136,7 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * kW4A4MaxStages + kW4A4MaxBufs + b); };
   // PAIR, CTA 0: "the peer's tiles of stage s have landed" (one remote arrival per stage by the peer's relay thread)
   auto pfull_bar = [&](int s) { return bar0 + 8u * (2 * kW4A4MaxStages + 2 * kW4A4MaxBufs + s); };
+  auto wres_bar = [&](int kb) { return bar0 + 8u * (3 * kW4A4MaxStages + 2 * kW4A4MaxBufs + kb); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < nst; ++s) {
@@ -140,6 +144,8 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
       tc::mbar_init(empty_bar(s), 1);
       tc::mbar_init(pfull_bar(s), 1);
     }
+    if (resident)
+      for (int kb = 0; kb < kW4A4MaxResident; ++kb) tc::mbar_init(wres_bar(kb), 1);
     for (int b = 0; b < p.nbuf; ++b) {
       tc::mbar_init(accf_bar(b), 1);
       tc::mbar_init(acce_bar(b), PAIR ? 2 * 4 * CG : 32 * 4 * CG);  // per drain warp of both CTAs / per drain thread
@@ -172,6 +178,13 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
   const int n_ft = PAIR ? p.n_ftiles / 2 : p.n_ftiles;
   const int ntiles = n_ft * p.n_ttiles;
   const int nkb = p.K / 128;
+  // Resident weights: a worker takes consecutive tiles in feature-major order and reloads the weights where the feature tile
+  // changes, at most about once; otherwise the workers stride over the tiles, feature tiles fastest.
+  const int tile0 = resident ? int((long long)(ntiles)*worker / nworkers) : worker;
+  const int tile_end = resident ? int((long long)(ntiles) * (worker + 1) / nworkers) : ntiles, tile_step = resident ? 1 : nworkers;
+  auto ft_of = [&](int tile) { return resident ? tile / p.n_ttiles : (PAIR ? 2 * (tile % n_ft) + int(rank) : tile % n_ft); };
+  auto tt_of = [&](int tile) { return resident ? tile % p.n_ttiles : tile / n_ft; };
+  const uint32_t ring = base + (resident ? uint32_t(nkb) * kW8TileBytes : 0u);  // the stages, behind the resident weights
 #ifdef ASRQ_TRACE
   const bool tr = p.trace != nullptr && int(blockIdx.x) == p.trace_block;
   auto mark = [&](int role, uint32_t i, int slot) {
@@ -187,18 +200,34 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
       uint32_t it = 0, ph = 0;
       int s = 0;
       bool ok = true;
-      for (int tile = worker; tile < ntiles && ok; tile += nworkers) {
-        const int ft = PAIR ? 2 * (tile % n_ft) + int(rank) : tile % n_ft, tt = tile / n_ft;
+      int ft_last = -1;
+      for (int tile = tile0; tile < tile_end && ok; tile += tile_step) {
+        const int ft = ft_of(tile), tt = tt_of(tile);
+        if (resident && ft != ft_last) {
+          // every stage consumed: no MMA reads the weights that are about to be replaced (nothing to wait for at first)
+          int s2 = s;
+          uint32_t ph2 = ph;
+          for (int j = 0; j < nst && ok; ++j) {
+            ok = tc::mbar_wait(empty_bar(s2), ph2 ^ 1u, p.status, 17);
+            if (++s2 == nst) { s2 = 0; ph2 ^= 1u; }
+          }
+          if (!ok) break;
+          for (int kb = 0; kb < nkb; ++kb) {
+            tc::mbar_arrive_expect_tx(wres_bar(kb), kW8TileBytes);
+            tc::tma_load_2d(base + kb * kW8TileBytes, tmw_p, kb * 128, ft * 128, wres_bar(kb));
+          }
+          ft_last = ft;
+        }
         const int row_w = ft * 128, row_a = tt * p.bt + (PAIR ? int(rank) * (p.bt / 2) : 0);
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           if (!tc::mbar_wait(empty_bar(s), ph ^ 1u, p.status, 11)) { ok = false; break; }
           mark(0, it, 0);
-          const uint32_t sb = base + s * stage_bytes;
+          const uint32_t sb = ring + s * stage_bytes;
           // every CTA's loads complete on its own barrier (a load that counts its bytes on the peer's
           // barrier measured far slower); the peer's relay thread forwards "landed" once per stage
-          tc::mbar_arrive_expect_tx(full_bar(s), kW8TileBytes + bbytes);
-          tc::tma_load_2d(sb, tmw_p, kb * 128, row_w, full_bar(s));
-          tc::tma_load_2d(sb + kW8TileBytes, tma_p, kb * 128, row_a, full_bar(s));
+          tc::mbar_arrive_expect_tx(full_bar(s), stage_bytes);
+          if (!resident) tc::tma_load_2d(sb, tmw_p, kb * 128, row_w, full_bar(s));
+          tc::tma_load_2d(sb + (resident ? 0u : kW8TileBytes), tma_p, kb * 128, row_a, full_bar(s));
           mark(0, it, 1);
           if (++s == nst) { s = 0; ph ^= 1u; }
         }
@@ -222,7 +251,14 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
       uint32_t buf = 0, bph = 0;        // accumulator buffer of group ac and the parity of its use count
       int s = 0, gb = 0;
       bool ok = true;
-      for (int tile = worker; tile < ntiles && ok; tile += nworkers) {
+      int ft_last = -1;
+      uint32_t wph = 1;  // parity of the weights' arrivals
+      for (int tile = tile0; tile < tile_end && ok; tile += tile_step) {
+        const bool fresh = resident && ft_of(tile) != ft_last;
+        if (fresh) {
+          ft_last = ft_of(tile);
+          wph ^= 1u;
+        }
         for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
           // Both issuers observe every phase of every stage barrier, also for the other one's K blocks:
           // a waiter that skipped a phase could mistake an older, still incomplete phase of the same
@@ -237,12 +273,16 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
               ok = tc::mbar_wait_spin(acce_bar(buf), bph ^ 1u, p.status, 12);
               if (!ok) break;
             }
+            if (fresh) {  // (the number of groups is even: a K block of the weights always belongs to the same issuer)
+              ok = tc::mbar_wait_spin(wres_bar(kb), wph, p.status, 18);
+              if (!ok) break;
+            }
             tc::fence_after_sync();
             mark(1, it, 0);
-            const uint32_t sb = base + s * stage_bytes;
+            const uint32_t sb = ring + s * stage_bytes;
             const uint32_t d_tmem = tmem_base + buf * uint32_t(p.bt);
             // a K step of 32 bytes = +2 in the descriptor's 16-byte address field
-            const uint64_t da = tc::smem_desc_sw128(sb), db = tc::smem_desc_sw128(sb + kW8TileBytes);
+            const uint64_t da = tc::smem_desc_sw128(resident ? base + kb * kW8TileBytes : sb), db = tc::smem_desc_sw128(resident ? sb : sb + kW8TileBytes);
             if (el) {
               if (PAIR) {
                 tc::mma_8bit_pair<F8>(d_tmem, da, db, idesc, uint32_t(gb != 0));
@@ -285,7 +325,7 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
       uint32_t ph = 0;
       int s = 0;
       bool ok = true;
-      for (int tile = worker; tile < ntiles && ok; tile += nworkers) {
+      for (int tile = tile0; tile < tile_end && ok; tile += tile_step) {
         for (int kb = 0; kb < nkb; ++kb) {
           if (!tc::mbar_wait(full_bar(s), ph, p.status, 16)) { ok = false; break; }
           tc::mbar_arrive_cluster_relaxed(pfull0 + 8u * s);
@@ -300,8 +340,8 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
     const int nch = wcols >> 4;        // 16-column chunks: 1..NCH
     uint32_t ac = 0, buf = 0, aph = 0;
     bool ok = true;
-    for (int tile = worker; tile < ntiles && ok; tile += nworkers) {
-      const int ft = PAIR ? 2 * (tile % n_ft) + int(rank) : tile % n_ft, tt = tile / n_ft;
+    for (int tile = tile0; tile < tile_end && ok; tile += tile_step) {
+      const int ft = ft_of(tile), tt = tt_of(tile);
       const int f = ft * 128 + qd * 32 + lane;
       const __half* swrow = p.sw + size_t(f) * p.groups;
       float2 accf[8 * NCH];  // running fp32 sums, two columns per register pair (packed fp32 FMA)
@@ -407,9 +447,10 @@ w4a4_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_consta
 // warps).  The accumulator buffers fill tensor memory: min(4, 512 / BT) of them.
 struct W4A4Tile {
   int bt, cg;
+  bool resident = false;
 };
 // `N` and `sm_count` are halved by the caller for the CTA-pair kernel (feature-tile pairs over CTA pairs).
-static W4A4Tile w4a4_pick_tile(int64_t M, int64_t N, int sm_count) {
+static W4A4Tile w4a4_pick_tile(int64_t M, int64_t N, int64_t K, int group_size, bool pair, int sm_count) {
   const int bt_env = option(kOptW4a4Bt);  // tuning knob
   if (bt_env > 0 && bt_env <= 192 && (bt_env % 48 == 0 || bt_env % 64 == 0))
     return {bt_env, bt_env % 48 == 0 ? 3 : 4};
@@ -424,6 +465,14 @@ static W4A4Tile w4a4_pick_tile(int64_t M, int64_t N, int sm_count) {
       best_cost = cost;
       best = {bt, 3};
     }
+  }
+  // Resident weights (K <= 1024).  Otherwise a group brings 16 KB of weights and bt * 128 B of activations for 2 bt clocks of
+  // MMAs, and an SM takes in about 45 B/clk: 880 clocks per group at 192 columns.  With the weights kept over a worker's
+  // consecutive token tiles only the activations come, 364 clocks for 128 columns (four accumulator buffers), after one load of
+  // the weights, or two where the worker's tiles span two feature tiles; it pays from two or three tiles per worker on.
+  if (!pair && K <= 128 * kW4A4MaxResident && K / group_size % 2 == 0) {
+    const int64_t tiles = nft * ((M + 127) / 128), rounds = (tiles + sm_count - 1) / sm_count;
+    if (double(rounds) * 370 + 2 * 364 < best_cost * 4.23) best = {128, 4, true};
   }
   return best;
 }
@@ -477,16 +526,18 @@ int w4a4_gemm_int8(const uint8_t* w8, const uint8_t* a8, const float* sa, const 
   // number of feature tiles.  Option "w4a4_pair" = 0 / 1 forces the choice (tuning knob).
   const int pair_env = option(kOptW4a4Pair);
   const bool pair = (N / 128) % 2 == 0 && sm_count >= 2 && pair_env != 0 && (pair_env == 1 || kW4A4PairDefault);
-  const W4A4Tile tile = pair ? w4a4_pick_tile(M, N / 2, sm_count / 2) : w4a4_pick_tile(M, N, sm_count);
+  const W4A4Tile tile = pair ? w4a4_pick_tile(M, N / 2, K, group_size, true, sm_count / 2) : w4a4_pick_tile(M, N, K, group_size, false, sm_count);
+  p.resident = tile.resident;
   p.bt = tile.bt;
   p.nbuf = 512 / p.bt >= 4 ? 4 : 2;  // even, so that a buffer always belongs to the same issuer
   p.n_ftiles = int(N / 128);
   p.n_ttiles = int((M + p.bt - 1) / p.bt);
   p.bf16 = dtype == ASRQ_BF16;
-  const size_t stage_bytes = kW8TileBytes + size_t(pair ? p.bt / 2 : p.bt) * 128;
-  const size_t budget = 227 * 1024 - 1024 - 512;
+  const size_t stage_bytes = (p.resident ? 0 : kW8TileBytes) + size_t(pair ? p.bt / 2 : p.bt) * 128;
+  const size_t kept = p.resident ? size_t(K / 128) * kW8TileBytes : 0;
+  const size_t budget = 227 * 1024 - 1024 - 512 - kept;
   p.nstages = int(std::min<size_t>(kW4A4MaxStages, budget / stage_bytes));
-  const size_t smem = 1024 + p.nstages * stage_bytes;
+  const size_t smem = 1024 + kept + p.nstages * stage_bytes;
 
   CUtensorMap tmw, tma;
   int rc = make_tmap_2d(&tmw, w8, 1, false, uint64_t(K), uint64_t(N), 128, 128, true);
