@@ -61,6 +61,7 @@ SIGNATURES = {
                                  c_void_p]),
     "asrq_bias_glu": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p]),
     "asrq_bias_affine_silu": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "asrq_argmax_rows": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int, c_void_p]),
     "asrq_half_step": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p]),
     "asrq_bias_add_transposed": (c_int, [c_void_p] * 4 + [c_int64, c_int64, c_int64, c_int, c_void_p]),
     "asrq_silu_mul": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p]),

@@ -46,6 +46,7 @@ int conv_elementwise(const void* in, const void* bias, const void* scale, const 
 int bias_add_transposed(const void* x, const void* conv, const void* bias, void* out, int64_t B, int64_t T, int64_t C, int dtype, cudaStream_t stream);
 int half_step(const void* x, const void* y, void* out, int64_t n, int dtype, cudaStream_t stream);
 int dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, int dtype, int sm_count, cudaStream_t stream);
+int argmax_rows(const void* y, long long* tok, long long* ids, const long long* pos, void* scratch, int64_t B, int64_t N, int dtype, cudaStream_t stream);
 int hadamard_quant_int4(const void* x, uint8_t* qa, float* sa, int64_t M, int64_t K, int hadamard, int dtype,
                         int out_int8, cudaStream_t stream);
 int w4a4_linear_tc(const void* x, const uint8_t* qw, const void* sw, const void* bias, void* y, int64_t M, int64_t N,
@@ -464,6 +465,21 @@ int asrq_bias_affine_silu(const void* in, const void* bias, const void* scale, c
   if (!scale || !shift) return fail(ASRQ_ERR_NULL, "asrq_bias_affine_silu: NULL pointer");
   if (B == 0 || T == 0) return ASRQ_OK;
   return conv_elementwise(in, bias, scale, shift, out, B, C, T, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_argmax_rows(const void* logits, int64_t* tokens, int64_t* ids, const int64_t* pos_device, void* scratch, int64_t B, int64_t N, int dtype,
+                     void* stream) {
+  last_error().clear();
+  if (!logits || !tokens || !scratch || (ids && !pos_device)) return fail(ASRQ_ERR_NULL, "asrq_argmax_rows: logits, tokens and scratch must not be NULL; ids needs pos_device");
+  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_argmax_rows: dtype %d", dtype);
+  if (B < 0 || B > 65535 || N <= 0 || N > (int64_t(1) << 30)) return fail(ASRQ_ERR_SHAPE, "asrq_argmax_rows: B=%lld N=%lld", (long long)B, (long long)N);
+  if (reinterpret_cast<uintptr_t>(scratch) % 8) return fail(ASRQ_ERR_ALIGN, "asrq_argmax_rows: scratch must be 8-byte aligned");
+  const DeviceFacts* f;
+  int rc;
+  if ((rc = device_facts(&f))) return rc;
+  if (B == 0) return ASRQ_OK;
+  return argmax_rows(logits, reinterpret_cast<long long*>(tokens), reinterpret_cast<long long*>(ids), reinterpret_cast<const long long*>(pos_device), scratch, B, N,
+                     dtype, static_cast<cudaStream_t>(stream));
 }
 
 int asrq_half_step(const void* x, const void* y, void* out, int64_t n, int dtype, void* stream) {

@@ -42,6 +42,64 @@ __device__ __forceinline__ uint4 ldg_stream16(const void* p) {
   return v;
 }
 
+// The next token of every row: the index of the largest logit (the first of equals; a NaN is larger than any number, as in torch),
+// in kArgmaxParts blocks per row that meet by one atomic maximum of (ordered value, ~index) and a counter; the last of a row
+// writes and leaves both at zero.  Bound: latency, some hundred KB per row from L2; the library's reduction in one block per row
+// took 8 to 23 us of a step, and a copy and an indexed copy followed it.
+constexpr int kArgmaxParts = 16;
+template <bool BF16, bool PAIRS>
+__global__ void __launch_bounds__(256)
+argmax_rows_kernel(const uint16_t* __restrict__ y, long long* __restrict__ tok, long long* __restrict__ ids, const long long* __restrict__ pos,
+                   unsigned long long* __restrict__ best, unsigned* __restrict__ arrived, int N) {
+  __shared__ unsigned long long part[8];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int row = blockIdx.y;
+  const uint16_t* src = y + size_t(row) * N;
+  auto ordered = [](uint32_t b) {  // monotone in the value; zeros equal; NaN above everything
+    if ((b & 0x7fffu) > (BF16 ? 0x7f80u : 0x7c00u)) return 0xffffu;
+    if (b == 0x8000u) b = 0u;
+    return (b & 0x8000u) ? (~b & 0xffffu) : (b | 0x8000u);
+  };
+  uint32_t top = 0, at = 0;  // every number's order is above zero
+  auto see = [&](uint32_t bits, int i) {
+    const uint32_t o = ordered(bits);
+    if (o > top) {
+      top = o;
+      at = uint32_t(i);
+    }
+  };
+  if (PAIRS) {
+    const int n2 = N / 2, lo = int((long long)n2 * blockIdx.x / kArgmaxParts), hi = int((long long)n2 * (blockIdx.x + 1) / kArgmaxParts);
+#pragma unroll 4
+    for (int i = lo + threadIdx.x; i < hi; i += 256) {
+      const uint32_t w = reinterpret_cast<const uint32_t*>(src)[i];
+      see(w & 0xffffu, 2 * i);
+      see(w >> 16, 2 * i + 1);
+    }
+  } else {
+    const int lo = int((long long)N * blockIdx.x / kArgmaxParts), hi = int((long long)N * (blockIdx.x + 1) / kArgmaxParts);
+    for (int i = lo + threadIdx.x; i < hi; i += 256) see(src[i], i);
+  }
+  unsigned long long key = (static_cast<unsigned long long>(top) << 32) | (top ? 0xffffffffu - at : 0u);
+  auto larger = [](unsigned long long a, unsigned long long b) { return a > b ? a : b; };
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) key = larger(key, __shfl_xor_sync(0xffffffffu, key, o));
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = key;
+  __syncthreads();
+  if (threadIdx.x) return;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) key = larger(key, part[i]);
+  atomicMax(best + row, key);
+  __threadfence();
+  if (atomicAdd(arrived + row, 1u) != kArgmaxParts - 1) return;
+  __threadfence();
+  const long long t = static_cast<long long>(0xffffffffu - uint32_t(atomicExch(best + row, 0ull)));
+  arrived[row] = 0u;
+  tok[row] = t;
+  if (ids) ids[*pos * gridDim.y + row] = t;
+}
+
 // x: M x K, w: N x K, y: M x N, all 16-bit of one type; K a multiple of 32; shared memory: head_smem(NT, K) bytes.
 // PER_SM: blocks that share an SM; AHEAD: K steps of weight loads in flight per warp.
 template <bool BF16, int NT, int PER_SM>
@@ -175,6 +233,26 @@ int dense_head(const void* x, const void* w, void* y, int64_t M, int64_t N, int6
   cfg.numAttrs = option(kOptNoPdl) ? 0 : 1;
   ASRQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<const uint16_t*>(x), static_cast<const uint16_t*>(w),
                                    static_cast<uint16_t*>(y), int(M), int(N), int(K)));
+  return ASRQ_OK;
+}
+
+// scratch: 16 bytes per row, zero between calls
+int argmax_rows(const void* y, long long* tok, long long* ids, const long long* pos, void* scratch, int64_t B, int64_t N, int dtype, cudaStream_t stream) {
+  unsigned long long* best = static_cast<unsigned long long*>(scratch);
+  unsigned* arrived = reinterpret_cast<unsigned*>(best + B);
+  const bool pairs = N % 2 == 0 && reinterpret_cast<uintptr_t>(y) % 4 == 0;
+  auto kern = dtype == ASRQ_BF16 ? (pairs ? argmax_rows_kernel<true, true> : argmax_rows_kernel<true, false>)
+                                 : (pairs ? argmax_rows_kernel<false, true> : argmax_rows_kernel<false, false>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kArgmaxParts, unsigned(B));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = option(kOptNoPdl) ? 0 : 1;
+  ASRQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<const uint16_t*>(y), tok, ids, pos, best, arrived, int(N)));
   return ASRQ_OK;
 }
 

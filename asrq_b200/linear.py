@@ -154,6 +154,16 @@ def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.
     return out
 
 
+def argmax_rows(logits: torch.Tensor, tokens: torch.Tensor, scratch: torch.Tensor, ids: torch.Tensor = None, pos: torch.Tensor = None) -> None:
+    """``tokens.copy_(logits.argmax(-1))`` for contiguous (B, N) 16-bit logits; with ``ids`` (steps, B) and ``pos`` (one int64 on the
+    device) also ``ids[pos] = tokens``.  ``scratch``: 2 B int64, zero before the first call, which every call leaves at zero."""
+    dt = _require_cuda_16bit(logits, "argmax_rows")
+    B, n = logits.shape
+    with _on_device(logits.device):
+        _lib.call("asrq_argmax_rows", logits.data_ptr(), tokens.data_ptr(), None if ids is None else ids.data_ptr(), None if pos is None else pos.data_ptr(),
+                  scratch.data_ptr(), B, n, dt, torch.cuda.current_stream(logits.device).cuda_stream)
+
+
 def _conv_step(fn: str, tensors, out: torch.Tensor, sizes) -> torch.Tensor:
     dt = _require_cuda_16bit(tensors[0], fn)
     with _on_device(out.device):

@@ -23,7 +23,7 @@ import torch.nn.functional as F
 
 from . import packing
 from .convert import linearq_from_linear
-from .linear import LinearQ, add_rmsnorm, decode_grouped_attention, dense_head, qk_norm_rope, silu_mul
+from .linear import LinearQ, add_rmsnorm, argmax_rows, decode_grouped_attention, dense_head, qk_norm_rope, silu_mul
 from .whisper import _cat_linearq
 
 try:
@@ -227,13 +227,17 @@ class Qwen3Engine:
         x, h = add_rmsnorm(x, att, L["ln2"], self.eps)
         return x, L["down"](silu_mul(L["gu"](h)))
 
+    @property
+    def own_attention(self) -> bool:
+        return self.hd == 128 and self.nq == 2 * self.nkv
+
     def _block_step(self, L, x, delta, kc, vc, mask):
         """:meth:`_block` for one new position per sequence, which lives on the device: q/k norm, rotary embedding, cache write
         and attention are one kernel for heads of 128 in pairs (Qwen3's), else the prompt's kernel and a masked attention."""
         B = x.shape[0]
         x, h = add_rmsnorm(x, delta, L["ln1"], self.eps)
         qkv = L["qkv"](h)
-        if self.hd == 128 and self.nq == 2 * self.nkv:
+        if self.own_attention:
             a = decode_grouped_attention(qkv, L["qn"], L["kn"], self.cos, self.sin, kc, vc, self.pos, self.nq, self.eps, self.hd ** -0.5)
         else:
             q = qk_norm_rope(qkv, L["qn"], L["kn"], self.cos, self.sin, kc, vc, self.pos, B, 1, self.nq, self.nkv, self.eps)
@@ -258,6 +262,7 @@ class Qwen3Engine:
         self.vc = [torch.zeros(B, self.nkv, max_len, self.hd, device=dev, dtype=dt) for _ in self.layers]
         self.pos = torch.zeros(1, device=dev, dtype=torch.long)
         self.tok = torch.zeros(B, device=dev, dtype=torch.long)
+        self.pick = torch.zeros(2 * B, device=dev, dtype=torch.long)  # scratch of the argmax, zero between steps
         self.last_logits = torch.zeros(B, self.head.shape[0], device=dev, dtype=dt)
         self._alloc_key = key
         self._graph = None
@@ -285,14 +290,13 @@ class Qwen3Engine:
         and advances self.pos."""
         B = self.B
         x = self.embed[self.tok]
-        mask = (torch.arange(self.max_len, device=self.device) <= self.pos).view(1, 1, 1, self.max_len)
+        mask = None if self.own_attention else (torch.arange(self.max_len, device=self.device) <= self.pos).view(1, 1, 1, self.max_len)
         delta = None
         for i, L in enumerate(self.layers):
             x, delta = self._block_step(L, x, delta, self.kc[i], self.vc[i], mask)
         h = self._final(x, delta)
-        logits = dense_head(h, self.head)
-        self.last_logits.copy_(logits)
-        self.tok.copy_(logits.argmax(-1))
+        dense_head(h, self.head, out=self.last_logits)
+        argmax_rows(self.last_logits, self.tok, self.pick)
         self.pos.add_(1)
 
     def decode(self, steps: int, use_graph: bool = True, keep_logits: bool = False):

@@ -30,7 +30,7 @@ import torch.nn.functional as F
 
 from . import packing
 from .convert import linearq_from_linear
-from .linear import LinearQ, add_layernorm, decode_cross_attention, decode_self_attention, dense_head
+from .linear import LinearQ, add_layernorm, argmax_rows, decode_cross_attention, decode_self_attention, dense_head
 
 try:  # the model classes need transformers; the engine does not
     from transformers.models.whisper.modeling_whisper import (WhisperAttention, WhisperConfig, WhisperDecoder,
@@ -395,6 +395,7 @@ class WhisperEngine:
         self.pos = torch.zeros(1, dtype=torch.long, device=dev)          # its position
         self.mask = torch.full((1, 1, 1, max_len), float("-inf"), device=dev, dtype=dt)  # 0 where a key exists
         self.out_ids = torch.zeros(max_len, batch, dtype=torch.long, device=dev)
+        self.pick = torch.zeros(2 * batch, dtype=torch.long, device=dev)  # scratch of the argmax, zero between steps
         self.logits = torch.empty(batch, self.head.shape[0], device=dev, dtype=dt)
         self._alloc_key = key
         self._graph = None
@@ -449,9 +450,7 @@ class WhisperEngine:
             x = L["fc2"].forward_fused(L["fc1"].forward_fused(h, gelu=True), residual=x)
         x = self.dec_ln(x).squeeze(1)
         dense_head(x, self.head, out=self.logits)
-        nxt = torch.argmax(self.logits, dim=-1)
-        self.out_ids.index_copy_(0, self.pos, nxt.unsqueeze(0))
-        self.tok.copy_(nxt)
+        argmax_rows(self.logits, self.tok, self.pick, self.out_ids, self.pos)
         self.pos.add_(1)
 
     def _ensure_graph(self):

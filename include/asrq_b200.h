@@ -176,6 +176,14 @@ int asrq_add_rmsnorm(const void* x, const void* delta, const void* gamma, float 
                      int64_t rows, int64_t dim, int dtype, void* stream);
 
 /*
+ * The greedy token of every row of logits (B x N): the index of the largest value, the first of equals, a NaN before any number.
+ * tokens: B int64.  ids (optional): also stored at ids[*pos_device * B + row].  scratch: 16 * B bytes, 8-byte aligned, zero before
+ * the first call and left at zero; calls that share it must be ordered.
+ */
+int asrq_argmax_rows(const void* logits, int64_t* tokens, int64_t* ids, const int64_t* pos_device, void* scratch, int64_t B, int64_t N, int dtype,
+                     void* stream);
+
+/*
  * The elementwise steps of a Conformer block's convolution module around its convolutions, contiguous tensors of `dtype`, every
  * step rounded to it as the sequence of modules rounds:
  *   asrq_bias_glu             in B x 2C x T -> out B x C x T: u = in + bias (2C), u[:, :C] * sigmoid(u[:, C:]);
