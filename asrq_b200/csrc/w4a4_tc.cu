@@ -88,7 +88,6 @@ struct W4A4TcParams {
   unsigned* status;
   long long* trace;  // builds with -DASRQ_TRACE: when not NULL, block `trace_block` records clock64() at pipeline milestones
   int M, N, K, groups, blocks_per_group, bt, nbuf, nstages, n_ftiles, n_ttiles, bf16, trace_block;
-  int resident;  // the feature tile's weights stay in shared memory over consecutive token tiles
 };
 
 constexpr int kW4A4MaxBufs = 4;
@@ -113,7 +112,8 @@ constexpr int kW4A4MaxResident = 8;  // K blocks of resident weights (128 KB)
 // from 16 KB + BT*128 to 16 KB + BT*64 per K block.  CTA 0 issues for both, its full[] barriers count
 // the bytes of both CTAs' loads, commits are multicast to both CTAs' empty[]/accf[] barriers, and the
 // drain warps of both CTAs arrive on CTA 0's acce[] barriers.
-template <bool DUMP, bool F8, int CG, int NCH, bool PAIR>
+// RES: the feature tile's weights stay in shared memory over consecutive token tiles (as a run-time switch it cost the other form 2 %).
+template <bool DUMP, bool F8, int CG, int NCH, bool PAIR, bool RES>
 __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUtensorMap* tma_p, const W4A4TcParams& p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * kW4A4MaxStages + 2 * kW4A4MaxBufs + kW4A4MaxResident];
@@ -122,7 +122,7 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
   const uint32_t raw_addr = tc::smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   const uint32_t bbytes = uint32_t(PAIR ? p.bt / 2 : p.bt) * 128u;  // this CTA's activation rows of a K block
-  const bool resident = !PAIR && p.resident != 0;
+  constexpr bool resident = !PAIR && RES;
   const uint32_t stage_bytes = (resident ? 0u : kW8TileBytes) + bbytes;
   const uint32_t rank = PAIR ? tc::cluster_ctarank() : 0u;
   const int worker = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x);     // tile-loop start and stride:
@@ -429,17 +429,17 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
   }
 }
 
-template <bool DUMP, bool F8, int CG, int NCH>
+template <bool DUMP, bool F8, int CG, int NCH, bool RES = false>
 __global__ void __launch_bounds__(w4a4_threads(CG), 1)
 w4a4_tc_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tma,
                const W4A4TcParams p) {
-  w4a4_tc_body<DUMP, F8, CG, NCH, false>(&tmw, &tma, p);
+  w4a4_tc_body<DUMP, F8, CG, NCH, false, RES>(&tmw, &tma, p);
 }
 template <bool DUMP, bool F8, int CG, int NCH>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(w4a4_threads(CG), 1)
 w4a4_tc_pair_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tma,
                     const W4A4TcParams p) {
-  w4a4_tc_body<DUMP, F8, CG, NCH, true>(&tmw, &tma, p);
+  w4a4_tc_body<DUMP, F8, CG, NCH, true, false>(&tmw, &tma, p);
 }
 
 // Token-tile width.  Two drain geometries: three column groups (BT a multiple of 48, up to 192, up to
@@ -527,14 +527,13 @@ int w4a4_gemm_int8(const uint8_t* w8, const uint8_t* a8, const float* sa, const 
   const int pair_env = option(kOptW4a4Pair);
   const bool pair = (N / 128) % 2 == 0 && sm_count >= 2 && pair_env != 0 && (pair_env == 1 || kW4A4PairDefault);
   const W4A4Tile tile = pair ? w4a4_pick_tile(M, N / 2, K, group_size, true, sm_count / 2) : w4a4_pick_tile(M, N, K, group_size, false, sm_count);
-  p.resident = tile.resident;
   p.bt = tile.bt;
   p.nbuf = 512 / p.bt >= 4 ? 4 : 2;  // even, so that a buffer always belongs to the same issuer
   p.n_ftiles = int(N / 128);
   p.n_ttiles = int((M + p.bt - 1) / p.bt);
   p.bf16 = dtype == ASRQ_BF16;
-  const size_t stage_bytes = (p.resident ? 0 : kW8TileBytes) + size_t(pair ? p.bt / 2 : p.bt) * 128;
-  const size_t kept = p.resident ? size_t(K / 128) * kW8TileBytes : 0;
+  const size_t stage_bytes = (tile.resident ? 0 : kW8TileBytes) + size_t(pair ? p.bt / 2 : p.bt) * 128;
+  const size_t kept = tile.resident ? size_t(K / 128) * kW8TileBytes : 0;
   const size_t budget = 227 * 1024 - 1024 - 512 - kept;
   p.nstages = int(std::min<size_t>(kW4A4MaxStages, budget / stage_bytes));
   const size_t smem = 1024 + kept + p.nstages * stage_bytes;
@@ -554,7 +553,10 @@ int w4a4_gemm_int8(const uint8_t* w8, const uint8_t* a8, const float* sa, const 
     else
       kern = fmt == 2 ? (acc_dump ? w4a4_tc_pair_kernel<true, true, 4, 2> : w4a4_tc_pair_kernel<false, true, 4, 2>)
                       : (acc_dump ? w4a4_tc_pair_kernel<true, false, 4, 2> : w4a4_tc_pair_kernel<false, false, 4, 2>);
-  } else if (tile.cg == 3)
+  } else if (tile.resident)
+    kern = fmt == 2 ? (acc_dump ? w4a4_tc_kernel<true, true, 4, 2, true> : w4a4_tc_kernel<false, true, 4, 2, true>)
+                    : (acc_dump ? w4a4_tc_kernel<true, false, 4, 2, true> : w4a4_tc_kernel<false, false, 4, 2, true>);
+  else if (tile.cg == 3)
     kern = fmt == 2 ? (acc_dump ? w4a4_tc_kernel<true, true, 3, 4> : w4a4_tc_kernel<false, true, 3, 4>)
                     : (acc_dump ? w4a4_tc_kernel<true, false, 3, 4> : w4a4_tc_kernel<false, false, 3, 4>);
   else
