@@ -401,12 +401,14 @@ qk_norm_rope_kernel(const uint16_t* __restrict__ qkv, const uint16_t* __restrict
   }
 }
 
-// kEpiVecs 16-byte vectors per thread in flight.  Bound: memory (with one vector at a time and the type, the activation and the
-// residual tested per element it ran at half of that).
-constexpr int kEpiVecs = 4;
+// 16-byte vectors per thread in flight: four for the activation, whose arithmetic they hide, in one pass per block; one for the
+// residual, whose three streams then move through memory together (12288 x 48000: 730 us a pass against 850 with four).  Bound:
+// memory (with the type, the activation and the residual tested per element the activation ran at half of that).
+constexpr int kEpiVecsResidual = 1, kEpiVecsActivation = 4;
 template <bool bf16, bool GELU, bool RES>
 __global__ void __launch_bounds__(256)
 epilogue16_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ residual, size_t n_vec) {
+  constexpr int kEpiVecs = RES ? kEpiVecsResidual : kEpiVecsActivation;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (size_t i0 = size_t(blockIdx.x) * (256 * kEpiVecs) + threadIdx.x; i0 < n_vec; i0 += size_t(gridDim.x) * (256 * kEpiVecs)) {
@@ -416,7 +418,7 @@ epilogue16_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ residua
       const size_t i = i0 + k * 256;
       if (i < n_vec) {
         a[k] = reinterpret_cast<const uint4*>(y)[i];
-        if (RES) r[k] = __ldcs(reinterpret_cast<const uint4*>(residual) + i);
+        if (RES) r[k] = reinterpret_cast<const uint4*>(residual)[i];
       }
     }
 #pragma unroll
@@ -533,7 +535,8 @@ int qk_norm_rope(const void* qkv, const void* qw, const void* kw, const void* co
 // y = act(y) / y = residual + y over M x N 16-bit elements (M*N a multiple of 8, pointers 16-byte aligned)
 int epilogue16_apply(void* y, const void* residual, int64_t M, int64_t N, int act, int dtype, int sm_count, cudaStream_t stream) {
   const size_t n_vec = size_t(M) * size_t(N) / 8;
-  const unsigned blocks = unsigned(std::max<size_t>(1, std::min<size_t>(size_t(sm_count) * 8, (n_vec + 256 * kEpiVecs - 1) / (256 * kEpiVecs))));
+  const size_t per_block = 256 * (residual ? kEpiVecsResidual : kEpiVecsActivation), all = (n_vec + per_block - 1) / per_block;
+  const unsigned blocks = unsigned(std::max<size_t>(1, std::min<size_t>(all, residual ? size_t(sm_count) * 8 : 0x7fffffffu)));
   auto run = [&](auto kern) { return launch_pdl(kern, dim3(blocks), dim3(256), stream, out_ptr(y), in_ptr(residual), n_vec); };
   const bool gelu = act == kActGelu;
   if (dtype == ASRQ_BF16) {
