@@ -277,8 +277,9 @@ row_norm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ del
 }
 
 // gu: rows x 2*inter (gate columns first, then up), out: rows x inter; eight elements per thread and row, kSiluRows rows in
-// flight.  Bound: memory; with one row at a time, a division to find it and exact quotients it took 2.2x the time of its bytes.
-// The exponential and the quotient are a few fp32 ulps off, under a rounding to 16 bits.
+// flight.  Bound: issue of the exponential and the IEEE quotient beside the memory (6144 wide, fp16: 64 rows 2.4 us, 16512 rows
+// 120 us or 5.07 TB/s; bf16 2.4 and 135).  __expf and __fdividef take 2.0 and 98 (2.1 and 106) but are tens of fp32 ulps off for
+// large negative gates, and the quotient is 0 from a divisor of 2^126 on: bf16 gates of -87.5 to -88.5 lost their result.
 constexpr int kSiluRows = 2;
 template <bool bf16>
 __global__ void __launch_bounds__(256)
@@ -305,7 +306,7 @@ silu_mul_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float gv = in16(uint16_t(gw[j] >> (16 * h)), bf16), uv = in16(uint16_t(uw[j] >> (16 * h)), bf16);
-          const float sv = in16(float_to_out16(__fdividef(gv, 1.f + __expf(-gv)), bf16), bf16);  // silu, rounded as the module rounds it
+          const float sv = in16(float_to_out16(gv / (1.f + expf(-gv)), bf16), bf16);  // silu, rounded as the module rounds it
           o2[h] = float_to_out16(sv * uv, bf16);
         }
         ow[j] = uint32_t(o2[0]) | (uint32_t(o2[1]) << 16);

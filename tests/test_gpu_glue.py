@@ -101,6 +101,22 @@ def test_silu_mul(rows, inter, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_silu_mul_every_gate(dtype):
+    """silu of every finite 16-bit gate down to -88.5 (below it exp(-gate) leaves fp32) against 64 bits.  With up = 1 the product
+    is exact, and in front of the one rounding to 16 bits the exponential (1 ulp), the sum and the quotient (half an ulp each)
+    leave at most 2 fp32 ulps; the interval allows 3."""
+    gate = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(dtype)
+    gate = gate[gate.isfinite() & (gate >= -88.5)]
+    gate = torch.cat((gate, gate.new_zeros(-gate.numel() % 8)))
+    out = asrq_b200.silu_mul(torch.cat((gate, torch.ones_like(gate))).to(DEV)).cpu().double()
+    ref = gate.double() / (1 + torch.exp(-gate.double()))
+    e = 3 * 2.0 ** -23
+    a, b = (ref * (1 - e)).to(dtype).double(), (ref * (1 + e)).to(dtype).double()
+    bad = (out < torch.minimum(a, b)) | (out > torch.maximum(a, b))
+    assert not bool(bad.any()), (int(bad.sum()), gate[bad][:8].tolist(), out[bad][:8].tolist(), ref[bad][:8].tolist())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("m,k,n", [(32, 1280, 51866), (1, 1280, 51866), (20, 2048, 4099), (32, 2048, 16384), (7, 96, 50), (32, 3200, 1000)])
 def test_dense_head(m, k, n, dtype):
     """The floating-point output head against fp32 on the same values (the reduction order differs from the library
