@@ -6,6 +6,11 @@
 // checks, the same allocation, the same C-ABI call -- for the ordinary case, and return None for everything else (wrong
 // types, CPU tensors, other devices, non-contiguous operands, empty inputs, tensor subclasses, dispatch modes), which the
 // Python code then handles and reports exactly as before.
+//
+// The interpreter lock is held while Python objects are looked at, and given up around the allocations and the C-ABI calls, as
+// torch's own operators and ctypes do: an allocation or a launch may wait (for memory, for room in the launch queue), and
+// neither the program's other threads nor a host function on the stream that needs the lock may have to wait with it.  What
+// the call uses is held by reference across it, since another thread may replace a layer's buffers or grow the workspace.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -51,8 +56,16 @@ inline bool int_of(PyObject* dict, PyObject* name, long long* out) {
   return true;
 }
 
+// Gives up the interpreter lock for a scope (an exception takes it again on its way out).
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 struct Layer {
-  const at::Tensor *weight, *scales, *zeros, *bias;  // bias NULL: none
+  at::Tensor weight, scales, zeros, bias;  // bias undefined: none
   PyObject* dict;
   long long k, n, bits, group;
 };
@@ -71,30 +84,32 @@ bool layer_of(PyObject* self, const c10::Device& dev, Layer* L) {
   };
   PyObject *w, *s, *z, *b;
   if (!operand(N.weight, &w) || !operand(N.scales, &s) || !operand(N.zeros, &z) || !operand(N.bias, &b)) return false;
-  L->weight = plain(w);
-  L->scales = plain(s);
-  L->zeros = plain(z);
-  L->bias = b == Py_None ? nullptr : plain(b);
-  if (!L->weight || !L->scales || !L->zeros || (b != Py_None && !L->bias)) return false;
-  if (L->weight->scalar_type() != at::kByte || L->scales->scalar_type() != at::kHalf || L->zeros->scalar_type() != at::kHalf) return false;
-  for (const at::Tensor* t : {L->weight, L->scales, L->zeros})
+  const at::Tensor *wt = plain(w), *st = plain(s), *zt = plain(z), *bt = plain(b);
+  if (!wt || !st || !zt || (b != Py_None && !bt)) return false;
+  if (wt->scalar_type() != at::kByte || st->scalar_type() != at::kHalf || zt->scalar_type() != at::kHalf) return false;
+  for (const at::Tensor* t : {wt, st, zt})
     if (t->device() != dev || !t->is_contiguous()) return false;
-  if (L->bias && (L->bias->scalar_type() != at::kHalf || L->bias->device() != dev)) return false;
+  if (bt && (bt->scalar_type() != at::kHalf || bt->device() != dev)) return false;
+  L->weight = *wt;
+  L->scales = *st;
+  L->zeros = *zt;
+  if (bt) L->bias = *bt;
   return int_of(d, N.in_features, &L->k) && int_of(d, N.out_features, &L->n) && int_of(d, N.bits, &L->bits) && int_of(d, N.group_size, &L->group);
 }
 
 // fp16 / bf16 activations on the current CUDA device, contiguous, at least one row
-bool activations(PyObject* o, const at::Tensor** x, int* dtype) {
-  *x = plain(o);
-  if (!*x || !(*x)->is_cuda() || (*x)->dim() < 1 || !(*x)->is_contiguous() || (*x)->numel() == 0) return false;
-  const auto st = (*x)->scalar_type();
+bool activations(PyObject* o, at::Tensor* x, int* dtype) {
+  const at::Tensor* t = plain(o);
+  if (!t || !t->is_cuda() || t->dim() < 1 || !t->is_contiguous() || t->numel() == 0) return false;
+  const auto st = t->scalar_type();
   if (st != at::kHalf && st != at::kBFloat16) return false;
+  *x = *t;
   *dtype = st == at::kHalf ? ASRQ_F16 : ASRQ_BF16;
-  return (*x)->device().index() == c10::cuda::current_device() && !modes_active();
+  return t->device().index() == c10::cuda::current_device() && !modes_active();
 }
 
 // The stream's workspace if it is there and large enough.
-bool workspace(int dev, cudaStream_t stream, size_t need, void** ptr, size_t* bytes) {
+bool workspace(int dev, cudaStream_t stream, size_t need, at::Tensor* ws) {
   PyObject* key = PyTuple_New(2);
   if (!key) return false;
   PyTuple_SET_ITEM(key, 0, PyLong_FromLong(dev));
@@ -103,8 +118,7 @@ bool workspace(int dev, cudaStream_t stream, size_t need, void** ptr, size_t* by
   Py_DECREF(key);
   const at::Tensor* t = plain(v);
   if (!t || size_t(t->numel()) < need) return false;
-  *ptr = t->data_ptr();
-  *bytes = size_t(t->numel());
+  *ws = *t;
   return true;
 }
 
@@ -128,40 +142,43 @@ PyObject* linearq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyErr_SetString(PyExc_TypeError, "linearq_forward(layer, input, residual, gelu)");
     return nullptr;
   }
-  const at::Tensor* x;
+  at::Tensor x;
   int dtype;
   Layer L;
-  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x->device(), &L) || (L.bits != 2 && L.bits != 4) || x->size(-1) != L.k) {
+  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x.device(), &L) || (L.bits != 2 && L.bits != 4) || x.size(-1) != L.k) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
-  const int64_t m = x->numel() / L.k;
-  const at::Tensor* res = nullptr;
+  const int64_t m = x.numel() / L.k;
+  at::Tensor res;
   if (a[2] != Py_None) {
-    res = plain(a[2]);
-    if (!res || res->scalar_type() != x->scalar_type() || res->device() != x->device() || res->numel() != m * L.n || !res->is_contiguous()) Py_RETURN_NONE;
+    const at::Tensor* r = plain(a[2]);
+    if (!r || r->scalar_type() != x.scalar_type() || r->device() != x.device() || r->numel() != m * L.n || !r->is_contiguous()) Py_RETURN_NONE;
+    res = *r;
   }
-  const bool gelu = a[3] == Py_True;
-  const int dev = x->device().index();
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
-  void* ws;
-  size_t ws_bytes;
-  if (!workspace(dev, stream, asrq_workspace_bytes(ASRQ_WS_LINEARQ, m, L.n, L.k), &ws, &ws_bytes)) {
+  const bool gelu = a[3] == Py_True, fused = res.defined() || gelu;
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+  at::Tensor ws;
+  if (!workspace(x.device().index(), stream, asrq_workspace_bytes(ASRQ_WS_LINEARQ, m, L.n, L.k), &ws)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;  // the Python path makes it
   }
-  at::Tensor y = output_like(*x, L.n);
-  g_calls.fetch_add(1, std::memory_order_relaxed);
-  const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
+  at::Tensor y;
   int rc;
-  if (!res && !gelu)
-    rc = asrq_linearq_a16(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(), bias,
-                          y.data_ptr(), m, L.n, L.k, int(L.group), dtype, ws, ws_bytes, stream);
-  else
-    rc = asrq_linearq_a16_fused(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(),
-                                bias, res ? res->data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype, gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE, ws,
-                                ws_bytes, stream);
-  if (rc) return failed(!res && !gelu ? "asrq_linearq_a16" : "asrq_linearq_a16_fused", rc);
+  {
+    Unlocked unlocked;
+    y = output_like(x, L.n);
+    g_calls.fetch_add(1, std::memory_order_relaxed);
+    const void* bias = L.bias.defined() ? L.bias.data_ptr() : nullptr;
+    if (!fused)
+      rc = asrq_linearq_a16(int(L.bits), x.data_ptr(), static_cast<const uint8_t*>(L.weight.data_ptr()), L.scales.data_ptr(), L.zeros.data_ptr(), bias,
+                            y.data_ptr(), m, L.n, L.k, int(L.group), dtype, ws.data_ptr(), size_t(ws.numel()), stream);
+    else
+      rc = asrq_linearq_a16_fused(int(L.bits), x.data_ptr(), static_cast<const uint8_t*>(L.weight.data_ptr()), L.scales.data_ptr(), L.zeros.data_ptr(),
+                                  bias, res.defined() ? res.data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype,
+                                  gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE, ws.data_ptr(), size_t(ws.numel()), stream);
+  }
+  if (rc) return failed(fused ? "asrq_linearq_a16_fused" : "asrq_linearq_a16", rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
 }
@@ -173,25 +190,26 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyErr_SetString(PyExc_TypeError, "linearqq_forward(layer, input)");
     return nullptr;
   }
-  const at::Tensor* x;
+  at::Tensor x;
   int dtype;
   Layer L;
-  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x->device(), &L) || x->size(-1) != L.k || L.group <= 0) {
+  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x.device(), &L) || x.size(-1) != L.k || L.group <= 0) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
   PyObject* had_o = PyDict_GetItemWithError(L.dict, N.hadamard);
   if (had_o != Py_True && had_o != Py_False) Py_RETURN_NONE;
   const int had = had_o == Py_True;
-  const int64_t m = x->numel() / L.k;
-  const int dev = x->device().index();
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
-  const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
-  void* ws;
-  size_t ws_bytes;
+  const int64_t m = x.numel() / L.k;
+  const int dev = x.device().index();
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+  const void* bias = L.bias.defined() ? L.bias.data_ptr() : nullptr;
+  at::Tensor ws, sc, y;
+  const char* fn;
+  int rc;
   // the activation codes and their scales: one scratch allocation (codes first, the scales at the next multiple of 256 bytes)
   auto scratch = [&](int64_t code_bytes) {
-    return at::detail::empty_cuda({(code_bytes + 255) / 256 * 256 + m * 4}, at::kByte, x->device(), std::nullopt);
+    return at::detail::empty_cuda({(code_bytes + 255) / 256 * 256 + m * 4}, at::kByte, x.device(), std::nullopt);
   };
   if (m >= 64 && L.n % 128 == 0 && L.k % 128 == 0 && L.group % 128 == 0 && L.k % L.group == 0) {
     PyObject* op = PyObject_GetAttr(a[0], N.operand);
@@ -200,37 +218,47 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const bool i8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "int8") == 0;
     // the prepared weight, if it was derived from this very buffer in this state
     PyObject *w8_o = PyDict_GetItemWithError(L.dict, N.w8), *key = PyDict_GetItemWithError(L.dict, N.w8_key);
-    const at::Tensor* w8 = plain(w8_o);
-    const bool fresh = (f8 || i8) && w8 && w8->device() == x->device() && key && PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 4 &&
-                       PyLong_AsVoidPtr(PyTuple_GET_ITEM(key, 0)) == L.weight->data_ptr() &&
-                       PyLong_AsLongLong(PyTuple_GET_ITEM(key, 1)) == (long long)L.weight->_version() && PyUnicode_Compare(PyTuple_GET_ITEM(key, 3), op) == 0;
+    const at::Tensor* w8_t = plain(w8_o);
+    const bool fresh = (f8 || i8) && w8_t && w8_t->device() == x.device() && key && PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 4 &&
+                       PyLong_AsVoidPtr(PyTuple_GET_ITEM(key, 0)) == L.weight.data_ptr() &&
+                       PyLong_AsLongLong(PyTuple_GET_ITEM(key, 1)) == (long long)L.weight._version() && PyUnicode_Compare(PyTuple_GET_ITEM(key, 3), op) == 0;
     Py_DECREF(op);
     if (PyErr_Occurred()) return nullptr;
-    if (!fresh || !workspace(dev, stream, 256, &ws, &ws_bytes)) Py_RETURN_NONE;
-    at::Tensor sc = scratch(m * L.k), y = output_like(*x, L.n);
+    if (!fresh || !workspace(dev, stream, 256, &ws)) Py_RETURN_NONE;
+    const at::Tensor w8 = *w8_t;
+    Unlocked unlocked;
+    sc = scratch(m * L.k);
+    y = output_like(x, L.n);
     uint8_t* a8 = static_cast<uint8_t*>(sc.data_ptr());
     float* sa = reinterpret_cast<float*>(a8 + (m * L.k + 255) / 256 * 256);
     g_calls.fetch_add(2, std::memory_order_relaxed);
-    int rc = (f8 ? asrq_hadamard_quant_f8 : asrq_hadamard_quant_int8)(x->data_ptr(), a8, sa, m, L.k, had, dtype, stream);
-    if (rc) return failed(f8 ? "asrq_hadamard_quant_f8" : "asrq_hadamard_quant_int8", rc);
-    rc = (f8 ? asrq_w4a4_gemm_f8 : asrq_w4a4_gemm_int8)(a8, sa, static_cast<const uint8_t*>(w8->data_ptr()), L.scales->data_ptr(), bias, y.data_ptr(), nullptr, m,
-                                                        L.n, L.k, int(L.group), dtype, ws, ws_bytes, stream);
-    if (rc) return failed(f8 ? "asrq_w4a4_gemm_f8" : "asrq_w4a4_gemm_int8", rc);
-    return THPVariable_Wrap(std::move(y));
+    fn = f8 ? "asrq_hadamard_quant_f8" : "asrq_hadamard_quant_int8";
+    rc = (f8 ? asrq_hadamard_quant_f8 : asrq_hadamard_quant_int8)(x.data_ptr(), a8, sa, m, L.k, had, dtype, stream);
+    if (!rc) {
+      fn = f8 ? "asrq_w4a4_gemm_f8" : "asrq_w4a4_gemm_int8";
+      rc = (f8 ? asrq_w4a4_gemm_f8 : asrq_w4a4_gemm_int8)(a8, sa, static_cast<const uint8_t*>(w8.data_ptr()), L.scales.data_ptr(), bias, y.data_ptr(), nullptr, m,
+                                                          L.n, L.k, int(L.group), dtype, ws.data_ptr(), size_t(ws.numel()), stream);
+    }
+  } else {
+    if (!workspace(dev, stream, asrq_workspace_bytes(ASRQ_WS_W4A4_GEMM, m, L.n, L.k), &ws)) {
+      if (PyErr_Occurred()) return nullptr;
+      Py_RETURN_NONE;
+    }
+    Unlocked unlocked;
+    sc = scratch(m * (L.k / 2));
+    y = output_like(x, L.n);
+    uint8_t* qa = static_cast<uint8_t*>(sc.data_ptr());
+    float* sa = reinterpret_cast<float*>(qa + (m * (L.k / 2) + 255) / 256 * 256);
+    g_calls.fetch_add(2, std::memory_order_relaxed);
+    fn = "asrq_hadamard_quant_int4";
+    rc = asrq_hadamard_quant_int4(x.data_ptr(), qa, sa, m, L.k, had, dtype, stream);
+    if (!rc) {
+      fn = "asrq_w4a4_gemm";
+      rc = asrq_w4a4_gemm(qa, sa, static_cast<const uint8_t*>(L.weight.data_ptr()), L.scales.data_ptr(), bias, y.data_ptr(), nullptr, m, L.n, L.k, int(L.group),
+                          dtype, ws.data_ptr(), size_t(ws.numel()), stream);
+    }
   }
-  if (!workspace(dev, stream, asrq_workspace_bytes(ASRQ_WS_W4A4_GEMM, m, L.n, L.k), &ws, &ws_bytes)) {
-    if (PyErr_Occurred()) return nullptr;
-    Py_RETURN_NONE;
-  }
-  at::Tensor sc = scratch(m * (L.k / 2)), y = output_like(*x, L.n);
-  uint8_t* qa = static_cast<uint8_t*>(sc.data_ptr());
-  float* sa = reinterpret_cast<float*>(qa + (m * (L.k / 2) + 255) / 256 * 256);
-  g_calls.fetch_add(2, std::memory_order_relaxed);
-  int rc = asrq_hadamard_quant_int4(x->data_ptr(), qa, sa, m, L.k, had, dtype, stream);
-  if (rc) return failed("asrq_hadamard_quant_int4", rc);
-  rc = asrq_w4a4_gemm(qa, sa, static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), bias, y.data_ptr(), nullptr, m, L.n, L.k, int(L.group),
-                      dtype, ws, ws_bytes, stream);
-  if (rc) return failed("asrq_w4a4_gemm", rc);
+  if (rc) return failed(fn, rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
 }

@@ -1,5 +1,8 @@
 """The module calls' native host path against the Python one: same bits, the same errors, and it sees replaced and
 modified buffers."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -79,3 +82,65 @@ def test_unusual_calls_go_the_python_way():
     q.group_size = 96                                   # the library's own refusal
     with pytest.raises(asrq_b200._lib.AsrqError):
         q(x.contiguous())
+
+
+def _in_threads(works):
+    errors = []
+
+    def guarded(work):
+        try:
+            work()
+        except BaseException as e:  # noqa: BLE001 (reported by the test's own thread)
+            errors.append(e)
+    threads = [threading.Thread(target=guarded, args=(w,)) for w in works]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors, errors
+
+
+def test_threads_on_streams_of_their_own():
+    q, qq = _layers(512, 256, True)
+    xs = [torch.randn(m, 512, device=DEV).half() for m in (1, 16, 33, 80)]
+    want = [(q(x), q.forward_fused(x, gelu=True), qq(x)) for x in xs]
+    torch.cuda.synchronize()
+
+    def work(x, w):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(200):
+                for got, ref in zip((q(x), q.forward_fused(x, gelu=True), qq(x)), w):
+                    assert torch.equal(got, ref)
+    _in_threads([lambda x=x, w=w: work(x, w) for x, w in zip(xs, want)])
+    asrq_b200.check_status()
+
+
+@pytest.mark.parametrize("quantized_activations", [False, True])
+def test_a_waiting_launch_leaves_the_interpreter_to_others(quantized_activations):
+    """A thread fills the launch queue of a stream that a timed kernel holds up for about two seconds, and waits in a launch for
+    room; this thread's Python goes on meanwhile."""
+    layer = _layers(512, 256, True)[quantized_activations]
+    x = torch.randn(80, 512, device=DEV).half()
+    stream = torch.cuda.Stream()
+    done, took = threading.Event(), []
+
+    def work():
+        with torch.cuda.stream(stream):
+            layer(x)                                    # workspace and prepared weight exist
+            stream.synchronize()
+            torch.cuda._sleep(int(4e9))
+            t0 = time.perf_counter()
+            for _ in range(4000):                       # several times what the queue holds
+                layer(x)
+            took.append(time.perf_counter() - t0)
+            done.set()
+    worker = threading.Thread(target=work)
+    worker.start()
+    gap, last = 0.0, time.perf_counter()
+    while not done.is_set() and worker.is_alive():
+        time.sleep(0.001)
+        now = time.perf_counter()
+        gap, last = max(gap, now - last), now
+    worker.join()
+    torch.cuda.synchronize()
+    assert took and took[0] > 1.0, took                 # the launches did have to wait
+    assert gap < 0.5, gap
+    asrq_b200.check_status()
