@@ -108,6 +108,13 @@ def load() -> ctypes.CDLL:
         raise ImportError(
             f"{LIB_PATH} or {NATIVE_PATH} is missing: build it with `python -m asrq_b200.build` (needs nvcc). "
             "asrq_b200 has no CPU or PyTorch fallback.")
+    from . import linear
+    if linear._native is None:  # built since the package was imported, or there and not to be loaded
+        try:
+            linear._load_native()
+        except ImportError as e:
+            raise ImportError(f"{NATIVE_PATH} does not load ({e}): build it again with `python -m asrq_b200.build` for this "
+                              "Python and torch") from e
     lib = ctypes.CDLL(LIB_PATH)
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)

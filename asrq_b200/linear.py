@@ -21,11 +21,21 @@ _CHECK = os.environ.get("ASRQ_B200_CHECK_STATUS", "0") == "1"
 # one scratch buffer per (device, stream): kernels on one stream run in order, so they can share it
 _workspaces: dict = {}
 
-try:  # the ordinary case of a module call in native code (csrc/host.cpp); built together with the library
-    from . import _native
-    _native.bind(_workspaces, _lib.check)
-except ImportError:  # not built: the first call raises (see _lib.load)
-    _native = None
+_native = None
+
+
+def _load_native() -> None:
+    """The ordinary case of a module call in native code (csrc/host.cpp); built together with the library."""
+    global _native
+    from . import _native as module
+    module.bind(_workspaces, _lib.check)
+    _native = module
+
+
+try:
+    _load_native()
+except ImportError:  # not built, or it does not load: packing works without it, the first call raises (see _lib.load)
+    pass
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:

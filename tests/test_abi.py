@@ -3,6 +3,8 @@ on the host before touching a device.  No compute calls here (no GPU needed)."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -116,3 +118,24 @@ def test_options_are_set_and_read_back():
     with pytest.raises(_lib.AsrqError) as e:
         _lib.set_option("no_such_switch", 1)
     assert e.value.code == -2
+
+
+def test_a_native_module_that_does_not_load_is_reported(tmp_path):
+    """The package imports (packing needs no native code) and the first call says what is wrong; built afterwards, it is taken up."""
+    src, pkg = os.path.dirname(_lib.LIB_PATH), tmp_path / "asrq_b200"
+    pkg.mkdir()
+    for f in os.listdir(src):
+        if f.endswith(".py") or f == os.path.basename(_lib.LIB_PATH):
+            os.symlink(os.path.join(src, f), pkg / f)
+    native = pkg / os.path.basename(_lib.NATIVE_PATH)
+    native.write_bytes(b"not a module")
+    code = ("import os, asrq_b200\n"
+            "from asrq_b200 import _lib, linear\n"
+            f"assert asrq_b200.__file__.startswith({str(pkg)!r})\n"
+            "try:\n    _lib.load()\n"
+            "except ImportError as e:\n    assert '_native.so does not load' in str(e), e\n"
+            "else:\n    raise SystemExit('a broken native module went unnoticed')\n"
+            f"os.remove({str(native)!r}); os.symlink({_lib.NATIVE_PATH!r}, {str(native)!r})\n"
+            "_lib.load(); assert linear._native is not None and _lib.CALLS == 0\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
