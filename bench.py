@@ -1329,11 +1329,11 @@ def main():
         args.warmup = 3
     args.warmup = max(args.warmup, 3) if args.impl == "ours" else args.warmup
 
+    if args.impl == "reference":
+        run_reference(args, int(os.environ.get("RANK", "0")))   # none of this library is imported, nor its native code mapped
+        return
     from asrq_b200 import dp
     rank, local_rank, world = dp.env_world()
-    if args.impl == "reference":
-        run_reference(args, rank)
-        return
     if not torch.cuda.is_available():
         raise SystemExit("bench.py: no CUDA device; the asrq_b200 path has no CPU fallback")
     torch.cuda.set_device(local_rank)

@@ -31,6 +31,18 @@ def test_reference_arm_line(workload, metric, unit):
     assert d["vs_baseline"] is None and d["higher_is_better"] is True and d["config"]["workload"].startswith(workload + ":")
 
 
+def test_reference_arm_maps_nothing_of_this_library():
+    """The arm that the library is compared with imports none of it: no module of the package, none of its shared objects."""
+    code = ("import os, runpy, sys\n"
+            "sys.argv = ['bench.py', '--impl', 'reference', '--workload', 'c1', '--steps', '1', '--warmup', '0']\n"
+            "runpy.run_path('bench.py', run_name='__main__')\n"
+            "mapped = {l.split()[-1] for l in open('/proc/self/maps') if 'asrq_b200' in l}\n"
+            "named = [m for m in sys.modules if m.split('.')[0] == 'asrq_b200']\n"
+            "assert not mapped and not named, (mapped, named)\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_ours_arm_refuses_to_run_without_a_gpu():
     import torch
     if torch.cuda.is_available():
