@@ -69,6 +69,8 @@ SIGNATURES = {
                                   c_int64, c_int64, c_int, c_int, c_int, c_int64, ctypes.c_float, c_int, c_void_p]),
     "asrq_decode_self_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int64, ctypes.c_float,
                                            c_int, c_void_p]),
+    "asrq_decode_self_attention_settled": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int64, ctypes.c_float,
+                                                   c_int, c_void_p]),
     "asrq_decode_cross_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int64, c_int64, ctypes.c_float,
                                             c_int, c_int, c_void_p]),
     "asrq_decode_grouped_attention": (c_int, [c_void_p] * 9 + [c_int64, c_int, c_int, c_int, c_int64, ctypes.c_float, ctypes.c_float, c_int,

@@ -35,7 +35,7 @@ int qk_norm_rope(const void* qkv, const void* qw, const void* kw, const void* co
                  long long pos_host, void* q_out, void* k_cache, void* v_cache, int64_t B, int64_t T, int nq, int nkv, int hd,
                  int64_t max_len, float eps, int dtype, cudaStream_t stream);
 int decode_self_attention(const void* qkv, void* kv, const long long* pos_dev, void* out, int64_t B, int H, int hd, int64_t max_len,
-                          float scale, int dtype, int sm_count, cudaStream_t stream);
+                          float scale, bool settled, int dtype, int sm_count, cudaStream_t stream);
 int decode_cross_attention(const void* q, const void* k, const void* v, void* out, int64_t B, int H, int hd, int64_t keys, int64_t row_stride,
                            float scale, bool settled, int dtype, int sm_count, cudaStream_t stream);
 int decode_grouped_attention(const void* qkv, const void* qw, const void* kw, const void* cos_t, const void* sin_t, const long long* pos_dev,
@@ -537,21 +537,32 @@ int asrq_qk_norm_rope(const void* qkv, const void* q_weight, const void* k_weigh
                       k_cache, v_cache, B, T, n_q_heads, n_kv_heads, head_dim, max_len, eps, dtype, static_cast<cudaStream_t>(stream));
 }
 
-int asrq_decode_self_attention(const void* qkv, void* kv_cache, const int64_t* pos_device, void* out, int64_t B, int n_heads,
-                               int head_dim, int64_t max_len, float scale, int dtype, void* stream) {
+static int self_attention(const char* who, const void* qkv, void* kv_cache, const int64_t* pos_device, void* out, int64_t B, int n_heads,
+                          int head_dim, int64_t max_len, float scale, bool settled, int dtype, void* stream) {
   last_error().clear();
-  if (!qkv || !kv_cache || !pos_device || !out) return fail(ASRQ_ERR_NULL, "asrq_decode_self_attention: no argument may be NULL");
-  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "asrq_decode_self_attention: dtype %d", dtype);
+  if (!qkv || !kv_cache || !pos_device || !out) return fail(ASRQ_ERR_NULL, "%s: no argument may be NULL", who);
+  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "%s: dtype %d", who, dtype);
   if (B < 0 || n_heads <= 0 || (head_dim != 64 && head_dim != 128) || max_len <= 0 || max_len > 512 || B * n_heads > (int64_t(1) << 28))
-    return fail(ASRQ_ERR_SHAPE, "asrq_decode_self_attention: B=%lld heads=%d head_dim=%d (64 or 128) max_len=%lld (at most 512)",
-                (long long)B, n_heads, head_dim, (long long)max_len);
-  if (!aligned16(kv_cache)) return fail(ASRQ_ERR_ALIGN, "asrq_decode_self_attention: kv_cache must be 16-byte aligned");
+    return fail(ASRQ_ERR_SHAPE, "%s: B=%lld heads=%d head_dim=%d (64 or 128) max_len=%lld (at most 512)", who, (long long)B, n_heads,
+                head_dim, (long long)max_len);
+  if (!aligned16(kv_cache)) return fail(ASRQ_ERR_ALIGN, "%s: kv_cache must be 16-byte aligned", who);
   const DeviceFacts* f;
   int rc;
   if ((rc = device_facts(&f))) return rc;
   if (B == 0) return ASRQ_OK;
   return decode_self_attention(qkv, kv_cache, reinterpret_cast<const long long*>(pos_device), out, B, n_heads, head_dim, max_len, scale,
-                               dtype, f->sm_count, static_cast<cudaStream_t>(stream));
+                               settled, dtype, f->sm_count, static_cast<cudaStream_t>(stream));
+}
+
+int asrq_decode_self_attention(const void* qkv, void* kv_cache, const int64_t* pos_device, void* out, int64_t B, int n_heads,
+                               int head_dim, int64_t max_len, float scale, int dtype, void* stream) {
+  return self_attention("asrq_decode_self_attention", qkv, kv_cache, pos_device, out, B, n_heads, head_dim, max_len, scale, false, dtype, stream);
+}
+
+int asrq_decode_self_attention_settled(const void* qkv, void* kv_cache, const int64_t* pos_device, void* out, int64_t B, int n_heads,
+                                       int head_dim, int64_t max_len, float scale, int dtype, void* stream) {
+  return self_attention("asrq_decode_self_attention_settled", qkv, kv_cache, pos_device, out, B, n_heads, head_dim, max_len, scale, true, dtype,
+                        stream);
 }
 
 int asrq_decode_cross_attention(const void* q, const void* k, const void* v, void* out, int64_t B, int n_heads, int head_dim, int64_t keys,

@@ -9,7 +9,8 @@
 // sequence took 8.5 us with one warp per item, each lane walking its keys' 128-byte rows alone.  Here an item is a block
 // of 4 or 8 warps, or a cluster of up to 8 such blocks when that fills the chip better.  HD / 8 lanes share a key (16 bytes
 // each), a warp has eight such loads of keys and eight of values in flight, and the first of them go out BEFORE the stream
-// dependency: everything below the new position was written by earlier steps.  Eight keys' partial scores are summed over the
+// dependency where the caller says that the cache is settled: in a decoder everything below the new position was written by
+// earlier steps.  Eight keys' partial scores are summed over the
 // lanes together by halving (7-8 shuffles instead of 24-32), after which every lane holds other keys' scores and the
 // exponentials are not computed twice.  Warps and blocks meet as (maximum, sum, weighted values), blocks through the shared
 // memory of the cluster's first.  fp32 scores, softmax and accumulation.
@@ -371,7 +372,7 @@ int launch_attn(const AttnParams& p, int64_t items, int64_t max_keys, int sm_cou
 }  // namespace
 
 int decode_self_attention(const void* qkv, void* kv, const long long* pos_dev, void* out, int64_t B, int H, int hd, int64_t max_len,
-                          float scale, int dtype, int sm_count, cudaStream_t stream) {
+                          float scale, bool settled, int dtype, int sm_count, cudaStream_t stream) {
   AttnParams p = {};
   p.qkv = static_cast<const uint16_t*>(qkv);
   p.k = static_cast<uint16_t*>(kv);
@@ -382,7 +383,7 @@ int decode_self_attention(const void* qkv, void* kv, const long long* pos_dev, v
   p.sh = (long long)max_len * hd;
   p.st = hd;
   p.q_row = 3 * H * hd;
-  p.early = 1;
+  p.early = settled;
   p.hkv = H;
   p.scale = scale;
   p.bf16 = dtype == ASRQ_BF16;

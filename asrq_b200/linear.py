@@ -150,16 +150,18 @@ def qk_norm_rope(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tens
     return q
 
 
-def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
+def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.Tensor, scale: float = 1.0, settled: bool = False) -> torch.Tensor:
     """Self-attention of one decoding step with the cache write: ``qkv`` (B, 3 * d) from a fused projection, ``kv_cache``
-    (2, B, heads, max_len, head_dim), ``pos`` a one-element int64 CUDA tensor (the new token's position).  Returns (B, d)."""
+    (2, B, heads, max_len, head_dim), ``pos`` a one-element int64 CUDA tensor (the new token's position).  Returns (B, d).
+    ``settled``: the position and the cache below it are older than the library's kernels just ahead on the stream (a decoder's
+    are), so they may be fetched while these still run."""
     dt = _require_cuda_16bit(qkv, "decode_self_attention")
     _, B, H, max_len, hd = kv_cache.shape
     q2 = qkv.reshape(B, 3 * H * hd)
     q2 = q2 if q2.is_contiguous() else q2.contiguous()
     out = torch.empty((B, H * hd), dtype=qkv.dtype, device=qkv.device)
     with _on_device(qkv.device):
-        _lib.call("asrq_decode_self_attention", q2.data_ptr(), kv_cache.data_ptr(), pos.data_ptr(), out.data_ptr(), B, H, hd, max_len,
+        _lib.call("asrq_decode_self_attention_settled" if settled else "asrq_decode_self_attention", q2.data_ptr(), kv_cache.data_ptr(), pos.data_ptr(), out.data_ptr(), B, H, hd, max_len,
                   float(scale), dt, torch.cuda.current_stream(qkv.device).cuda_stream)
     return out
 
@@ -221,7 +223,9 @@ def decode_cross_attention(q: torch.Tensor, kv: torch.Tensor, heads: int, scale:
 def decode_grouped_attention(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
                              k_cache: torch.Tensor, v_cache: torch.Tensor, pos: torch.Tensor, n_q: int, eps: float, scale: float) -> torch.Tensor:
     """:func:`qk_norm_rope` for one new position and the attention over the cache in one kernel: ``qkv`` (B, (n_q + 2 n_kv) * 128),
-    caches (B, n_kv, max_len, 128), ``pos`` a one-element int64 CUDA tensor; two query heads per key head.  Returns (B, n_q * 128)."""
+    caches (B, n_kv, max_len, 128), ``pos`` a one-element int64 CUDA tensor; two query heads per key head.  Returns (B, n_q * 128).
+    The position and the cache below it are fetched ahead of the stream dependency: behind :func:`qk_norm_rope` into the same
+    cache an ordinary kernel or copy has to come first."""
     dt = _require_cuda_16bit(qkv, "decode_grouped_attention")
     B, nkv, max_len, hd = k_cache.shape
     out = torch.empty((B, n_q * hd), dtype=qkv.dtype, device=qkv.device)

@@ -429,7 +429,7 @@ class WhisperEngine:
             qkv = L["qkv"](h)
             if self.fused_self_attention:
                 # this position's key and value into the cache and the attention over the cache: one kernel
-                a = decode_self_attention(qkv, self.kv_self[i], self.pos, 1.0 if L["q_folded"] else scaling).unsqueeze(1)
+                a = decode_self_attention(qkv, self.kv_self[i], self.pos, 1.0 if L["q_folded"] else scaling, settled=True).unsqueeze(1)
             else:
                 q = qkv[..., :self.d]
                 if not L["q_folded"]:

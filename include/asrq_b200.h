@@ -237,6 +237,14 @@ int asrq_decode_self_attention(const void* qkv, void* kv_cache, const int64_t* p
                                int head_dim, int64_t max_len, float scale, int dtype, void* stream);
 
 /*
+ * The same for a cache and a position that are settled: *pos_device and the cache below it are read ahead of the stream
+ * dependency.  Calls of this function and of the one above may follow each other at once; other kernels of this library that
+ * write the cache or the position need an ordinary kernel or copy in between (a decoding step has many).
+ */
+int asrq_decode_self_attention_settled(const void* qkv, void* kv_cache, const int64_t* pos_device, void* out, int64_t B, int n_heads,
+                                       int head_dim, int64_t max_len, float scale, int dtype, void* stream);
+
+/*
  * The cross-attention of one decoding step: one query per sequence and head against `keys` given keys and values.  q, out:
  * B x (n_heads * head_dim); key t of sequence b and head h at k + (b * keys + t) * row_stride + h * head_dim values, the value
  * likewise at v: what a fused key/value projection of the encoder states leaves ([k | v] rows: row_stride 2 * n_heads *
@@ -251,8 +259,9 @@ int asrq_decode_cross_attention(const void* q, const void* k, const void* v, voi
  * The self-attention of one decoding step of a grouped-query decoder with what surrounds it: per-head RMS norm of queries and
  * keys, rotary embedding, the cache write at *pos_device, and the attention over positions 0..pos.  qkv, the tables and the
  * caches as for asrq_qk_norm_rope with T = 1; out: B x (n_q_heads * head_dim).  n_q_heads = 2 n_kv_heads, head_dim 128.
- * The cache below the position is read ahead of the stream dependency: calls of this function may follow each other at once,
- * other kernels of this library that write the cache (asrq_qk_norm_rope) need an ordinary kernel or copy in between.
+ * The position, the cache below it and the tables' row of it are read ahead of the stream dependency: calls of this function
+ * may follow each other at once, other kernels of this library that write any of these (asrq_qk_norm_rope) need an ordinary
+ * kernel or copy in between.
  */
 int asrq_decode_grouped_attention(const void* qkv, const void* q_weight, const void* k_weight, const void* cos_table, const void* sin_table,
                                   const int64_t* pos_device, void* k_cache, void* v_cache, void* out, int64_t B, int n_q_heads, int n_kv_heads,

@@ -60,3 +60,25 @@ def test_grouped(B, nkv, pos, dtype):
     k, v = (t[:, :, :pos + 1].repeat_interleave(2, 1) for t in (kc, vc))
     ref = _softmax_attention(q, k, v, hd ** -0.5).reshape(B, nq * hd)
     assert (y.double() - ref).abs().max() < (2e-3 if dtype == torch.float16 else 1.6e-2)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_self_behind_the_kernel_that_wrote_the_cache(hd):
+    """A prompt's keys and values written by the library's own kernel, some waves of blocks long, directly ahead: the call waits
+    for them.  (With ``settled`` the caller says that it need not; the same bits when that is so.)"""
+    B, H, T, max_len = 32, 16, 200, 256
+    g = torch.Generator().manual_seed(hd)
+    prompt = torch.randn(B * T, 3 * H * hd, generator=g).half().cuda()
+    qkv = torch.randn(B, 3 * H * hd, generator=g).half().cuda()
+    w, pos = torch.ones(hd, dtype=torch.half, device="cuda"), torch.tensor([T], device="cuda")
+    cos = torch.randn(max_len, hd, generator=g).half().cuda()
+    kv = torch.zeros(2, B, H, max_len, hd, dtype=torch.half, device="cuda")
+    want = None
+    for _ in range(10):
+        kv.zero_()
+        linear.qk_norm_rope(prompt, w, w, cos, cos, kv[0], kv[1], 0, B, T, H, H, 1e-6)
+        y = linear.decode_self_attention(qkv, kv, pos, hd ** -0.5)
+        if want is None:
+            torch.cuda.synchronize()
+            want = linear.decode_self_attention(qkv, kv, pos, hd ** -0.5, settled=True)
+        assert torch.equal(y, want)
