@@ -34,13 +34,13 @@ PyObject* g_workspaces = nullptr;    // linear._workspaces: (device index, strea
 PyObject* g_check = nullptr;         // _lib.check(function name, status): raises AsrqError
 
 struct Names {
-  PyObject *buffers, *weight, *scales, *zeros, *bias, *in_features, *out_features, *bits, *group_size, *hadamard, *operand, *w8, *w8_key;
+  PyObject *buffers, *weight, *scales, *zeros, *bias, *in_features, *out_features, *bits, *group_size, *hadamard, *operand, *w8;
 } N;
 
 bool intern_names() {
   auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
   N = {s("_buffers"), s("weight"), s("scales"), s("zeros"), s("bias"), s("in_features"), s("out_features"), s("bits"), s("group_size"),
-       s("hadamard"), s("operand"), s("_w8"), s("_w8_key")};
+       s("hadamard"), s("operand"), s("_w8")};
   return !PyErr_Occurred();
 }
 
@@ -216,16 +216,21 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!op) return nullptr;
     const bool f8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "f8") == 0;
     const bool i8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "int8") == 0;
-    // the prepared weight, if it was derived from this very buffer in this state
-    PyObject *w8_o = PyDict_GetItemWithError(L.dict, N.w8), *key = PyDict_GetItemWithError(L.dict, N.w8_key);
-    const at::Tensor* w8_t = plain(w8_o);
-    const bool fresh = (f8 || i8) && w8_t && w8_t->device() == x.device() && key && PyTuple_Check(key) && PyTuple_GET_SIZE(key) == 4 &&
-                       PyLong_AsVoidPtr(PyTuple_GET_ITEM(key, 0)) == L.weight.data_ptr() &&
-                       PyLong_AsLongLong(PyTuple_GET_ITEM(key, 1)) == (long long)L.weight._version() && PyUnicode_Compare(PyTuple_GET_ITEM(key, 3), op) == 0;
+    // the prepared weight (linear._Prepared), if it was derived from this very buffer in this state
+    PyObject* prepared = PyDict_GetItemWithError(L.dict, N.w8);
+    at::Tensor w8;
+    if ((f8 || i8) && prepared && PyTuple_Check(prepared) && PyTuple_GET_SIZE(prepared) == 4) {
+      const at::Tensor *t = plain(PyTuple_GET_ITEM(prepared, 0)), *src = plain(PyTuple_GET_ITEM(prepared, 1));
+      if (t && src && t->device() == x.device() && src->device() == x.device() && src->data_ptr() == L.weight.data_ptr() &&
+          PyLong_AsLongLong(PyTuple_GET_ITEM(prepared, 2)) == (long long)L.weight._version() && PyUnicode_Compare(PyTuple_GET_ITEM(prepared, 3), op) == 0)
+        w8 = *t;
+    }
     Py_DECREF(op);
     if (PyErr_Occurred()) return nullptr;
-    if (!fresh || !workspace(dev, stream, 256, &ws)) Py_RETURN_NONE;
-    const at::Tensor w8 = *w8_t;
+    if (!w8.defined() || !workspace(dev, stream, 256, &ws)) {
+      if (PyErr_Occurred()) return nullptr;
+      Py_RETURN_NONE;
+    }
     Unlocked unlocked;
     sc = scratch(m * L.k);
     y = output_like(x, L.n);

@@ -389,6 +389,19 @@ class LinearQ(nn.Module):
                 f"group_size={self.group_size}, bias={self.bias is not None}")
 
 
+class _Prepared(tuple):
+    """(operand, an alias of the packed weight it was derived from, that weight's version, the operand's format).  The alias keeps
+    the weight's memory, so that an equal address means the same memory.  A copy of a layer, or a pickled one, derives its own."""
+    __slots__ = ()
+
+    def of(self, weight: torch.Tensor, operand: str) -> bool:
+        src = self[1]
+        return (src.data_ptr(), src.device, self[2], self[3]) == (weight.data_ptr(), weight.device, weight._version, operand)
+
+    def __reduce_ex__(self, protocol):
+        return type(None), ()
+
+
 class LinearQQ(LinearQ):
     """W4A4 linear: online Hadamard rotation + per-token int4 activations, grouped int4 weights.
 
@@ -450,15 +463,17 @@ class LinearQQ(LinearQ):
 
     def _prepared_weight(self) -> torch.Tensor:
         """8-bit operand form of ``weight`` (natural k order), derived on first use and whenever the
-        packed buffer is replaced or modified; not part of ``state_dict``."""
-        key = (self.weight.data_ptr(), self.weight._version, self.weight.device, self.operand)
-        if getattr(self, "_w8_key", None) != key:
-            n, k = self.out_features, self.in_features
-            w8 = torch.empty((n, k), dtype=torch.uint8, device=self.weight.device)
-            _lib.call(self._entry("prepare"), self.weight.data_ptr(), w8.data_ptr(), n, k,
-                      torch.cuda.current_stream(self.weight.device).cuda_stream)
-            self._w8, self._w8_key = w8, key
-        return self._w8
+        packed buffer is replaced or modified; not part of ``state_dict``.  (A change that the tensor's version
+        counter does not see, as through ``weight.data``, is not seen here either.)"""
+        weight, operand = self.weight, self.operand
+        stream = torch.cuda.current_stream(weight.device)
+        p = getattr(self, "_w8", None)
+        if type(p) is _Prepared and p.of(weight, operand):
+            return p[0]
+        w8 = torch.empty((self.out_features, self.in_features), dtype=torch.uint8, device=weight.device)
+        _lib.call(self._entry("prepare"), weight.data_ptr(), w8.data_ptr(), self.out_features, self.in_features, stream.cuda_stream)
+        self._w8 = _Prepared((w8, weight.detach(), weight._version, operand))
+        return w8
 
     def _tensor_core_ok(self, m: int) -> bool:
         n, k, g = self.out_features, self.in_features, self.group_size

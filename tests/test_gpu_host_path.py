@@ -1,5 +1,7 @@
 """The module calls' native host path against the Python one: same bits, the same errors, and it sees replaced and
 modified buffers."""
+import copy
+import pickle
 import threading
 import time
 
@@ -144,3 +146,22 @@ def test_a_waiting_launch_leaves_the_interpreter_to_others(quantized_activations
     assert took and took[0] > 1.0, took                 # the launches did have to wait
     assert gap < 0.5, gap
     asrq_b200.check_status()
+
+
+def test_prepared_weight_is_the_weights_own():
+    """The derived 8-bit operand goes with the memory of the packed weight, not with its address; a copied layer derives its own."""
+    x = torch.randn(80, 512, device=DEV).half()
+    a, b, c = (_layers(512, 256, True, seed=s)[1] for s in (0, 1, 2))
+    want_a, want_c = a(x), c(x)
+    for other in (copy.deepcopy(a), pickle.loads(pickle.dumps(a))):
+        assert torch.equal(other(x), want_a)
+    address = a.weight.data_ptr()
+    a.load_quantized_params(b.scales, b.zeros, b.weight.clone())   # gives the first weight back, no call with this one
+    held = []
+    for _ in range(64):                                            # the third weight at the first one's address, if that is free
+        held.append(c.weight.clone())
+        if held[-1].data_ptr() == address:
+            break
+    a.load_quantized_params(c.scales, c.zeros, held[-1])
+    a.bias = c.bias
+    assert torch.equal(a(x), want_c)
