@@ -472,7 +472,8 @@ class LinearQQ(LinearQ):
             return p[0]
         w8 = torch.empty((self.out_features, self.in_features), dtype=torch.uint8, device=weight.device)
         _lib.call(self._entry("prepare"), weight.data_ptr(), w8.data_ptr(), self.out_features, self.in_features, stream.cuda_stream)
-        self._w8 = _Prepared((w8, weight.detach(), weight._version, operand))
+        if not torch.cuda.is_current_stream_capturing():  # what is captured exists only once the graph has run
+            self._w8 = _Prepared((w8, weight.detach(), weight._version, operand))
         return w8
 
     def _tensor_core_ok(self, m: int) -> bool:

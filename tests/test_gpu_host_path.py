@@ -165,3 +165,16 @@ def test_prepared_weight_is_the_weights_own():
     a.load_quantized_params(c.scales, c.zeros, held[-1])
     a.bias = c.bias
     assert torch.equal(a(x), want_c)
+
+
+def test_prepared_weight_derived_under_capture():
+    """What a capture derives exists only once the graph has run: a call outside makes its own."""
+    qq = _layers(512, 256, True)[1]
+    x = torch.randn(80, 512, device=DEV).half()
+    want = _layers(512, 256, True)[1](x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = qq(x)
+    assert torch.equal(qq(x), want)
+    graph.replay()
+    assert torch.equal(y, want)
