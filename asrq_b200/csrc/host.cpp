@@ -122,6 +122,14 @@ bool workspace(int dev, cudaStream_t stream, size_t need, at::Tensor* ws) {
   return true;
 }
 
+bool contains(PyObject* streams, cudaStream_t stream) {
+  PyObject* handle = PyLong_FromVoidPtr(stream);
+  if (!handle) return false;
+  const int in = PySet_Contains(streams, handle);
+  Py_DECREF(handle);
+  return in == 1;
+}
+
 at::Tensor output_like(const at::Tensor& x, int64_t n) {
   c10::SmallVector<int64_t, 5> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = n;
@@ -216,13 +224,14 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!op) return nullptr;
     const bool f8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "f8") == 0;
     const bool i8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "int8") == 0;
-    // the prepared weight (linear._Prepared), if it was derived from this very buffer in this state
+    // the prepared weight (linear._Prepared), if it was derived from this very buffer in this state and this stream is behind that
     PyObject* prepared = PyDict_GetItemWithError(L.dict, N.w8);
     at::Tensor w8;
-    if ((f8 || i8) && prepared && PyTuple_Check(prepared) && PyTuple_GET_SIZE(prepared) == 4) {
+    if ((f8 || i8) && prepared && PyTuple_Check(prepared) && PyTuple_GET_SIZE(prepared) == 6) {
       const at::Tensor *t = plain(PyTuple_GET_ITEM(prepared, 0)), *src = plain(PyTuple_GET_ITEM(prepared, 1));
       if (t && src && t->device() == x.device() && src->device() == x.device() && src->data_ptr() == L.weight.data_ptr() &&
-          PyLong_AsLongLong(PyTuple_GET_ITEM(prepared, 2)) == (long long)L.weight._version() && PyUnicode_Compare(PyTuple_GET_ITEM(prepared, 3), op) == 0)
+          PyLong_AsLongLong(PyTuple_GET_ITEM(prepared, 2)) == (long long)L.weight._version() && PyUnicode_Compare(PyTuple_GET_ITEM(prepared, 3), op) == 0 &&
+          contains(PyTuple_GET_ITEM(prepared, 4), stream))
         w8 = *t;
     }
     Py_DECREF(op);

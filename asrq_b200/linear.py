@@ -390,8 +390,9 @@ class LinearQ(nn.Module):
 
 
 class _Prepared(tuple):
-    """(operand, an alias of the packed weight it was derived from, that weight's version, the operand's format).  The alias keeps
-    the weight's memory, so that an equal address means the same memory.  A copy of a layer, or a pickled one, derives its own."""
+    """(operand, an alias of the packed weight it was derived from, that weight's version, the operand's format, the streams that
+    are ordered behind the derivation, its event).  The alias keeps the weight's memory, so that an equal address means the same
+    memory; another stream waits for the event once.  A copy of a layer, or a pickled one, derives its own."""
     __slots__ = ()
 
     def of(self, weight: torch.Tensor, operand: str) -> bool:
@@ -467,13 +468,17 @@ class LinearQQ(LinearQ):
         counter does not see, as through ``weight.data``, is not seen here either.)"""
         weight, operand = self.weight, self.operand
         stream = torch.cuda.current_stream(weight.device)
+        capturing = torch.cuda.is_current_stream_capturing()
         p = getattr(self, "_w8", None)
         if type(p) is _Prepared and p.of(weight, operand):
+            if stream.cuda_stream not in p[4] and not capturing:
+                stream.wait_event(p[5])
+                p[4].add(stream.cuda_stream)
             return p[0]
         w8 = torch.empty((self.out_features, self.in_features), dtype=torch.uint8, device=weight.device)
         _lib.call(self._entry("prepare"), weight.data_ptr(), w8.data_ptr(), self.out_features, self.in_features, stream.cuda_stream)
-        if not torch.cuda.is_current_stream_capturing():  # what is captured exists only once the graph has run
-            self._w8 = _Prepared((w8, weight.detach(), weight._version, operand))
+        if not capturing:  # what is being captured exists only once the graph has run: its own calls derive it again
+            self._w8 = _Prepared((w8, weight.detach(), weight._version, operand, {stream.cuda_stream}, stream.record_event()))
         return w8
 
     def _tensor_core_ok(self, m: int) -> bool:

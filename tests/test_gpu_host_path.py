@@ -178,3 +178,22 @@ def test_prepared_weight_derived_under_capture():
     assert torch.equal(qq(x), want)
     graph.replay()
     assert torch.equal(y, want)
+
+
+def test_prepared_weight_on_another_stream():
+    """A stream that did not derive the operand waits for the one that did."""
+    x = torch.randn(80, 512, device=DEV).half()
+    want = _layers(512, 256, True)[1](x)
+    qq = _layers(512, 256, True)[1]
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(two):
+        _layers(512, 256, True)[1](x)                              # this stream's workspace exists
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(int(2e8))                                # about a tenth of a second
+        qq(x)
+    with torch.cuda.stream(two):
+        first, second = qq(x), qq(x)                               # by the Python path, then by the native one
+    torch.cuda.synchronize()
+    assert torch.equal(first, want) and torch.equal(second, want)
+    asrq_b200.check_status()
