@@ -20,6 +20,7 @@ _CHECK = os.environ.get("ASRQ_B200_CHECK_STATUS", "0") == "1"
 
 # one scratch buffer per (device, stream): kernels on one stream run in order, so they can share it
 _workspaces: dict = {}
+_outgrown: list = []  # earlier, smaller ones: a captured graph may hold their address
 
 _native = None
 
@@ -42,6 +43,9 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
+        if ws is not None:
+            _outgrown.append(ws)
+            nbytes = max(nbytes, 2 * ws.numel())  # what is kept stays below what is in use
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
         _workspaces[key] = ws
     return ws

@@ -197,3 +197,20 @@ def test_prepared_weight_on_another_stream():
     torch.cuda.synchronize()
     assert torch.equal(first, want) and torch.equal(second, want)
     asrq_b200.check_status()
+
+
+def test_a_workspace_that_was_outgrown_stays():
+    """A captured graph holds the address of the workspace that its stream had: that memory is given to nobody else when a
+    wider layer needs more, and what is kept is bounded by what is in use."""
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        key = (torch.cuda.current_device(), stream.cuda_stream)
+        linear._workspaces.pop(key, None)
+        small = linear._workspace(torch.device(DEV), 1 << 20)
+        address, kept = small.data_ptr(), len(linear._outgrown)
+        del small
+        for n in (3 << 20, 9 << 20, 10 << 20, 30 << 20):
+            linear._workspace(torch.device(DEV), n)
+        others = [torch.empty(1 << 20, dtype=torch.uint8, device=DEV) for _ in range(64)]
+        assert all(t.data_ptr() != address for t in others)
+        assert sum(t.numel() for t in linear._outgrown[kept:]) <= linear._workspaces[key].numel()
