@@ -19,6 +19,8 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -279,6 +281,27 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 
 PyObject* calls(PyObject*, PyObject*) { return PyLong_FromLongLong(g_calls.load(std::memory_order_relaxed)); }
 
+// zeros_now(bytes, device) -> uint8 tensor that is zero on return, also while a stream is under capture: zeros made on that stream
+// would be the graph's, there only once it has run, in memory of the graph's.
+PyObject* zeros_now(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
+  long long bytes;
+  int device;
+  if (!PyArg_ParseTuple(args, "Li", &bytes, &device)) return nullptr;
+  at::Tensor t;
+  {
+    Unlocked unlocked;
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    const c10::cuda::CUDAStream side = c10::cuda::getStreamFromPool(false, c10::DeviceIndex(device));
+    c10::cuda::CUDAStreamGuard guard(side);
+    t = at::detail::empty_cuda({bytes}, at::kByte, c10::Device(c10::kCUDA, c10::DeviceIndex(device)), std::nullopt);
+    C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, size_t(bytes), side.stream()));
+    C10_CUDA_CHECK(cudaStreamSynchronize(side.stream()));
+  }
+  return THPVariable_Wrap(std::move(t));
+  END_HANDLE_TH_ERRORS
+}
+
 // bind(workspaces dict, check function)
 PyObject* bind(PyObject*, PyObject* args) {
   PyObject *ws, *check;
@@ -296,6 +319,7 @@ PyMethodDef kMethods[] = {
     {"linearq_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linearq_forward)), METH_FASTCALL, nullptr},
     {"linearqq_forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linearqq_forward)), METH_FASTCALL, nullptr},
     {"calls", calls, METH_NOARGS, nullptr},
+    {"zeros_now", zeros_now, METH_VARARGS, nullptr},
     {"bind", bind, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

@@ -46,7 +46,8 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
         if ws is not None:
             _outgrown.append(ws)
             nbytes = max(nbytes, 2 * ws.numel())  # what is kept stays below what is in use
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        from . import _native as native  # (not the switch between the two call paths above)
+        ws = native.zeros_now(max(nbytes, 1 << 20), device.index)
         _workspaces[key] = ws
     return ws
 

@@ -214,3 +214,29 @@ def test_a_workspace_that_was_outgrown_stays():
         others = [torch.empty(1 << 20, dtype=torch.uint8, device=DEV) for _ in range(64)]
         assert all(t.data_ptr() != address for t in others)
         assert sum(t.numel() for t in linear._outgrown[kept:]) <= linear._workspaces[key].numel()
+
+
+def test_a_workspace_made_under_capture():
+    """Two layers captured one after the other on a stream that has no workspace yet: the second graph runs without the first
+    ever having run.  (Scales at an odd address take the kernel that counts in the workspace.)"""
+    q = _layers(2048, 256, False)[0]
+    q.scales = torch.cat((q.scales.new_zeros(1), q.scales.flatten()))[1:].view_as(q.scales)
+    x = torch.randn(1, 2048, device=DEV).half()
+    want = q(x)
+    stream = torch.cuda.Stream()
+    linear._workspaces.pop((torch.cuda.current_device(), stream.cuda_stream), None)
+    first = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(first, stream=stream):
+        torch.full((1 << 20,), 255, dtype=torch.uint8, device=DEV)     # what the graphs' memory holds then
+    first.replay()
+    torch.cuda.synchronize()
+    graphs, ys = [torch.cuda.CUDAGraph() for _ in range(2)], []
+    for graph in graphs:
+        with torch.cuda.graph(graph, stream=stream, pool=first.pool()):
+            ys.append(q(x))
+    ws = linear._workspaces[(torch.cuda.current_device(), stream.cuda_stream)]
+    assert not bool(ws[:256 + 4 * 4096].any())                     # status and counters
+    for y, graph in zip(ys[::-1], graphs[::-1]):
+        graph.replay()
+        assert torch.equal(y, want)
+    asrq_b200.check_status()
