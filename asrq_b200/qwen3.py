@@ -24,7 +24,7 @@ import torch.nn.functional as F
 from . import packing
 from .convert import linearq_from_linear
 from .linear import LinearQ, add_rmsnorm, argmax_rows, decode_grouped_attention, dense_head, qk_norm_rope, silu_mul
-from .whisper import _cat_linearq
+from .whisper import _baked_in, _cat_linearq, _same
 
 try:
     from transformers.models.qwen3.modeling_qwen3 import (Qwen3Attention, Qwen3Config, Qwen3DecoderLayer,
@@ -141,7 +141,6 @@ class Qwen3Engine:
         self.eps = config.rms_norm_eps
         self.layers: List[dict] = []
         self._graph = None
-        self._graph_key = None
 
     # ---- construction -------------------------------------------------------------------------
     def _rotary_table(self, max_len: int):
@@ -252,7 +251,7 @@ class Qwen3Engine:
     # ---- prefill / decode -------------------------------------------------------------------------
     def _alloc(self, B: int, max_len: int):
         """Static state for a batch size and a maximal length; kept (with the captured graph) across calls."""
-        key = (B, max_len)
+        key = (B, max_len, self.head.shape[0])
         if getattr(self, "_alloc_key", None) == key:
             return
         dev, dt = self.device, self.dtype
@@ -303,7 +302,8 @@ class Qwen3Engine:
         """Runs ``steps`` further tokens after :meth:`prefill`; returns ids (B, steps) [and logits (steps, B, V)]."""
         ids = torch.empty(steps, self.B, dtype=torch.long, device=self.device)
         lg = torch.empty(steps, self.B, self.head.shape[0], dtype=self.dtype, device=self.device) if keep_logits else None
-        if use_graph and self._graph is None:
+        ops = _baked_in(self.layers + [self.norm, self.embed, self.head, self.eps]) if use_graph else []
+        if use_graph and not (self._graph is not None and _same(ops, self._graph_ops)):
             st = torch.cuda.Stream(self.device)
             st.wait_stream(torch.cuda.current_stream(self.device))
             tok0, pos0 = self.tok.clone(), self.pos.clone()
@@ -318,7 +318,7 @@ class Qwen3Engine:
             torch.cuda.current_stream(self.device).wait_stream(st)
             self.tok.copy_(tok0)
             self.pos.copy_(pos0)
-            self._graph = g
+            self._graph, self._graph_ops = g, ops
         for s in range(steps):
             if use_graph:
                 self._graph.replay()

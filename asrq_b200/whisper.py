@@ -173,6 +173,25 @@ def _cat_linearq(parts: List[LinearQ]) -> LinearQ:
     return f
 
 
+def _baked_in(values) -> list:
+    """Everything of an engine's operands that a captured step holds the address or value of."""
+    out = []
+    for v in values:
+        if isinstance(v, dict):
+            out += _baked_in(v.values())
+        elif isinstance(v, LinearQ):
+            out += [v._buffers.get(n, v.__dict__.get(n)) for n in ("weight", "scales", "zeros", "bias")] + [v.bits, v.group_size]
+        elif isinstance(v, _Norm):
+            out += [v.w, v.b, v.eps]
+        else:
+            out.append(v)
+    return out
+
+
+def _same(a: list, b: list) -> bool:
+    return len(a) == len(b) and all(x is y or (type(x) in (bool, int, float) and x == y) for x, y in zip(a, b))
+
+
 class _Norm:
     """Layer norm through the library's kernel (one launch; fp32 statistics, 16-bit in and out)."""
     __slots__ = ("w", "b", "eps")
@@ -228,7 +247,6 @@ class WhisperEngine:
         self.enc_layers: List[dict] = []
         self.dec_layers: List[dict] = []
         self._graph = None
-        self._graph_key = None
 
     # ---- construction -------------------------------------------------------------------------
     @classmethod
@@ -375,7 +393,7 @@ class WhisperEngine:
 
     # ---- decoder ------------------------------------------------------------------------------
     def _alloc(self, batch: int, src_len: int, max_len: int):
-        key = (batch, src_len, max_len)
+        key = (batch, src_len, max_len, self.head.shape[0])
         if getattr(self, "_alloc_key", None) == key:
             return
         dev, dt, nl = self.device, self.dtype, len(self.dec_layers)
@@ -454,7 +472,9 @@ class WhisperEngine:
         self.pos.add_(1)
 
     def _ensure_graph(self):
-        if self._graph is not None:
+        ops = _baked_in(self.dec_layers + [self.embed, self.dec_pos, self.dec_ln, self.head, self.fused_self_attention, self.cross_kv_views,
+                                           self.own_cross_attention_items])
+        if self._graph is not None and _same(ops, self._graph_ops):
             return
         # warm-up on a side stream (lazy initialisation inside libraries must not happen under capture),
         # then capture; the buffers are reset by generate() before every use
@@ -470,7 +490,7 @@ class WhisperEngine:
             with torch.cuda.graph(g, stream=side):
                 self._step()
         torch.cuda.current_stream(self.device).wait_stream(side)
-        self._graph = g
+        self._graph, self._graph_ops = g, ops
 
     @torch.no_grad()
     def decode(self, enc: torch.Tensor, steps: int, start_token: Optional[int] = None, use_graph: bool = True,

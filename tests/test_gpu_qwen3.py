@@ -71,3 +71,23 @@ def test_engine_random_init_qwen3_1p7b_widths():
     b = eng.generate(emb, 5).clone()
     assert a.shape == (64, 5) and torch.equal(a, b)
     asrq_b200.check_status()
+
+
+def test_engine_captures_again_for_replaced_operands():
+    """The captured step is replayed only while the weights are the ones that it was captured with."""
+    cfg, fm, q = toy_models()
+    eng = Q.Qwen3Engine.from_model(q.half().to(DEV))
+    emb = fm.model.embed_tokens(_inputs(cfg, batch=4, T=7)).detach().half().to(DEV)
+    eng.generate(emb, 4)
+    first, held = eng._graph, (eng.head, eng.layers[0]["o"].weight)
+    eng.generate(emb, 4)
+    assert eng._graph is first
+    o = eng.layers[0]["o"]
+    for change in (lambda: setattr(eng, "head", eng.head.flip(0).contiguous()),
+                   lambda: o.load_quantized_params(o.scales, o.zeros, o.weight.flip(0).contiguous())):
+        change()
+        want = eng.generate(emb, 4, use_graph=False).clone(), eng.last_logits.clone()
+        got = eng.generate(emb, 4).clone(), eng.last_logits.clone()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert len(held) == 2
+    asrq_b200.check_status()

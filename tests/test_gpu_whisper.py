@@ -89,3 +89,22 @@ def test_engine_random_init_large_width_runs_and_is_deterministic():
     c = eng.generate(x[:2], steps=8)
     assert torch.equal(c, a[:2])
     asrq_b200.check_status()
+
+
+def test_engine_captures_again_for_replaced_operands():
+    """The captured step is replayed only while the weights are the ones that it was captured with."""
+    cfg, m, x, ids, logits, enc = _model()
+    eng = W.WhisperEngine.from_model(m)
+    eng.generate(x, steps=4)
+    first, held = eng._graph, (eng.head, eng.dec_layers[0]["fc1"].weight)
+    eng.generate(x, steps=4)
+    assert eng._graph is first
+    for change in (lambda: setattr(eng, "head", eng.head.flip(0).contiguous()),
+                   lambda: eng.dec_layers[0]["fc1"].load_quantized_params(eng.dec_layers[0]["fc1"].scales, eng.dec_layers[0]["fc1"].zeros,
+                                                                          eng.dec_layers[0]["fc1"].weight.flip(0).contiguous())):
+        change()
+        want = eng.generate(x, steps=4, use_graph=False).clone(), eng.logits.clone()
+        got = eng.generate(x, steps=4).clone(), eng.logits.clone()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert len(held) == 2
+    asrq_b200.check_status()
