@@ -8,9 +8,12 @@
 //   * a block owns ONE work item -- a tile of 128 features x BT tokens and a part of K.  Its activation tiles and packed
 //     weights pass through a ring of stages in shared memory, which for decode batches holds all of them at once;
 //   * it triggers its dependents as its first instruction and is small enough (448 threads, <= 73
-//     registers, < 113 KB) for two launches to share an SM.  Packed weights are fetched by TMA and the
-//     first three K blocks are dequantised BEFORE griddepcontrol.wait: weights do not depend on the
-//     kernel before, so the next launch's weight traffic and unpacking run under this launch's tail;
+//     registers) for two blocks to share an SM where the plan's shared memory allows (up to 112 KB: 1280
+//     inputs at up to 32 tokens 73-105 KB, 2048 -> 2048 at 64 tokens 97).  Larger plans have the SM to themselves
+//     (64 tokens: 2048 -> 4096 145 KB, 2048 -> 6144 181, 2048 -> 12288 217) and the next launch takes the SMs that
+//     this one leaves idle or is done with.  Packed weights are fetched by TMA and the first three K blocks are
+//     dequantised BEFORE griddepcontrol.wait: weights do not depend on the kernel before, so the next launch's
+//     weight traffic and unpacking run under this launch's tail where it has an SM by then;
 //   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32 to 256 TMEM columns)
 //     are fetched, as many as there are stages at once; tcgen05.mma kind::f16 128 x BT x 16, fp32 accumulator in tensor memory;
 //   * the K parts of a tile are a thread-block cluster and meet in distributed shared memory: every block leaves its
@@ -361,7 +364,7 @@ int skinny_capacity(int split, size_t smem) {
 // Token tile and K parts: the pair with the least estimated time among those whose blocks run in one wave.  The estimate (us)
 // follows the measurements of 17 to 1500 tokens on eight layer shapes: 4 for launch, first fetches and stores, 0.34 per K block
 // (dequantisation and its hand-over; the MMAs of 256 columns hide behind it), 0.011 per column of the tile for its way out of
-// tensor memory, 0.6 for the clusters' two barriers.
+// tensor memory, 0.6 for the clusters' two barriers.  It has no term for two blocks on an SM: no plan counts on a second one.
 bool skinny_search(int64_t M, int64_t N, int64_t K, int sm_count, SkinnyPlan* pl) {
   const int64_t nft = N / 128, nkb = K / 64;
   pl->us = 1e30;

@@ -17,8 +17,9 @@ pytestmark = pytest.mark.gpu
     (65, 1280, 1280, 4), (96, 2048, 2048, 4), (97, 1280, 3840, 2), (128, 1280, 5120, 4), (128, 64, 128, 4),
     (20, 6144, 2048, 4), (64, 6144, 2048, 4),   # six parts of sixteen
     (31, 8192, 128, 4),    # eight parts of sixteen
-    (24, 2048, 12288, 4),  # more tiles than one wave takes: the persistent kernel
-    (65, 2048, 12288, 4),
+    (24, 2048, 12288, 4),  # one part, 32 K blocks through a ring of sixteen stages
+    (65, 2048, 12288, 4), (128, 2048, 12288, 2),   # of eleven and of eight
+    (24, 256, 19200, 4), (128, 128, 19072, 2),     # 150 and 149 feature tiles, more than one wave: the other kernels
     (129, 1280, 1280, 4), (257, 5120, 1280, 4), (300, 6144, 2048, 2),   # several token tiles; stages used many times
     (511, 2048, 2048, 4), (1000, 5120, 1280, 4), (1300, 6144, 256, 4), (2048, 5120, 256, 2),
 ])
