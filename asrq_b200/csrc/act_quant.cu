@@ -218,9 +218,12 @@ quant_int4_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, floa
 // Values live as pairs, so every butterfly but the one inside the pair is a packed fp32 add and a packed subtract (add.f32x2 /
 // fma.f32x2) on two pairs.  Rows of the transpose are padded by four floats: its 4-byte writes and 16-byte reads are free of bank
 // conflicts.
-// Bound: instruction issue (about 500 clocks per token of 4096 and SM, 110 per token of 1024) as long as enough warps hide the
-// latencies.  One warp per token of 4096 (128 values a lane, nine warps per SM, 41 KB of straight-line code) took 24.5 us for 6000
-// tokens; shuffles for 1024 took 1100 instructions per token.
+// Bound: the latencies of a token's own chain -- load, barrier, transpose, barrier, store -- with the sixteen warps per SM that 104
+// registers leave (eight tokens of 4096): of the issue slots 44% are taken, of DRAM's time 23%, no pipe is above 31%, and the
+// stalls are spread over shared memory, fixed latencies and loads.  In chains of launches, us, one warp per token of 4096 and five
+// levels of shuffles for 1024 -> this kernel: 4096 wide, 6000 tokens 25.4 -> 24.3 (3.0 TB/s; 11 by bytes), 250 tokens 5.0 -> 4.3,
+// one 4.6 -> 2.7; 1024 wide 14.3 -> 7.1, 4.4 -> 2.0, 4.2 -> 1.8.  Long calls of 4096 gain next to nothing, short ones the overlap of
+// launches.  256, 512 and 2048, which no layer of the models here has, stay with the kernel above: 512 and 2048 are no squares.
 // The division by sqrt(K) = 32 or 64 is exact and is applied to the scale only: rint((v/64) / (s/64)) is rint(v/s) bit for bit.
 // Quantisation without a division per element: t_lo = fma(v, inv_lo, magic), t_hi = fma(v, inv_hi,
 // magic) with inv_lo < 1/s < inv_hi (2^-22 apart) bracket the exact quotient, and adding 1.5*2^23
