@@ -1,8 +1,8 @@
 // The steps either side of a quantized layer in a decoder block, as kernels of their own:
 //
-//   add_layernorm   x' = x + delta (optional), h = LayerNorm(x') * gamma + beta, one warp per row, fp32
-//                   statistics on the 16-bit-rounded x' (what the unfused sequence "add, then layer_norm"
-//                   computes), 16-bit in and out;
+//   add_layernorm   x' = x + delta (optional), h = LayerNorm(x') * gamma + beta, one warp per row (a block per
+//                   row up to 296 rows, as for the RMS norm), fp32 statistics on the 16-bit-rounded x' (what
+//                   the unfused sequence "add, then layer_norm" computes), 16-bit in and out;
 //   add_rmsnorm     x' = x + delta (optional), h = (x' / rms(x')) rounded to 16 bits, then * gamma: the RMS norm of
 //                   the Qwen3 decoder blocks (statistics in fp32, the normalised value rounded before the weight
 //                   multiplies it, as the module does);
