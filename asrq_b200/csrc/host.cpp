@@ -66,8 +66,28 @@ struct Unlocked {
   ~Unlocked() { PyEval_RestoreThread(state); }
 };
 
+// A tensor held by its Python object.  (Copies of the at::Tensor, an atomic count each that reaches the Python object too, made a
+// call of 4.9 us one of 5.2.)
+class Held {
+ public:
+  Held() = default;
+  Held(const Held&) = delete;
+  ~Held() { Py_XDECREF(o_); }
+  void operator=(PyObject* o) {
+    Py_INCREF(o);
+    Py_XDECREF(o_);
+    o_ = o;
+  }
+  explicit operator bool() const { return o_ != nullptr; }
+  const at::Tensor& operator*() const { return THPVariable_Unpack(o_); }
+  const at::Tensor* operator->() const { return &THPVariable_Unpack(o_); }
+
+ private:
+  PyObject* o_ = nullptr;
+};
+
 struct Layer {
-  at::Tensor weight, scales, zeros, bias;  // bias undefined: none
+  Held weight, scales, zeros, bias;  // bias empty: none
   PyObject* dict;
   long long k, n, bits, group;
 };
@@ -92,26 +112,26 @@ bool layer_of(PyObject* self, const c10::Device& dev, Layer* L) {
   for (const at::Tensor* t : {wt, st, zt})
     if (t->device() != dev || !t->is_contiguous()) return false;
   if (bt && (bt->scalar_type() != at::kHalf || bt->device() != dev)) return false;
-  L->weight = *wt;
-  L->scales = *st;
-  L->zeros = *zt;
-  if (bt) L->bias = *bt;
+  L->weight = w;
+  L->scales = s;
+  L->zeros = z;
+  if (bt) L->bias = b;
   return int_of(d, N.in_features, &L->k) && int_of(d, N.out_features, &L->n) && int_of(d, N.bits, &L->bits) && int_of(d, N.group_size, &L->group);
 }
 
 // fp16 / bf16 activations on the current CUDA device, contiguous, at least one row
-bool activations(PyObject* o, at::Tensor* x, int* dtype) {
+bool activations(PyObject* o, Held* x, int* dtype) {
   const at::Tensor* t = plain(o);
   if (!t || !t->is_cuda() || t->dim() < 1 || !t->is_contiguous() || t->numel() == 0) return false;
   const auto st = t->scalar_type();
   if (st != at::kHalf && st != at::kBFloat16) return false;
-  *x = *t;
+  *x = o;
   *dtype = st == at::kHalf ? ASRQ_F16 : ASRQ_BF16;
   return t->device().index() == c10::cuda::current_device() && !modes_active();
 }
 
 // The stream's workspace if it is there and large enough.
-bool workspace(int dev, cudaStream_t stream, size_t need, at::Tensor* ws) {
+bool workspace(int dev, cudaStream_t stream, size_t need, Held* ws) {
   PyObject* key = PyTuple_New(2);
   if (!key) return false;
   PyTuple_SET_ITEM(key, 0, PyLong_FromLong(dev));
@@ -120,7 +140,7 @@ bool workspace(int dev, cudaStream_t stream, size_t need, at::Tensor* ws) {
   Py_DECREF(key);
   const at::Tensor* t = plain(v);
   if (!t || size_t(t->numel()) < need) return false;
-  *ws = *t;
+  *ws = v;
   return true;
 }
 
@@ -152,24 +172,24 @@ PyObject* linearq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyErr_SetString(PyExc_TypeError, "linearq_forward(layer, input, residual, gelu)");
     return nullptr;
   }
-  at::Tensor x;
+  Held x;
   int dtype;
   Layer L;
-  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x.device(), &L) || (L.bits != 2 && L.bits != 4) || x.size(-1) != L.k) {
+  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x->device(), &L) || (L.bits != 2 && L.bits != 4) || x->size(-1) != L.k) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
-  const int64_t m = x.numel() / L.k;
-  at::Tensor res;
+  const int64_t m = x->numel() / L.k;
+  Held res;
   if (a[2] != Py_None) {
     const at::Tensor* r = plain(a[2]);
-    if (!r || r->scalar_type() != x.scalar_type() || r->device() != x.device() || r->numel() != m * L.n || !r->is_contiguous()) Py_RETURN_NONE;
-    res = *r;
+    if (!r || r->scalar_type() != x->scalar_type() || r->device() != x->device() || r->numel() != m * L.n || !r->is_contiguous()) Py_RETURN_NONE;
+    res = a[2];
   }
-  const bool gelu = a[3] == Py_True, fused = res.defined() || gelu;
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-  at::Tensor ws;
-  if (!workspace(x.device().index(), stream, asrq_workspace_bytes(ASRQ_WS_LINEARQ, m, L.n, L.k), &ws)) {
+  const bool gelu = a[3] == Py_True, fused = bool(res) || gelu;
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  Held ws;
+  if (!workspace(x->device().index(), stream, asrq_workspace_bytes(ASRQ_WS_LINEARQ, m, L.n, L.k), &ws)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;  // the Python path makes it
   }
@@ -177,16 +197,16 @@ PyObject* linearq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   int rc;
   {
     Unlocked unlocked;
-    y = output_like(x, L.n);
+    y = output_like(*x, L.n);
     g_calls.fetch_add(1, std::memory_order_relaxed);
-    const void* bias = L.bias.defined() ? L.bias.data_ptr() : nullptr;
+    const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
     if (!fused)
-      rc = asrq_linearq_a16(int(L.bits), x.data_ptr(), static_cast<const uint8_t*>(L.weight.data_ptr()), L.scales.data_ptr(), L.zeros.data_ptr(), bias,
-                            y.data_ptr(), m, L.n, L.k, int(L.group), dtype, ws.data_ptr(), size_t(ws.numel()), stream);
+      rc = asrq_linearq_a16(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(), bias,
+                            y.data_ptr(), m, L.n, L.k, int(L.group), dtype, ws->data_ptr(), size_t(ws->numel()), stream);
     else
-      rc = asrq_linearq_a16_fused(int(L.bits), x.data_ptr(), static_cast<const uint8_t*>(L.weight.data_ptr()), L.scales.data_ptr(), L.zeros.data_ptr(),
-                                  bias, res.defined() ? res.data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype,
-                                  gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE, ws.data_ptr(), size_t(ws.numel()), stream);
+      rc = asrq_linearq_a16_fused(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(),
+                                  bias, res ? res->data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype,
+                                  gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE, ws->data_ptr(), size_t(ws->numel()), stream);
   }
   if (rc) return failed(fused ? "asrq_linearq_a16_fused" : "asrq_linearq_a16", rc);
   return THPVariable_Wrap(std::move(y));
@@ -200,26 +220,27 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyErr_SetString(PyExc_TypeError, "linearqq_forward(layer, input)");
     return nullptr;
   }
-  at::Tensor x;
+  Held x;
   int dtype;
   Layer L;
-  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x.device(), &L) || x.size(-1) != L.k || L.group <= 0) {
+  if (!activations(a[1], &x, &dtype) || !layer_of(a[0], x->device(), &L) || x->size(-1) != L.k || L.group <= 0) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
   PyObject* had_o = PyDict_GetItemWithError(L.dict, N.hadamard);
   if (had_o != Py_True && had_o != Py_False) Py_RETURN_NONE;
   const int had = had_o == Py_True;
-  const int64_t m = x.numel() / L.k;
-  const int dev = x.device().index();
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-  const void* bias = L.bias.defined() ? L.bias.data_ptr() : nullptr;
-  at::Tensor ws, sc, y;
+  const int64_t m = x->numel() / L.k;
+  const int dev = x->device().index();
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
+  const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
+  Held ws, w8;
+  at::Tensor sc, y;
   const char* fn;
   int rc;
   // the activation codes and their scales: one scratch allocation (codes first, the scales at the next multiple of 256 bytes)
   auto scratch = [&](int64_t code_bytes) {
-    return at::detail::empty_cuda({(code_bytes + 255) / 256 * 256 + m * 4}, at::kByte, x.device(), std::nullopt);
+    return at::detail::empty_cuda({(code_bytes + 255) / 256 * 256 + m * 4}, at::kByte, x->device(), std::nullopt);
   };
   if (m >= 64 && L.n % 128 == 0 && L.k % 128 == 0 && L.group % 128 == 0 && L.k % L.group == 0) {
     PyObject* op = PyObject_GetAttr(a[0], N.operand);
@@ -228,32 +249,31 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const bool i8 = PyUnicode_Check(op) && PyUnicode_CompareWithASCIIString(op, "int8") == 0;
     // the prepared weight (linear._Prepared), if it was derived from this very buffer in this state and this stream is behind that
     PyObject* prepared = PyDict_GetItemWithError(L.dict, N.w8);
-    at::Tensor w8;
     if ((f8 || i8) && prepared && PyTuple_Check(prepared) && PyTuple_GET_SIZE(prepared) == 6) {
       const at::Tensor *t = plain(PyTuple_GET_ITEM(prepared, 0)), *src = plain(PyTuple_GET_ITEM(prepared, 1));
-      if (t && src && t->device() == x.device() && src->device() == x.device() && src->data_ptr() == L.weight.data_ptr() &&
-          PyLong_AsLongLong(PyTuple_GET_ITEM(prepared, 2)) == (long long)L.weight._version() && PyUnicode_Compare(PyTuple_GET_ITEM(prepared, 3), op) == 0 &&
+      if (t && src && t->device() == x->device() && src->device() == x->device() && src->data_ptr() == L.weight->data_ptr() &&
+          PyLong_AsLongLong(PyTuple_GET_ITEM(prepared, 2)) == (long long)L.weight->_version() && PyUnicode_Compare(PyTuple_GET_ITEM(prepared, 3), op) == 0 &&
           contains(PyTuple_GET_ITEM(prepared, 4), stream))
-        w8 = *t;
+        w8 = PyTuple_GET_ITEM(prepared, 0);
     }
     Py_DECREF(op);
     if (PyErr_Occurred()) return nullptr;
-    if (!w8.defined() || !workspace(dev, stream, 256, &ws)) {
+    if (!w8 || !workspace(dev, stream, 256, &ws)) {
       if (PyErr_Occurred()) return nullptr;
       Py_RETURN_NONE;
     }
     Unlocked unlocked;
     sc = scratch(m * L.k);
-    y = output_like(x, L.n);
+    y = output_like(*x, L.n);
     uint8_t* a8 = static_cast<uint8_t*>(sc.data_ptr());
     float* sa = reinterpret_cast<float*>(a8 + (m * L.k + 255) / 256 * 256);
     g_calls.fetch_add(2, std::memory_order_relaxed);
     fn = f8 ? "asrq_hadamard_quant_f8" : "asrq_hadamard_quant_int8";
-    rc = (f8 ? asrq_hadamard_quant_f8 : asrq_hadamard_quant_int8)(x.data_ptr(), a8, sa, m, L.k, had, dtype, stream);
+    rc = (f8 ? asrq_hadamard_quant_f8 : asrq_hadamard_quant_int8)(x->data_ptr(), a8, sa, m, L.k, had, dtype, stream);
     if (!rc) {
       fn = f8 ? "asrq_w4a4_gemm_f8" : "asrq_w4a4_gemm_int8";
-      rc = (f8 ? asrq_w4a4_gemm_f8 : asrq_w4a4_gemm_int8)(a8, sa, static_cast<const uint8_t*>(w8.data_ptr()), L.scales.data_ptr(), bias, y.data_ptr(), nullptr, m,
-                                                          L.n, L.k, int(L.group), dtype, ws.data_ptr(), size_t(ws.numel()), stream);
+      rc = (f8 ? asrq_w4a4_gemm_f8 : asrq_w4a4_gemm_int8)(a8, sa, static_cast<const uint8_t*>(w8->data_ptr()), L.scales->data_ptr(), bias, y.data_ptr(), nullptr, m,
+                                                          L.n, L.k, int(L.group), dtype, ws->data_ptr(), size_t(ws->numel()), stream);
     }
   } else {
     if (!workspace(dev, stream, asrq_workspace_bytes(ASRQ_WS_W4A4_GEMM, m, L.n, L.k), &ws)) {
@@ -262,16 +282,16 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     }
     Unlocked unlocked;
     sc = scratch(m * (L.k / 2));
-    y = output_like(x, L.n);
+    y = output_like(*x, L.n);
     uint8_t* qa = static_cast<uint8_t*>(sc.data_ptr());
     float* sa = reinterpret_cast<float*>(qa + (m * (L.k / 2) + 255) / 256 * 256);
     g_calls.fetch_add(2, std::memory_order_relaxed);
     fn = "asrq_hadamard_quant_int4";
-    rc = asrq_hadamard_quant_int4(x.data_ptr(), qa, sa, m, L.k, had, dtype, stream);
+    rc = asrq_hadamard_quant_int4(x->data_ptr(), qa, sa, m, L.k, had, dtype, stream);
     if (!rc) {
       fn = "asrq_w4a4_gemm";
-      rc = asrq_w4a4_gemm(qa, sa, static_cast<const uint8_t*>(L.weight.data_ptr()), L.scales.data_ptr(), bias, y.data_ptr(), nullptr, m, L.n, L.k, int(L.group),
-                          dtype, ws.data_ptr(), size_t(ws.numel()), stream);
+      rc = asrq_w4a4_gemm(qa, sa, static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), bias, y.data_ptr(), nullptr, m, L.n, L.k, int(L.group),
+                          dtype, ws->data_ptr(), size_t(ws->numel()), stream);
     }
   }
   if (rc) return failed(fn, rc);
