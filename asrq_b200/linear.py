@@ -478,6 +478,7 @@ class LinearQQ(LinearQ):
         if type(p) is _Prepared and p.of(weight, operand):
             if stream.cuda_stream not in p[4] and not capturing:
                 stream.wait_event(p[5])
+                p[0].record_stream(stream)  # replaced, its memory waits for this stream's work too
                 p[4].add(stream.cuda_stream)
             return p[0]
         w8 = torch.empty((self.out_features, self.in_features), dtype=torch.uint8, device=weight.device)

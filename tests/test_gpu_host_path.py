@@ -199,6 +199,29 @@ def test_prepared_weight_on_another_stream():
     asrq_b200.check_status()
 
 
+def test_prepared_weight_outlives_the_streams_that_use_it():
+    """The layer gets another weight while a call on a second stream is still to run: that call's operand is not reused for
+    the first stream's tensors meanwhile."""
+    x = torch.randn(80, 512, device=DEV).half()
+    qq, other = (_layers(512, 256, True, seed=s)[1] for s in (0, 1))
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(one):
+        want = qq(x)                                               # derives
+        other(x)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(two):
+        qq(x)
+        torch.cuda._sleep(int(2e8))                                # about a tenth of a second
+        y = qq(x)
+    held = qq.scales, qq.zeros, qq.weight                          # a program's own part of it
+    with torch.cuda.stream(one):
+        qq.load_quantized_params(other.scales, other.zeros, other.weight)
+        qq(x)                                                      # gives the first operand back
+        junk = [torch.full((512 * 256,), 255, dtype=torch.uint8, device=DEV) for _ in range(32)]
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and len(junk) == 32 and len(held) == 3
+
+
 def test_a_workspace_that_was_outgrown_stays():
     """A captured graph holds the address of the workspace that its stream had: that memory is given to nobody else when a
     wider layer needs more, and what is kept is bounded by what is in use."""
