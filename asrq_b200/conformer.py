@@ -169,15 +169,19 @@ class FastConformerStandIn:
     graph_shapes = 4    # graphs kept, the least recently used given back first
 
     def _operands(self):
-        """Everything a captured encode has baked in: a graph is replayed only while all of it is what it was."""
+        """Everything a captured encode has baked in (the layers' derived operands among it), held with the graph: it is
+        replayed only while all of it is what it was."""
         ops = [LinearQQ.operand, self.heads, self.conv_kernel, len(self.layers)]
         for L in self.layers:
-            for v in L.values():
+            for name, v in L.items():
                 if isinstance(v, tuple):
                     ops.extend(v)
                 else:
                     bufs = v._buffers
                     ops.extend((bufs.get("weight"), bufs.get("scales"), bufs.get("bias"), bufs["weight"]._version))
+                    if name not in ("q", "k", "v", "pos"):  # (which run as parts of the joined layers)
+                        ops.append(v.__dict__.get("_w8"))
+        ops.extend(m.__dict__.get("_w8") for m in self._qkv + [self._pos])
         ops.extend(self.sub_out)
         return ops
 
@@ -195,7 +199,7 @@ class FastConformerStandIn:
                 if key not in self._seen:
                     self._seen.add(key)
                     return None
-                hit = self._capture(x, ops)
+                hit = self._capture(x)
                 while len(self._graphs) >= self.graph_shapes:
                     self._graphs.pop(next(iter(self._graphs)))["done"].synchronize()  # not while it runs
             self._graphs[key] = hit  # most recently used last
@@ -207,7 +211,7 @@ class FastConformerStandIn:
             hit["done"].record(stream)
             return out
 
-    def _capture(self, x: torch.Tensor, ops) -> dict:
+    def _capture(self, x: torch.Tensor) -> dict:
         xs = x.clone()
         cur, side = torch.cuda.current_stream(self.device), torch.cuda.Stream(self.device)
         side.wait_stream(cur)
@@ -220,7 +224,7 @@ class FastConformerStandIn:
             out = self._blocks(xs, pe)
         done = torch.cuda.Event()
         done.record(cur)
-        return {"graph": g, "x": xs, "pe": pe, "out": out, "ops": ops, "done": done}
+        return {"graph": g, "x": xs, "pe": pe, "out": out, "ops": self._operands(), "done": done}
 
     @torch.no_grad()
     def encode(self, feats: torch.Tensor, hook=None) -> torch.Tensor:

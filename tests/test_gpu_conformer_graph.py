@@ -27,6 +27,23 @@ def test_encode_is_the_blocks_bit_for_bit(b, frames):
     assert not enc._joined_ok() and torch.equal(enc.encode(_feats(b, frames)), plain(_feats(b, frames)))
 
 
+def test_a_captured_shape_keeps_its_derived_operands(monkeypatch):
+    """Operands derived anew (another 8-bit form in between) are other memory: the captured encode is not replayed over what
+    the first ones left, and an unchanged encoder captures once."""
+    enc = C.FastConformerStandIn("cuda", n_layers=2, d_model=256, ffn=512, heads=4, mel=80, sub_channels=64, seed=4)
+    f = _feats(1, 800)
+    want = [enc.encode(f) for _ in range(4)][0]
+    graph = next(iter(enc._graphs.values()))["graph"]
+    enc.encode(f)
+    assert next(iter(enc._graphs.values()))["graph"] is graph
+    with monkeypatch.context() as m:
+        m.setattr(C.LinearQQ, "operand", "int8")
+        assert torch.equal(enc.encode(_feats(1, 960)), enc.encode(_feats(1, 960), hook=lambda *_: None))
+    torch.cuda.synchronize()
+    junk = [torch.full((256 * n,), 77, dtype=torch.uint8, device="cuda") for n in (256, 512, 768) for _ in range(32)]
+    assert torch.equal(enc.encode(f), want) and len(junk) == 96
+
+
 def test_captured_shapes_are_bounded_and_shared_by_streams():
     enc = C.FastConformerStandIn("cuda", n_layers=2, d_model=256, ffn=512, heads=4, mel=80, sub_channels=64, seed=4)
     for frames in range(400, 400 + 16 * (enc.graph_shapes + 2), 16):
