@@ -84,6 +84,12 @@ class _on_device:
         return False
 
 
+def _expect(ok: bool, what: str) -> None:
+    """What a kernel takes as given about its operands (it gets addresses and sizes only)."""
+    if not ok:
+        raise ValueError(what)
+
+
 def add_layernorm(x: torch.Tensor, delta, weight: torch.Tensor, bias: torch.Tensor, eps: float = 1e-5, write_sum: bool = True):
     """``(x + delta, layer_norm(x + delta) * weight + bias)`` in one kernel (``delta`` may be None: then the
     first result is ``x`` itself).  16-bit tensors on a CUDA device; the last dimension is normalised."""
@@ -162,6 +168,8 @@ def decode_self_attention(qkv: torch.Tensor, kv_cache: torch.Tensor, pos: torch.
     are), so they may be fetched while these still run."""
     dt = _require_cuda_16bit(qkv, "decode_self_attention")
     _, B, H, max_len, hd = kv_cache.shape
+    _expect(kv_cache.is_contiguous() and kv_cache.shape[0] == 2 and kv_cache.dtype == qkv.dtype and kv_cache.device == pos.device == qkv.device and
+            pos.dtype == torch.int64, "decode_self_attention: kv_cache must be contiguous (2, B, heads, max_len, head_dim) of qkv's type, pos int64")
     q2 = qkv.reshape(B, 3 * H * hd)
     q2 = q2 if q2.is_contiguous() else q2.contiguous()
     out = torch.empty((B, H * hd), dtype=qkv.dtype, device=qkv.device)
@@ -176,6 +184,10 @@ def argmax_rows(logits: torch.Tensor, tokens: torch.Tensor, scratch: torch.Tenso
     device) also ``ids[pos] = tokens``.  ``scratch``: 2 B int64, zero before the first call, which every call leaves at zero."""
     dt = _require_cuda_16bit(logits, "argmax_rows")
     B, n = logits.shape
+    _expect(logits.is_contiguous() and all(t is None or (t.is_contiguous() and t.dtype == torch.int64 and t.device == logits.device)
+                                           for t in (tokens, scratch, ids, pos)) and tokens.numel() >= B and scratch.numel() >= 2 * B and
+            (ids is None or (pos is not None and ids.numel() % max(B, 1) == 0)),
+            "argmax_rows: contiguous (B, N) logits, int64 tokens (B), scratch (2 B), ids (steps, B) with pos on the same device")
     with _on_device(logits.device):
         _lib.call("asrq_argmax_rows", logits.data_ptr(), tokens.data_ptr(), None if ids is None else ids.data_ptr(), None if pos is None else pos.data_ptr(),
                   scratch.data_ptr(), B, n, dt, torch.cuda.current_stream(logits.device).cuda_stream)
@@ -183,30 +195,37 @@ def argmax_rows(logits: torch.Tensor, tokens: torch.Tensor, scratch: torch.Tenso
 
 def _conv_step(fn: str, tensors, out: torch.Tensor, sizes) -> torch.Tensor:
     dt = _require_cuda_16bit(tensors[0], fn)
+    _expect(all(t.dtype == out.dtype and t.device == out.device for t in tensors), f"{fn}: tensors of one type on one device")
+    tensors = [t if t.is_contiguous() else t.contiguous() for t in tensors]
     with _on_device(out.device):
         _lib.call(fn, *(t.data_ptr() for t in tensors), out.data_ptr(), *sizes, dt, torch.cuda.current_stream(out.device).cuda_stream)
     return out
 
 
 def bias_glu(x: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
-    """``glu(x + bias)`` over the channels of a contiguous (B, 2C, T) convolution output, in one pass."""
+    """``glu(x + bias)`` over the channels of a (B, 2C, T) convolution output, in one pass."""
     B, c2, T = x.shape
+    _expect(c2 % 2 == 0 and bias.numel() == c2, f"bias_glu: an even number of channels and a bias of as many values (x {tuple(x.shape)}, bias {bias.numel()})")
     return _conv_step("asrq_bias_glu", (x, bias), x.new_empty(B, c2 // 2, T), (B, c2 // 2, T))
 
 
 def bias_affine_silu(x: torch.Tensor, bias: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor) -> torch.Tensor:
-    """``silu((x + bias) * scale + shift)`` per channel of a contiguous (B, C, T) convolution output, in one pass."""
-    return _conv_step("asrq_bias_affine_silu", (x, bias, scale, shift), torch.empty_like(x), x.shape)
+    """``silu((x + bias) * scale + shift)`` per channel of a (B, C, T) convolution output, in one pass."""
+    _expect(bias.numel() == scale.numel() == shift.numel() == x.shape[1], "bias_affine_silu: bias, scale and shift of one value per channel")
+    return _conv_step("asrq_bias_affine_silu", (x, bias, scale, shift), x.new_empty(x.shape), x.shape)
 
 
 def half_step(x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
-    """``x + 0.5 * y``, contiguous tensors of a multiple of 8 values, in one pass."""
-    return _conv_step("asrq_half_step", (x, y), torch.empty_like(x), (x.numel(),))
+    """``x + 0.5 * y``, tensors of as many values, a multiple of 8, in one pass."""
+    _expect(x.numel() == y.numel(), f"half_step: {tuple(x.shape)} and {tuple(y.shape)}")
+    return _conv_step("asrq_half_step", (x, y), x.new_empty(x.shape), (x.numel(),))
 
 
 def bias_add_transposed(x: torch.Tensor, conv: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
-    """``x + (conv + bias).transpose(1, 2)``: x (B, T, C), conv (B, C, T), both contiguous, in one pass."""
-    return _conv_step("asrq_bias_add_transposed", (x, conv, bias), torch.empty_like(x), x.shape)
+    """``x + (conv + bias).transpose(1, 2)``: x (B, T, C), conv (B, C, T), in one pass."""
+    _expect(conv.shape == (x.shape[0], x.shape[2], x.shape[1]) and bias.numel() == x.shape[2],
+            f"bias_add_transposed: x {tuple(x.shape)}, conv {tuple(conv.shape)}, bias {bias.numel()}")
+    return _conv_step("asrq_bias_add_transposed", (x, conv, bias), x.new_empty(x.shape), x.shape)
 
 
 def decode_cross_attention(q: torch.Tensor, kv: torch.Tensor, heads: int, scale: float = 1.0, settled: bool = False) -> torch.Tensor:
@@ -216,6 +235,8 @@ def decode_cross_attention(q: torch.Tensor, kv: torch.Tensor, heads: int, scale:
     dt = _require_cuda_16bit(q, "decode_cross_attention")
     B, T, d2 = kv.shape
     d = d2 // 2
+    _expect(kv.is_contiguous() and kv.dtype == q.dtype and kv.device == q.device and d2 == 2 * d and d % heads == 0 and q.numel() == B * d,
+            f"decode_cross_attention: contiguous kv (B, T, 2 d) of q's type and q (B, d) (kv {tuple(kv.shape)}, q {tuple(q.shape)}, {heads} heads)")
     q2 = q.reshape(B, d)
     q2 = q2 if q2.is_contiguous() else q2.contiguous()
     out = torch.empty((B, d), dtype=q.dtype, device=q.device)
@@ -233,6 +254,11 @@ def decode_grouped_attention(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight
     cache an ordinary kernel or copy has to come first."""
     dt = _require_cuda_16bit(qkv, "decode_grouped_attention")
     B, nkv, max_len, hd = k_cache.shape
+    _expect(v_cache.shape == k_cache.shape and qkv.numel() == B * (n_q + 2 * nkv) * hd and min(cos.numel(), sin.numel()) >= max_len * hd and
+            q_weight.numel() == k_weight.numel() == hd and pos.dtype == torch.int64 and pos.device == qkv.device and
+            all(t.is_contiguous() and t.dtype == qkv.dtype and t.device == qkv.device for t in (qkv, q_weight, k_weight, cos, sin, k_cache, v_cache)),
+            "decode_grouped_attention: contiguous tensors of one type; qkv (B, (n_q + 2 n_kv) head_dim), caches (B, n_kv, max_len, head_dim), "
+            "tables (max_len, head_dim), pos int64")
     out = torch.empty((B, n_q * hd), dtype=qkv.dtype, device=qkv.device)
     with _on_device(qkv.device):
         _lib.call("asrq_decode_grouped_attention", qkv.data_ptr(), q_weight.data_ptr(), k_weight.data_ptr(), cos.data_ptr(), sin.data_ptr(),
@@ -251,7 +277,8 @@ def dense_head(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor = None) 
     m, n = x2.shape[0], weight.shape[0]
     if out is None:
         out = torch.empty((m, n), dtype=x.dtype, device=x.device)
-    if m > 32 or k % 32 or k > 3200 or weight.dtype != x.dtype or not weight.is_contiguous():
+    if (m > 32 or k % 32 or k > 3200 or weight.dtype != x.dtype or not weight.is_contiguous() or weight.shape[1] != k or out.numel() != m * n or
+            out.dtype != x.dtype or not out.is_contiguous()):
         torch.matmul(x2, weight.t(), out=out)
         return out.reshape(*x.shape[:-1], n)
     x2 = x2 if x2.is_contiguous() else x2.contiguous()
