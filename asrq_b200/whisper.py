@@ -21,6 +21,7 @@ Two things live here.
 from __future__ import annotations
 
 import math
+import operator
 import os
 from typing import Dict, List, Optional
 
@@ -180,7 +181,8 @@ def _baked_in(values) -> list:
         if isinstance(v, dict):
             out += _baked_in(v.values())
         elif isinstance(v, LinearQ):
-            out += [v._buffers.get(n, v.__dict__.get(n)) for n in ("weight", "scales", "zeros", "bias")] + [v.bits, v.group_size]
+            at, buf = v.__dict__, v._buffers  # (attribute access by name costs a module's call each)
+            out += (buf.get("weight"), buf.get("scales"), buf.get("zeros"), buf.get("bias") if "bias" in buf else at.get("bias"), at["bits"], at["group_size"])
         elif isinstance(v, _Norm):
             out += [v.w, v.b, v.eps]
         else:
@@ -189,7 +191,8 @@ def _baked_in(values) -> list:
 
 
 def _same(a: list, b: list) -> bool:
-    return len(a) == len(b) and all(x is y or (type(x) in (bool, int, float) and x == y) for x, y in zip(a, b))
+    return len(a) == len(b) and (all(map(operator.is_, a, b)) or
+                                 all(x is y or (type(x) in (bool, int, float) and x == y) for x, y in zip(a, b)))
 
 
 class _Norm:
