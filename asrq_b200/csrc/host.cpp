@@ -26,6 +26,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <atomic>
+#include <map>
+#include <mutex>
 
 #include "../../include/asrq_b200.h"
 
@@ -301,6 +303,21 @@ PyObject* linearqq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 
 PyObject* calls(PyObject*, PyObject*) { return PyLong_FromLongLong(g_calls.load(std::memory_order_relaxed)); }
 
+// A stream of this file's own per device: never under capture, which one of the pool that torch hands out round and round may be.
+c10::cuda::CUDAStream own_stream(c10::DeviceIndex device) {
+  static std::mutex mu;
+  static std::map<int, cudaStream_t> streams;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = streams.find(device);
+  if (it == streams.end()) {
+    c10::cuda::CUDAGuard guard(device);
+    cudaStream_t s;
+    C10_CUDA_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    it = streams.emplace(device, s).first;
+  }
+  return c10::cuda::getStreamFromExternal(it->second, device);
+}
+
 // zeros_now(bytes, device) -> uint8 tensor that is zero on return, also while a stream is under capture: zeros made on that stream
 // would be the graph's, there only once it has run, in memory of the graph's.
 PyObject* zeros_now(PyObject*, PyObject* args) {
@@ -312,7 +329,7 @@ PyObject* zeros_now(PyObject*, PyObject* args) {
   {
     Unlocked unlocked;
     c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
-    const c10::cuda::CUDAStream side = c10::cuda::getStreamFromPool(false, c10::DeviceIndex(device));
+    const c10::cuda::CUDAStream side = own_stream(c10::DeviceIndex(device));
     c10::cuda::CUDAStreamGuard guard(side);
     t = at::detail::empty_cuda({bytes}, at::kByte, c10::Device(c10::kCUDA, c10::DeviceIndex(device)), std::nullopt);
     C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, size_t(bytes), side.stream()));

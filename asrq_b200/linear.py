@@ -9,6 +9,7 @@ fallback -- a CPU tensor, or a missing library, raises.
 from __future__ import annotations
 
 import os
+import threading
 
 import torch
 import torch.nn as nn
@@ -21,6 +22,7 @@ _CHECK = os.environ.get("ASRQ_B200_CHECK_STATUS", "0") == "1"
 # one scratch buffer per (device, stream): kernels on one stream run in order, so they can share it
 _workspaces: dict = {}
 _outgrown: list = []  # earlier, smaller ones: a captured graph may hold their address
+_growing = threading.Lock()
 
 _native = None
 
@@ -43,12 +45,15 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
-        if ws is not None:
-            _outgrown.append(ws)
-            nbytes = max(nbytes, 2 * ws.numel())  # what is kept stays below what is in use
-        from . import _native as native  # (not the switch between the two call paths above)
-        ws = native.zeros_now(max(nbytes, 1 << 20), device.index)
-        _workspaces[key] = ws
+        with _growing:  # one thread makes it; a second one that another thread had in use would not outlive its call
+            ws = _workspaces.get(key)
+            if ws is None or ws.numel() < nbytes:
+                if ws is not None:
+                    _outgrown.append(ws)
+                    nbytes = max(nbytes, 2 * ws.numel())  # what is kept stays below what is in use
+                from . import _native as native  # (not the switch between the two call paths above)
+                ws = native.zeros_now(max(nbytes, 1 << 20), device.index)
+                _workspaces[key] = ws
     return ws
 
 

@@ -263,3 +263,27 @@ def test_a_workspace_made_under_capture():
         graph.replay()
         assert torch.equal(y, want)
     asrq_b200.check_status()
+
+
+def test_workspaces_of_many_streams_and_threads():
+    """Every stream of torch's pool under capture in its turn, none of them with a workspace yet; then threads that ask for one
+    stream's workspace at once and get the same."""
+    q = _layers(512, 256, True)[0]
+    x = torch.randn(4, 512, device=DEV).half()
+    want = q(x)
+    for _ in range(40):
+        stream = torch.cuda.Stream()
+        linear._workspaces.pop((torch.cuda.current_device(), stream.cuda_stream), None)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            y = q(x)
+        graph.replay()
+        assert torch.equal(y, want)
+    stream, got = torch.cuda.Stream(), []
+    linear._workspaces.pop((torch.cuda.current_device(), stream.cuda_stream), None)
+
+    def work():
+        with torch.cuda.stream(stream):
+            got.append(linear._workspace(torch.device(DEV), 1 << 20).data_ptr())
+    _in_threads([work] * 8)
+    assert len(got) == 8 and len(set(got)) == 1
