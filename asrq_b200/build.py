@@ -21,7 +21,7 @@ LIB = os.path.join(PKG, "libasrq_b200.so")
 NATIVE = os.path.join(PKG, "_native.so")  # the module calls' host path (csrc/host.cpp), a CPython extension on torch's C++ API
 OBJ_DIR = os.path.join(PKG, "build")
 
-SOURCES = ["api.cu", "gemv_a16.cu", "gemv_a16_splitk.cu", "gemv_a16_staged.cu", "gemm_a16_tc.cu", "gemm_a16_tc2.cu", "gemm_a16_skinny.cu", "act_quant.cu", "glue.cu", "offline.cu", "dense_head.cu", "decode_attn.cu", "conformer.cu", "w4a4_mma.cu", "w4a4_tc.cu"]
+SOURCES = ["api.cu", "gemv_a16.cu", "gemv_a16_splitk.cu", "gemv_a16_staged.cu", "gemm_a16_tc.cu", "gemm_a16_tc2.cu", "gemm_a16_dense.cu", "gemm_a16_skinny.cu", "act_quant.cu", "glue.cu", "offline.cu", "dense_head.cu", "decode_attn.cu", "conformer.cu", "w4a4_mma.cu", "w4a4_tc.cu"]
 HEADERS = ["common.cuh", "tcgen05.cuh", "dequant.cuh", os.path.join("..", "..", "include", "asrq_b200.h")]
 
 NVCC_FLAGS = [

@@ -22,6 +22,12 @@ size_t gemm_tc_workspace_bytes(int64_t M, int64_t N);
 int gemm_a16_tc(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                 void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
                 size_t workspace_bytes, int sm_count, cudaStream_t stream, const Epilogue& ep, bool* fused);
+size_t gemm_a16_dense_workspace_bytes(int64_t N, int64_t K);
+double gemm_a16_dense_estimate(int64_t M, int64_t N, int64_t K, int sm_count, bool gelu, bool residual);
+bool gemm_a16_dense_supports(int64_t M, int64_t N, int64_t K, int group_size);
+int gemm_a16_dense(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias, void* y, int64_t M,
+                   int64_t N, int64_t K, int group_size, int dtype, void* workspace, size_t workspace_bytes, int sm_count,
+                   cudaStream_t stream, const Epilogue& ep);
 int add_layernorm(const void* x, const void* delta, const void* gamma, const void* beta, float eps, void* x_out, void* h_out,
                   int64_t rows, int64_t dim, int dtype, cudaStream_t stream);
 int epilogue16_apply(void* y, const void* residual, int64_t M, int64_t N, int act, int dtype, int sm_count, cudaStream_t stream);
@@ -201,8 +207,8 @@ int g_tmap_next = 0;
 }  // namespace
 
 int make_tmap_2d(CUtensorMap* out, const void* base, int elem_bytes, bool bf16, uint64_t inner, uint64_t rows,
-                 uint32_t box_inner, uint32_t box_rows, bool swizzle128) {
-  const TmapKey key = {base, inner, rows, box_inner, box_rows, elem_bytes, (bf16 ? 1 : 0) | (swizzle128 ? 2 : 0)};
+                 uint32_t box_inner, uint32_t box_rows, TmapSwizzle swizzle) {
+  const TmapKey key = {base, inner, rows, box_inner, box_rows, elem_bytes, (bf16 ? 1 : 0) | (int(swizzle) << 1)};
   {
     std::lock_guard<std::mutex> lock(g_tmap_mutex);
     for (const TmapEntry& e : g_tmap_cache)
@@ -222,7 +228,9 @@ int make_tmap_2d(CUtensorMap* out, const void* base, int elem_bytes, bool bf16, 
   const cuuint32_t estr[2] = {1, 1};
   if (strides[0] % 16) return fail(ASRQ_ERR_ALIGN, "row pitch %llu is not a multiple of 16 bytes", (unsigned long long)strides[0]);
   const CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                        swizzle == kSwizzle128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                        : swizzle == kSwizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(ASRQ_ERR_SHAPE, "cuTensorMapEncodeTiled failed with CUresult %d", int(r));
   std::lock_guard<std::mutex> lock(g_tmap_mutex);
@@ -278,6 +286,8 @@ int current_device_sm_count(int* sm_count) {
 
 // M at or below which LinearQ.forward goes to the skinny kernel.
 constexpr int64_t kGemvMaxM = 32;
+// M from which the dequantise-once form is considered: below, it lost on every layer shape measured (1280 to 6144 inputs).
+constexpr int64_t kDenseMinM = 768;
 
 }  // namespace asrq
 
@@ -290,13 +300,19 @@ int asrq_version(void) { return 100; }
 
 const char* asrq_last_error_string(void) { return last_error().c_str(); }
 
+// What the dequantise-once form asks of the workspace for a call of this size (0: the call does not take it)
+static size_t dense_workspace(int64_t M, int64_t N, int64_t K) {
+  return M >= kDenseMinM && gemm_a16_dense_supports(M, N, K, 64) ? gemm_a16_dense_workspace_bytes(N, K) : 0;
+}
+
 size_t asrq_workspace_bytes(int kind, int64_t M, int64_t N, int64_t K) {
   switch (kind) {
     case ASRQ_WS_A16_GEMV:
-    case ASRQ_WS_LINEARQ:
       return gemv_workspace_bytes(N);
+    case ASRQ_WS_LINEARQ:
+      return std::max(gemv_workspace_bytes(N), dense_workspace(M, N, K));
     case ASRQ_WS_A16_GEMM:
-      return gemm_tc_workspace_bytes(M, N);
+      return std::max(gemm_tc_workspace_bytes(M, N), dense_workspace(M, N, K));
     case ASRQ_WS_W4A4_GEMM:
       return w4a4_tc_workspace_bytes(M, N, K);
     default:
@@ -339,6 +355,24 @@ static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scale
   // as fast; the widest, 2048 -> 12288, us: 15.5 / 16.7 / 17.8 at 64 / 96 / 128 tokens against 16.2 / 16.4 / 16.7.
   const double one_wave = option(kOptMidKernel) != 1 && option(kOptTcPair) < 0 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0
                               ? gemm_a16_skinny_estimate(M, N, K, group_size, f->sm_count, workspace_bytes) : -1.0;
+  // Large calls: the weights dequantised once and the epilogue in the GEMM, where that is estimated below both the others (measured:
+  // 1.0 to 1.5 times as fast without epilogue from 2000 tokens on, 1.2 to 1.9 times with one, 0.6 to 1.0 at 600).
+  const int pair = option(kOptTcPair);
+  if ((pair == 2 ? any_m || M >= 32 : pair < 0 && M >= kDenseMinM) && gemm_a16_dense_supports(M, N, K, group_size) && aligned16(ep.residual) &&
+      workspace_bytes >= gemm_a16_dense_workspace_bytes(N, K)) {
+    const bool gelu = ep.act == kActGelu, res = ep.residual != nullptr;
+    const double dense = gemm_a16_dense_estimate(M, N, K, f->sm_count, gelu, res);
+    // the persistent kernel's K blocks under load, 0.33 us rising to 0.5 from about 140 of them on, and the epilogue's pass
+    const double blocks = std::max(0.0, gemm_a16_tc_estimate(M, N, K, group_size, f->sm_count) - 5.5);
+    const double unpacking = 6.0 + blocks * std::min(1.6, 1.06 + 0.0122 * std::max(0.0, blocks - 9.4)) + (gelu || res ? 1.0 + 1.3e-6 * double(M) * double(N) : 0.0);
+    // the one-wave kernel's epilogue has nothing to run under
+    const double whole_k = one_wave * 1.06 + (gelu ? 1.5 + 1.2e-6 * double(M) * double(N) : 0.0) + (res ? 2.0 + 1.5e-6 * double(M) * double(N) : 0.0);
+    if (pair == 2 || (dense * 1.04 < unpacking && (one_wave <= 0 || dense * 1.04 < whole_k))) {
+      *fused = true;
+      return gemm_a16_dense(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, f->sm_count,
+                            static_cast<cudaStream_t>(stream), ep);
+    }
+  }
   if (one_wave > 0 && (M <= 128 || one_wave < gemm_a16_tc_estimate(M, N, K, group_size, f->sm_count))) {
     *fused = true;
     return gemm_a16_skinny(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes,

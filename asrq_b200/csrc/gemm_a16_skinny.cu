@@ -476,9 +476,9 @@ int gemm_a16_skinny(int bits, const void* x, const uint8_t* w, const void* scale
 #endif
   const bool bf16 = dtype == ASRQ_BF16;
   CUtensorMap tmx, tmw;
-  int rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, uint32_t(pl.bt), true);
+  int rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, uint32_t(pl.bt), kSwizzle128);
   if (rc) return rc;
-  rc = make_tmap_2d(&tmw, w, 1, false, uint64_t(K) * bits / 8, uint64_t(N), uint32_t(8 * bits), 128, false);
+  rc = make_tmap_2d(&tmw, w, 1, false, uint64_t(K) * bits / 8, uint64_t(N), uint32_t(8 * bits), 128, kSwizzleNone);
   if (rc) return rc;
   if (bits == 4)
     return bf16 ? launch_skinny<4, true>(tmx, tmw, p, pl.grid, pl.smem, stream)

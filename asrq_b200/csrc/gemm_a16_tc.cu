@@ -553,9 +553,9 @@ int gemm_a16_tc(int bits, const void* x, const uint8_t* w, const void* scales, c
 
   const bool bf16 = dtype == ASRQ_BF16;
   CUtensorMap tmx, tmw;
-  int rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, uint32_t(p.bt), true);
+  int rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, uint32_t(p.bt), kSwizzle128);
   if (rc) return rc;
-  rc = make_tmap_2d(&tmw, w, 1, false, uint64_t(K) * bits / 8, uint64_t(N), uint32_t(8 * bits), 128, false);
+  rc = make_tmap_2d(&tmw, w, 1, false, uint64_t(K) * bits / 8, uint64_t(N), uint32_t(8 * bits), 128, kSwizzleNone);
   if (rc) return rc;
   p.ksplit = gemm_tc_pick_split(M, N, K, p.bt, sm_count);
   if (p.ksplit > 1 && (workspace_bytes < kPartialOffset + size_t(4) * N * p.n_ttiles * p.bt * p.ksplit ||

@@ -566,9 +566,9 @@ int gemm_a16_tc2(int bits, const void* x, const uint8_t* w, const void* scales, 
 
   const bool bf16 = dtype == ASRQ_BF16;
   CUtensorMap tmx, tmw;
-  int rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, uint32_t(p.bt / 2), true);
+  int rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, uint32_t(p.bt / 2), kSwizzle128);
   if (rc) return rc;
-  rc = make_tmap_2d(&tmw, w, 1, false, uint64_t(K) * bits / 8, uint64_t(N), uint32_t(8 * bits), 128, false);
+  rc = make_tmap_2d(&tmw, w, 1, false, uint64_t(K) * bits / 8, uint64_t(N), uint32_t(8 * bits), 128, kSwizzleNone);
   if (rc) return rc;
   const int nclusters = int(std::min<int64_t>(int64_t(p.n_fpairs) * p.n_ttiles, max_clusters));
   const int grid = 2 * nclusters;

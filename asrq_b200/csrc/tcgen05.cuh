@@ -425,9 +425,10 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 
 // ---- host: tensor maps ----------------------------------------------------------------------
 // 2-D row-major tensor of `rows` x `inner` elements of `elem_bytes` bytes (1 or 2),
-// box `box_inner` x `box_rows`.  swizzle128: 128-byte swizzle (box_inner*elem_bytes == 128)
-// or none.  Returns 0 or a negative ASRQ status.
+// box `box_inner` x `box_rows`.  A swizzle spans the box's rows: box_inner * elem_bytes is 128 or 64 for it.
+// Returns 0 or a negative ASRQ status.
+enum TmapSwizzle { kSwizzleNone = 0, kSwizzle128 = 1, kSwizzle64 = 2 };
 int make_tmap_2d(CUtensorMap* out, const void* base, int elem_bytes, bool bf16, uint64_t inner, uint64_t rows,
-                 uint32_t box_inner, uint32_t box_rows, bool swizzle128);
+                 uint32_t box_inner, uint32_t box_rows, TmapSwizzle swizzle);
 
 }  // namespace asrq

@@ -539,9 +539,9 @@ int w4a4_gemm_int8(const uint8_t* w8, const uint8_t* a8, const float* sa, const 
   const size_t smem = 1024 + kept + p.nstages * stage_bytes;
 
   CUtensorMap tmw, tma;
-  int rc = make_tmap_2d(&tmw, w8, 1, false, uint64_t(K), uint64_t(N), 128, 128, true);
+  int rc = make_tmap_2d(&tmw, w8, 1, false, uint64_t(K), uint64_t(N), 128, 128, kSwizzle128);
   if (rc) return rc;
-  rc = make_tmap_2d(&tma, a8, 1, false, uint64_t(K), uint64_t(M), 128, uint32_t(pair ? p.bt / 2 : p.bt), true);
+  rc = make_tmap_2d(&tma, a8, 1, false, uint64_t(K), uint64_t(M), 128, uint32_t(pair ? p.bt / 2 : p.bt), kSwizzle128);
   if (rc) return rc;
   const int grid = pair ? 2 * int(std::min<int64_t>(int64_t(p.n_ftiles / 2) * p.n_ttiles, sm_count / 2))
                         : int(std::min<int64_t>(int64_t(p.n_ftiles) * p.n_ttiles, sm_count));

@@ -115,7 +115,9 @@ int asrq_w4a16_gemv_static(const void* x, const uint8_t* w, const void* scales, 
  * For M <= 256 the K range of an output tile may be divided among several blocks
  * (fp32 parts in the workspace, added in a fixed order); with a workspace smaller
  * than asrq_workspace_bytes(ASRQ_WS_A16_GEMM, M, N, K) but at least 256 bytes the
- * call still runs, unsplit.
+ * call still runs, unsplit.  From 768 tokens on that size has room for the layer's 16-bit
+ * weights: large calls write them there once and run a plain 16-bit GEMM (same bits); with a
+ * smaller workspace they unpack inside the GEMM.
  * Replaces matmul_f16xint4 / matmul_f16xint2 for M > 64
  * (asrq/matmulq/csrc/bindings.cpp:44-57, 607-650, 705-747).
  */
@@ -398,7 +400,8 @@ int asrq_w4a4_gemm_f8(const uint8_t* a8, const float* sa, const uint8_t* w8, con
  *   gemv_cpw (0), gemv_loop (-1)   strip-per-block decode kernel: steps per warp, rounds variant
  *   tc_split (0)          1: no split K in the prefill kernel
  *   tc_bt (0), w4a4_bt (0)         token-tile width of the tcgen05 kernels (0 auto)
- *   tc_pair (-1), w4a4_pair (-1)   CTA-pair variants: -1 auto, 0 off, 1 on
+ *   tc_pair (-1), w4a4_pair (-1)   CTA-pair variants: -1 auto, 0 off, 1 on; tc_pair 2: the form that
+ *                         unpacks the weights once per call, where the workspace has room for them
  *   tc_pair_release (0)   CTA-pair prefill kernel: 1 = release/acquire at cluster scope on the
  *                         cross-CTA "operand written" hand-off (slower), 0 = relaxed arrival
  *   trace (0), trace_block (0)     only in builds with -DASRQ_TRACE: pipeline clock marks
