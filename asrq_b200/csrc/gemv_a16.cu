@@ -7,7 +7,14 @@
 // two (a subnormal), which mma.sync.m16n8k16 multiplies exactly with the fp16 activations and
 // accumulates in fp32.  Fields at different bit positions ("types") go to different accumulators
 // and are combined, scaled by the group's scale and offset by zero * sum(x) once per quantisation
-// group in fp32; sum(x) over the group comes from one more MMA against a matrix of ones.
+// group in fp32; sum(x) over the group comes from MMAs against a matrix of ones (half as many).
+//
+// bf16 activations take the same route without conversion: a code in the low bits of 128.0's mantissa is 128 + code in bf16, and the
+// 128 * sum(x) too much goes with the zero's term.  Turning the activations into fp16 instead cost a pack instruction of a
+// quarter of the issue rate or less per pair in every block, and their range.  Chains of launches, before (fp16 codes, converted
+// activations, twice the MMAs against ones) -> now, us: 6144 -> 2048, 2-bit, 16 tokens, bf16 9.8 -> 6.2, fp16 6.9 -> 6.0; 2048 -> 12288, 4-bit,
+// one token 9.2 -> 6.5 and 7.1 -> 6.0; 1280 -> 1280, 4-bit, one token 3.6 -> 3.0 and 3.0 -> 2.85; 2-bit at 8 tokens of 1280 -> 3840
+// in fp16 went from 3.6 to 4.0.
 //
 // Work split: a warp owns a strip of 16 weight rows (rows g and g+8 per lane, g = lane/4) over one
 // to four "steps" (a step = 64 bytes of a row per lane quad = 128 k for 4-bit, 256 k for 2-bit),
@@ -44,7 +51,7 @@ struct GemvParams {
   const __half* zeros;
   const __half* bias;
   uint16_t* y;
-  int M, N, K, groups_per_row, KQ, CPW, bf16;  // CPW repeats the kernel's template argument
+  int M, N, K, groups_per_row, KQ, CPW;  // CPW repeats the kernel's template argument
   // fused steps either side of the layer (see Epilogue): residual addition or activation
   const uint16_t* residual;
   int act;
@@ -55,30 +62,43 @@ struct GemvParams {
 constexpr int kGemvMaxWarps = 16;
 constexpr int kGemvMaxSteps = 4;
 
-// d = a * b (+ c): m16n8k16, fp16 operands, fp32 accumulation
+// d = a * b (+ c): m16n8k16, fp16 or bf16 operands, fp32 accumulation
+template <bool BF16>
 __device__ __forceinline__ void mma_acc(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                         uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  if (BF16)
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+template <bool BF16>
 __device__ __forceinline__ void mma_new(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                         uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%10,%10,%10,%10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+  if (BF16)
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+  else
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
-
-__device__ __forceinline__ uint32_t bf16x2_to_f16x2_sat(uint32_t v) {
-  float lo = __uint_as_float(v << 16);
-  float hi = __uint_as_float(v & 0xffff0000u);
-  lo = fminf(fmaxf(lo, -65504.f), 65504.f);
-  hi = fminf(fmaxf(hi, -65504.f), 65504.f);
-  return h2_as_u32(__floats2half2_rn(lo, hi));
+// two 16-bit activations as floats
+template <bool BF16>
+__device__ __forceinline__ float2 two_floats(uint32_t v) {
+  return BF16 ? make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)) : __half22float2(u32_as_h2(v));
 }
 
 // streaming loads of W words (never re-read by this kernel: keep them out of L1)
@@ -131,6 +151,14 @@ __device__ __forceinline__ unsigned long long gemv_globaltimer() {
   return t;
 }
 
+// Registers a thread.  TIGHT: the form of two 4-bit steps per warp that leaves room for three blocks of eight warps on an SM, for layers
+// that need them to be resident at once (2048 -> 6144, one token, us: 4.1 in one wave, 4.6 in two of the other form; that is
+// faster where one wave is enough: 2048 -> 2048, eight tokens, 3.7 against 4.8).
+constexpr bool gemv_has_tight(int bits, int mh, int cpw) { return bits == 4 && mh == 1 && cpw == 2; }
+constexpr int gemv_registers(int bits, int mh, int cpw, bool loop, bool tight) {
+  return bits == 4 && mh == 1 && !loop && cpw == 1 ? 40 : (tight ? 80 : 128);
+}
+
 // BITS: 4 or 2.  MH: token halves (1: M <= 8, 2: M <= 16).  GPS: quantisation groups per step
 // (1, 2 or 4; the group size is 128/GPS k for 4-bit and 256/GPS k for 2-bit).  CPW: steps per warp
 // (1, 2 or 4, CPW * GPS <= 8).  XC: M <= 2, the activation sums are made on the CUDA cores instead of
@@ -141,8 +169,8 @@ __device__ __forceinline__ unsigned long long gemv_globaltimer() {
 // 2.0-2.5 for one round per warp.  Requesting the next round's words before this round's arithmetic,
 // in registers or through a cp.async ring in shared memory, measured slower: the variant is bound by
 // per-warp latency with 12-16 warps per SM at 128 registers, not by bytes in flight.)
-template <int BITS, int MH, int GPS, int CPW, bool XC, bool TRACE, bool LOOP = false>
-__global__ void __launch_bounds__(kGemvMaxWarps * 32, (CPW == 1 && MH == 1 && BITS == 4 && !LOOP) ? 3 : 1)
+template <int BITS, bool BF16, int MH, int GPS, int CPW, bool XC, bool TRACE, bool LOOP = false, bool TIGHT = false>
+__global__ void __maxnreg__(gemv_registers(BITS, MH, CPW, LOOP, TIGHT))
 gemv_a16_kernel(const GemvParams p) {
   constexpr int CPWORD = 32 / BITS;   // codes per 32-bit word (8 / 16)
   constexpr int STEPK = 16 * CPWORD;  // k per step (128 / 256)
@@ -153,7 +181,8 @@ gemv_a16_kernel(const GemvParams p) {
   constexpr int FR = 4 * MH;          // output registers per lane
   constexpr uint32_t FIELD = (1u << BITS) - 1u;
   constexpr uint32_t MASK0 = FIELD | (FIELD << 16);
-  constexpr uint32_t ONES = 0x3c003c00u;  // (1.0, 1.0)
+  constexpr uint32_t ONES = BF16 ? 0x3f803f80u : 0x3c003c00u;  // (1.0, 1.0)
+  constexpr int NA = BF16 ? 2 : NT;   // accumulators of a group (bf16: every type has the same weight, two for the chains' length)
 
   __shared__ float red[kGemvMaxWarps * FR * 32];
   const int tid = threadIdx.x;
@@ -253,11 +282,7 @@ gemv_a16_kernel(const GemvParams p) {
       for (int v = 0; v < WPC * XR / 4; ++v) {
         uint4 u = make_uint4(0, 0, 0, 0);
         if (m < p.M) {
-          u = __ldg(xp + v);
-          if (p.bf16) {
-            u.x = bf16x2_to_f16x2_sat(u.x); u.y = bf16x2_to_f16x2_sat(u.y);
-            u.z = bf16x2_to_f16x2_sat(u.z); u.w = bf16x2_to_f16x2_sat(u.w);
-          }
+          asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(xp + v));
         }
         dst[mh][(4 * v) / XR][(4 * v) % XR + 0] = u.x; dst[mh][(4 * v) / XR][(4 * v) % XR + 1] = u.y;
         dst[mh][(4 * v) / XR][(4 * v) % XR + 2] = u.z; dst[mh][(4 * v) / XR][(4 * v) % XR + 3] = u.w;
@@ -282,16 +307,33 @@ gemv_a16_kernel(const GemvParams p) {
           tr[3] = gemv_clock_after(xr[0][0][0]);
           tr[4] = gemv_clock_after(qa[0][0] ^ qb[0][0]);
         }
-        // raw fields times activations: acc[mh][type], and the plain activation sums accx[mh]
-        float acc[MH][NT][4], accx[MH][4];
+        // raw fields times activations.  The plain activation sums come from MMAs whose A operand is the activations and whose B
+        // operand is ones: a token's B fragment is, in the same lane, the upper or lower half of an A fragment, so one such MMA takes
+        // two of them (both token halves, or two field positions): three MMAs where ones times each fragment took four.  (2-bit weights
+        // at 3 to 8 tokens keep ones times each fragment, whose sums are in the lanes that need them: the same time in fp16, and in bf16 the
+        // registers of 2048 -> 2048 in one wave, 3.7 against 4.8 us.)
+        constexpr bool PAIR = BITS == 4 || MH == 2;
+        constexpr int XN = PAIR && BITS == 4 && !LOOP && WPC * MH > 1 ? 2 : 1;  // their accumulators, in turn (registers permitting: the chain's length)
+        float acc[MH][NA][4], accx[XN][4];
+        uint32_t xa0 = 0u, xa2 = 0u;  // the first fragment of the pair
 #pragma unroll
         for (int t = 0; t < WPC; ++t) {
           const uint32_t q0 = qa[i][j * WPC + t], q1 = qb[i][j * WPC + t];
           const uint32_t q0h = q0 >> 8, q1h = q1 >> 8;
 #pragma unroll
           for (int ty = 0; ty < NT; ++ty) {
-            const uint32_t mask = MASK0 << (BITS * ty);
-            const uint32_t a0 = q0 & mask, a1 = q1 & mask, a2 = q0h & mask, a3 = q1h & mask;
+            uint32_t a0, a1, a2, a3;
+            if (BF16) {
+              // the code in the low bits of 128.0's mantissa: 128 + code
+              const int sh = BITS * ty;
+              a0 = lop3_and_or(q0 >> sh, MASK0, 0x43004300u);
+              a1 = lop3_and_or(q1 >> sh, MASK0, 0x43004300u);
+              a2 = lop3_and_or(q0 >> (8 + sh), MASK0, 0x43004300u);
+              a3 = lop3_and_or(q1 >> (8 + sh), MASK0, 0x43004300u);
+            } else {
+              const uint32_t mask = MASK0 << (BITS * ty);
+              a0 = q0 & mask; a1 = q1 & mask; a2 = q0h & mask; a3 = q1h & mask;
+            }
 #pragma unroll
             for (int mh = 0; mh < MH; ++mh) {
               // element a of the word pairs with element a + CPWORD/2: codes e_a and e_(a + CPWORD/2)
@@ -300,16 +342,27 @@ gemv_a16_kernel(const GemvParams p) {
               const uint32_t sel = (ty & 1) ? 0x7632u : 0x5410u;
               const uint32_t b0 = prmt(xw[ty / 2], xw[(ty + CPWORD / 2) / 2], sel);
               const uint32_t b1 = prmt(xw[(ty + NT) / 2], xw[(ty + NT + CPWORD / 2) / 2], sel);
-              if (t == 0) {
-                mma_new(acc[mh][ty], a0, a1, a2, a3, b0, b1);
+              if (t == 0 && ty < NA) {
+                mma_new<BF16>(acc[mh][ty % NA], a0, a1, a2, a3, b0, b1);
               } else {
-                mma_acc(acc[mh][ty], a0, a1, a2, a3, b0, b1);
+                mma_acc<BF16>(acc[mh][ty % NA], a0, a1, a2, a3, b0, b1);
               }
-              if (!XC) {
+              if (!XC && !PAIR) {
                 if (t == 0 && ty == 0) {
-                  mma_new(accx[mh], ONES, ONES, ONES, ONES, b0, b1);
+                  mma_new<BF16>(accx[0], ONES, ONES, ONES, ONES, b0, b1);
                 } else {
-                  mma_acc(accx[mh], ONES, ONES, ONES, ONES, b0, b1);
+                  mma_acc<BF16>(accx[0], ONES, ONES, ONES, ONES, b0, b1);
+                }
+              } else if (!XC) {
+                const bool second = MH == 2 ? mh == 1 : (ty & 1) == 1;
+                const int nth = MH == 2 ? t * NT + ty : (t * NT + ty) / 2;
+                if (!second) {
+                  xa0 = b0;
+                  xa2 = b1;
+                } else if (nth < XN) {
+                  mma_new<BF16>(accx[nth % XN], xa0, b0, xa2, b1, ONES, ONES);
+                } else {
+                  mma_acc<BF16>(accx[nth % XN], xa0, b0, xa2, b1, ONES, ONES);
                 }
               }
             }
@@ -321,12 +374,7 @@ gemv_a16_kernel(const GemvParams p) {
             float sum = 0.f;
 #pragma unroll
             for (int v = 0; v < HPL / 4; ++v) {
-              uint2 u = xu[tok][v];
-              if (p.bf16) {
-                u.x = bf16x2_to_f16x2_sat(u.x);
-                u.y = bf16x2_to_f16x2_sat(u.y);
-              }
-              const float2 f0 = __half22float2(u32_as_h2(u.x)), f1 = __half22float2(u32_as_h2(u.y));
+              const float2 f0 = two_floats<BF16>(xu[tok][v].x), f1 = two_floats<BF16>(xu[tok][v].y);
               sum += f0.x; sum += f0.y; sum += f1.x; sum += f1.y;
             }
 #pragma unroll
@@ -338,18 +386,41 @@ gemv_a16_kernel(const GemvParams p) {
         // once per group: combine the types (a field at bit BITS*ty carries 2^(BITS*ty) times its code;
         // a code in the lowest field is code * 2^-24 as an fp16 number), scale, add zero * sum(x)
         const int gidx = i * GPS + j;
-        const float s0 = table_entry(ts0, gidx) * 16777216.f, s1 = table_entry(ts1, gidx) * 16777216.f;
-        const float z0 = table_entry(tz0, gidx), z1 = table_entry(tz1, gidx);
+        // (bf16: every code is 128 too large, so sum(x) takes zero - 128 * scale)
+        constexpr float kUnit = BF16 ? 1.f : 16777216.f;
+        const float s0 = table_entry(ts0, gidx) * kUnit, s1 = table_entry(ts1, gidx) * kUnit;
+        const float z0 = BF16 ? fmaf(-128.f, s0, table_entry(tz0, gidx)) : table_entry(tz0, gidx);
+        const float z1 = BF16 ? fmaf(-128.f, s1, table_entry(tz1, gidx)) : table_entry(tz1, gidx);
+        float xt[MH][2];  // sums of tokens 2c and 2c + 1
+        if (!XC && PAIR) {  // from the lanes that hold tokens g and g + 8 (MH == 1: two parts of token g's)
+          float lo = accx[0][0], hi = accx[0][2];
+          if (XN > 1) {
+            lo += accx[XN - 1][0];
+            hi += accx[XN - 1][2];
+          }
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            xt[0][r] = __shfl_sync(0xffffffffu, MH == 2 ? lo : lo + hi, 4 * (2 * c + r));
+            if (MH == 2) xt[MH - 1][r] = __shfl_sync(0xffffffffu, hi, 4 * (2 * c + r));
+          }
+        } else if (!XC) {
+          xt[0][0] = accx[0][0];
+          xt[0][1] = accx[0][1];
+        }
 #pragma unroll
         for (int mh = 0; mh < MH; ++mh)
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
-            float tsum = acc[mh][NT - 1][r];
+            float tsum;
+            if (BF16) {
+              tsum = acc[mh][0][r] + acc[mh][1][r];
+            } else {
+              tsum = acc[mh][NA - 1][r];
 #pragma unroll
-            for (int ty = NT - 2; ty >= 0; --ty) tsum = fmaf(tsum, 1.f / float(1 << BITS), acc[mh][ty][r]);
+              for (int ty = NA - 2; ty >= 0; --ty) tsum = fmaf(tsum, 1.f / float(1 << BITS), acc[mh][ty][r]);
+            }
             yv[mh][r] = fmaf(tsum, r < 2 ? s0 : s1, yv[mh][r]);
-            const float xsum = XC ? xs[r & 1][gidx] : accx[mh][r & 1];
-            yv[mh][r] = fmaf(xsum, r < 2 ? z0 : z1, yv[mh][r]);
+            yv[mh][r] = fmaf(XC ? xs[r & 1][gidx] : xt[mh][r & 1], r < 2 ? z0 : z1, yv[mh][r]);
           }
       }
     }
@@ -366,10 +437,10 @@ gemv_a16_kernel(const GemvParams p) {
       if (!first) bias_first = ldg_half(p.bias + n);
       v += bias_first;
     }
-    uint16_t y16 = float_to_out16(v, p.bf16);
+    uint16_t y16 = float_to_out16(v, BF16);
     if (p.act != kActNone || p.residual) {
       if (p.residual && !first) res_first = p.residual[idx];
-      y16 = epilogue16(y16, p.act, p.residual != nullptr, res_first, p.bf16);
+      y16 = epilogue16(y16, p.act, p.residual != nullptr, res_first, BF16);
     }
     p.y[idx] = y16;
   };
@@ -398,59 +469,71 @@ gemv_a16_kernel(const GemvParams p) {
 
 using GemvKernel = void (*)(const GemvParams);
 
-template <int BITS, int MH, int GPS, int CPW>
-GemvKernel kernel_for(bool xc, bool trace) {
+template <int BITS, bool BF16, int MH, int GPS, int CPW>
+GemvKernel kernel_for(bool xc, bool trace, bool tight) {
 #ifdef ASRQ_TRACE
   if (trace) {
-    if (MH == 1 && xc) return gemv_a16_kernel<BITS, 1, GPS, CPW, true, true>;
-    return gemv_a16_kernel<BITS, MH, GPS, CPW, false, true>;
+    if (MH == 1 && xc) return gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, true>;
+    return gemv_a16_kernel<BITS, BF16, MH, GPS, CPW, false, true>;
   }
 #endif
   (void)trace;  // the shipped library holds no trace variants
-  if (MH == 1 && xc) return gemv_a16_kernel<BITS, 1, GPS, CPW, true, false>;
-  return gemv_a16_kernel<BITS, MH, GPS, CPW, false, false>;
+  if (gemv_has_tight(BITS, MH, CPW) && tight) {
+    constexpr bool T = gemv_has_tight(BITS, MH, CPW);
+    return xc ? gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, false, false, T> : gemv_a16_kernel<BITS, BF16, MH, GPS, CPW, false, false, false, T>;
+  }
+  if (MH == 1 && xc) return gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, false>;
+  return gemv_a16_kernel<BITS, BF16, MH, GPS, CPW, false, false>;
 }
-template <int BITS, int MH>
-GemvKernel kernel_for(int gps, int cpw, bool xc, bool trace) {
+template <int BITS, bool BF16, int MH>
+GemvKernel kernel_for(int gps, int cpw, bool xc, bool trace, bool tight) {
   switch (gps * 8 + cpw) {
-    case 1 * 8 + 1: return kernel_for<BITS, MH, 1, 1>(xc, trace);
-    case 1 * 8 + 2: return kernel_for<BITS, MH, 1, 2>(xc, trace);
-    case 1 * 8 + 4: return kernel_for<BITS, MH, 1, 4>(xc, trace);
-    case 2 * 8 + 1: return kernel_for<BITS, MH, 2, 1>(xc, trace);
-    case 2 * 8 + 2: return kernel_for<BITS, MH, 2, 2>(xc, trace);
-    case 2 * 8 + 4: return kernel_for<BITS, MH, 2, 4>(xc, trace);
-    case 4 * 8 + 1: return kernel_for<BITS, MH, 4, 1>(xc, trace);
-    case 4 * 8 + 2: return kernel_for<BITS, MH, 4, 2>(xc, trace);
+    case 1 * 8 + 1: return kernel_for<BITS, BF16, MH, 1, 1>(xc, trace, tight);
+    case 1 * 8 + 2: return kernel_for<BITS, BF16, MH, 1, 2>(xc, trace, tight);
+    case 1 * 8 + 4: return kernel_for<BITS, BF16, MH, 1, 4>(xc, trace, tight);
+    case 2 * 8 + 1: return kernel_for<BITS, BF16, MH, 2, 1>(xc, trace, tight);
+    case 2 * 8 + 2: return kernel_for<BITS, BF16, MH, 2, 2>(xc, trace, tight);
+    case 2 * 8 + 4: return kernel_for<BITS, BF16, MH, 2, 4>(xc, trace, tight);
+    case 4 * 8 + 1: return kernel_for<BITS, BF16, MH, 4, 1>(xc, trace, tight);
+    case 4 * 8 + 2: return kernel_for<BITS, BF16, MH, 4, 2>(xc, trace, tight);
     default: return nullptr;
   }
 }
 // LOOP variants: the most steps per round the group table allows (CPW * GPS <= 8), no trace build
-template <int BITS, int MH>
+template <int BITS, bool BF16, int MH>
 GemvKernel loop_kernel_for(int gps, bool xc, int* cpw) {
   *cpw = gps == 4 ? 2 : 4;
   if (MH == 1 && xc) {
     switch (gps) {
-      case 1: return gemv_a16_kernel<BITS, 1, 1, 4, true, false, true>;
-      case 2: return gemv_a16_kernel<BITS, 1, 2, 4, true, false, true>;
-      case 4: return gemv_a16_kernel<BITS, 1, 4, 2, true, false, true>;
+      case 1: return gemv_a16_kernel<BITS, BF16, 1, 1, 4, true, false, true>;
+      case 2: return gemv_a16_kernel<BITS, BF16, 1, 2, 4, true, false, true>;
+      case 4: return gemv_a16_kernel<BITS, BF16, 1, 4, 2, true, false, true>;
       default: return nullptr;
     }
   }
   switch (gps) {
-    case 1: return gemv_a16_kernel<BITS, MH, 1, 4, false, false, true>;
-    case 2: return gemv_a16_kernel<BITS, MH, 2, 4, false, false, true>;
-    case 4: return gemv_a16_kernel<BITS, MH, 4, 2, false, false, true>;
+    case 1: return gemv_a16_kernel<BITS, BF16, MH, 1, 4, false, false, true>;
+    case 2: return gemv_a16_kernel<BITS, BF16, MH, 2, 4, false, false, true>;
+    case 4: return gemv_a16_kernel<BITS, BF16, MH, 4, 2, false, false, true>;
     default: return nullptr;
   }
 }
-GemvKernel loop_kernel_for(int bits, int mh, int gps, bool xc, int* cpw) {
-  if (bits == 4) return mh == 1 ? loop_kernel_for<4, 1>(gps, xc, cpw) : loop_kernel_for<4, 2>(gps, xc, cpw);
-  return mh == 1 ? loop_kernel_for<2, 1>(gps, xc, cpw) : loop_kernel_for<2, 2>(gps, xc, cpw);
+template <int BITS, bool BF16>
+GemvKernel loop_kernel_for(int mh, int gps, bool xc, int* cpw) {
+  return mh == 1 ? loop_kernel_for<BITS, BF16, 1>(gps, xc, cpw) : loop_kernel_for<BITS, BF16, 2>(gps, xc, cpw);
+}
+GemvKernel loop_kernel_for(int bits, bool bf16, int mh, int gps, bool xc, int* cpw) {
+  if (bits == 4) return bf16 ? loop_kernel_for<4, true>(mh, gps, xc, cpw) : loop_kernel_for<4, false>(mh, gps, xc, cpw);
+  return bf16 ? loop_kernel_for<2, true>(mh, gps, xc, cpw) : loop_kernel_for<2, false>(mh, gps, xc, cpw);
 }
 
-GemvKernel kernel_for(int bits, int mh, int gps, int cpw, bool xc, bool trace) {
-  if (bits == 4) return mh == 1 ? kernel_for<4, 1>(gps, cpw, xc, trace) : kernel_for<4, 2>(gps, cpw, xc, trace);
-  return mh == 1 ? kernel_for<2, 1>(gps, cpw, xc, trace) : kernel_for<2, 2>(gps, cpw, xc, trace);
+template <int BITS, bool BF16>
+GemvKernel kernel_for(int mh, int gps, int cpw, bool xc, bool trace, bool tight) {
+  return mh == 1 ? kernel_for<BITS, BF16, 1>(gps, cpw, xc, trace, tight) : kernel_for<BITS, BF16, 2>(gps, cpw, xc, trace, tight);
+}
+GemvKernel kernel_for(int bits, bool bf16, int mh, int gps, int cpw, bool xc, bool trace, bool tight) {
+  if (bits == 4) return bf16 ? kernel_for<4, true>(mh, gps, cpw, xc, trace, tight) : kernel_for<4, false>(mh, gps, cpw, xc, trace, tight);
+  return bf16 ? kernel_for<2, true>(mh, gps, cpw, xc, trace, tight) : kernel_for<2, false>(mh, gps, cpw, xc, trace, tight);
 }
 
 // How one launch splits K inside a block: a warp takes CPW steps (1, 2 or 4) and KQ warps (1..16)
@@ -463,7 +546,7 @@ struct GemvSplit {
   int R = 1;        // rounds per warp (LOOP variants)
 };
 
-GemvSplit gemv_pick_split(int bits, int mh, int gps, bool xc, bool trace, int64_t N, int64_t K, int sm_count) {
+GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool trace, int64_t N, int64_t K, int sm_count) {
   const int stepk = bits == 4 ? 128 : 256;
   const int steps = int(K / stepk);
   const int cpw_env = option(kOptGemvCpw);  // tuning knob
@@ -475,15 +558,23 @@ GemvSplit gemv_pick_split(int bits, int mh, int gps, bool xc, bool trace, int64_
     if (steps % cpw || steps / cpw > kGemvMaxWarps || cpw * gps > 8) continue;
     if (cpw_env && cpw != cpw_env) continue;
     const int kq = steps / cpw;
-    GemvKernel k = kernel_for(bits, mh, gps, cpw, xc, trace);
-    if (!k) continue;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kq, 0) != cudaSuccess || per_sm < 1) {
-      cudaGetLastError();
-      continue;
+    GemvKernel k = nullptr;
+    long waves = 0;
+    for (int tight = 0; tight <= int(gemv_has_tight(bits, mh, cpw) && !trace); ++tight) {
+      GemvKernel form = kernel_for(bits, bf16, mh, gps, cpw, xc, trace, tight != 0);
+      if (!form) continue;
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form, 32 * kq, 0) != cudaSuccess || per_sm < 1) {
+        cudaGetLastError();
+        continue;
+      }
+      const long slots = long(per_sm) * sm_count;
+      const long w = (long(N / 16) + slots - 1) / slots;
+      if (k && w >= waves) continue;  // the tight form only where it saves a wave
+      k = form;
+      waves = w;
     }
-    const long slots = long(per_sm) * sm_count;
-    const long waves = (long(N / 16) + slots - 1) / slots;
+    if (!k) continue;
     // Fewest waves first.  Among those, 8 to 12 warps per block measured fastest on the decode
     // shapes (16 warps pay more for the shared-memory reduction and the block-wide barrier, 4 to 6
     // leave too few loads in flight): the largest count up to 12, else the smallest above.
@@ -501,7 +592,7 @@ GemvSplit gemv_pick_split(int bits, int mh, int gps, bool xc, bool trace, int64_
   const bool large = N * K * bits / 8 >= (int64_t(16) << 20);
   if (!trace && loop_env != 0 && (!best.kern || (best_waves > 1 && (large || loop_env == 1)))) {
     int cpw = 0;
-    GemvKernel k = loop_kernel_for(bits, mh, gps, xc, &cpw);
+    GemvKernel k = loop_kernel_for(bits, bf16, mh, gps, xc, &cpw);
     static const int kq_order[] = {4, 8, 2, 16, 1};
     for (int kq : kq_order) {
       if (!k || steps % (kq * cpw)) continue;
@@ -516,8 +607,8 @@ GemvSplit gemv_pick_split(int bits, int mh, int gps, bool xc, bool trace, int64_
   return best;
 }
 
-// the choice costs a few occupancy queries: keep it per (bits, class, groups per step, N, K, device SMs)
-GemvSplit cached_split(int bits, int cls, int gps, bool trace, int64_t N, int64_t K, int sm_count) {
+// the choice costs a few occupancy queries: keep it per (bits, type, class, groups per step, N, K, device SMs)
+GemvSplit cached_split(int bits, bool bf16, int cls, int gps, bool trace, int64_t N, int64_t K, int sm_count) {
   struct Entry {
     uint64_t key;
     GemvSplit sp;
@@ -533,13 +624,13 @@ GemvSplit cached_split(int bits, int cls, int gps, bool trace, int64_t N, int64_
     }
   }
   const uint64_t key = (uint64_t(N) << 40) ^ (uint64_t(K) << 16) ^ (uint64_t(sm_count) << 6) ^ (uint64_t(gps) << 3) ^
-                       (uint64_t(cls) << 1) ^ uint64_t(bits == 4);
+                       (uint64_t(cls) << 1) ^ uint64_t(bits == 4) ^ (uint64_t(bf16) << 63);
   {
     std::lock_guard<std::mutex> lock(mu);
     for (const Entry& e : cache)
       if (e.key == key) return e.sp;
   }
-  const GemvSplit sp = gemv_pick_split(bits, cls == 2 ? 2 : 1, gps, cls == 0, trace, N, K, sm_count);
+  const GemvSplit sp = gemv_pick_split(bits, bf16, cls == 2 ? 2 : 1, gps, cls == 0, trace, N, K, sm_count);
   std::lock_guard<std::mutex> lock(mu);
   if (cache.size() < 4096) cache.push_back({key, sp});
   return sp;
@@ -619,7 +710,7 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
   for (int cls = 0; cls < 3; ++cls) {
     const bool needed = cls == 2 ? M > 8 : (cls == 1 ? (M % 16 > 2 && M % 16 <= 8) : (M % 16 >= 1 && M % 16 <= 2));
     if (!needed) continue;
-    split[cls] = cached_split(bits, cls, gps, trace, N, K, sm_count);
+    split[cls] = cached_split(bits, dtype == ASRQ_BF16, cls, gps, trace, N, K, sm_count);
     if (!split[cls].kern)
       return gemv_a16_splitk(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace,
                              workspace_bytes, sm_count, stream, max_split);
@@ -632,7 +723,6 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
   p.N = int(N);
   p.K = int(K);
   p.groups_per_row = int(K / group_size);
-  p.bf16 = dtype == ASRQ_BF16;
   p.act = ep.act;
   *fused = true;
   // diagnostic marks go to the (otherwise unused) partial-sum area of the workspace
