@@ -13,11 +13,13 @@
 // round-half-even, packed two's-complement nibbles, even k in the low nibble.
 #include <cuda_fp8.h>
 
-#include "common.cuh"
+#include <algorithm>
+
+#include "tcgen05.cuh"
 
 namespace asrq {
 
-int ensure_dynamic_smem(const void* kernel, size_t bytes);
+int current_device_sm_count(int* sm_count);
 
 constexpr int kQuantWarps = 4;
 
@@ -209,8 +211,7 @@ quant_int4_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, floa
 
 // K = 1024 and 4096: 32 and 64 threads per token, each with 32 and 64 values, and ONE transpose through shared memory where the
 // kernel above has five levels of shuffles:
-//   phase A  thread t holds the T consecutive elements t * T + e (staged through shared memory, so that the loads are whole
-//            lines): strides 1 .. T / 2;
+//   phase A  thread t holds the T consecutive elements t * T + e: strides 1 .. T / 2;
 //   phase B  thread u holds the elements o * T + u, o = 0..T-1: strides T .. K / 2.  Four neighbouring threads transpose their
 //            4 x 4 bytes of codes by two shuffles per word, so that a warp stores whole 32-byte sectors.
 // The strides are taken in ascending order, as everywhere in this file: another order rounds differently, and behind four bits a
@@ -218,12 +219,7 @@ quant_int4_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, floa
 // Values live as pairs, so every butterfly but the one inside the pair is a packed fp32 add and a packed subtract (add.f32x2 /
 // fma.f32x2) on two pairs.  Rows of the transpose are padded by four floats: its 4-byte writes and 16-byte reads are free of bank
 // conflicts.
-// Bound: the latencies of a token's own chain -- load, barrier, transpose, barrier, store -- with the sixteen warps per SM that 104
-// registers leave (eight tokens of 4096): of the issue slots 44% are taken, of DRAM's time 23%, no pipe is above 31%, and the
-// stalls are spread over shared memory, fixed latencies and loads.  In chains of launches, us, one warp per token of 4096 and five
-// levels of shuffles for 1024 -> this kernel: 4096 wide, 6000 tokens 25.4 -> 24.3 (3.0 TB/s; 11 by bytes), 250 tokens 5.0 -> 4.3,
-// one 4.6 -> 2.7; 1024 wide 14.3 -> 7.1, 4.4 -> 2.0, 4.2 -> 1.8.  Long calls of 4096 gain next to nothing, short ones the overlap of
-// launches.  256, 512 and 2048, which no layer of the models here has, stay with the kernel above: 512 and 2048 are no squares.
+// 256, 512 and 2048, which no layer of the models here has, stay with the kernel above: 512 and 2048 are no squares.
 // The division by sqrt(K) = 32 or 64 is exact and is applied to the scale only: rint((v/64) / (s/64)) is rint(v/s) bit for bit.
 // Quantisation without a division per element: t_lo = fma(v, inv_lo, magic), t_hi = fma(v, inv_hi,
 // magic) with inv_lo < 1/s < inv_hi (2^-22 apart) bracket the exact quotient, and adding 1.5*2^23
@@ -239,28 +235,39 @@ __device__ __noinline__ float4 quant4_exact(float2 v01, float2 v23, float s) {
                      __fadd_rn(rintf(__fdiv_rn(v23.x, s)), 12582912.f), __fadd_rn(rintf(__fdiv_rn(v23.y, s)), 12582912.f));
 }
 
-// codes of four values: OUT 0 and 1 as bytes b0..b3 = low byte of each t (t = magic + code), OUT 2 as e4m3 bytes
+// Codes of eight values as two words: OUT 0 and 1 as bytes b0..b3 = low byte of each t (t = magic + code), OUT 2 as e4m3 bytes
 template <int OUT>
-__device__ __forceinline__ uint32_t quant4_bytes(float2 v01, float2 v23, float2 inv_lo, float2 inv_hi, float s) {
+__device__ __forceinline__ void quant8_bytes(const float2 (&v)[4], float2 inv_lo, float2 inv_hi, float s, uint32_t (&out)[2]) {
   const float2 magic = make_float2(12582912.f, 12582912.f);
-  float2 a = __ffma2_rn(v01, inv_lo, magic), b = __ffma2_rn(v23, inv_lo, magic);
-  const float2 a2 = __ffma2_rn(v01, inv_hi, magic), b2 = __ffma2_rn(v23, inv_hi, magic);
-  const uint32_t diff = (__float_as_uint(a.x) ^ __float_as_uint(a2.x)) | (__float_as_uint(a.y) ^ __float_as_uint(a2.y)) |
-                        (__float_as_uint(b.x) ^ __float_as_uint(b2.x)) | (__float_as_uint(b.y) ^ __float_as_uint(b2.y));
+  float2 a[4];
+  uint32_t diff = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    a[i] = __ffma2_rn(v[i], inv_lo, magic);
+    const float2 h = __ffma2_rn(v[i], inv_hi, magic);
+    diff |= __float_as_uint(a[i].x) ^ __float_as_uint(h.x);
+    diff |= __float_as_uint(a[i].y) ^ __float_as_uint(h.y);
+  }
   if (diff != 0) {  // an element within 4e-6 of a rounding boundary: IEEE division
-    const float4 e = quant4_exact(v01, v23, s);
-    a = make_float2(e.x, e.y);
-    b = make_float2(e.z, e.w);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 e = quant4_exact(v[2 * i], v[2 * i + 1], s);
+      a[2 * i] = make_float2(e.x, e.y);
+      a[2 * i + 1] = make_float2(e.z, e.w);
+    }
   }
-  if (OUT == 2) {
-    const float2 nm = make_float2(-12582912.f, -12582912.f);
-    a = __fadd2_rn(a, nm);  // exact: the code as a float
-    b = __fadd2_rn(b, nm);
-    return e4m3x2(a.x, a.y) | (e4m3x2(b.x, b.y) << 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    float2 p = a[2 * i], q = a[2 * i + 1];
+    if (OUT == 2) {
+      const float2 nm = make_float2(-12582912.f, -12582912.f);
+      p = __fadd2_rn(p, nm);  // exact: the code as a float
+      q = __fadd2_rn(q, nm);
+      out[i] = e4m3x2(p.x, p.y) | (e4m3x2(q.x, q.y) << 16);
+    } else {
+      out[i] = prmt(prmt(__float_as_uint(p.x), __float_as_uint(p.y), 0x0040u), prmt(__float_as_uint(q.x), __float_as_uint(q.y), 0x0040u), 0x5410u);
+    }
   }
-  const uint32_t p01 = prmt(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040u);
-  const uint32_t p23 = prmt(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040u);
-  return prmt(p01, p23, 0x5410u);
 }
 
 // log2 levels over an array of pairs: strides of 1 .. N / 2 pairs
@@ -282,60 +289,98 @@ __device__ __forceinline__ void inside_pairs(float2 (&P)[N]) {
   for (int j = 0; j < N; ++j) P[j] = make_float2(P[j].x + P[j].y, P[j].x - P[j].y);
 }
 
-template <int K, int T>
-constexpr int kHadTokens = T == 64 ? 1 : 4;  // per block
-
-template <int K, int T, int OUT, bool BF16>
-__global__ void __launch_bounds__(T * kHadTokens<K, T>, T == 64 ? 8 : 5)
-hadamard_transpose_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {
-  constexpr int PITCH = T + 4, TOKENS = kHadTokens<K, T>, UNITS = T / 8;  // 16-byte units per thread
-  static_assert(K == T * T, "one row of the transpose per thread");
-  __shared__ __align__(16) float rows_all[TOKENS][T * PITCH];  // the 16-bit input is staged in its first half
-  __shared__ float part[2];
+template <int N>
+__device__ __forceinline__ float largest(const float2 (&P)[N]) {
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < N; ++j) amax = fmaxf(amax, fmaxf(fabsf(P[j].x), fabsf(P[j].y)));
+#pragma unroll
+  for (int mask = 16; mask > 0; mask >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, mask));
+  return amax;
+}
+// scale of the unnormalised values, with the bracket of its reciprocal; the token's scale is that / sqrt(K) (exact)
+struct CodeScale {
+  float s;
+  float2 inv_lo, inv_hi;
+};
+template <int K>
+__device__ __forceinline__ CodeScale code_scale(float amax, float* sa) {
+  CodeScale c;
+  c.s = __fdiv_rn(amax, 7.f);
+  const bool zero = c.s == 0.f;
+  if (sa) *sa = zero ? 1e-3f : c.s * (K == 4096 ? 0.015625f : 0.03125f);
+  if (zero) c.s = 1.f;  // every value is 0: any scale gives code 0
+  const float inv = __fdiv_rn(1.f, c.s);
+  const float il = inv * (1.f - 2.384185791015625e-07f), ih = inv * (1.f + 2.384185791015625e-07f);  // 2^-22
+  c.inv_lo = make_float2(il, il);
+  c.inv_hi = make_float2(ih, ih);
+  return c;
+}
+// Codes of twice four values that lie a row of memory apart each, held by each of four neighbouring lanes at neighbouring places
+// of these rows: after the exchange a lane has four neighbouring places of row (lane & 3) of either four, which go to elements
+// at0 and at1 of the token.
+template <int K, int OUT>
+__device__ __forceinline__ void store_codes(const float2 (&v)[4], const CodeScale& c, int lane, uint8_t* __restrict__ qa, int64_t token, int at0, int at1) {
+  const uint32_t sel1 = (lane & 2) ? 0x3276u : 0x5410u, sel2 = (lane & 1) ? 0x3715u : 0x6240u;
+  uint32_t w[2];
+  quant8_bytes<OUT>(v, c.inv_lo, c.inv_hi, c.s, w);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    uint32_t b = prmt(w[i], __shfl_xor_sync(0xffffffffu, w[i], 2), sel1);
+    b = prmt(b, __shfl_xor_sync(0xffffffffu, b, 1), sel2);
+    const int at = i ? at1 : at0;
+    if (OUT >= 1) {
+      *reinterpret_cast<uint32_t*>(qa + size_t(token) * K + at) = OUT == 1 ? (b << 4) & 0xf0f0f0f0u : b;
+    } else {
+      const uint32_t n = b & 0x0f0f0f0fu, m = n | (n >> 4);  // bytes 0 and 2 hold two nibbles each, element 0 lowest
+      *reinterpret_cast<uint16_t*>(qa + size_t(token) * (K / 2) + at / 2) = uint16_t((m & 0xffu) | ((m >> 8) & 0xff00u));
+    }
+  }
+}
+template <bool BF16, int N>
+__device__ __forceinline__ void unpack8(const uint4& q, float2 (&P)[N], int at) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    P[at + e] = BF16 ? make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u)) : __half22float2(u32_as_h2(w[e]));
+}
+// K = 1024: a warp per token, four to a block
+template <int OUT, bool BF16>
+__global__ void __launch_bounds__(128, 5)
+hadamard_1024_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {
+  constexpr int K = 1024, T = 32, PITCH = T + 4, UNITS = T / 8;  // 16-byte units per thread
+  __shared__ __align__(16) float rows_all[4][T * PITCH];  // the 16-bit input is staged in its first half
   // A GEMM launched behind this kernel with programmatic stream serialisation may be scheduled once
   // every block of this grid has started, and set itself up on SMs the last wave leaves idle; it
   // orders itself with griddepcontrol.wait before it touches this kernel's output.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int t = threadIdx.x % T, token = blockIdx.x * TOKENS + threadIdx.x / T;
+  const int t = threadIdx.x % T, token = blockIdx.x * 4 + threadIdx.x / T;
   float* rows = rows_all[threadIdx.x / T];
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (token >= M) return;  // a whole warp, which meets no other (T = 32), or nobody (T = 64)
-  auto meet = [&]() {
-    if (T == 64) {
-      __syncthreads();
-    } else {
-      __syncwarp();
-    }
-  };
+  if (token >= M) return;  // a whole warp, which meets no other
   const uint4* src = reinterpret_cast<const uint4*>(x + size_t(token) * K) + t;
   uint4* stage = reinterpret_cast<uint4*>(rows);
-  auto slot = [](int owner, int j) { return owner * UNITS + (T == 64 ? (j ^ (owner & 7)) : (j ^ ((owner >> 1) & 3))); };  // conflict-free both ways
+  auto slot = [](int owner, int j) { return owner * UNITS + (j ^ ((owner >> 1) & 3)); };  // conflict-free both ways
   uint4 raw[UNITS];
 #pragma unroll
   for (int i = 0; i < UNITS; ++i) raw[i] = __ldg(src + i * T);
 #pragma unroll
   for (int i = 0; i < UNITS; ++i) stage[slot((i * T + t) / UNITS, (i * T + t) % UNITS)] = raw[i];
-  meet();
+  __syncwarp();
   {
     float2 P[T / 2];
 #pragma unroll
-    for (int i = 0; i < UNITS; ++i) {
-      const uint4 q = stage[slot(t, i)];
-      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        P[4 * i + e] = BF16 ? make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u)) : __half22float2(u32_as_h2(w[e]));
-    }
+    for (int i = 0; i < UNITS; ++i) unpack8<BF16>(stage[slot(t, i)], P, 4 * i);
     inside_pairs(P);
     butterflies(P);
-    meet();  // the staged rows have been read
+    __syncwarp();  // the staged rows have been read
 #pragma unroll
     for (int i = 0; i < T / 2; ++i) {
       rows[(2 * i) * PITCH + t] = P[i].x;
       rows[(2 * i + 1) * PITCH + t] = P[i].y;
     }
   }
-  meet();
+  __syncwarp();
   float2 Q[T / 2];
 #pragma unroll
   for (int k = 0; k < T / 4; ++k) {
@@ -345,60 +390,123 @@ hadamard_transpose_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restr
   }
   inside_pairs(Q);
   butterflies(Q);
-  float amax = 0.f;
+  const CodeScale c = code_scale<K>(largest(Q), t == 0 ? sa + token : nullptr);
 #pragma unroll
-  for (int j = 0; j < T / 2; ++j) amax = fmaxf(amax, fmaxf(fabsf(Q[j].x), fabsf(Q[j].y)));
-#pragma unroll
-  for (int mask = 16; mask > 0; mask >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, mask));
-  if (T == 64) {
-    if ((t & 31) == 0) part[t >> 5] = amax;
-    meet();
-    amax = fmaxf(part[0], part[1]);
+  for (int k = 0; k < T / 8; ++k) {
+    const float2 v[4] = {Q[4 * k], Q[4 * k + 1], Q[4 * k + 2], Q[4 * k + 3]};
+    const int at = (8 * k + (t & 3)) * T + (t & ~3);
+    store_codes<K, OUT>(v, c, t, qa, token, at, at + 4 * T);
   }
-  // scale of the unnormalised values; the token's scale is that / sqrt(K) (exact)
-  float s = __fdiv_rn(amax, 7.f);
-  const bool zero = s == 0.f;
-  if (t == 0) sa[token] = zero ? 1e-3f : s * (K == 4096 ? 0.015625f : 0.03125f);
-  if (zero) s = 1.f;  // every value is 0: any scale gives code 0
-  const float inv = __fdiv_rn(1.f, s);
-  const float il = inv * (1.f - 2.384185791015625e-07f), ih = inv * (1.f + 2.384185791015625e-07f);  // 2^-22
-  const float2 inv_lo = make_float2(il, il), inv_hi = make_float2(ih, ih);
-  const uint32_t sel1 = (t & 2) ? 0x3276u : 0x5410u, sel2 = (t & 1) ? 0x3715u : 0x6240u;
-  const size_t first = size_t(t & 3) * T + (t & ~3);  // this thread's four elements of o = 4 k + (t & 3)
+}
+
+// The wait for this block's own copy, bounded like every wait of the library.
+__device__ __forceinline__ bool wait_landed(uint32_t bar, uint32_t parity) {
+  if (tc::mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (clock64() - t0 <= tc::kWaitCycles)
+    if (tc::mbar_try_wait(bar, parity)) return true;
+  return false;
+}
+
+// K = 4096: 64 threads per token, each with 64 values, in blocks that walk the tokens.
+// A token's 8 KB arrive by one bulk copy, asked for as soon as the token before has been read from the same place, and lie as in
+// memory.  Thread t's 128 bytes all start in the same bank, so it takes its eight 16-byte units in the order i ^ r, r = t % 8.  Place i
+// then holds unit i ^ r, and for the strides between units (8, 16, 32) the partners of a butterfly have changed places where their
+// bit of r is set: the sum is the same, the difference has the other sign, which changes nothing in how it rounds.  After phase A
+// place i holds unit i with the sign (-1)^popcount(i & r): over the o of phase B a Walsh function, under which the butterflies of
+// strides T, 2 T and 4 T exchange their results.  Place m after phase B is o = m ^ s, s = t / 8, and the codes are stored accordingly;
+// no sign is ever put back.
+// Bound: instruction issue (about 2 300 warp instructions a token, a third of them packed ones and conversions that issue at half rate
+// or less; ncu: 56% of the issue slots).  128 threads of 32 values with two transposes and 32 warps per SM: 24.9 us for 6 000
+// tokens; more warps of this code, at 80 registers: no change.  Chains of launches, loads in the chain and a branch per four codes -> this
+// form, us: one token 2.6 -> 2.3, 250 4.6 -> 4.0, 6 000 23.6 -> 22.6, 16 000 57.8 -> 53.9; the 1024-wide kernel with a branch per eight codes
+// 1.74 -> 1.57, 2.0 -> 1.87, 6.9 -> 6.8, 13.45 -> 13.7.
+template <int OUT, bool BF16>
+__global__ void __launch_bounds__(64, 8)
+hadamard_4096_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {
+  constexpr int K = 4096, T = 64, PITCH = T + 4, UNITS = T / 8;
+  __shared__ __align__(128) uint4 stage[K / 8];
+  __shared__ __align__(16) float rows[T * PITCH];
+  __shared__ float part[2];
+  __shared__ __align__(8) uint64_t full;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int t = threadIdx.x;
+  const uint32_t bar = tc::smem_u32(&full), dst = tc::smem_u32(stage);
+  auto fetch = [&](int token) {
+    tc::mbar_arrive_expect_tx(bar, K * 2);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(x + size_t(token) * K), "r"(K * 2), "r"(bar)
+                 : "memory");
+  };
+  if (t == 0) {
+    tc::mbar_init(bar, 1);
+    tc::fence_barrier_init();
+    tc::fence_proxy_async_smem();
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (t == 0) fetch(blockIdx.x);
+  __syncthreads();
+  const int s = t >> 3;
+  uint32_t ph = 0;
+  for (int token = blockIdx.x; token < M; token += gridDim.x, ph ^= 1u) {
+    const bool landed = wait_landed(bar, ph);
+    {
+      float2 P[T / 2];
 #pragma unroll
-  for (int k = 0; k < T / 4; ++k) {
-    uint32_t w = quant4_bytes<OUT>(Q[2 * k], Q[2 * k + 1], inv_lo, inv_hi, s);  // element u of o = 4 k .. 4 k + 3
-    w = prmt(w, __shfl_xor_sync(0xffffffffu, w, 2), sel1);
-    w = prmt(w, __shfl_xor_sync(0xffffffffu, w, 1), sel2);  // elements u & ~3 .. of o = 4 k + (t & 3)
-    const size_t at = first + size_t(4 * k) * T;
-    if (OUT >= 1) {
-      *reinterpret_cast<uint32_t*>(qa + size_t(token) * K + at) = OUT == 1 ? (w << 4) & 0xf0f0f0f0u : w;
-    } else {
-      const uint32_t n = w & 0x0f0f0f0fu, m = n | (n >> 4);  // bytes 0 and 2 hold two nibbles each, element 0 lowest
-      *reinterpret_cast<uint16_t*>(qa + size_t(token) * (K / 2) + at / 2) = uint16_t((m & 0xffu) | ((m >> 8) & 0xff00u));
+      for (int i = 0; i < UNITS; ++i) unpack8<BF16>(stage[t * UNITS + (i ^ (t & 7))], P, 4 * i);
+      inside_pairs(P);
+      butterflies(P);
+#pragma unroll
+      for (int i = 0; i < T / 2; ++i) {
+        rows[(2 * i) * PITCH + t] = P[i].x;
+        rows[(2 * i + 1) * PITCH + t] = P[i].y;
+      }
+    }
+    __syncthreads();  // the transpose is written and the staged bytes have been read
+    if (t == 0 && token + int(gridDim.x) < M) fetch(token + gridDim.x);
+    float2 Q[T / 2];
+#pragma unroll
+    for (int k = 0; k < T / 4; ++k) {
+      const float4 z = *reinterpret_cast<const float4*>(rows + t * PITCH + 4 * k);
+      Q[2 * k] = make_float2(z.x, z.y);
+      Q[2 * k + 1] = make_float2(z.z, z.w);
+    }
+    inside_pairs(Q);
+    butterflies(Q);
+    const float m = largest(Q);
+    if ((t & 31) == 0) part[t >> 5] = m;
+    __syncthreads();  // also: the transpose has been read, the next token's may be written
+    const CodeScale c = code_scale<K>(fmaxf(part[0], part[1]), t == 0 ? sa + token : nullptr);
+    if (!landed && t == 0) sa[token] = __int_as_float(0x7fc00000);  // gave up waiting: the token's outputs are NaN
+#pragma unroll
+    for (int k = 0; k < T / 8; ++k) {
+      const float2 v[4] = {Q[4 * k], Q[4 * k + 1], Q[4 * k + 2], Q[4 * k + 3]};
+      const int at = ((8 * k + (t & 3)) ^ s) * T + (t & ~3);
+      store_codes<K, OUT>(v, c, t, qa, token, at, at ^ (4 * T));
     }
   }
 }
 
-template <int K, int T, int OUT, bool BF16>
-static int launch_transpose_quant(const uint16_t* xp, uint8_t* qa, float* sa, int64_t M, cudaStream_t stream) {
-  constexpr int TOKENS = kHadTokens<K, T>;
+static int launch_had(void (*kern)(const uint16_t*, uint8_t*, float*, int), int64_t blocks, int threads, const uint16_t* xp, uint8_t* qa, float* sa,
+                      int64_t M, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned((M + TOKENS - 1) / TOKENS));
-  cfg.blockDim = dim3(T * TOKENS);
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(threads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = option(kOptNoPdl) ? 0 : 1;
-  ASRQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, hadamard_transpose_quant_kernel<K, T, OUT, BF16>, xp, qa, sa, int(M)));
+  ASRQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, xp, qa, sa, int(M)));
   return ASRQ_OK;
 }
 
 template <int OUT>
 static int launch_quant(const uint16_t* xp, uint8_t* qa, float* sa, int64_t M, int64_t K, int hadamard, int bf16,
                         cudaStream_t stream) {
+  int sm_count = 0;
+  if (const int rc = current_device_sm_count(&sm_count)) return rc;
   const int blocks = int((M + kQuantWarps - 1) / kQuantWarps);
   const int thr = kQuantWarps * 32;
   if (!hadamard) {
@@ -409,10 +517,11 @@ static int launch_quant(const uint16_t* xp, uint8_t* qa, float* sa, int64_t M, i
       case 256: hadamard_quant_kernel<8, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
       case 512: hadamard_quant_kernel<16, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
       case 1024:
-        return bf16 ? launch_transpose_quant<1024, 32, OUT, true>(xp, qa, sa, M, stream) : launch_transpose_quant<1024, 32, OUT, false>(xp, qa, sa, M, stream);
+        return launch_had(bf16 ? hadamard_1024_quant_kernel<OUT, true> : hadamard_1024_quant_kernel<OUT, false>, (M + 3) / 4, 128, xp, qa, sa, M, stream);
       case 2048: hadamard_quant_kernel<64, OUT><<<blocks, thr, 0, stream>>>(xp, qa, sa, int(M), int(K), bf16); break;
       case 4096:
-        return bf16 ? launch_transpose_quant<4096, 64, OUT, true>(xp, qa, sa, M, stream) : launch_transpose_quant<4096, 64, OUT, false>(xp, qa, sa, M, stream);
+        return launch_had(bf16 ? hadamard_4096_quant_kernel<OUT, true> : hadamard_4096_quant_kernel<OUT, false>, std::min<int64_t>(M, 8 * sm_count), 64, xp,
+                          qa, sa, M, stream);
       default:
         return fail(ASRQ_ERR_SHAPE, "hadamard_quant_int4: K must be 256, 512, 1024, 2048 or 4096 (K=%lld)",
                     (long long)K);

@@ -314,3 +314,13 @@ def test_w4a4_gemm_rejects_bad_group_size():
             _lib.call("asrq_w4a4_gemm", p.data_ptr(), p.data_ptr(), p.data_ptr(), p.data_ptr(), None, p.data_ptr(), None,
                       8, 64, 128, gs, _lib.F16, p.data_ptr(), p.numel(), None)
         assert e.value.code == -2
+
+
+@pytest.mark.parametrize("m", [1, 1184, 1185, 2500])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_blocks_that_walk_the_tokens(m, dtype):
+    """K = 4096: a block takes tokens blockIdx, blockIdx + 8 per SM, ... through one staging place (1 184 blocks on 148 SMs)."""
+    x = (torch.randn(m, 4096, generator=torch.Generator().manual_seed(m)) * torch.linspace(0.1, 9.0, m)[:, None]).to(dtype)
+    qa, sa = _quant_gpu(x, True, dtype)
+    _, s_ref, p_ref = O.hadamard_quant_int4(x, True)
+    assert torch.equal(sa, s_ref) and torch.equal(qa, p_ref)
