@@ -18,6 +18,10 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
              void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
              size_t workspace_bytes, int sm_count, cudaStream_t stream, int max_split, const Epilogue& ep, bool* fused);
 size_t gemv_workspace_bytes(int64_t N);
+bool gemv_a16_pre_supports(int bits, int pre, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int sm_count);
+int gemv_a16_pre(int bits, int pre, const void* x, const void* gamma, const void* beta, float eps, const uint8_t* w, const void* scales, const void* zeros,
+                 const void* bias, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int sm_count, cudaStream_t stream,
+                 const Epilogue& ep);
 size_t gemm_tc_workspace_bytes(int64_t M, int64_t N);
 int gemm_a16_tc(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                 void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
@@ -448,6 +452,44 @@ int asrq_linearq_a16_fused(int bits, const void* x, const uint8_t* w, const void
   ep.residual = residual;
   ep.act = act;
   return linearq_a16(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream, ep);
+}
+
+static int check_pre(const char* who, int bits, int pre, int64_t M, int64_t N, int64_t K, int dtype) {
+  last_error().clear();
+  if (bits != 2 && bits != 4) return fail(ASRQ_ERR_SHAPE, "%s: bits must be 2 or 4 (got %d)", who, bits);
+  if (pre != kPreLayerNorm && pre != kPreRmsNorm && pre != kPreSilu) return fail(ASRQ_ERR_SHAPE, "%s: pre %d", who, pre);
+  if (dtype != ASRQ_F16 && dtype != ASRQ_BF16) return fail(ASRQ_ERR_DTYPE, "%s: dtype %d", who, dtype);
+  if (M < 0 || N <= 0 || K <= 0) return fail(ASRQ_ERR_SHAPE, "%s: M=%lld N=%lld K=%lld", who, (long long)M, (long long)N, (long long)K);
+  return ASRQ_OK;
+}
+
+int asrq_linearq_a16_pre_covers(int bits, int pre, int64_t M, int64_t N, int64_t K, int group_size, int dtype) {
+  int rc = check_pre("asrq_linearq_a16_pre_covers", bits, pre, M, N, K, dtype);
+  const DeviceFacts* f;
+  if (rc || (rc = device_facts(&f))) return rc > 0 ? -rc : rc;
+  return option(kOptGemvKernel) == 0 && option(kOptGemvCpw) == 0 && option(kOptGemvLoop) < 0 && option(kOptTrace) == 0 &&
+         gemv_a16_pre_supports(bits, pre, M, N, K, group_size, dtype, f->sm_count);
+}
+
+int asrq_linearq_a16_pre(int bits, int pre, const void* x, const void* gamma, const void* beta, float eps, const uint8_t* w, const void* scales,
+                         const void* zeros, const void* bias, const void* residual, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype,
+                         int act, void* stream) {
+  int rc = check_pre("asrq_linearq_a16_pre", bits, pre, M, N, K, dtype);
+  if (rc) return rc;
+  if (!x || !w || !scales || !zeros || !y || (pre != kPreSilu && !gamma) || (pre == kPreLayerNorm && !beta))
+    return fail(ASRQ_ERR_NULL, "asrq_linearq_a16_pre: x, w, scales, zeros, y and the norm's weights must not be NULL");
+  if (act != kActNone && act != kActGelu) return fail(ASRQ_ERR_SHAPE, "asrq_linearq_a16_pre: act %d", act);
+  if (!aligned16(x) || !aligned16(w) || !aligned16(y) || !aligned16(scales) || !aligned16(zeros) || reinterpret_cast<uintptr_t>(gamma) % 8 ||
+      reinterpret_cast<uintptr_t>(beta) % 8)
+    return fail(ASRQ_ERR_ALIGN, "asrq_linearq_a16_pre: x, w, y, scales and zeros must be 16-byte, gamma and beta 8-byte aligned");
+  const DeviceFacts* f;
+  if ((rc = device_facts(&f))) return rc;
+  if (M == 0) return ASRQ_OK;
+  Epilogue ep;
+  ep.residual = residual;
+  ep.act = act;
+  return gemv_a16_pre(bits, pre, x, gamma, pre == kPreLayerNorm ? beta : nullptr, eps, w, scales, zeros, bias, y, M, N, K, group_size, dtype, f->sm_count,
+                      static_cast<cudaStream_t>(stream), ep);
 }
 
 int asrq_add_layernorm(const void* x, const void* delta, const void* gamma, const void* beta, float eps, void* x_out,

@@ -151,6 +151,8 @@ struct Epilogue {
   const void* residual = nullptr;  // same shape and type as y, or NULL
   int act = kActNone;
 };
+// What may come before: the activations of a layer as the norm of the residual stream, or as silu(gate) * up (ASRQ_PRE_* of the header).
+constexpr int kPreLayerNorm = ASRQ_PRE_LAYERNORM, kPreRmsNorm = ASRQ_PRE_RMSNORM, kPreSilu = ASRQ_PRE_SILU_MUL;
 __device__ __forceinline__ float out16_to_float(uint16_t b, bool bf16) {
   return bf16 ? bf16_bits_to_float(b) : __half2float(__ushort_as_half(b));
 }

@@ -55,11 +55,16 @@ struct GemvParams {
   // fused steps either side of the layer (see Epilogue): residual addition or activation
   const uint16_t* residual;
   int act;
+  // PRE variants: what happens to x on its way in (see GemvPre); x rows of K values, of 2 K for kPreSilu
+  int pre;
+  const uint16_t *gamma, *beta;
+  float eps;
   int R;                                       // rounds (LOOP variants): a warp takes R runs of CPW steps, KQ * CPW steps apart
   unsigned long long* trace;  // builds with -DASRQ_TRACE: per-warp clock marks (8 words per warp), NULL otherwise
 };
 
 constexpr int kGemvMaxWarps = 16;
+constexpr int kGemvPreMaxK = 8192;
 constexpr int kGemvMaxSteps = 4;
 
 // d = a * b (+ c): m16n8k16, fp16 or bf16 operands, fp32 accumulation
@@ -94,6 +99,18 @@ __device__ __forceinline__ void mma_new(float (&d)[4], uint32_t a0, uint32_t a1,
         "{%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// Loads of activations, in program order behind the stream dependency.  (__ldg promises the compiler that nothing writes there while the
+// kernel runs, so it may move such a load ahead of griddepcontrol.wait, when the kernel before is still writing: seen in a graph.)
+__device__ __forceinline__ uint4 ld_x4(const void* p) {
+  uint4 u;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p) : "memory");
+  return u;
+}
+__device__ __forceinline__ uint2 ld_x2(const void* p) {
+  uint2 u;
+  asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(p) : "memory");
+  return u;
 }
 // two 16-bit activations as floats
 template <bool BF16>
@@ -155,22 +172,26 @@ __device__ __forceinline__ unsigned long long gemv_globaltimer() {
 // that need them to be resident at once (2048 -> 6144, one token, us: 4.1 in one wave, 4.6 in two of the other form; that is
 // faster where one wave is enough: 2048 -> 2048, eight tokens, 3.7 against 4.8).
 constexpr bool gemv_has_tight(int bits, int mh, int cpw) { return bits == 4 && mh == 1 && cpw == 2; }
-constexpr int gemv_registers(int bits, int mh, int cpw, bool loop, bool tight) {
-  return bits == 4 && mh == 1 && !loop && cpw == 1 ? 40 : (tight ? 80 : 128);
+constexpr int gemv_registers(int bits, int mh, int cpw, bool loop, bool tight, bool pre) {
+  return bits == 4 && mh == 1 && !loop && cpw == 1 ? (pre ? 64 : 40) : (tight ? 80 : 128);
 }
 
 // BITS: 4 or 2.  MH: token halves (1: M <= 8, 2: M <= 16).  GPS: quantisation groups per step
 // (1, 2 or 4; the group size is 128/GPS k for 4-bit and 256/GPS k for 2-bit).  CPW: steps per warp
 // (1, 2 or 4, CPW * GPS <= 8).  XC: M <= 2, the activation sums are made on the CUDA cores instead of
 // by an MMA against ones (the legacy MMA pipe is this kernel's second bottleneck).
+// PRE: one or two tokens whose norm (or silu(gate) * up) is computed here, by every block for itself, instead of by a launch of its own.  A
+// decoding step of one sequence is a chain of launches: the norm between two of them took 1.9 us, here it adds the statistics'
+// shuffles and a barrier.  A warp needs the row's statistics but only its own part of K: it loads that part (which XC's sums want
+// anyway), meets the others over two numbers, and reads its MMA fragments from its part of shared memory instead of L2.
 // LOOP: layers too large for one resident wave.  Blocks are small (a few warps), several share an SM
 // at different points of their lives, and a warp walks K in R rounds, so that loads of one block
 // are in flight while another computes.  (Measured on 32-128 MB layers at M=1: 2.7-3.4 TB/s against
 // 2.0-2.5 for one round per warp.  Requesting the next round's words before this round's arithmetic,
 // in registers or through a cp.async ring in shared memory, measured slower: the variant is bound by
 // per-warp latency with 12-16 warps per SM at 128 registers, not by bytes in flight.)
-template <int BITS, bool BF16, int MH, int GPS, int CPW, bool XC, bool TRACE, bool LOOP = false, bool TIGHT = false>
-__global__ void __maxnreg__(gemv_registers(BITS, MH, CPW, LOOP, TIGHT))
+template <int BITS, bool BF16, int MH, int GPS, int CPW, bool XC, bool TRACE, bool LOOP = false, bool TIGHT = false, bool PRE = false>
+__global__ void __maxnreg__(gemv_registers(BITS, MH, CPW, LOOP, TIGHT, PRE))
 gemv_a16_kernel(const GemvParams p) {
   constexpr int CPWORD = 32 / BITS;   // codes per 32-bit word (8 / 16)
   constexpr int STEPK = 16 * CPWORD;  // k per step (128 / 256)
@@ -185,6 +206,8 @@ gemv_a16_kernel(const GemvParams p) {
   constexpr int NA = BF16 ? 2 : NT;   // accumulators of a group (bf16: every type has the same weight, two for the chains' length)
 
   __shared__ float red[kGemvMaxWarps * FR * 32];
+  __shared__ float2 stat[PRE ? 2 : 1][kGemvMaxWarps];  // PRE: sums and sums of squared distances
+  extern __shared__ __align__(16) uint16_t xsh[];      // PRE: the tokens as the product sees them
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;  // warp = K part inside the block
   const int g = lane >> 2, c = lane & 3;
@@ -223,6 +246,8 @@ gemv_a16_kernel(const GemvParams p) {
   };
   uint16_t res_first = 0;
   float bias_first = 0.f;
+  constexpr int PV = PRE ? CPW * STEPK / 128 : 1;
+  uint2 gam[PV], bet[PV];
   uint32_t qa[CPW][4], qb[CPW][4], ts0[4], tz0[4], ts1[4], tz1[4];
 #pragma unroll 1
   for (int rd = 0; rd < rounds; ++rd) {
@@ -243,6 +268,14 @@ gemv_a16_kernel(const GemvParams p) {
   if (rd == 0) {
     // the bias and the residual of this warp's first output register, fetched under the arithmetic
     if (p.bias && p.KQ > 1 && warp < FR) bias_first = ldg_half(p.bias + n_base + g + ((warp >> 1) & 1) * 8);
+    if (PRE && p.pre != kPreSilu) {  // the norm's weights are constants
+      const int e = step0 * STEPK + lane * (CPW * STEPK / 32);
+#pragma unroll
+      for (int v = 0; v < PV; ++v) {
+        gam[v] = __ldg(reinterpret_cast<const uint2*>(p.gamma + e) + v);
+        bet[v] = p.beta ? __ldg(reinterpret_cast<const uint2*>(p.beta + e) + v) : make_uint2(0, 0);
+      }
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.residual && p.KQ > 1 && warp < FR) {
       const int n = n_base + g + ((warp >> 1) & 1) * 8, m = 8 * (warp >> 2) + 2 * c + (warp & 1);
@@ -259,13 +292,96 @@ gemv_a16_kernel(const GemvParams p) {
   float xs[2][NG];
   uint2 xu[2][HPL / 4];
   if (XC) {
+    const size_t row = PRE && p.pre == kPreSilu ? 2 * size_t(p.K) : size_t(p.K);
 #pragma unroll
     for (int tok = 0; tok < 2; ++tok) {
-      const uint16_t* xp = p.x + size_t(tok) * p.K + step0 * STEPK + lane * HPL;
+      const uint16_t* xp = p.x + tok * row + step0 * STEPK + lane * HPL;
 #pragma unroll
       for (int v = 0; v < HPL / 4; ++v)
-        xu[tok][v] = tok < p.M ? __ldg(reinterpret_cast<const uint2*>(xp) + v) : make_uint2(0, 0);
+        xu[tok][v] = tok < p.M ? ld_x2(reinterpret_cast<const uint2*>(xp) + v) : make_uint2(0, 0);
     }
+  }
+  if (PRE) {
+    uint4 xr8[2];  // for the statistics: the warp's 256 elements of each token
+#pragma unroll
+    for (int tok = 0; tok < 2; ++tok)
+      xr8[tok] = p.pre != kPreSilu && tok < p.M && warp * 256 < p.K ? ld_x4(reinterpret_cast<const uint4*>(p.x + size_t(tok) * p.K + warp * 256) + lane)
+                                                                    : make_uint4(0, 0, 0, 0);
+    // HPL values of a token in place: f(value, position in the lane's run) -> value, rounded to the type, kept and put into shared memory
+    auto each = [&](int tok, auto f) {
+      uint16_t* dst = xsh + size_t(tok) * p.K + step0 * STEPK + lane * HPL;
+#pragma unroll
+      for (int v = 0; v < HPL / 4; ++v) {
+        const float2 a = two_floats<BF16>(xu[tok][v].x), b = two_floats<BF16>(xu[tok][v].y);
+        xu[tok][v].x = uint32_t(float_to_out16(f(a.x, 4 * v), BF16)) | (uint32_t(float_to_out16(f(a.y, 4 * v + 1), BF16)) << 16);
+        xu[tok][v].y = uint32_t(float_to_out16(f(b.x, 4 * v + 2), BF16)) | (uint32_t(float_to_out16(f(b.y, 4 * v + 3), BF16)) << 16);
+        reinterpret_cast<uint2*>(dst)[v] = xu[tok][v];
+      }
+    };
+    auto half_of = [&](const uint2* t, int i) {  // i is a compile-time value after unrolling
+      const uint32_t w = (i & 2) ? t[i >> 2].y : t[i >> 2].x;
+      return out16_to_float(uint16_t((i & 1) ? (w >> 16) : (w & 0xffffu)), BF16);
+    };
+    if (p.pre == kPreSilu) {
+      // one token (gemv_a16_pre_supports), as silu_mul_kernel: the gate's factor rounded as the module rounds it
+      uint2 up[HPL / 4];
+#pragma unroll
+      for (int v = 0; v < HPL / 4; ++v) up[v] = ld_x2(reinterpret_cast<const uint2*>(p.x + p.K + step0 * STEPK + lane * HPL) + v);
+      each(0, [&](float gv, int i) { return out16_to_float(float_to_out16(gv / (1.f + expf(-gv)), BF16), BF16) * half_of(up, i); });
+    } else {
+      // statistics with the bits of row_norm_kernel: warp q takes elements 256 q .. 256 q + 255, eight a lane, and the parts are added in
+      // order (K / 256 <= KQ: gemv_a16_pre_supports)
+      const bool layer = p.pre == kPreLayerNorm;
+      const int nw = p.K / 256;
+      float mean[2] = {0.f, 0.f}, rs[2];
+      auto eighth = [&](int tok, int i) {
+        const uint32_t w = i < 2 ? xr8[tok].x : (i < 4 ? xr8[tok].y : (i < 6 ? xr8[tok].z : xr8[tok].w));
+        return out16_to_float(uint16_t((i & 1) ? (w >> 16) : (w & 0xffffu)), BF16);
+      };
+      if (layer) {
+#pragma unroll
+        for (int tok = 0; tok < 2; ++tok) {
+          if (tok >= p.M) break;
+          float sum = 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sum += eighth(tok, i);
+#pragma unroll
+          for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          if (lane == 0) stat[tok][warp].x = sum;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int tok = 0; tok < 2; ++tok) {
+          if (tok >= p.M) break;
+          float t = 0.f;
+          for (int q = 0; q < nw; ++q) t += stat[tok][q].x;
+          mean[tok] = t / float(p.K);
+        }
+      }
+#pragma unroll
+      for (int tok = 0; tok < 2; ++tok) {
+        if (tok >= p.M) break;
+        float sq = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sq = fmaf(eighth(tok, i) - mean[tok], eighth(tok, i) - mean[tok], sq);
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (lane == 0) stat[tok][warp].y = sq;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int tok = 0; tok < 2; ++tok) {
+        if (tok >= p.M) break;
+        float t = 0.f;
+        for (int q = 0; q < nw; ++q) t += stat[tok][q].y;
+        rs[tok] = rsqrtf(t / float(p.K) + p.eps);
+        if (layer)
+          each(tok, [&](float v, int i) { return ln_apply(v, mean[tok], rs[tok], half_of(gam, i), half_of(bet, i)); });
+        else  // the normalised value is rounded before the weight multiplies it, as in add_rmsnorm
+          each(tok, [&](float v, int i) { return out16_to_float(float_to_out16(v * rs[tok], BF16), BF16) * half_of(gam, i); });
+      }
+    }
+    __syncwarp();  // a warp reads what it wrote
   }
 
   // activations of token g (+8) for the k of this lane's WPC words of group gi, natural order;
@@ -281,8 +397,10 @@ gemv_a16_kernel(const GemvParams p) {
 #pragma unroll
       for (int v = 0; v < WPC * XR / 4; ++v) {
         uint4 u = make_uint4(0, 0, 0, 0);
-        if (m < p.M) {
-          asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(xp + v));
+        if (PRE) {
+          if (m < p.M) u = *reinterpret_cast<const uint4*>(xsh + size_t(m) * p.K + kbase + 8 * v);
+        } else if (m < p.M) {
+          u = ld_x4(xp + v);
         }
         dst[mh][(4 * v) / XR][(4 * v) % XR + 0] = u.x; dst[mh][(4 * v) / XR][(4 * v) % XR + 1] = u.y;
         dst[mh][(4 * v) / XR][(4 * v) % XR + 2] = u.z; dst[mh][(4 * v) / XR][(4 * v) % XR + 3] = u.w;
@@ -470,7 +588,7 @@ gemv_a16_kernel(const GemvParams p) {
 using GemvKernel = void (*)(const GemvParams);
 
 template <int BITS, bool BF16, int MH, int GPS, int CPW>
-GemvKernel kernel_for(bool xc, bool trace, bool tight) {
+GemvKernel kernel_for(bool xc, bool trace, bool tight, bool pre) {
 #ifdef ASRQ_TRACE
   if (trace) {
     if (MH == 1 && xc) return gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, true>;
@@ -478,24 +596,28 @@ GemvKernel kernel_for(bool xc, bool trace, bool tight) {
   }
 #endif
   (void)trace;  // the shipped library holds no trace variants
-  if (gemv_has_tight(BITS, MH, CPW) && tight) {
-    constexpr bool T = gemv_has_tight(BITS, MH, CPW);
+  constexpr bool T = gemv_has_tight(BITS, MH, CPW);
+  if (pre) {
+    if (MH != 1) return nullptr;
+    return T && tight ? gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, false, false, T, true> : gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, false, false, false, true>;
+  }
+  if (T && tight) {
     return xc ? gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, false, false, T> : gemv_a16_kernel<BITS, BF16, MH, GPS, CPW, false, false, false, T>;
   }
   if (MH == 1 && xc) return gemv_a16_kernel<BITS, BF16, 1, GPS, CPW, true, false>;
   return gemv_a16_kernel<BITS, BF16, MH, GPS, CPW, false, false>;
 }
 template <int BITS, bool BF16, int MH>
-GemvKernel kernel_for(int gps, int cpw, bool xc, bool trace, bool tight) {
+GemvKernel kernel_for(int gps, int cpw, bool xc, bool trace, bool tight, bool pre) {
   switch (gps * 8 + cpw) {
-    case 1 * 8 + 1: return kernel_for<BITS, BF16, MH, 1, 1>(xc, trace, tight);
-    case 1 * 8 + 2: return kernel_for<BITS, BF16, MH, 1, 2>(xc, trace, tight);
-    case 1 * 8 + 4: return kernel_for<BITS, BF16, MH, 1, 4>(xc, trace, tight);
-    case 2 * 8 + 1: return kernel_for<BITS, BF16, MH, 2, 1>(xc, trace, tight);
-    case 2 * 8 + 2: return kernel_for<BITS, BF16, MH, 2, 2>(xc, trace, tight);
-    case 2 * 8 + 4: return kernel_for<BITS, BF16, MH, 2, 4>(xc, trace, tight);
-    case 4 * 8 + 1: return kernel_for<BITS, BF16, MH, 4, 1>(xc, trace, tight);
-    case 4 * 8 + 2: return kernel_for<BITS, BF16, MH, 4, 2>(xc, trace, tight);
+    case 1 * 8 + 1: return kernel_for<BITS, BF16, MH, 1, 1>(xc, trace, tight, pre);
+    case 1 * 8 + 2: return kernel_for<BITS, BF16, MH, 1, 2>(xc, trace, tight, pre);
+    case 1 * 8 + 4: return kernel_for<BITS, BF16, MH, 1, 4>(xc, trace, tight, pre);
+    case 2 * 8 + 1: return kernel_for<BITS, BF16, MH, 2, 1>(xc, trace, tight, pre);
+    case 2 * 8 + 2: return kernel_for<BITS, BF16, MH, 2, 2>(xc, trace, tight, pre);
+    case 2 * 8 + 4: return kernel_for<BITS, BF16, MH, 2, 4>(xc, trace, tight, pre);
+    case 4 * 8 + 1: return kernel_for<BITS, BF16, MH, 4, 1>(xc, trace, tight, pre);
+    case 4 * 8 + 2: return kernel_for<BITS, BF16, MH, 4, 2>(xc, trace, tight, pre);
     default: return nullptr;
   }
 }
@@ -528,12 +650,12 @@ GemvKernel loop_kernel_for(int bits, bool bf16, int mh, int gps, bool xc, int* c
 }
 
 template <int BITS, bool BF16>
-GemvKernel kernel_for(int mh, int gps, int cpw, bool xc, bool trace, bool tight) {
-  return mh == 1 ? kernel_for<BITS, BF16, 1>(gps, cpw, xc, trace, tight) : kernel_for<BITS, BF16, 2>(gps, cpw, xc, trace, tight);
+GemvKernel kernel_for(int mh, int gps, int cpw, bool xc, bool trace, bool tight, bool pre) {
+  return mh == 1 ? kernel_for<BITS, BF16, 1>(gps, cpw, xc, trace, tight, pre) : kernel_for<BITS, BF16, 2>(gps, cpw, xc, trace, tight, pre);
 }
-GemvKernel kernel_for(int bits, bool bf16, int mh, int gps, int cpw, bool xc, bool trace, bool tight) {
-  if (bits == 4) return bf16 ? kernel_for<4, true>(mh, gps, cpw, xc, trace, tight) : kernel_for<4, false>(mh, gps, cpw, xc, trace, tight);
-  return bf16 ? kernel_for<2, true>(mh, gps, cpw, xc, trace, tight) : kernel_for<2, false>(mh, gps, cpw, xc, trace, tight);
+GemvKernel kernel_for(int bits, bool bf16, int mh, int gps, int cpw, bool xc, bool trace, bool tight, bool pre) {
+  if (bits == 4) return bf16 ? kernel_for<4, true>(mh, gps, cpw, xc, trace, tight, pre) : kernel_for<4, false>(mh, gps, cpw, xc, trace, tight, pre);
+  return bf16 ? kernel_for<2, true>(mh, gps, cpw, xc, trace, tight, pre) : kernel_for<2, false>(mh, gps, cpw, xc, trace, tight, pre);
 }
 
 // How one launch splits K inside a block: a warp takes CPW steps (1, 2 or 4) and KQ warps (1..16)
@@ -543,7 +665,8 @@ GemvKernel kernel_for(int bits, bool bf16, int mh, int gps, int cpw, bool xc, bo
 struct GemvSplit {
   int KQ, CPW;
   GemvKernel kern;
-  int R = 1;        // rounds per warp (LOOP variants)
+  int R = 0;        // rounds per warp (LOOP variants)
+  bool tight = false;
 };
 
 GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool trace, int64_t N, int64_t K, int sm_count) {
@@ -560,8 +683,9 @@ GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool tr
     const int kq = steps / cpw;
     GemvKernel k = nullptr;
     long waves = 0;
+    bool k_tight = false;
     for (int tight = 0; tight <= int(gemv_has_tight(bits, mh, cpw) && !trace); ++tight) {
-      GemvKernel form = kernel_for(bits, bf16, mh, gps, cpw, xc, trace, tight != 0);
+      GemvKernel form = kernel_for(bits, bf16, mh, gps, cpw, xc, trace, tight != 0, false);
       if (!form) continue;
       int per_sm = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form, 32 * kq, 0) != cudaSuccess || per_sm < 1) {
@@ -573,6 +697,7 @@ GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool tr
       if (k && w >= waves) continue;  // the tight form only where it saves a wave
       k = form;
       waves = w;
+      k_tight = tight != 0;
     }
     if (!k) continue;
     // Fewest waves first.  Among those, 8 to 12 warps per block measured fastest on the decode
@@ -583,6 +708,7 @@ GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool tr
       best.KQ = kq;
       best.CPW = cpw;
       best.kern = k;
+      best.tight = k_tight;
       best_waves = waves;
     }
   }
@@ -636,13 +762,13 @@ GemvSplit cached_split(int bits, bool bf16, int cls, int gps, bool trace, int64_
   return sp;
 }
 
-int launch_gemv(const GemvSplit& sp, const GemvParams& p, cudaStream_t stream) {
+int launch_gemv(const GemvSplit& sp, const GemvParams& p, cudaStream_t stream, size_t smem = 0) {
   // Programmatic dependent launch: consecutive decode kernels overlap their weight fetch with the
   // predecessor's tail (the kernel orders itself with griddepcontrol.wait).
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.N / 16);
   cfg.blockDim = dim3(32 * p.KQ);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -715,7 +841,7 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
       return gemv_a16_splitk(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace,
                              workspace_bytes, sm_count, stream, max_split);
   }
-  GemvParams p;
+  GemvParams p = {};
   p.w = w;
   p.scales = static_cast<const __half*>(scales);
   p.zeros = static_cast<const __half*>(zeros);
@@ -736,11 +862,58 @@ int gemv_a16(int bits, const void* x, const uint8_t* w, const void* scales, cons
     const GemvSplit& sp = split[mb <= 8 ? (mb <= 2 ? 0 : 1) : 2];
     p.KQ = sp.KQ;
     p.CPW = sp.CPW;
-    p.R = sp.R;
+    p.R = sp.R > 0 ? sp.R : 1;
     const int rc = launch_gemv(sp, p, stream);
     if (rc) return rc;
   }
   return ASRQ_OK;
+}
+
+// The kernel of a call with a step ahead of the layer, with the split that the layer alone has (so that it gives the same bits), or
+// none.  One token for silu(gate) * up: every block computes it, 0.9 us a token for 6144 values.
+static GemvSplit pre_split(int bits, int pre, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int sm_count) {
+  GemvSplit none = {0, 0, nullptr};
+  const int gps = groups_per_step(bits, group_size);
+  if (M < 1 || M > (pre == kPreSilu ? 1 : 2) || N % 16 || K % ((128 / bits) * 4) || K > kGemvPreMaxK || N > int64_t(4096) * 16 || !gps || K % group_size) return none;
+  GemvSplit sp = cached_split(bits, dtype == ASRQ_BF16, 0, gps, false, N, K, sm_count);
+  if (!sp.kern || sp.R) return none;
+  // statistics as row_norm_kernel makes them: a warp per 256 elements
+  if (pre != kPreSilu && (K % 256 || K > 2048 || sp.KQ < K / 256)) return none;
+  sp.kern = kernel_for(bits, dtype == ASRQ_BF16, 1, gps, sp.CPW, true, false, sp.tight, true);
+  return sp;
+}
+bool gemv_a16_pre_supports(int bits, int pre, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int sm_count) {
+  return pre_split(bits, pre, M, N, K, group_size, dtype, sm_count).kern != nullptr;
+}
+
+int gemv_a16_pre(int bits, int pre, const void* x, const void* gamma, const void* beta, float eps, const uint8_t* w, const void* scales, const void* zeros,
+                 const void* bias, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int sm_count, cudaStream_t stream,
+                 const Epilogue& ep) {
+  const GemvSplit sp = pre_split(bits, pre, M, N, K, group_size, dtype, sm_count);
+  if (!sp.kern)
+    return fail(ASRQ_ERR_SHAPE, "w%da16 with a step ahead: M=%lld N=%lld K=%lld g=%d not covered (ask asrq_linearq_a16_pre_covers)", bits, (long long)M,
+                (long long)N, (long long)K, group_size);
+  GemvParams p = {};
+  p.x = static_cast<const uint16_t*>(x);
+  p.pre = pre;
+  p.gamma = static_cast<const uint16_t*>(gamma);
+  p.beta = static_cast<const uint16_t*>(beta);
+  p.eps = eps;
+  p.w = w;
+  p.scales = static_cast<const __half*>(scales);
+  p.zeros = static_cast<const __half*>(zeros);
+  p.bias = static_cast<const __half*>(bias);
+  p.y = static_cast<uint16_t*>(y);
+  p.residual = static_cast<const uint16_t*>(ep.residual);
+  p.act = ep.act;
+  p.M = int(M);
+  p.N = int(N);
+  p.K = int(K);
+  p.groups_per_row = int(K / group_size);
+  p.KQ = sp.KQ;
+  p.CPW = sp.CPW;
+  p.R = 1;
+  return launch_gemv(sp, p, stream, size_t(2) * size_t(M) * size_t(K));
 }
 
 }  // namespace asrq

@@ -426,6 +426,39 @@ class LinearQ(nn.Module):
                 f"group_size={self.group_size}, bias={self.bias is not None}")
 
 
+PRE_LAYERNORM, PRE_RMSNORM, PRE_SILU_MUL = 1, 2, 3  # asrq_linearq_a16_pre
+
+
+def linear_after(layer: LinearQ, pre: int, x: torch.Tensor, weight=None, bias=None, eps: float = 0.0, residual=None, gelu: bool = False):
+    """``layer.forward_fused(h, residual, gelu)`` where ``h`` is the step ahead of the layer: the layer norm or RMS norm of the
+    residual stream ``x``, or ``silu(gate) * up`` of a fused projection's output ``x``.  For one or two rows (one for the last)
+    both are one kernel; otherwise None, and the caller does them one after the other."""
+    k, n = layer.in_features, layer.out_features
+    width = 2 * k if pre == PRE_SILU_MUL else k
+    rows = x.numel() // width
+    if (rows > 2 or not x.is_cuda or x.shape[-1] != width or not x.is_contiguous() or x.dtype not in _DTYPES or
+            _lib.load().asrq_linearq_a16_pre_covers(layer.bits, pre, rows, n, k, layer.group_size, _DTYPES[x.dtype]) != 1):
+        return None
+    layer._check_buffers(x)
+    if residual is not None and not (residual.numel() == rows * n and residual.is_contiguous() and residual.dtype == x.dtype and residual.device == x.device):
+        return None
+    for t in (weight, bias):
+        if t is not None and not (t.numel() == k and t.is_contiguous() and t.dtype == x.dtype and t.device == x.device):
+            return None
+    if any(t is not None and t.data_ptr() % 16 for t in (x, layer.weight, layer.scales, layer.zeros, weight, bias)):
+        return None
+    y = torch.empty((*x.shape[:-1], n), dtype=x.dtype, device=x.device)
+
+    def ptr(t):
+        return None if t is None else t.data_ptr()
+
+    with _on_device(x.device):
+        _lib.call("asrq_linearq_a16_pre", layer.bits, pre, x.data_ptr(), ptr(weight), ptr(bias), float(eps), layer.weight.data_ptr(),
+                  layer.scales.data_ptr(), layer.zeros.data_ptr(), ptr(layer.bias), ptr(residual), y.data_ptr(), rows, n, k, layer.group_size,
+                  _DTYPES[x.dtype], _lib.ACT_GELU if gelu else _lib.ACT_NONE, torch.cuda.current_stream(x.device).cuda_stream)
+    return y
+
+
 class _Prepared(tuple):
     """(operand, an alias of the packed weight it was derived from, that weight's version, the operand's format, the streams that
     are ordered behind the derivation, its event).  The alias keeps the weight's memory, so that an equal address means the same

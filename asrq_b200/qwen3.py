@@ -23,7 +23,8 @@ import torch.nn.functional as F
 
 from . import packing
 from .convert import linearq_from_linear
-from .linear import LinearQ, add_rmsnorm, argmax_rows, decode_grouped_attention, dense_head, qk_norm_rope, silu_mul
+from .linear import (PRE_RMSNORM, PRE_SILU_MUL, LinearQ, add_rmsnorm, argmax_rows, decode_grouped_attention, dense_head, linear_after, qk_norm_rope,
+                     silu_mul)
 from .whisper import _baked_in, _cat_linearq, _same
 
 try:
@@ -234,14 +235,25 @@ class Qwen3Engine:
         """:meth:`_block` for one new position per sequence, which lives on the device: q/k norm, rotary embedding, cache write
         and attention are one kernel for heads of 128 in pairs (Qwen3's), else the prompt's kernel and a masked attention."""
         B = x.shape[0]
-        x, h = add_rmsnorm(x, delta, L["ln1"], self.eps)
-        qkv = L["qkv"](h)
+        # one or two sequences: the norms inside the projections behind them, the residual in the epilogue of those ahead (the same bits)
+        qkv = linear_after(L["qkv"], PRE_RMSNORM, x, L["ln1"], None, self.eps) if delta is None else None
+        lean = qkv is not None
+        if not lean:
+            x, h = add_rmsnorm(x, delta, L["ln1"], self.eps)
+            qkv = L["qkv"](h)
         if self.own_attention:
             a = decode_grouped_attention(qkv, L["qn"], L["kn"], self.cos, self.sin, kc, vc, self.pos, self.nq, self.eps, self.hd ** -0.5)
         else:
             q = qk_norm_rope(qkv, L["qn"], L["kn"], self.cos, self.sin, kc, vc, self.pos, B, 1, self.nq, self.nkv, self.eps)
             a = F.scaled_dot_product_attention(q, kc, vc, attn_mask=mask, enable_gqa=self.nq != self.nkv)
             a = a.transpose(1, 2).reshape(B, self.nq * self.hd)
+        if lean:
+            x = L["o"].forward_fused(a, residual=x)
+            gu = linear_after(L["gu"], PRE_RMSNORM, x, L["ln2"], None, self.eps)
+            if gu is None:
+                gu = L["gu"](add_rmsnorm(x, None, L["ln2"], self.eps)[1])
+            y = linear_after(L["down"], PRE_SILU_MUL, gu, residual=x)
+            return (L["down"].forward_fused(silu_mul(gu), residual=x) if y is None else y), None
         x, h = add_rmsnorm(x, L["o"](a), L["ln2"], self.eps)
         return x, L["down"](silu_mul(L["gu"](h)))
 

@@ -158,6 +158,25 @@ int asrq_linearq_a16_fused(int bits, const void* x, const uint8_t* w, const void
                            void* stream);
 
 /*
+ * asrq_linearq_a16_fused with the step ahead of the layer in the same kernel, for a decoding step of one or two
+ * sequences, where that step is a launch as long as the layer's own:
+ *   ASRQ_PRE_LAYERNORM  x[M,K] is the residual stream, the layer sees layer_norm(x) * gamma + beta;
+ *   ASRQ_PRE_RMSNORM    ... rms_norm(x) * gamma (rounded as asrq_add_rmsnorm rounds), beta NULL;
+ *   ASRQ_PRE_SILU_MUL   x[M,2K] is a fused gate/up projection, the layer sees silu(gate) * up; gamma, beta NULL.
+ * gamma and beta in x's type, 8-byte aligned, constants like the weights (read ahead of the stream dependency);
+ * scales and zeros 16-byte aligned.  Needs no workspace.  asrq_linearq_a16_pre_covers says whether a call is taken
+ * (1 or 0; negative: error): others do the step and the layer as two calls.
+ */
+#define ASRQ_PRE_LAYERNORM 1
+#define ASRQ_PRE_RMSNORM 2
+#define ASRQ_PRE_SILU_MUL 3
+int asrq_linearq_a16_pre_covers(int bits, int pre, int64_t M, int64_t N, int64_t K, int group_size, int dtype);
+int asrq_linearq_a16_pre(int bits, int pre, const void* x, const void* gamma, const void* beta, float eps,
+                         const uint8_t* w, const void* scales, const void* zeros, const void* bias,
+                         const void* residual, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype,
+                         int act, void* stream);
+
+/*
  * x' = x + delta (delta may be NULL), h = LayerNorm(x') * gamma + beta over the last dimension.
  * x, delta, x_out (optional; may alias x), h_out: rows x dim in the 16-bit type `dtype`; gamma, beta: dim
  * values of that type.  Statistics in fp32 on the 16-bit-rounded x' (what "add, then layer_norm" computes).
