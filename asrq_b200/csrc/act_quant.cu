@@ -363,7 +363,8 @@ hadamard_1024_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__
   auto slot = [](int owner, int j) { return owner * UNITS + (j ^ ((owner >> 1) & 3)); };  // conflict-free both ways
   uint4 raw[UNITS];
 #pragma unroll
-  for (int i = 0; i < UNITS; ++i) raw[i] = __ldg(src + i * T);
+  for (int i = 0; i < UNITS; ++i)  // (behind the wait: __ldg could be moved ahead of it)
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(raw[i].x), "=r"(raw[i].y), "=r"(raw[i].z), "=r"(raw[i].w) : "l"(src + i * T) : "memory");
 #pragma unroll
   for (int i = 0; i < UNITS; ++i) stage[slot((i * T + t) / UNITS, (i * T + t) % UNITS)] = raw[i];
   __syncwarp();

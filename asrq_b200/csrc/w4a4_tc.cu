@@ -408,7 +408,7 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
           for (int j = 0; j < 16; ++j) {
             const int tok = tok0 + ch * 16 + j;
             const float a = (j & 1) ? accf[ch * 8 + (j >> 1)].y : accf[ch * 8 + (j >> 1)].x;
-            if (tok < p.M) p.y[size_t(tok) * p.N + f] = float_to_out16(a * __ldg(p.sa + tok) + bias, p.bf16);
+            if (tok < p.M) p.y[size_t(tok) * p.N + f] = float_to_out16(a * __ldcg(p.sa + tok) + bias, p.bf16);
           }
         }
       }
