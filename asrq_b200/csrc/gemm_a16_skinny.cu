@@ -7,25 +7,31 @@
 //
 //   * a block owns ONE work item -- a tile of 128 features x BT tokens and a part of K.  Its activation tiles and packed
 //     weights pass through a ring of stages in shared memory, which for decode batches holds all of them at once;
-//   * it triggers its dependents as its first instruction and is small enough (448 threads, <= 73
-//     registers) for two blocks to share an SM where the plan's shared memory allows (up to 112 KB: 1280
-//     inputs at up to 32 tokens 73-105 KB, 2048 -> 2048 at 64 tokens 97).  Larger plans have the SM to themselves
-//     (64 tokens: 2048 -> 4096 145 KB, 2048 -> 6144 181, 2048 -> 12288 217) and the next launch takes the SMs that
-//     this one leaves idle or is done with.  Packed weights are fetched by TMA and the first three K blocks are
-//     dequantised BEFORE griddepcontrol.wait: weights do not depend on the kernel before, so the next launch's
-//     weight traffic and unpacking run under this launch's tail where it has an SM by then;
+//   * weights are unpacked into TENSOR MEMORY, as the MMA's A operand (tcgen05.st; a lane is a weight row, 32 columns a K block of 64;
+//     three or six such slots beside the accumulator).  Through shared memory a K block cost 128 clocks of stores, 128 of the
+//     MMA's reads and a proxy fence beside the 190 that packed weights and activations take: shared memory was busy for three
+//     quarters of the block's 620 clocks;
+//   * it triggers its dependents as its first instruction, and up to 64 tokens two blocks share an SM where the plan's shared memory
+//     allows (up to 112 KB).  Packed weights are fetched by TMA and the first three or six K blocks are dequantised BEFORE
+//     griddepcontrol.wait: weights do not depend on the kernel before, so the next launch's weight traffic and unpacking run under
+//     this launch's tail where it has an SM by then;
 //   * after the wait only the activation tiles (tokens as the MMA's N dimension: 32 to 256 TMEM columns)
 //     are fetched, as many as there are stages at once; tcgen05.mma kind::f16 128 x BT x 16, fp32 accumulator in tensor memory;
 //   * the K parts of a tile are a thread-block cluster and meet in distributed shared memory: every block leaves its
-//     fp32 part in its own shared memory (over A slots and stages, whose MMAs are done), and after one cluster barrier each
+//     fp32 part in its own shared memory (over the stages, whose MMAs are done), and after one cluster barrier each
 //     adds its share of the tokens over all parts in part order, with all of its threads, adds the bias, converts
 //     and stores.  Through the workspace (partial tiles, a counter per tile, the last block adding) the same step
 //     cost a release to memory, an atomic and two to four L2 round trips of one block while the others were done.
 //
 // Roles (14 warps): warp 0 TMA producer, warp 1 MMA issuer (owns the tensor-memory allocation), warps
-// 2-13 three dequant groups of 128 threads (one weight row per thread, group d takes K blocks d, d+3, ...
-// and owns A slot d); the first group (warps 2-5, one per TMEM lane quadrant) then runs the epilogue.
-// No TMA multicast.  Every wait is bounded.
+// 2-13 three dequant groups of 128 threads (one weight row per thread, group d takes K blocks d, d+3, ...); the first group
+// (warps 2-5, one per TMEM lane quadrant) then runs the epilogue.  No TMA multicast.  Every wait is bounded.
+//
+// Bound: the chain's latencies and, where a block has many K blocks, the dequant groups' own (0.27 us a block; 0.23 with the
+// arithmetic left out).  Chains of launches, W4, unpacking through shared memory -> this form, us at 32 / 64 / 128 / 259 tokens:
+// 1280 -> 1280 4.3 / 4.6 / 5.9 / 6.6 -> 3.9 / 4.1 / 5.5 / 6.4; 1280 -> 5120 6.1 / 6.8 / 8.1 / 11.8 -> 5.0 / 6.0 / 8.0 / 11.0; 2048 -> 4096 6.7 / 7.5 /
+// 8.7 / 12.6 -> 5.3 / 6.6 / 8.7 / 11.3; 2048 -> 12288 15.3 / 16.1 / 17.9 -> 12.9 / 14.0 / 15.6; 6144 -> 2048 10.5 / 11.4 / 12.4 / 16.5 -> 8.5 / 10.0 / 12.1 /
+// 15.7; bf16 2048 -> 4096 at 80 to 128 tokens 0.2 us slower.  More slots than the MMAs' round trip needs changed nothing.
 //
 // Prompts of some hundred tokens: the persistent kernels give a tile the whole of K, and with few tiles most SMs idle (1280 x 5120
 // at 260 to 1500 tokens: 31 us on 20 to 60 of them).  Here K is cut so that one wave fills the chip.
@@ -45,11 +51,18 @@ constexpr int kSkWarps = 14;
 constexpr int kSkThreads = 32 * kSkWarps;
 constexpr int kSkMaxStages = 16;                // K blocks of 64 in shared memory at once
 constexpr int kSkMaxSplit = 8;
+constexpr int kSkMaxSlots = 6;
+constexpr uint32_t kSkSlotCols = 32;            // a dequantised A slot in tensor memory: 128 lanes x 64 16-bit elements
 constexpr int kSkMaxM = 2048;
-constexpr uint32_t kSkATile = 128 * 128;        // one dequantised A slot: 128 rows x 64 16-bit elements
 constexpr size_t kSkMaxSmem = 226 * 1024;
 constexpr size_t kSkTwoPerSm = 112 * 1024;      // two blocks share an SM
 constexpr uint32_t kSkWSlot = 4096;             // packed weights of one K block (<= 128 x 32 B)
+
+// Columns of tensor memory to allocate (a power of two).  256 at most up to 128 tokens: two blocks share an SM's 512.
+__host__ __device__ constexpr uint32_t skinny_tmem_cols(int bt, int slots) {
+  const uint32_t need = uint32_t(bt) + uint32_t(slots) * kSkSlotCols;
+  return need <= 128 ? 128u : (need <= 256 ? 256u : 512u);
+}
 
 struct SkinnyParams {
   const __half* scales;
@@ -60,6 +73,7 @@ struct SkinnyParams {
   uint16_t* y;
   unsigned* status;
   int M, N, K, group_size, groups_per_row, bt, n_tt, ksplit, nkb, stages;
+  int slots;  // A slots in tensor memory, a multiple of three: K block kb is in slot kb % slots
   unsigned long long* trace;  // builds with -DASRQ_TRACE: 8 globaltimer marks per block, NULL otherwise
 };
 
@@ -83,7 +97,7 @@ __global__ void __launch_bounds__(kSkThreads, 2)
 gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
                        const SkinnyParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * kSkMaxStages + 7];
+  __shared__ __align__(8) uint64_t bars[3 * kSkMaxStages + 1 + 2 * kSkMaxSlots];
   __shared__ uint32_t tmem_slot;
   // the next launch on the stream may start its own set-up, weight fetch and first dequantisation now
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -97,8 +111,8 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   const int ks = blockIdx.x % p.ksplit, tile = blockIdx.x / p.ksplit, tt = tile % p.n_tt, ft = tile / p.n_tt;
   const int kb0 = ks * p.nkb / p.ksplit, kb1 = (ks + 1) * p.nkb / p.ksplit, kbn = kb1 - kb0, nst = p.stages;
   const uint32_t xbytes = uint32_t(p.bt) * 128u;
-  // [A slot x 3] [activation tile x stages] [packed weights x stages]
-  const uint32_t x_base = 3 * kSkATile, w_base = x_base + uint32_t(nst) * xbytes;
+  // [activation tile x stages] [packed weights x stages]
+  const uint32_t x_base = 0, w_base = uint32_t(nst) * xbytes;
   constexpr uint32_t wbytes = 128u * 8u * BITS;
   const uint32_t bar0 = tc::smem_u32(bars);
   auto w_bar = [&](int st) { return bar0 + 8u * st; };
@@ -106,8 +120,9 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
   auto sfree_bar = [&](int st) { return bar0 + 8u * (2 * kSkMaxStages + st); };  // the stage's MMAs are done
   const uint32_t accf_bar = bar0 + 8u * (3 * kSkMaxStages);
   auto deq_bar = [&](int a) { return accf_bar + 8u + 8u * a; };
-  auto afree_bar = [&](int a) { return accf_bar + 32u + 8u * a; };
-  const uint32_t tmem_cols = p.bt <= 32 ? 32u : (p.bt <= 64 ? 64u : (p.bt <= 128 ? 128u : 256u));
+  auto afree_bar = [&](int a) { return accf_bar + 8u + 8u * (kSkMaxSlots + a); };
+  // tensor memory: [accumulator, bt columns] [A slots]
+  const uint32_t a_col = uint32_t(p.bt), tmem_cols = skinny_tmem_cols(p.bt, p.slots);
 
   // The bias of the four features this thread stores (the same in each of its steps): a constant, and fetched here a first touch
   // of memory that the last step would otherwise wait for.
@@ -122,8 +137,8 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
       tc::mbar_init(sfree_bar(st), 1);
     }
     tc::mbar_init(accf_bar, 1);
-    for (int a = 0; a < 3; ++a) {
-      tc::mbar_init(deq_bar(a), 128);
+    for (int a = 0; a < p.slots; ++a) {
+      tc::mbar_init(deq_bar(a), 4);  // the four warps of the group
       tc::mbar_init(afree_bar(a), 1);
     }
     tc::fence_barrier_init();
@@ -172,48 +187,49 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    const bool el = tc::elect_one();
+    // The warp's own latency is part of every K block's chain: the next block's barriers are tested in the stream of this block's MMAs
+    // (see mma4_ts_commit_probe), and waited for only where that found one incomplete.
+    const uint32_t el = tc::elect_one() ? 1u : 0u;
     const uint32_t idesc = tc::instr_desc(1u, BF16 ? 1u : 0u, 128u, uint32_t(p.bt));
-    int st = 0;
-    uint32_t ph = 0;
+    int st = 0, a = 0;
+    uint32_t ph = 0, aph = 0, ready = 0;
     bool ok = tc::mbar_wait_spin(x_bar(0), 0u, p.status, 31);
     if (lane == 0) SK_MARK(4);
     for (int kb = 0; kb < kbn && ok; ++kb) {
-      const int a = kb % 3;
-      if (RING && kb) ok = tc::mbar_wait_spin(x_bar(st), ph, p.status, 31);
-      ok = ok && tc::mbar_wait_spin(deq_bar(a), uint32_t(kb / 3) & 1u, p.status, 32);
-      if (!ok) break;
-      tc::fence_after_sync();
-      const uint64_t da = tc::smem_desc_sw128(base + a * kSkATile);
-      const uint64_t db = tc::smem_desc_sw128(base + x_base + st * xbytes);
-      if (el) {
-        tc::mma_f16(tmem_base, da, db, idesc, uint32_t(kb != 0));
-        tc::mma_f16(tmem_base, da + 2, db + 2, idesc, 1u);
-        tc::mma_f16(tmem_base, da + 4, db + 4, idesc, 1u);
-        tc::mma_f16(tmem_base, da + 6, db + 6, idesc, 1u);
-        tc::mma_commit(afree_bar(a));
-        if (RING && kb + nst < kbn) tc::mma_commit(sfree_bar(st));
-        if (kb + 1 == kbn) tc::mma_commit(accf_bar);
+      if (!ready) {
+        if (RING && kb) ok = tc::mbar_wait_spin(x_bar(st), ph, p.status, 31);
+        ok = ok && tc::mbar_wait_spin(deq_bar(a), aph, p.status, 32);
+        if (!ok) break;
       }
-      if (++st == nst && RING) { st = 0; ph ^= 1u; }
+      tc::fence_after_sync();
+      int st_n = st + 1, a_n = a + 1;
+      uint32_t ph_n = ph, aph_n = aph;
+      if (st_n == nst && RING) { st_n = 0; ph_n ^= 1u; }
+      if (a_n == p.slots) { a_n = 0; aph_n ^= 1u; }
+      ready = tc::mma4_ts_commit_probe(el, tmem_base, tmem_base + a_col + uint32_t(a) * kSkSlotCols, tc::smem_desc_sw128(base + x_base + st * xbytes), idesc,
+                                       uint32_t(kb != 0), afree_bar(a), RING && kb + nst < kbn, sfree_bar(RING ? st : 0), deq_bar(a_n), aph_n,
+                                       x_bar(RING ? st_n : 0), RING ? ph_n : 0u);
+      if (el && kb + 1 == kbn) tc::mma_commit(accf_bar);
+      st = st_n; a = a_n; ph = ph_n; aph = aph_n;
     }
     if (lane == 0) SK_MARK(5);
   } else {
     // ------------------------------ dequant (three groups) ------------------------------
     const int dgroup = (warp - 2) >> 2;
-    const int t = ((warp - 2) & 3) * 32 + lane;  // weight row inside the tile
+    const int t = (warp & 3) * 32 + lane;  // weight row inside the tile = lane of tensor memory (a warp reaches quadrant warp % 4)
+    const uint32_t a_lane = tmem_base + (uint32_t((warp & 3) * 32) << 16) + a_col;
     const int kbpg = p.group_size / 64;
     bool ok = true;
     auto load_sz = [&](int kb) {
       const size_t idx = (size_t(ft) * 128 + t) * p.groups_per_row + (kb0 + kb) / kbpg;
       return uint32_t(__half_as_ushort(__ldg(p.scales + idx))) | (uint32_t(__half_as_ushort(__ldg(p.zeros + idx))) << 16);
     };
-    uint32_t sz_next = RING && dgroup < kbn ? load_sz(dgroup) : 0u;
-    int st = dgroup;  // a ring that goes round has at least four stages
-    uint32_t ph = 0;
+    uint32_t sz_next = dgroup < kbn ? load_sz(dgroup) : 0u;  // a block of this group ahead
+    int st = dgroup, a = dgroup;  // a ring that goes round has at least four stages
+    uint32_t ph = 0, aph = 1;     // aph: parity of the slot's last release; the first pass waits for none
     for (int kb = dgroup; kb < kbn && ok; kb += 3) {
-      const uint32_t sz = RING ? sz_next : load_sz(kb);
-      if (RING && kb + 3 < kbn) sz_next = load_sz(kb + 3);
+      const uint32_t sz = sz_next;
+      if (kb + 3 < kbn) sz_next = load_sz(kb + 3);
       const __half sh = __ushort_as_half(uint16_t(sz & 0xffffu)), zh = __ushort_as_half(uint16_t(sz >> 16));
       uint32_t s2, z2;
       if (BF16) {
@@ -223,36 +239,35 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
         s2 = h2_as_u32(__half2half2(sh));
         z2 = h2_as_u32(__half2half2(zh));
       }
-      // the slot's previous K block (three back) must have been consumed by its MMAs
-      if (kb >= 3) ok = tc::mbar_wait(afree_bar(dgroup), uint32_t(kb / 3 - 1) & 1u, p.status, 33);
-      ok = ok && tc::mbar_wait(w_bar(st), ph, p.status, 34);
+      bool okw = tc::mbar_wait(w_bar(st), ph, p.status, 34);
+      // the slot's previous K block must have been consumed by its MMAs
+      if (kb >= p.slots) okw = okw && tc::mbar_wait(afree_bar(a), aph, p.status, 33);
+      // one decision for the warp, and its lanes together: the store to tensor memory is a warp-wide instruction
+      ok = __all_sync(0xffffffffu, okw);
       if (!ok) break;
+      __syncwarp();
       const uint4* wp = reinterpret_cast<const uint4*>(smem + w_base + st * kSkWSlot + t * (8 * BITS));
-      uint8_t* arow = smem + dgroup * kSkATile + t * 128;
       constexpr int NV = BITS / 2;  // 16-byte vectors of packed weights per row per K block
+      uint32_t o[32];               // the row's 64 elements in pairs, in k order: one 32-bit column of tensor memory each
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         const uint4 qv = wp[v];
         const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w};
+        constexpr int PW = 32 / BITS / 2;  // output pairs per word: 4 or 8
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          constexpr int PW = 32 / BITS / 2;  // output pairs per word: 4 or 8
-          uint32_t o[PW];
-          dequant_word<BITS, BF16>(qw[j], s2, z2, o);
-#pragma unroll
-          for (int cc = 0; cc < PW / 4; ++cc) {
-            const int chunk = (v * 4 + j) * (PW / 4) + cc;  // 16-byte chunk (8 elements) in the row
-            *reinterpret_cast<uint4*>(arow + ((chunk ^ (t & 7)) << 4)) =
-                make_uint4(o[4 * cc], o[4 * cc + 1], o[4 * cc + 2], o[4 * cc + 3]);
-          }
-        }
+        for (int j = 0; j < 4; ++j) dequant_word<BITS, BF16>(qw[j], s2, z2, o + (v * 4 + j) * PW);
       }
-      tc::fence_proxy_async_smem();
-      tc::mbar_arrive(deq_bar(dgroup));
+      if (kb >= p.slots) tc::fence_after_sync();
+      tc::tmem_st_32x32(a_lane + uint32_t(a) * kSkSlotCols, o);
+      tc::tmem_st_wait();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(deq_bar(a));
+      a += 3;
+      if (a >= p.slots) { a -= p.slots; aph ^= 1u; }
       st += 3;
       if (RING && st >= nst) { st -= nst; ph ^= 1u; }
     }
-    ok = __all_sync(0xffffffffu, ok);  // a wait that gave up in any lane ends the warp's work
     if (dgroup == 0 && ok) {
       // ------------------------------ epilogue (warps 2-5: lane quadrants 2, 3, 0, 1) ------------------------------
       const int qd = warp & 3;
@@ -263,7 +278,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
         tc::fence_after_sync();
         if (warp == 2 && lane == 0) SK_MARK(6);
         const uint32_t taddr = tmem_base + (uint32_t(qd * 32) << 16);
-        // this block's part of the tile, fp32 [token][128 features], over A slots and stages
+        // this block's part of the tile, fp32 [token][128 features], over the stages
         float* part = reinterpret_cast<float*>(smem) + qd * 32 + lane;
         for (int ch = 0; ch < p.bt / 32; ++ch) {
           uint32_t r[32];
@@ -327,7 +342,7 @@ gemm_a16_skinny_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_con
 }
 
 struct SkinnyPlan {
-  int bt, n_tt, ksplit, nkb, stages, grid;
+  int bt, n_tt, ksplit, nkb, stages, slots, grid;
   size_t smem;
   double us;  // estimate
 };
@@ -362,7 +377,7 @@ int skinny_capacity(int split, size_t smem) {
 }
 
 // Token tile and K parts: the pair with the least estimated time among those whose blocks run in one wave.  The estimate (us)
-// follows the measurements of 17 to 1500 tokens on eight layer shapes: 4 for launch, first fetches and stores, 0.34 per K block
+// follows the measurements of 17 to 1500 tokens on eight layer shapes: 4 for launch, first fetches and stores, 0.31 per K block
 // (dequantisation and its hand-over; the MMAs of 256 columns hide behind it), 0.011 per column of the tile for its way out of
 // tensor memory, 0.6 for the clusters' two barriers.  It has no term for two blocks on an SM: no plan counts on a second one.
 bool skinny_search(int64_t M, int64_t N, int64_t K, int sm_count, SkinnyPlan* pl) {
@@ -373,13 +388,17 @@ bool skinny_search(int64_t M, int64_t N, int64_t K, int sm_count, SkinnyPlan* pl
     const int64_t n_tt = (M + bt - 1) / bt, tiles = nft * n_tt;
     if (tiles > sm_count) continue;
     const size_t stage = size_t(bt) * 128 + kSkWSlot;
-    const int64_t fit = std::min<int64_t>(kSkMaxStages, int64_t((kSkMaxSmem - 1024 - 3 * kSkATile) / stage));
+    const int64_t fit = std::min<int64_t>(kSkMaxStages, int64_t((kSkMaxSmem - 1024) / stage));
     for (int64_t sp = 1; sp <= kSkMaxSplit && sp <= nkb && tiles * sp <= sm_count; ++sp) {
       const int64_t kb = (nkb + sp - 1) / sp, stages = std::min(kb, fit);
-      const size_t smem = 1024 + std::max(3 * kSkATile + size_t(stages) * stage, size_t(bt) * 512);
-      const double us = 4.0 + 0.34 * double(kb) + 0.011 * bt + (sp > 1 ? 0.6 : 0.0);
+      const int slots = kb <= 3 || bt + 6 * int(kSkSlotCols) > 256 ? 3 : 6;
+      // A block with all of tensor memory shares its SM with nobody: one of another launch's cluster could hold it up in its allocation
+      // while it is itself waited for in its own.  From 96 tokens on a block has its SM to itself, too: two of one launch on one SM beside
+      // SMs that the launch before still held took 7.4-8.7 us where one each takes 6.6-7.4 (1280 -> 3840 at 96 and 128 tokens, 2048 -> 2048 at 96).
+      const size_t smem = skinny_tmem_cols(bt, slots) == 512 ? kSkMaxSmem : std::max(bt >= 96 ? kSkTwoPerSm + 1024 : 0, 1024 + std::max(size_t(stages) * stage, size_t(bt) * 512));
+      const double us = 4.0 + 0.31 * double(kb) + 0.011 * bt + (sp > 1 ? 0.6 : 0.0);
       if (us >= pl->us || (sp > 1 && skinny_capacity(int(sp), smem) < tiles * sp)) continue;
-      *pl = {bt, int(n_tt), int(sp), int(nkb), int(stages), int(tiles * sp), smem, us};
+      *pl = {bt, int(n_tt), int(sp), int(nkb), int(stages), slots, int(tiles * sp), smem, us};
     }
   }
   return pl->us < 1e30;
@@ -464,6 +483,7 @@ int gemm_a16_skinny(int bits, const void* x, const uint8_t* w, const void* scale
   p.nkb = pl.nkb;
   p.n_tt = pl.n_tt;
   p.stages = pl.stages;
+  p.slots = pl.slots;
   p.trace = nullptr;
 #ifdef ASRQ_TRACE
   if (option(kOptTrace) && workspace_bytes >= (8u << 20)) {  // marks of the launches since the option last changed

@@ -233,15 +233,42 @@ __device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Same with the A operand in tensor memory (lane = row, 32-bit column c = elements 2c and 2c+1 of a
-// 16-bit type): a K step of 16 elements is 8 columns.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                           uint32_t accumulate) {
+// One K block of 64 with the A operand in tensor memory (lane = row, 32-bit column c = elements 2c and 2c + 1 of a 16-bit type: a K step of
+// 16 elements is 8 columns) in a single instruction stream, as mma4_commit_probe_pair for one CTA: tests of the NEXT
+// block's two barriers, four MMAs (in the lane with el != 0), a commit to `commit_bar` and, with `second` != 0, one to `second_bar`.
+// Returns 1 when both probed barriers had completed their phases.
+__device__ __forceinline__ uint32_t mma4_ts_commit_probe(uint32_t el, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                                         uint32_t accumulate, uint32_t commit_bar, uint32_t second, uint32_t second_bar,
+                                                         uint32_t probe_a, uint32_t parity_a, uint32_t probe_b, uint32_t parity_b) {
+  uint32_t ready;
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t"
+      ".reg .pred pe, ps, pacc, pt, p1, p2;\n\t"
+      ".reg .b32 a1, a2, a3;\n\t"
+      ".reg .b64 b1, b2, b3;\n\t"
+      "setp.ne.b32 pe, %1, 0;\n\t"
+      "setp.ne.and.b32 ps, %8, 0, pe;\n\t"
+      "setp.ne.b32 pacc, %6, 0;\n\t"
+      "setp.eq.b32 pt, %1, %1;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p1, [%10], %11;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p2, [%12], %13;\n\t"
+      "add.u32 a1, %3, 8;\n\tadd.s64 b1, %4, 2;\n\t"
+      "add.u32 a2, %3, 16;\n\tadd.s64 b2, %4, 4;\n\t"
+      "add.u32 a3, %3, 24;\n\tadd.s64 b3, %4, 6;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [%3], %4, %5, pacc;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a1], b1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a2], b2, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a3], b3, %5, pt;\n\t"
+      "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
+      "@ps tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%9];\n\t"
+      "and.pred p1, p1, p2;\n\t"
+      "selp.u32 %0, 1, 0, p1;\n\t"
+      "}"
+      : "=r"(ready)
+      : "r"(el), "r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(commit_bar), "r"(second), "r"(second_bar), "r"(probe_a),
+        "r"(parity_a), "r"(probe_b), "r"(parity_b)
       : "memory");
+  return ready;
 }
 // Arrives once on `bar` when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {

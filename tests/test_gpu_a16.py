@@ -538,3 +538,22 @@ def test_mid_kernel_takes_the_qwen3_down_projection(m):
     with lib_option("mid_kernel", 1):
         y_old = run_a16_abi("asrq_w4a16_gemv" if m <= 32 else "asrq_w4a16_gemm", case)
     assert_close_rows(y_old, _ref32(case), what=f"down projection m{m}, other kernels")
+
+
+@pytest.mark.parametrize("bits,dtype", [(4, torch.float16), (2, torch.float16), (4, torch.bfloat16), (2, torch.bfloat16)])
+@pytest.mark.parametrize("m,k,n", [(17, 128, 128), (33, 192, 256), (64, 448, 128), (97, 2048, 128), (128, 2048, 12288), (193, 1280, 1280), (257, 5120, 256)])
+def test_one_wave_kernel_tensor_memory_slots(m, k, n, bits, dtype):
+    """Weights unpacked into tensor memory: fewer, as many and more K blocks than slots (three or six), rings of stages that go round,
+    token tiles of 32 to 256 columns (half of tensor memory and all of it)."""
+    gen = torch.Generator().manual_seed(m + k + n)
+    w = torch.randn(n, k, generator=gen) * 0.02
+    codes, scales, zeros, _ = O.rtn_codes(w, bits, 64, False)
+    case = dict(x=torch.randn(m, k, generator=gen).to(dtype), weight=O.pack_codes(codes, bits), scales=scales.half(), zeros=zeros.half(),
+                bias=(torch.randn(n, generator=gen) * 0.02).half(), bits=bits, group_size=64)
+    y = run_a16_abi(f"asrq_w{bits}a16_gemm", case, dtype=dtype)
+    ref = _ref32(case, dtype)
+    extra = None
+    if dtype == torch.bfloat16:  # the MMA takes weights rounded to bf16 (2^-9 of each): six standard deviations of that, and half an output ulp
+        wd = codes.float() * scales.half().float().repeat_interleave(64, dim=1) + zeros.half().float().repeat_interleave(64, dim=1)
+        extra = bf16_half_ulp(ref) + 6 * 2.0 ** -9 / 3 ** 0.5 * ((case["x"].float() ** 2) @ (wd ** 2).t()).sqrt()
+    assert_close_rows(y, ref, extra=extra, what=f"one wave w{bits} m{m} {k}->{n}")
