@@ -404,11 +404,18 @@ __device__ __forceinline__ void w4a4_tc_body(const CUtensorMap* tmw_p, const CUt
 #pragma unroll
       for (int ch = 0; ch < NCH; ++ch) {
         if (ch < nch) {
+          // the tokens' scales: the kernel before wrote them, so in program order, and all of them ahead of the stores, which could alias
+          float sa[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            sa[j] = 0.f;
+            if (tok0 + ch * 16 + j < p.M) asm volatile("ld.global.f32 %0, [%1];" : "=f"(sa[j]) : "l"(p.sa + tok0 + ch * 16 + j) : "memory");
+          }
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int tok = tok0 + ch * 16 + j;
             const float a = (j & 1) ? accf[ch * 8 + (j >> 1)].y : accf[ch * 8 + (j >> 1)].x;
-            if (tok < p.M) p.y[size_t(tok) * p.N + f] = float_to_out16(a * __ldcg(p.sa + tok) + bias, p.bf16);
+            if (tok < p.M) p.y[size_t(tok) * p.N + f] = float_to_out16(a * sa[j] + bias, p.bf16);
           }
         }
       }

@@ -324,3 +324,31 @@ def test_blocks_that_walk_the_tokens(m, dtype):
     qa, sa = _quant_gpu(x, True, dtype)
     _, s_ref, p_ref = O.hadamard_quant_int4(x, True)
     assert torch.equal(sa, s_ref) and torch.equal(qa, p_ref)
+
+
+@pytest.mark.parametrize("k,n", [(128, 64), (1024, 1024), (1024, 4096), (2048, 192), (4096, 1024)])
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 33, 63, 64])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_few_tokens_have_the_bits_of_the_tile_kernel(m, k, n, dtype):
+    """Up to 64 tokens the groups of a block's features are shared out among its warps; their sums are scaled and added in the order of
+    the register-tile kernel, which a call that asks for the accumulators takes.  Codes at both ends of their range among them."""
+    gen = torch.Generator().manual_seed(m + k + n)
+    qa = torch.randint(0, 256, (m, k // 2), generator=gen, dtype=torch.uint8)
+    qw = torch.randint(0, 256, (n, k // 2), generator=gen, dtype=torch.uint8)
+    qa[0], qw[0], qw[1] = 0x99, 0x88, 0x77  # -7 against -8 and 7 throughout: the largest sums
+    sa = torch.rand(m, generator=gen) * 0.1
+    sw = (torch.rand(n, k // 128, generator=gen) * 0.02).half()
+    bias = torch.randn(n, generator=gen).half()
+    qa, qw, sa, sw, bias = (t.to(DEV) for t in (qa, qw, sa, sw, bias))
+    ws = torch.zeros(max(256, _lib.workspace_bytes(_lib.WS_W4A4_GEMM, m, n, k)), dtype=torch.uint8, device=DEV)
+    dump = torch.empty(m, n, k // 128, dtype=torch.int32, device=DEV)
+    dt = _lib.F16 if dtype == torch.float16 else _lib.BF16
+
+    def run(acc):
+        y = padded((m, n), dtype, DEV)
+        _lib.call("asrq_w4a4_gemm", qa.data_ptr(), sa.data_ptr(), qw.data_ptr(), sw.data_ptr(), bias.data_ptr(), y.data_ptr(), acc, m, n, k, 128, dt,
+                  ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        check_canary(y, "output")
+        return y
+
+    assert torch.equal(run(None), run(dump.data_ptr()))
