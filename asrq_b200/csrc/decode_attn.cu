@@ -7,7 +7,7 @@
 //
 // Bound: the bytes of the cache when there are many (sequence, head) items, else latency: a launch of 64 keys for one
 // sequence took 8.5 us with one warp per item, each lane walking its keys' 128-byte rows alone.  Here an item is a block
-// of 4 or 8 warps, or a cluster of up to 8 such blocks when that fills the chip better.  HD / 8 lanes share a key (16 bytes
+// of 2, 4 or 8 warps, or a cluster of up to 8 such blocks when that fills the chip better.  HD / 8 lanes share a key (16 bytes
 // each), a warp has eight such loads of keys and eight of values in flight, and the first of them go out BEFORE the stream
 // dependency where the caller says that the cache is settled: in a decoder everything below the new position was written by
 // earlier steps.  Eight keys' partial scores are summed over the
@@ -312,8 +312,8 @@ decode_attn_kernel(const AttnParams p) {
 // Blocks of `warps` warps, in clusters of `split`, that the device holds at once (the clusters of a size leave SMs unused)
 template <int HD, int QH, int KIND>
 int resident_blocks(int split, int warps, int sm_count) {
-  static std::atomic<int> known[9][2];  // one kind of device: asked once per process
-  std::atomic<int>& k = known[split][warps == 4];
+  static std::atomic<int> known[9][9];  // one kind of device: asked once per process
+  std::atomic<int>& k = known[split][warps];
   int n = k.load(std::memory_order_relaxed);
   if (n) return n;
   cudaLaunchConfig_t cfg = {};
@@ -337,14 +337,15 @@ template <int HD, int QH, int KIND>
 int launch_attn(const AttnParams& p, int64_t items, int64_t max_keys, int sm_count, cudaStream_t stream) {
   // Blocks per item and warps per block: the pair with the least (waves of resident blocks) x (batches a warp walks, plus 2 for
   // the launch, the query and the merge, plus 1 for the cluster's merge); the fewest blocks among equals, since the cache may be
-  // much shorter than max_keys.  Over 20 to 640 items of 30 to 1500 keys the pair that this picks measured within 12% of the
+  // much shorter than max_keys.  Two warps keep many items of few keys in one wave (640 items, us: 10 keys 4.6 -> 3.2, 64 5.5 -> 4.1, 128
+  // 8.3 -> 6.9; 320 items of 1500 keys in clusters of three 29 -> 23).  Over 20 to 640 items of 30 to 1500 keys the pair that this picks measured within 12% of the
   // best of the fourteen (64-wide heads, 1500 keys, us: 20 items 5.7, 80 9.3, 160 14.7, 320 30, 640 50; one block of 8 warps per
   // item: 12.8, 13.8, 17.6, 31.7, 49.5).
   constexpr int BATCH = kU * 32 / (HD / 8);
   int split = 1, warps = kAttnWarps;
   int64_t best = INT64_MAX;
   for (int sp = 1; sp <= 8; ++sp)
-    for (int w : {8, 4}) {
+    for (int w : {8, 4, 2}) {
       const int64_t slots = resident_blocks<HD, QH, KIND>(sp, w, sm_count), waves = (items * sp + slots - 1) / slots;
       const int64_t cost = waves * ((max_keys + sp * w * BATCH - 1) / (sp * w * BATCH) + (sp > 1 ? 3 : 2));
       if (cost < best) {

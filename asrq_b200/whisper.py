@@ -242,8 +242,9 @@ class WhisperEngine:
 
     fused_self_attention = os.environ.get("ASRQ_B200_WHISPER_FUSED_SELF_ATTENTION", "1") == "1"
     # Cross-attention of a step: this library's kernel up to this many (sequence, head) pairs, the vendor library's above, which
-    # runs at the copy rate once there is a wave of them (a step of 160 pairs 1.53 against 1.64 ms, of 320 2.15 against 2.11).
-    own_cross_attention_items = int(os.environ.get("ASRQ_B200_WHISPER_OWN_CROSS_ITEMS", "296"))
+    # runs at the copy rate where this one needs a second wave of blocks (1500 keys, chains of launches, us: 280 pairs 18.3 against 23.9,
+    # 320 23.0 against 26.1, 360 31.3 against 28.8, 440 30.9 against 33.5, 560 34.4 against 40.5, 600 44.8 against 38.6).
+    own_cross_attention_items = int(os.environ.get("ASRQ_B200_WHISPER_OWN_CROSS_ITEMS", "590"))
     cross_kv_views = os.environ.get("ASRQ_B200_WHISPER_CROSS_KV_VIEWS", "1") == "1"
 
     def __init__(self, config, device, dtype=torch.float16):

@@ -1,5 +1,5 @@
 """Attention of one decoding step (csrc/decode_attn.cu) against fp32 PyTorch at the edges of its splits: a warp's batch is 32
-keys (head of 64) or 16 (head of 128), a block has 4 or 8 warps, an item 1 to 8 blocks."""
+keys (head of 64) or 16 (head of 128), a block has 2, 4 or 8 warps, an item 1 to 8 blocks."""
 import pytest
 import torch
 
@@ -15,7 +15,7 @@ def _softmax_attention(q, k, v, scale):  # q (B, H, hd), k / v (B, H, T, hd)
 
 @pytest.mark.parametrize("B,H,hd,keys,dtype", [
     (1, 1, 64, 1, torch.float16), (1, 20, 64, 1500, torch.float16), (2, 3, 128, 17, torch.bfloat16), (3, 20, 64, 257, torch.bfloat16),
-    (5, 20, 64, 1500, torch.float16), (32, 20, 64, 100, torch.float16), (40, 8, 128, 33, torch.float16),
+    (5, 20, 64, 1500, torch.float16), (32, 20, 64, 100, torch.float16), (40, 8, 128, 33, torch.float16), (16, 20, 64, 1500, torch.float16), (28, 20, 64, 191, torch.bfloat16),
 ])
 @pytest.mark.parametrize("settled", [False, True])
 def test_cross(B, H, hd, keys, dtype, settled):
