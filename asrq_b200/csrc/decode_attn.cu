@@ -337,16 +337,17 @@ template <int HD, int QH, int KIND>
 int launch_attn(const AttnParams& p, int64_t items, int64_t max_keys, int sm_count, cudaStream_t stream) {
   // Blocks per item and warps per block: the pair with the least (waves of resident blocks) x (batches a warp walks, plus 2 for
   // the launch, the query and the merge, plus 1 for the cluster's merge); the fewest blocks among equals, since the cache may be
-  // much shorter than max_keys.  Two warps keep many items of few keys in one wave (640 items, us: 10 keys 4.6 -> 3.2, 64 5.5 -> 4.1, 128
-  // 8.3 -> 6.9; 320 items of 1500 keys in clusters of three 29 -> 23).  Over 20 to 640 items of 30 to 1500 keys the pair that this picks measured within 12% of the
-  // best of the fourteen (64-wide heads, 1500 keys, us: 20 items 5.7, 80 9.3, 160 14.7, 320 30, 640 50; one block of 8 warps per
-  // item: 12.8, 13.8, 17.6, 31.7, 49.5).
+  // much shorter than max_keys.  Two warps keep many items of few keys in one wave (640 items, us: 10 keys 4.6 -> 3.2, 64
+  // 5.5 -> 4.1, 128 8.3 -> 6.9; 320 items of 1500 keys in clusters of three 29 -> 23).  Clusters of more than two blocks count a
+  // sixteenth fewer slots than the occupancy query gives: behind a running launch they do not pack as tightly (377 clusters of
+  // three by the query; 340 take one wave and 23.4 us, 360 take 32.4, and 29.7 as single blocks of four warps).
   constexpr int BATCH = kU * 32 / (HD / 8);
   int split = 1, warps = kAttnWarps;
   int64_t best = INT64_MAX;
   for (int sp = 1; sp <= 8; ++sp)
     for (int w : {8, 4, 2}) {
-      const int64_t slots = resident_blocks<HD, QH, KIND>(sp, w, sm_count), waves = (items * sp + slots - 1) / slots;
+      const int64_t held = resident_blocks<HD, QH, KIND>(sp, w, sm_count), slots = sp > 2 ? held * 15 / 16 : held;
+      const int64_t waves = (items * sp + slots - 1) / slots;
       const int64_t cost = waves * ((max_keys + sp * w * BATCH - 1) / (sp * w * BATCH) + (sp > 1 ? 3 : 2));
       if (cost < best) {
         best = cost;

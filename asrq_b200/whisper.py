@@ -241,9 +241,10 @@ class WhisperEngine:
     """
 
     fused_self_attention = os.environ.get("ASRQ_B200_WHISPER_FUSED_SELF_ATTENTION", "1") == "1"
-    # Cross-attention of a step: this library's kernel up to this many (sequence, head) pairs, the vendor library's above, which
-    # runs at the copy rate where this one needs a second wave of blocks (1500 keys, chains of launches, us: 280 pairs 18.3 against 23.9,
-    # 320 23.0 against 26.1, 360 31.3 against 28.8, 440 30.9 against 33.5, 560 34.4 against 40.5, 600 44.8 against 38.6).
+    # Cross-attention of a step: this library's kernel up to this many (sequence, head) pairs, which is where four-warp blocks stop
+    # fitting in one wave; the vendor library's above (1500 keys, chains of launches, us, this library's first: 280 pairs 18.5 against
+    # 23.7, 320 23.0 against 26.1, 360 29.5 against 28.4, 380 29.7 against 30.0, 440 30.6 against 33.2, 580 35.0 against 41.6, 600 44.3
+    # against 38.7; 360 to 370 pairs is the one stretch below the line where the vendor's is ahead).
     own_cross_attention_items = int(os.environ.get("ASRQ_B200_WHISPER_OWN_CROSS_ITEMS", "590"))
     cross_kv_views = os.environ.get("ASRQ_B200_WHISPER_CROSS_KV_VIEWS", "1") == "1"
 
