@@ -356,7 +356,7 @@ static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scale
   // Decode batches (17..128 tokens): the one-wave kernel, where it covers the layer (up to 148 feature tiles).  Above, while a tile
   // with all of K leaves SMs idle: where its estimate, which the fused epilogue is not even counted in, is the lower one.  Eight
   // layer shapes of 1280 to 6144 inputs, chains of launches, one-wave against the other kernels at 24 to 128 tokens: 1.25 to 2 times
-  // as fast; the widest, 2048 -> 12288, us: 15.5 / 16.7 / 17.8 at 64 / 96 / 128 tokens against 16.2 / 16.4 / 16.7.
+  // as fast; the widest, 2048 -> 12288, us: 14.0 / 14.7 / 15.6 at 64 / 96 / 128 tokens against 16.2 / 16.4 / 16.7.
   const double one_wave = option(kOptMidKernel) != 1 && option(kOptTcPair) < 0 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0
                               ? gemm_a16_skinny_estimate(M, N, K, group_size, f->sm_count, workspace_bytes) : -1.0;
   // Large calls: the weights dequantised once and the epilogue in the GEMM, where that is estimated below both the others (measured:
@@ -425,7 +425,7 @@ static int linearq_a16(int bits, const void* x, const uint8_t* w, const void* sc
   int rc;
   // From 17 tokens the tensor cores, unless switched off for 17..32: the mma.sync decode kernel takes sixteen tokens per
   // launch and is bound by the legacy MMA pipe (2048 -> 12288, us in a chain of launches: 23 for 24 tokens, 29 for 32; the one-wave
-  // kernel 14.1 and 14.3).
+  // kernel 12.7 and 12.9).
   if (tc_ok && (M > kGemvMaxM || (M > 16 && option(kOptMidKernel) != 1)))
     rc = a16_gemm(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream,
                   ep, &fused, true);
