@@ -429,10 +429,20 @@ class LinearQ(nn.Module):
 PRE_LAYERNORM, PRE_RMSNORM, PRE_SILU_MUL = 1, 2, 3  # asrq_linearq_a16_pre
 
 
+def calls_only_linearq(layer) -> bool:
+    """Whether calling ``layer`` runs :meth:`LinearQ.forward` and nothing else: no subclass or stand-in, no hooks, no replaced method."""
+    return (type(layer) is LinearQ and not layer._forward_hooks and not layer._forward_pre_hooks and "forward" not in layer.__dict__ and
+            "forward_fused" not in layer.__dict__ and not nn.modules.module._global_forward_hooks and
+            not nn.modules.module._global_forward_pre_hooks)
+
+
 def linear_after(layer: LinearQ, pre: int, x: torch.Tensor, weight=None, bias=None, eps: float = 0.0, residual=None, gelu: bool = False):
     """``layer.forward_fused(h, residual, gelu)`` where ``h`` is the step ahead of the layer: the layer norm or RMS norm of the
     residual stream ``x``, or ``silu(gate) * up`` of a fused projection's output ``x``.  For one or two rows (one for the last)
-    both are one kernel; otherwise None, and the caller does them one after the other."""
+    both are one kernel; otherwise None, and the caller does them one after the other; so also where a call of the layer does
+    more than its product (:func:`calls_only_linearq`)."""
+    if not calls_only_linearq(layer):
+        return None
     k, n = layer.in_features, layer.out_features
     width = 2 * k if pre == PRE_SILU_MUL else k
     rows = x.numel() // width
@@ -441,6 +451,8 @@ def linear_after(layer: LinearQ, pre: int, x: torch.Tensor, weight=None, bias=No
         return None
     layer._check_buffers(x)
     if residual is not None and not (residual.numel() == rows * n and residual.is_contiguous() and residual.dtype == x.dtype and residual.device == x.device):
+        return None
+    if layer.bias is not None and not layer.bias.is_contiguous():
         return None
     for t in (weight, bias):
         if t is not None and not (t.numel() == k and t.is_contiguous() and t.dtype == x.dtype and t.device == x.device):

@@ -23,8 +23,8 @@ import torch.nn.functional as F
 
 from . import packing
 from .convert import linearq_from_linear
-from .linear import (PRE_RMSNORM, PRE_SILU_MUL, LinearQ, add_rmsnorm, argmax_rows, decode_grouped_attention, dense_head, linear_after, qk_norm_rope,
-                     silu_mul)
+from .linear import (PRE_RMSNORM, PRE_SILU_MUL, LinearQ, add_rmsnorm, argmax_rows, calls_only_linearq, decode_grouped_attention, dense_head,
+                     linear_after, qk_norm_rope, silu_mul)
 from .whisper import _baked_in, _cat_linearq, _same
 
 try:
@@ -236,7 +236,8 @@ class Qwen3Engine:
         and attention are one kernel for heads of 128 in pairs (Qwen3's), else the prompt's kernel and a masked attention."""
         B = x.shape[0]
         # one or two sequences: the norms inside the projections behind them, the residual in the epilogue of those ahead (the same bits)
-        qkv = linear_after(L["qkv"], PRE_RMSNORM, x, L["ln1"], None, self.eps) if delta is None else None
+        lean = delta is None and all(calls_only_linearq(L[name]) for name in ("qkv", "o", "gu", "down"))
+        qkv = linear_after(L["qkv"], PRE_RMSNORM, x, L["ln1"], None, self.eps) if lean else None
         lean = qkv is not None
         if not lean:
             x, h = add_rmsnorm(x, delta, L["ln1"], self.eps)

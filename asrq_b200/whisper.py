@@ -205,10 +205,13 @@ class _Norm:
     def __call__(self, x):
         return add_layernorm(x, None, self.w, self.b, self.eps)[1]
 
-    def then(self, layer, x, gelu=False):
-        """``layer(self(x))`` (with GELU): one kernel for a row or two, else two."""
-        y = linear_after(layer, PRE_LAYERNORM, x, self.w, self.b, self.eps, gelu=gelu)
-        return layer.forward_fused(self(x), gelu=gelu) if y is None else y
+
+def _norm_then(norm, layer, x, gelu=False):
+    """``layer(norm(x))`` (with GELU): one kernel for a row or two, else two.  Either may have been replaced or hooked by the user."""
+    y = linear_after(layer, PRE_LAYERNORM, x, norm.w, norm.b, norm.eps, gelu=gelu) if type(norm) is _Norm else None
+    if y is not None:
+        return y
+    return layer.forward_fused(norm(x), gelu=True) if gelu else layer(norm(x))
 
 
 def _fold_query_scale(lq: LinearQ, rows: int, s: float) -> bool:
@@ -453,7 +456,7 @@ class WhisperEngine:
             self.mask.index_fill_(3, self.pos, 0.0)
         x = (self.embed[self.tok] + self.dec_pos[self.pos]).unsqueeze(1)  # (B, 1, d)
         for i, L in enumerate(self.dec_layers):
-            qkv = L["ln1"].then(L["qkv"], x)
+            qkv = _norm_then(L["ln1"], L["qkv"], x)
             if self.fused_self_attention:
                 # this position's key and value into the cache and the attention over the cache: one kernel
                 a = decode_self_attention(qkv, self.kv_self[i], self.pos, 1.0 if L["q_folded"] else scaling, settled=True).unsqueeze(1)
@@ -464,7 +467,7 @@ class WhisperEngine:
                 self.kv_self[i].index_copy_(3, self.pos, qkv[..., self.d:].view(b, 1, 2, self.heads_d, hd).permute(2, 0, 3, 1, 4))
                 a = self._attend(q, self.kv_self[i, 0], self.kv_self[i, 1], self.heads_d, self.mask)
             x = L["out"].forward_fused(a, residual=x)
-            q = L["lnx"].then(L["xq"], x)
+            q = _norm_then(L["lnx"], L["xq"], x)
             if self.cross_kv_views and hd in (64, 128) and b * self.heads_d <= self.own_cross_attention_items:
                 a = decode_cross_attention(q, self.xkv[i], self.heads_d, 1.0 if L["xq_folded"] else scaling, settled=True).unsqueeze(1)
             else:
@@ -472,7 +475,7 @@ class WhisperEngine:
                     q = q * scaling
                 a = self._attend(q, self.k_cross[i], self.v_cross[i], self.heads_d)
             x = L["xout"].forward_fused(a, residual=x)
-            x = L["fc2"].forward_fused(L["ln2"].then(L["fc1"], x, gelu=True), residual=x)
+            x = L["fc2"].forward_fused(_norm_then(L["ln2"], L["fc1"], x, gelu=True), residual=x)
         x = self.dec_ln(x).squeeze(1)
         dense_head(x, self.head, out=self.logits)
         argmax_rows(self.logits, self.tok, self.pick, self.out_ids, self.pos)

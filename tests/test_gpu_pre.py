@@ -3,9 +3,10 @@ import pytest
 import torch
 
 import asrq_b200
-from asrq_b200 import _lib, packing
+from asrq_b200 import _lib, packing, qwen3, whisper
 from asrq_b200.linear import PRE_LAYERNORM, PRE_RMSNORM, PRE_SILU_MUL, linear_after
 from gpu_util import DEV
+from tests.qwen3_util import toy_models
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +67,36 @@ def test_what_is_not_covered_is_left_to_the_caller():
     with pytest.raises(_lib.AsrqError):
         _lib.call("asrq_linearq_a16_pre", 4, PRE_RMSNORM, x.data_ptr(), g.data_ptr(), None, 1e-5, layer.weight.data_ptr(), layer.scales.data_ptr(),
                   layer.zeros.data_ptr(), None, None, x.data_ptr(), 3, 1280, 1280, 128, _lib.F16, 0, torch.cuda.current_stream().cuda_stream)
+
+
+class _Doubling(asrq_b200.LinearQ):
+    def forward(self, input):
+        return 2 * super().forward(input)
+
+
+def test_a_layer_that_does_more_than_its_product_is_called():
+    layer, gen = _layer(1280, 1280, 4, 128)
+    x = torch.randn(1, 1280, generator=gen, device=DEV).half()
+    norm = whisper._Norm(torch.ones(1280, device=DEV).half(), torch.zeros(1280, device=DEV).half())
+    want = layer(norm(x))
+    assert torch.equal(whisper._norm_then(norm, layer, x), want)
+    seen = []
+    hook = layer.register_forward_hook(lambda m, i, o: seen.append(o))
+    assert linear_after(layer, PRE_LAYERNORM, x, norm.w, norm.b, norm.eps) is None
+    assert torch.equal(whisper._norm_then(norm, layer, x), want) and len(seen) == 1
+    hook.remove()
+    layer.__class__ = _Doubling
+    assert torch.equal(whisper._norm_then(norm, layer, x), 2 * want)
+    assert torch.equal(whisper._norm_then(torch.nn.Identity(), torch.nn.Flatten(), x), x)   # neither the engine's own
+
+
+@pytest.mark.parametrize("name", ["qkv", "o", "gu", "down"])
+def test_qwen_step_of_one_sequence_runs_the_hooks_of_its_layers(name):
+    _, _, model = toy_models()
+    eng = qwen3.Qwen3Engine.from_model(model.half().to(DEV))
+    emb = torch.randn(1, 5, eng.embed.shape[1], generator=torch.Generator().manual_seed(0)).half().to(DEV)
+    want = eng.generate(emb, 3, use_graph=False).clone()
+    calls = []
+    eng.layers[0][name].register_forward_hook(lambda m, i, o: calls.append(o.shape))
+    assert torch.equal(eng.generate(emb, 3, use_graph=False), want)
+    assert len(calls) == 3                                                                  # the prompt and two steps
