@@ -55,6 +55,9 @@ SIGNATURES = {
     "asrq_linearq_a16": (c_int, [c_int] + _A16_ARGS),
     "asrq_linearq_a16_fused": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                        c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "asrq_linearq_a16_scratch_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int, c_int, c_int]),
+    "asrq_linearq_a16_scratch": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64,
+                                         c_int64, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_size_t, c_void_p]),
     "asrq_linearq_a16_pre_covers": (c_int, [c_int, c_int, c_int64, c_int64, c_int64, c_int, c_int]),
     "asrq_linearq_a16_pre": (c_int, [c_int, c_int, c_void_p, c_void_p, c_void_p, ctypes.c_float] + [c_void_p] * 6 +
                              [c_int64, c_int64, c_int64, c_int, c_int, c_int, c_void_p]),

@@ -26,11 +26,11 @@ size_t gemm_tc_workspace_bytes(int64_t M, int64_t N);
 int gemm_a16_tc(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                 void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
                 size_t workspace_bytes, int sm_count, cudaStream_t stream, const Epilogue& ep, bool* fused);
-size_t gemm_a16_dense_workspace_bytes(int64_t N, int64_t K);
+size_t gemm_a16_dense_scratch_bytes(int64_t N, int64_t K);
 double gemm_a16_dense_estimate(int64_t M, int64_t N, int64_t K, int sm_count, bool gelu, bool residual);
 bool gemm_a16_dense_supports(int64_t M, int64_t N, int64_t K, int group_size);
 int gemm_a16_dense(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias, void* y, int64_t M,
-                   int64_t N, int64_t K, int group_size, int dtype, void* workspace, size_t workspace_bytes, int sm_count,
+                   int64_t N, int64_t K, int group_size, int dtype, void* workspace, void* scratch, size_t scratch_bytes, int sm_count,
                    cudaStream_t stream, const Epilogue& ep);
 int add_layernorm(const void* x, const void* delta, const void* gamma, const void* beta, float eps, void* x_out, void* h_out,
                   int64_t rows, int64_t dim, int dtype, cudaStream_t stream);
@@ -304,19 +304,13 @@ int asrq_version(void) { return 100; }
 
 const char* asrq_last_error_string(void) { return last_error().c_str(); }
 
-// What the dequantise-once form asks of the workspace for a call of this size (0: the call does not take it)
-static size_t dense_workspace(int64_t M, int64_t N, int64_t K) {
-  return M >= kDenseMinM && gemm_a16_dense_supports(M, N, K, 64) ? gemm_a16_dense_workspace_bytes(N, K) : 0;
-}
-
 size_t asrq_workspace_bytes(int kind, int64_t M, int64_t N, int64_t K) {
   switch (kind) {
     case ASRQ_WS_A16_GEMV:
-      return gemv_workspace_bytes(N);
     case ASRQ_WS_LINEARQ:
-      return std::max(gemv_workspace_bytes(N), dense_workspace(M, N, K));
+      return gemv_workspace_bytes(N);
     case ASRQ_WS_A16_GEMM:
-      return std::max(gemm_tc_workspace_bytes(M, N), dense_workspace(M, N, K));
+      return gemm_tc_workspace_bytes(M, N);
     case ASRQ_WS_W4A4_GEMM:
       return w4a4_tc_workspace_bytes(M, N, K);
     default:
@@ -340,9 +334,35 @@ static int a16_gemv(int bits, const void* x, const uint8_t* w, const void* scale
                   f->sm_count, static_cast<cudaStream_t>(stream), kGemvMaxSplit, ep, fused);
 }
 
+// Estimated time of the one-wave kernel, or -1 where it does not take the call.
+static double one_wave_estimate(int64_t M, int64_t N, int64_t K, int group_size, const void* bias, size_t workspace_bytes, int sm_count) {
+  return option(kOptMidKernel) != 1 && option(kOptTcPair) < 0 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0
+             ? gemm_a16_skinny_estimate(M, N, K, group_size, sm_count, workspace_bytes) : -1.0;
+}
+
+// Whether a call takes the dequantise-once form, given the scratch that it needs: the dispatch and the query for that scratch ask here.
+// Large calls, where it is estimated below both the others (measured: 1.0 to 1.5 times as fast without epilogue from 2000 tokens on,
+// 1.2 to 1.9 times with one, 0.6 to 1.0 at 600).
+static bool takes_dense(int64_t M, int64_t N, int64_t K, int group_size, bool gelu, bool res, bool any_m, double one_wave, int sm_count) {
+  const int pair = option(kOptTcPair);
+  if (!(pair == 2 ? any_m || M >= 32 : pair < 0 && M >= kDenseMinM) || !gemm_a16_dense_supports(M, N, K, group_size)) return false;
+  if (pair == 2) return true;
+  const double dense = gemm_a16_dense_estimate(M, N, K, sm_count, gelu, res);
+  // the persistent kernel's K blocks under load, 0.33 us rising to 0.5 from about 140 of them on, and the epilogue's pass
+  const double blocks = std::max(0.0, gemm_a16_tc_estimate(M, N, K, group_size, sm_count) - 5.5);
+  const double unpacking = 6.0 + blocks * std::min(1.6, 1.06 + 0.0122 * std::max(0.0, blocks - 9.4)) + (gelu || res ? 1.0 + 1.3e-6 * double(M) * double(N) : 0.0);
+  // the one-wave kernel's epilogue has nothing to run under
+  const double whole_k = one_wave * 1.06 + (gelu ? 1.5 + 1.2e-6 * double(M) * double(N) : 0.0) + (res ? 2.0 + 1.5e-6 * double(M) * double(N) : 0.0);
+  return dense * 1.04 < unpacking && (one_wave <= 0 || dense * 1.04 < whole_k);
+}
+
+// scratch: memory of this call's own for the weights as 16-bit values, or NULL.  (Not the workspace: that is shared by what runs on a
+// stream, and a second call may be unpacking into it while this one's GEMM reads: two graphs that were captured on one stream, two
+// threads whose launches alternate.)
 static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
                     void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, void* workspace,
-                    size_t workspace_bytes, void* stream, const Epilogue& ep = Epilogue(), bool* fused = nullptr, bool any_m = false) {
+                    size_t workspace_bytes, void* stream, const Epilogue& ep = Epilogue(), bool* fused = nullptr, bool any_m = false,
+                    void* scratch = nullptr, size_t scratch_bytes = 0) {
   last_error().clear();
   bool fused_here = false;
   if (!fused) fused = &fused_here;
@@ -357,25 +377,12 @@ static int a16_gemm(int bits, const void* x, const uint8_t* w, const void* scale
   // with all of K leaves SMs idle: where its estimate, which the fused epilogue is not even counted in, is the lower one.  Eight
   // layer shapes of 1280 to 6144 inputs, chains of launches, one-wave against the other kernels at 24 to 128 tokens: 1.25 to 2 times
   // as fast; the widest, 2048 -> 12288, us: 14.0 / 14.7 / 15.6 at 64 / 96 / 128 tokens against 16.2 / 16.4 / 16.7.
-  const double one_wave = option(kOptMidKernel) != 1 && option(kOptTcPair) < 0 && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0
-                              ? gemm_a16_skinny_estimate(M, N, K, group_size, f->sm_count, workspace_bytes) : -1.0;
-  // Large calls: the weights dequantised once and the epilogue in the GEMM, where that is estimated below both the others (measured:
-  // 1.0 to 1.5 times as fast without epilogue from 2000 tokens on, 1.2 to 1.9 times with one, 0.6 to 1.0 at 600).
-  const int pair = option(kOptTcPair);
-  if ((pair == 2 ? any_m || M >= 32 : pair < 0 && M >= kDenseMinM) && gemm_a16_dense_supports(M, N, K, group_size) && aligned16(ep.residual) &&
-      workspace_bytes >= gemm_a16_dense_workspace_bytes(N, K)) {
-    const bool gelu = ep.act == kActGelu, res = ep.residual != nullptr;
-    const double dense = gemm_a16_dense_estimate(M, N, K, f->sm_count, gelu, res);
-    // the persistent kernel's K blocks under load, 0.33 us rising to 0.5 from about 140 of them on, and the epilogue's pass
-    const double blocks = std::max(0.0, gemm_a16_tc_estimate(M, N, K, group_size, f->sm_count) - 5.5);
-    const double unpacking = 6.0 + blocks * std::min(1.6, 1.06 + 0.0122 * std::max(0.0, blocks - 9.4)) + (gelu || res ? 1.0 + 1.3e-6 * double(M) * double(N) : 0.0);
-    // the one-wave kernel's epilogue has nothing to run under
-    const double whole_k = one_wave * 1.06 + (gelu ? 1.5 + 1.2e-6 * double(M) * double(N) : 0.0) + (res ? 2.0 + 1.5e-6 * double(M) * double(N) : 0.0);
-    if (pair == 2 || (dense * 1.04 < unpacking && (one_wave <= 0 || dense * 1.04 < whole_k))) {
-      *fused = true;
-      return gemm_a16_dense(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, f->sm_count,
-                            static_cast<cudaStream_t>(stream), ep);
-    }
+  const double one_wave = one_wave_estimate(M, N, K, group_size, bias, workspace_bytes, f->sm_count);
+  if (scratch && scratch_bytes >= gemm_a16_dense_scratch_bytes(N, K) &&
+      takes_dense(M, N, K, group_size, ep.act == kActGelu, ep.residual != nullptr, any_m, one_wave, f->sm_count)) {
+    *fused = true;
+    return gemm_a16_dense(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, scratch, scratch_bytes, f->sm_count,
+                          static_cast<cudaStream_t>(stream), ep);
   }
   if (one_wave > 0 && (M <= 128 || one_wave < gemm_a16_tc_estimate(M, N, K, group_size, f->sm_count))) {
     *fused = true;
@@ -409,9 +416,18 @@ int asrq_w2a16_gemm(const void* x, const uint8_t* w, const void* scales, const v
   return a16_gemm(2, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream);
 }
 
+// Whether LinearQ.forward goes to the tensor-core kernels.  From 17 tokens on, unless switched off for 17..32: the mma.sync decode kernel
+// takes sixteen tokens per launch and is bound by the legacy MMA pipe (2048 -> 12288, us in a chain of launches: 23 for 24 tokens, 29
+// for 32; the one-wave kernel 12.7 and 12.9).
+static bool linearq_takes_gemm(int64_t M, int64_t N, int64_t K, int group_size) {
+  const bool tc_ok = N % 128 == 0 && K % 64 == 0 && group_size > 0 && group_size % 64 == 0 && K % group_size == 0;
+  return tc_ok && (M > kGemvMaxM || (M > 16 && option(kOptMidKernel) != 1));
+}
+
 static int linearq_a16(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros,
                        const void* bias, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype,
-                       void* workspace, size_t workspace_bytes, void* stream, const Epilogue& ep) {
+                       void* workspace, size_t workspace_bytes, void* stream, const Epilogue& ep, void* scratch = nullptr,
+                       size_t scratch_bytes = 0) {
   if (bits != 2 && bits != 4) {
     last_error().clear();
     return fail(ASRQ_ERR_SHAPE, "asrq_linearq_a16: bits must be 2 or 4 (got %d)", bits);
@@ -420,15 +436,12 @@ static int linearq_a16(int bits, const void* x, const uint8_t* w, const void* sc
   if (ep.act != kActNone && ep.act != kActGelu) return fail(ASRQ_ERR_SHAPE, "asrq_linearq_a16_fused: act %d", ep.act);
   if (want_ep && ((M * N) % 8 || !aligned16(y) || !aligned16(ep.residual)))
     return fail(ASRQ_ERR_ALIGN, "asrq_linearq_a16_fused: y and residual must be 16-byte aligned and M*N a multiple of 8");
-  const bool tc_ok = N % 128 == 0 && K % 64 == 0 && group_size > 0 && group_size % 64 == 0 && K % group_size == 0;
+  if (!aligned16(scratch)) return fail(ASRQ_ERR_ALIGN, "asrq_linearq_a16_scratch: scratch must be 16-byte aligned");
   bool fused = false;
   int rc;
-  // From 17 tokens the tensor cores, unless switched off for 17..32: the mma.sync decode kernel takes sixteen tokens per
-  // launch and is bound by the legacy MMA pipe (2048 -> 12288, us in a chain of launches: 23 for 24 tokens, 29 for 32; the one-wave
-  // kernel 12.7 and 12.9).
-  if (tc_ok && (M > kGemvMaxM || (M > 16 && option(kOptMidKernel) != 1)))
+  if (linearq_takes_gemm(M, N, K, group_size))
     rc = a16_gemm(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream,
-                  ep, &fused, true);
+                  ep, &fused, true, scratch, scratch_bytes);
   else
     rc = a16_gemv(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream, ep, &fused);
   if (rc || !want_ep || fused || M == 0) return rc;
@@ -452,6 +465,24 @@ int asrq_linearq_a16_fused(int bits, const void* x, const uint8_t* w, const void
   ep.residual = residual;
   ep.act = act;
   return linearq_a16(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream, ep);
+}
+
+size_t asrq_linearq_a16_scratch_bytes(int64_t M, int64_t N, int64_t K, int group_size, int act, int has_residual) {
+  last_error().clear();
+  const DeviceFacts* f;
+  if (M <= 0 || N <= 0 || K <= 0 || !linearq_takes_gemm(M, N, K, group_size) || device_facts(&f)) return 0;
+  const double one_wave = M >= kDenseMinM ? one_wave_estimate(M, N, K, group_size, nullptr, kStatusBytes, f->sm_count) : -1.0;
+  return takes_dense(M, N, K, group_size, act == kActGelu, has_residual != 0, true, one_wave, f->sm_count) ? gemm_a16_dense_scratch_bytes(N, K) : 0;
+}
+
+int asrq_linearq_a16_scratch(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias,
+                             const void* residual, void* y, int64_t M, int64_t N, int64_t K, int group_size, int dtype, int act,
+                             void* workspace, size_t workspace_bytes, void* scratch, size_t scratch_bytes, void* stream) {
+  Epilogue ep;
+  ep.residual = residual;
+  ep.act = act;
+  return linearq_a16(bits, x, w, scales, zeros, bias, y, M, N, K, group_size, dtype, workspace, workspace_bytes, stream, ep, scratch,
+                     scratch_bytes);
 }
 
 static int check_pre(const char* who, int bits, int pre, int64_t M, int64_t N, int64_t K, int dtype) {

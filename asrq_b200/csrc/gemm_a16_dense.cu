@@ -2,7 +2,7 @@
 //
 // The kernels that unpack weights inside the GEMM do it again for every token tile: at 48 000 tokens the same 128 x 64 block of
 // weights is unpacked 188 times, beside the MMAs and at the same power budget, and their few epilogue warps have no issue slots
-// left for an activation.  Here `unpack_kernel` writes the layer's 16-bit weights into the caller's workspace (13 MB for
+// left for an activation.  Here `unpack_kernel` writes the layer's 16-bit weights into scratch of the call's own (13 MB for
 // 1280 -> 5120, which stay in L2) and `gemm_dense_kernel` takes both operands by TMA:
 //
 //   * activations are the MMA's A operand (256 tokens of a CTA pair, 128 per CTA = TMEM lanes), weights the B operand (up to
@@ -35,7 +35,6 @@ constexpr int kDnProducerWarp = 0, kDnMmaWarp = 1, kDnFirstEpilogueWarp = 4;
 constexpr uint32_t kDnXBytes = 128 * 128;   // a CTA's 128 tokens x 64 elements
 constexpr uint32_t kDnRingBytes = 6 * 2 * kDnXBytes;  // six stages with half of 256 features beside the tokens, more of narrower ones
 constexpr uint32_t kDnBoxBytes = 32 * 64;   // an epilogue warp's 32 tokens x 32 features
-constexpr size_t kDnWeightOffset = (kPartialOffset + 1023) / 1024 * 1024;  // of the 16-bit weights in the workspace
 
 struct DenseParams {
   const __half* bias;
@@ -74,7 +73,7 @@ __device__ __forceinline__ void dense_unit(const DenseParams& p, int u, int& tt,
 // ---- packed weights -> 16-bit weights, (N, K) row-major ------------------------------------------------------------
 // A thread takes 32-bit words of packed weights (8 or 16 outputs, one or two 16-byte stores; a warp reads 128 and writes 512 or
 // 1024 contiguous bytes); words, scales and zeros are constants and are fetched ahead of the stream dependency, the stores wait,
-// because the kernel before on the stream may still read the workspace.
+// because a kernel before on the stream may still use that memory.
 constexpr int kUnpackWords = 4;
 template <int BITS, bool BF16>
 __global__ void __launch_bounds__(256)
@@ -403,8 +402,8 @@ double pick_units(DenseParams* p, int64_t M, int64_t N, int max_clusters) {
 
 }  // namespace
 
-// Status block, counters and the 16-bit weights.
-size_t gemm_a16_dense_workspace_bytes(int64_t N, int64_t K) { return kDnWeightOffset + size_t(2) * size_t(N) * size_t(K); }
+// The 16-bit weights.
+size_t gemm_a16_dense_scratch_bytes(int64_t N, int64_t K) { return size_t(2) * size_t(N) * size_t(K); }
 
 // Estimated time in us, epilogue included: unpacking and two launches, and the rounds' K blocks at the clock that the power limit
 // leaves (1.8 GHz for a call of 20 us, 1.3 from about 70 us on).  Measured, W4, fp16, us: 21.1 for 1500 tokens of 1280 -> 5120, 33.7 for
@@ -421,21 +420,20 @@ bool gemm_a16_dense_supports(int64_t M, int64_t N, int64_t K, int group_size) {
 }
 
 int gemm_a16_dense(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros, const void* bias, void* y, int64_t M,
-                   int64_t N, int64_t K, int group_size, int dtype, void* workspace, size_t workspace_bytes, int sm_count,
+                   int64_t N, int64_t K, int group_size, int dtype, void* workspace, void* scratch, size_t scratch_bytes, int sm_count,
                    cudaStream_t stream, const Epilogue& ep) {
   if (!gemm_a16_dense_supports(M, N, K, group_size))
     return fail(ASRQ_ERR_SHAPE, "w%da16 gemm (dense): unsupported shape N=%lld K=%lld g=%d", bits, (long long)N, (long long)K, group_size);
-  if (workspace_bytes < gemm_a16_dense_workspace_bytes(N, K)) return fail(ASRQ_ERR_WORKSPACE, "w%da16 gemm (dense): workspace too small", bits);
-  if (!aligned16(x) || !aligned16(w) || !aligned16(y) || !aligned16(ep.residual))
-    return fail(ASRQ_ERR_ALIGN, "w%da16 gemm (dense): x, w, y and residual must be 16-byte aligned", bits);
+  if (!scratch || scratch_bytes < gemm_a16_dense_scratch_bytes(N, K)) return fail(ASRQ_ERR_WORKSPACE, "w%da16 gemm (dense): scratch too small", bits);
+  if (!aligned16(x) || !aligned16(w) || !aligned16(y) || !aligned16(ep.residual) || !aligned16(scratch))
+    return fail(ASRQ_ERR_ALIGN, "w%da16 gemm (dense): x, w, y, residual and scratch must be 16-byte aligned", bits);
   const bool bf16 = dtype == ASRQ_BF16;
-  void* w16 = static_cast<char*>(workspace) + kDnWeightOffset;
 
   const unsigned words_per_row = unsigned(K * bits / 32), n_words = unsigned(N) * words_per_row;
   const int blocks = int((n_words + 256u * kUnpackWords - 1) / (256u * kUnpackWords));
   auto unpack = [&](auto kern) {
     return launch(kern, blocks, 256, 0, stream, reinterpret_cast<const uint32_t*>(w), static_cast<const __half*>(scales),
-                  static_cast<const __half*>(zeros), static_cast<uint4*>(w16), n_words, words_per_row, unsigned(group_size * bits / 32),
+                  static_cast<const __half*>(zeros), static_cast<uint4*>(scratch), n_words, words_per_row, unsigned(group_size * bits / 32),
                   unsigned(K / group_size));
   };
   int rc = bits == 4 ? (bf16 ? unpack(unpack_kernel<4, true>) : unpack(unpack_kernel<4, false>))
@@ -454,8 +452,8 @@ int gemm_a16_dense(int bits, const void* x, const uint8_t* w, const void* scales
   p.stages = int(std::min<unsigned>(kDnMaxStages, kDnRingBytes / p.stage_bytes));
   CUtensorMap tmx, tmw, tmwt, tmy, tmr;
   if ((rc = make_tmap_2d(&tmx, x, 2, bf16, uint64_t(K), uint64_t(M), 64, 128, kSwizzle128))) return rc;
-  if ((rc = make_tmap_2d(&tmw, w16, 2, bf16, uint64_t(K), uint64_t(N), 64, 128, kSwizzle128))) return rc;
-  if ((rc = make_tmap_2d(&tmwt, w16, 2, bf16, uint64_t(K), uint64_t(N), 64, uint32_t(p.w * 16), kSwizzle128))) return rc;
+  if ((rc = make_tmap_2d(&tmw, scratch, 2, bf16, uint64_t(K), uint64_t(N), 64, 128, kSwizzle128))) return rc;
+  if ((rc = make_tmap_2d(&tmwt, scratch, 2, bf16, uint64_t(K), uint64_t(N), 64, uint32_t(p.w * 16), kSwizzle128))) return rc;
   if ((rc = make_tmap_2d(&tmy, y, 2, bf16, uint64_t(N), uint64_t(M), 32, 32, kSwizzle64))) return rc;
   tmr = tmy;
   if (ep.residual && (rc = make_tmap_2d(&tmr, ep.residual, 2, bf16, uint64_t(N), uint64_t(M), 32, 32, kSwizzle64))) return rc;

@@ -160,6 +160,18 @@ at::Tensor output_like(const at::Tensor& x, int64_t n) {
   return at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt);
 }
 
+// Memory of a large call's own for its weights as 16-bit values, from torch's allocator: on a shared stream a block that no other call
+// has, under capture the graph's.  Undefined where the call needs none, and where there is none to be had: the kernels that unpack inside
+// the GEMM run then.
+at::Tensor weights_scratch(int64_t bytes, const c10::Device& device) {
+  if (bytes == 0) return at::Tensor();
+  try {
+    return at::detail::empty_cuda({bytes}, at::kByte, device, std::nullopt);
+  } catch (const c10::OutOfMemoryError&) {
+    return at::Tensor();
+  }
+}
+
 PyObject* failed(const char* fn, int rc) {
   PyObject* r = PyObject_CallFunction(g_check, "si", fn, rc);
   Py_XDECREF(r);
@@ -202,13 +214,11 @@ PyObject* linearq_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     y = output_like(*x, L.n);
     g_calls.fetch_add(1, std::memory_order_relaxed);
     const void* bias = L.bias ? L.bias->data_ptr() : nullptr;
-    if (!fused)
-      rc = asrq_linearq_a16(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(), bias,
-                            y.data_ptr(), m, L.n, L.k, int(L.group), dtype, ws->data_ptr(), size_t(ws->numel()), stream);
-    else
-      rc = asrq_linearq_a16_fused(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(),
-                                  bias, res ? res->data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype,
-                                  gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE, ws->data_ptr(), size_t(ws->numel()), stream);
+    const int act = gelu ? ASRQ_ACT_GELU : ASRQ_ACT_NONE;
+    const at::Tensor w16 = weights_scratch(int64_t(asrq_linearq_a16_scratch_bytes(m, L.n, L.k, int(L.group), act, bool(res))), x->device());
+    rc = asrq_linearq_a16_scratch(int(L.bits), x->data_ptr(), static_cast<const uint8_t*>(L.weight->data_ptr()), L.scales->data_ptr(), L.zeros->data_ptr(),
+                                  bias, res ? res->data_ptr() : nullptr, y.data_ptr(), m, L.n, L.k, int(L.group), dtype, act, ws->data_ptr(),
+                                  size_t(ws->numel()), w16.defined() ? w16.data_ptr() : nullptr, w16.defined() ? size_t(w16.numel()) : 0, stream);
   }
   if (rc) return failed(fused ? "asrq_linearq_a16_fused" : "asrq_linearq_a16", rc);
   return THPVariable_Wrap(std::move(y));

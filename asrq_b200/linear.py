@@ -57,6 +57,17 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws
 
 
+def _weights_scratch(nbytes: int, device: torch.device):
+    """Memory of a large call's own for its weights as 16-bit values (asrq_linearq_a16_scratch): unlike the workspace not shared by
+    what runs on a stream.  None where the call needs none, and where there is none to be had: it then unpacks inside the GEMM."""
+    if nbytes == 0:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def check_status(device=None) -> None:
     """Synchronises the device and raises if a kernel on any of its streams reported a bounded wait that gave up."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
@@ -402,20 +413,22 @@ class LinearQ(nn.Module):
         stream = torch.cuda.current_stream(input.device).cuda_stream
         bias = None if self.bias is None else self.bias.data_ptr()
         with _on_device(input.device):
-            if residual is None and not gelu:
-                _lib.call("asrq_linearq_a16", self.bits, x2.data_ptr(), self.weight.data_ptr(), self.scales.data_ptr(),
-                          self.zeros.data_ptr(), bias, y.data_ptr(), m, n, k, self.group_size, dt, ws.data_ptr(),
-                          ws.numel(), stream)
+            r2 = None
+            if residual is not None:
+                if residual.dtype != input.dtype or residual.numel() != m * n or residual.device != input.device:
+                    raise ValueError("forward_fused: residual must have the output's shape, dtype and device")
+                r2 = residual.reshape(m, n)
+                r2 = r2 if r2.is_contiguous() else r2.contiguous()
+            act = _lib.ACT_GELU if gelu else _lib.ACT_NONE
+            w16 = _weights_scratch(_lib.load().asrq_linearq_a16_scratch_bytes(m, n, k, self.group_size, act, residual is not None), input.device)
+            args = (self.bits, x2.data_ptr(), self.weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(), bias)
+            if w16 is not None:
+                _lib.call("asrq_linearq_a16_scratch", *args, None if r2 is None else r2.data_ptr(), y.data_ptr(), m, n, k, self.group_size, dt, act,
+                          ws.data_ptr(), ws.numel(), w16.data_ptr(), w16.numel(), stream)
+            elif r2 is None and not gelu:
+                _lib.call("asrq_linearq_a16", *args, y.data_ptr(), m, n, k, self.group_size, dt, ws.data_ptr(), ws.numel(), stream)
             else:
-                r2 = None
-                if residual is not None:
-                    if residual.dtype != input.dtype or residual.numel() != m * n or residual.device != input.device:
-                        raise ValueError("forward_fused: residual must have the output's shape, dtype and device")
-                    r2 = residual.reshape(m, n)
-                    r2 = r2 if r2.is_contiguous() else r2.contiguous()
-                _lib.call("asrq_linearq_a16_fused", self.bits, x2.data_ptr(), self.weight.data_ptr(),
-                          self.scales.data_ptr(), self.zeros.data_ptr(), bias, None if r2 is None else r2.data_ptr(),
-                          y.data_ptr(), m, n, k, self.group_size, dt, _lib.ACT_GELU if gelu else _lib.ACT_NONE,
+                _lib.call("asrq_linearq_a16_fused", *args, None if r2 is None else r2.data_ptr(), y.data_ptr(), m, n, k, self.group_size, dt, act,
                           ws.data_ptr(), ws.numel(), stream)
         if _CHECK:
             check_status(input.device)

@@ -14,7 +14,9 @@
  *     here calls exit() (the reference's CUDA_CHECK does, csrc/cuda/common.h:5-12);
  *   - the caller owns all memory, including the scratch `workspace`
  *     (size from asrq_workspace_bytes); no entry point allocates, frees or
- *     synchronises, so all of them are safe on any stream;
+ *     synchronises, so all of them are safe on any stream.  A workspace belongs
+ *     to one call at a time: calls that share it are ordered, by one stream or
+ *     by the caller (graphs captured on one stream but replayed on two are not);
  *   - the buffers' device must be the CURRENT device of the calling thread (the library reads
  *     cudaGetDevice for its per-device facts and launches there);
  *   - constant operands (packed weights, scales, zeros, bias; a layer norm's weight and bias; the
@@ -115,9 +117,7 @@ int asrq_w4a16_gemv_static(const void* x, const uint8_t* w, const void* scales, 
  * For M <= 256 the K range of an output tile may be divided among several blocks
  * (fp32 parts in the workspace, added in a fixed order); with a workspace smaller
  * than asrq_workspace_bytes(ASRQ_WS_A16_GEMM, M, N, K) but at least 256 bytes the
- * call still runs, unsplit.  From 768 tokens on that size has room for the layer's 16-bit
- * weights: large calls write them there once and run a plain 16-bit GEMM (same bits); with a
- * smaller workspace they unpack inside the GEMM.
+ * call still runs, unsplit.
  * Replaces matmul_f16xint4 / matmul_f16xint2 for M > 64
  * (asrq/matmulq/csrc/bindings.cpp:44-57, 607-650, 705-747).
  */
@@ -156,6 +156,22 @@ int asrq_linearq_a16_fused(int bits, const void* x, const uint8_t* w, const void
                            const void* bias, const void* residual, void* y, int64_t M, int64_t N, int64_t K,
                            int group_size, int dtype, int act, void* workspace, size_t workspace_bytes,
                            void* stream);
+
+/*
+ * asrq_linearq_a16_fused with memory for the weights as 16-bit values: a large call (from 768 tokens) writes them there
+ * once and runs a plain 16-bit GEMM with the epilogue in it, where that is estimated faster than unpacking inside the
+ * GEMM.  Same bits.  asrq_linearq_a16_scratch_bytes: what such a call asks for (2*N*K), 0 for a call that does not take
+ * this form.  scratch may be NULL or too small: the call then unpacks inside the GEMM.  16-byte aligned; its contents on
+ * entry do not matter and nothing is kept in it.  It belongs to this call alone until the call's work is done:
+ * unlike the workspace it must not be shared by calls that the stream does not order, such as graphs that are replayed on
+ * different streams or threads whose calls on one stream may alternate.  act and residual as above, ASRQ_ACT_NONE and
+ * NULL for the plain layer.
+ */
+size_t asrq_linearq_a16_scratch_bytes(int64_t M, int64_t N, int64_t K, int group_size, int act, int has_residual);
+int asrq_linearq_a16_scratch(int bits, const void* x, const uint8_t* w, const void* scales, const void* zeros,
+                             const void* bias, const void* residual, void* y, int64_t M, int64_t N, int64_t K,
+                             int group_size, int dtype, int act, void* workspace, size_t workspace_bytes, void* scratch,
+                             size_t scratch_bytes, void* stream);
 
 /*
  * asrq_linearq_a16_fused with the step ahead of the layer in the same kernel, for a decoding step of one or two
@@ -420,7 +436,7 @@ int asrq_w4a4_gemm_f8(const uint8_t* a8, const float* sa, const uint8_t* w8, con
  *   tc_split (0)          1: no split K in the prefill kernel
  *   tc_bt (0), w4a4_bt (0)         token-tile width of the tcgen05 kernels (0 auto)
  *   tc_pair (-1), w4a4_pair (-1)   CTA-pair variants: -1 auto, 0 off, 1 on; tc_pair 2: the form that
- *                         unpacks the weights once per call, where the workspace has room for them
+ *                         unpacks the weights once per call, where the call has scratch for them
  *   tc_pair_release (0)   CTA-pair prefill kernel: 1 = release/acquire at cluster scope on the
  *                         cross-CTA "operand written" hand-off (slower), 0 = relaxed arrival
  *   trace (0), trace_block (0)     only in builds with -DASRQ_TRACE: pipeline clock marks

@@ -38,6 +38,15 @@ def test_workspace_bytes():
     assert _lib.workspace_bytes(99, 1, 1, 1) == 0
 
 
+def test_the_shared_workspace_holds_no_weights():
+    """What is written and read by one call of many launches has no place in memory that a stream's calls share: the size does not grow
+    with the layer's N * K from 768 tokens on."""
+    for kind in (_lib.WS_LINEARQ, _lib.WS_A16_GEMM):
+        for n, k in ((1280, 5120), (28672, 8192)):
+            assert _lib.workspace_bytes(kind, 48000, n, k) == _lib.workspace_bytes(kind, 767, n, k)
+    assert _lib.workspace_bytes(_lib.WS_LINEARQ, 48000, 1280, 5120) == _lib.workspace_bytes(_lib.WS_LINEARQ, 1, 1280, 5120)
+
+
 def test_null_and_dtype_rejected_before_launch():
     lib = _lib.load()
     buf = ctypes.create_string_buffer(4096 + 16)
