@@ -87,6 +87,32 @@ __device__ __forceinline__ float ldg_half(const __half* p) {
   return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short*>(p))));
 }
 
+// What the kernel before on the stream wrote must not be read ahead of griddepcontrol.wait, and a "memory" clobber there does not see to
+// it: __ldg, and a const __restrict__ kernel argument, promise the compiler that nothing writes that memory while the kernel runs, so it
+// may move such a load ahead of the wait, when the kernel before is still writing (seen in a graph: input-independent tokens).  Either
+// loads that stay in program order behind it, or a pointer that the compiler knows nothing of before it.
+__device__ __forceinline__ uint4 ld_x4(const void* p) {
+  uint4 u;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p) : "memory");
+  return u;
+}
+__device__ __forceinline__ uint2 ld_x2(const void* p) {
+  uint2 u;
+  asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(p) : "memory");
+  return u;
+}
+__device__ __forceinline__ uint16_t ld_x1(const void* p) {
+  uint16_t u;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(u) : "l"(p) : "memory");
+  return u;
+}
+template <typename T>
+__device__ __forceinline__ T* behind_wait(T* p) {
+  size_t a = __cvta_generic_to_global(p);  // still known to be global memory
+  asm volatile("" : "+l"(a) : : "memory");
+  return static_cast<T*>(__cvta_global_to_generic(a));
+}
+
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 

@@ -54,6 +54,8 @@ argmax_rows_kernel(const uint16_t* __restrict__ y, long long* __restrict__ tok, 
   __shared__ unsigned long long part[8];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  y = behind_wait(y);
+  pos = behind_wait(pos);
   const int row = blockIdx.y;
   const uint16_t* src = y + size_t(row) * N;
   auto ordered = [](uint32_t b) {  // monotone in the value; zeros equal; NaN above everything
@@ -137,6 +139,7 @@ dense_head_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  x = behind_wait(x);
   // activations -> shared memory (rows beyond M are zero)
   for (int i = threadIdx.x; i < kHeadTokens * (K / 8); i += blockDim.x) {
     const int r = i / (K / 8), c = (i - r * (K / 8)) * 8;

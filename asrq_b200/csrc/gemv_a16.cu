@@ -100,18 +100,6 @@ __device__ __forceinline__ void mma_new(float (&d)[4], uint32_t a0, uint32_t a1,
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
-// Loads of activations, in program order behind the stream dependency.  (__ldg promises the compiler that nothing writes there while the
-// kernel runs, so it may move such a load ahead of griddepcontrol.wait, when the kernel before is still writing: seen in a graph.)
-__device__ __forceinline__ uint4 ld_x4(const void* p) {
-  uint4 u;
-  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p) : "memory");
-  return u;
-}
-__device__ __forceinline__ uint2 ld_x2(const void* p) {
-  uint2 u;
-  asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(p) : "memory");
-  return u;
-}
 // two 16-bit activations as floats
 template <bool BF16>
 __device__ __forceinline__ float2 two_floats(uint32_t v) {

@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_a16_kernel(const GemvPar
       uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
       if (m < p.M) {
         const uint4* src = reinterpret_cast<const uint4*>(p.x + size_t(m) * p.K + k_begin + b * 16);
-        lo = __ldg(src);
-        hi = __ldg(src + 1);
+        lo = ld_x4(src);
+        hi = ld_x4(src + 1);
         if (p.bf16) {
           lo.x = bf16x2_to_f16x2_sat(lo.x); lo.y = bf16x2_to_f16x2_sat(lo.y);
           lo.z = bf16x2_to_f16x2_sat(lo.z); lo.w = bf16x2_to_f16x2_sat(lo.w);

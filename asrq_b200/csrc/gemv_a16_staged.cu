@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(32 * st_warps(MH), 2) gemv_a16_staged_kernel(c
         for (int v = 0; v < WPC * XR / 4; ++v) {
           uint4 u = make_uint4(0, 0, 0, 0);
           if (m < p.M) {
-            u = XS ? xp[v] : __ldcg(xp + v);  // not XS: L2 (written by the kernel before this one on the stream)
+            u = XS ? xp[v] : ld_x4(xp + v);  // not XS: written by the kernel before this one on the stream
             if (p.bf16) {
               u.x = st_bf16x2_to_f16x2_sat(u.x); u.y = st_bf16x2_to_f16x2_sat(u.y);
               u.z = st_bf16x2_to_f16x2_sat(u.z); u.w = st_bf16x2_to_f16x2_sat(u.w);

@@ -17,7 +17,8 @@
 //
 // All open with griddepcontrol.launch_dependents / .wait and are launched with programmatic stream
 // serialisation, so in a chain of this library's kernels (a decoder step replayed as a CUDA graph)
-// consecutive launches overlap their ramp-up with the predecessor's tail.
+// consecutive launches overlap their ramp-up with the predecessor's tail.  Behind the wait, what is not
+// a constant is read by ld_x4 and ld_x1 or through behind_wait (common.cuh).
 #include <algorithm>
 
 #include "common.cuh"
@@ -31,6 +32,41 @@ __device__ __forceinline__ float in16(uint16_t b, bool bf16) {
 }
 
 constexpr int kLnWarps = 8;
+
+// use(e, x[e] (+ delta[e], rounded)) for a lane's elements of a row of any width, in order, eight loads of each in flight
+template <bool bf16, bool DELTA, typename F>
+__device__ __forceinline__ void each_of_row(const uint16_t* x, const uint16_t* delta, int dim, int lane, F use) {
+  constexpr int kBatch = 8;
+  uint16_t a[kBatch], d[kBatch];
+  auto value = [&](int k) { return float_to_out16(DELTA ? in16(a[k], bf16) + in16(d[k], bf16) : in16(a[k], bf16), bf16); };
+  int e0 = lane;
+  for (; e0 + 32 * (kBatch - 1) < dim; e0 += 32 * kBatch) {
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) a[k] = ld_x1(x + e0 + 32 * k);
+    if (DELTA) {
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) d[k] = ld_x1(delta + e0 + 32 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) use(e0 + 32 * k, value(k));
+  }
+  // the rest: fewer than a batch
+#pragma unroll
+  for (int k = 0; k < kBatch - 1; ++k) {
+    if (e0 + 32 * k < dim) {
+      a[k] = ld_x1(x + e0 + 32 * k);
+      if (DELTA) d[k] = ld_x1(delta + e0 + 32 * k);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kBatch - 1; ++k)
+    if (e0 + 32 * k < dim) use(e0 + 32 * k, value(k));
+}
+template <bool bf16, typename F>
+__device__ __forceinline__ void each_of_row(const uint16_t* x, const uint16_t* delta, int dim, int lane, F use) {
+  if (delta) each_of_row<bf16, true>(x, delta, dim, lane, use);
+  else each_of_row<bf16, false>(x, delta, dim, lane, use);
+}
 
 // VEC: 16-byte vectors per lane (dim = 256 * VEC); generic dims take the strided loop with VEC = 0
 template <int VEC, bool bf16>
@@ -57,13 +93,14 @@ add_layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
   if constexpr (VEC > 0) {
     uint4 xr[VEC > 0 ? VEC : 1];  // the row (after the add, rounded to 16 bits), as the statistics see it
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const int e = (i * 32 + lane) * 8;
-      const uint4 a = *reinterpret_cast<const uint4*>(x + off + e);
-      if (delta) {
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-        const uint4 d = *reinterpret_cast<const uint4*>(delta + off + e);
-        const uint32_t dw[4] = {d.x, d.y, d.z, d.w};
+    for (int i = 0; i < VEC; ++i) xr[i] = ld_x4(x + off + (i * 32 + lane) * 8);
+    if (delta) {
+      uint4 d8[VEC > 0 ? VEC : 1];
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) d8[i] = ld_x4(delta + off + (i * 32 + lane) * 8);
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) {
+        const uint32_t aw[4] = {xr[i].x, xr[i].y, xr[i].z, xr[i].w}, dw[4] = {d8[i].x, d8[i].y, d8[i].z, d8[i].w};
         uint32_t ow[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -72,10 +109,11 @@ add_layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
           ow[j] = uint32_t(float_to_out16(lo, bf16)) | (uint32_t(float_to_out16(hi, bf16)) << 16);
         }
         xr[i] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-      } else {
-        xr[i] = a;
       }
-      if (x_out) *reinterpret_cast<uint4*>(x_out + off + e) = xr[i];
+    }
+    if (x_out) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) *reinterpret_cast<uint4*>(x_out + off + (i * 32 + lane) * 8) = xr[i];
     }
     float mean, rstd;
     ln_row_stats<(VEC > 0 ? VEC : 1)>(xr, dim, eps, bf16, mean, rstd);
@@ -99,39 +137,31 @@ add_layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
   } else {
     // any dimension: three passes over the row (the second and third hit L1/L2)
     float sum = 0.f;
-    for (int e = lane; e < dim; e += 32) {
-      float a = in16(x[off + e], bf16);
-      if (delta) a += in16(delta[off + e], bf16);
-      const uint16_t a16 = float_to_out16(a, bf16);
+    each_of_row<bf16>(x + off, delta ? delta + off : nullptr, dim, lane, [&](int e, uint16_t a16) {
       if (x_out) x_out[off + e] = a16;
       sum += in16(a16, bf16);
-    }
+    });
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float mean = sum / float(dim);
     float sq = 0.f;
-    for (int e = lane; e < dim; e += 32) {
-      float a = in16(x[off + e], bf16);
-      if (delta) a += in16(delta[off + e], bf16);
-      const float d = in16(float_to_out16(a, bf16), bf16) - mean;
+    each_of_row<bf16>(x + off, delta ? delta + off : nullptr, dim, lane, [&](int, uint16_t a16) {
+      const float d = in16(a16, bf16) - mean;
       sq = fmaf(d, d, sq);
-    }
+    });
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     const float rstd = rsqrtf(sq / float(dim) + eps);
-    for (int e = lane; e < dim; e += 32) {
-      float a = in16(x[off + e], bf16);
-      if (delta) a += in16(delta[off + e], bf16);
-      const float c = in16(float_to_out16(a, bf16), bf16);
-      h_out[off + e] = float_to_out16((c - mean) * rstd * in16(gamma[e], bf16) + in16(beta[e], bf16), bf16);
-    }
+    each_of_row<bf16>(x + off, delta ? delta + off : nullptr, dim, lane, [&](int e, uint16_t a16) {
+      h_out[off + e] = float_to_out16((in16(a16, bf16) - mean) * rstd * in16(gamma[e], bf16) + in16(beta[e], bf16), bf16);
+    });
   }
 }
 
 // One warp per row; VEC 16-byte vectors per lane when dim == 256 * VEC, else (VEC = 0) a strided loop.  All of a row's loads go
 // out before the first is used.
 template <int VEC, bool bf16>
-__global__ void __launch_bounds__(32 * kLnWarps)
+__global__ void __launch_bounds__(32 * kLnWarps, 2)
 add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ delta, const uint16_t* __restrict__ gamma,
                    float eps, uint16_t* __restrict__ x_out, uint16_t* __restrict__ h_out, int rows, int dim) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -150,10 +180,10 @@ add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
     float sq = 0.f;
     uint4 a8[VEC > 0 ? VEC : 1], d8[VEC > 0 ? VEC : 1];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) a8[i] = *reinterpret_cast<const uint4*>(x + off + (i * 32 + lane) * 8);
+    for (int i = 0; i < VEC; ++i) a8[i] = ld_x4(x + off + (i * 32 + lane) * 8);
     if (delta) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) d8[i] = *reinterpret_cast<const uint4*>(delta + off + (i * 32 + lane) * 8);
+      for (int i = 0; i < VEC; ++i) d8[i] = ld_x4(delta + off + (i * 32 + lane) * 8);
     }
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
@@ -196,23 +226,17 @@ add_rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
     }
   } else {
     float sq = 0.f;
-    for (int e = lane; e < dim; e += 32) {
-      float a = in16(x[off + e], bf16);
-      if (delta) a += in16(delta[off + e], bf16);
-      const uint16_t a16 = float_to_out16(a, bf16);
+    each_of_row<bf16>(x + off, delta ? delta + off : nullptr, dim, lane, [&](int e, uint16_t a16) {
       if (x_out) x_out[off + e] = a16;
       const float c = in16(a16, bf16);
       sq = fmaf(c, c, sq);
-    }
+    });
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     const float rs = rsqrtf(sq / float(dim) + eps);
-    for (int e = lane; e < dim; e += 32) {
-      float a = in16(x[off + e], bf16);
-      if (delta) a += in16(delta[off + e], bf16);
-      const float c = in16(float_to_out16(a, bf16), bf16);
-      h_out[off + e] = float_to_out16(in16(float_to_out16(c * rs, bf16), bf16) * in16(gamma[e], bf16), bf16);
-    }
+    each_of_row<bf16>(x + off, delta ? delta + off : nullptr, dim, lane, [&](int e, uint16_t a16) {
+      h_out[off + e] = float_to_out16(in16(float_to_out16(in16(a16, bf16) * rs, bf16), bf16) * in16(gamma[e], bf16), bf16);
+    });
   }
 }
 
@@ -230,10 +254,10 @@ row_norm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ del
   const uint4 gq = __ldg(reinterpret_cast<const uint4*>(gamma + e)), bq = LAYER ? __ldg(reinterpret_cast<const uint4*>(beta + e)) : make_uint4(0, 0, 0, 0);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const size_t off = size_t(blockIdx.x) * dim + e;
-  const uint4 a = *reinterpret_cast<const uint4*>(x + off);
+  const uint4 a = ld_x4(x + off);
   uint32_t w[4] = {a.x, a.y, a.z, a.w};
   if (delta) {
-    const uint4 d = *reinterpret_cast<const uint4*>(delta + off);
+    const uint4 d = ld_x4(delta + off);
     const uint32_t dw[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -286,6 +310,7 @@ __global__ void __launch_bounds__(256)
 silu_mul_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int rows, int inter) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  gu = behind_wait(gu);
   const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
   if (c >= inter) return;
   for (int r0 = blockIdx.y * kSiluRows; r0 < rows; r0 += gridDim.y * kSiluRows) {
@@ -331,6 +356,8 @@ qk_norm_rope_kernel(const uint16_t* __restrict__ qkv, const uint16_t* __restrict
   constexpr int LPH = HD / 8, PER = 32 / LPH, PASSES = kRopeHeads / PER;  // lanes per head, heads per pass
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  qkv = behind_wait(qkv);
+  pos_dev = behind_wait(pos_dev);
   const int lane = threadIdx.x & 31, sub = lane % LPH, hg = lane / LPH;
   const int heads = nq + 2 * nkv;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), head0 = blockIdx.y * kRopeHeads;
@@ -412,6 +439,8 @@ epilogue16_kernel(uint16_t* __restrict__ y, const uint16_t* __restrict__ residua
   constexpr int kEpiVecs = RES ? kEpiVecsResidual : kEpiVecsActivation;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  y = behind_wait(y);
+  residual = behind_wait(residual);
   for (size_t i0 = size_t(blockIdx.x) * (256 * kEpiVecs) + threadIdx.x; i0 < n_vec; i0 += size_t(gridDim.x) * (256 * kEpiVecs)) {
     uint4 a[kEpiVecs], r[kEpiVecs];
 #pragma unroll
