@@ -368,19 +368,27 @@ class LinearQ(nn.Module):
             raise NotImplementedError("bits must be 2 or 4")
         return q * scale + zero
 
-    def _check_buffers(self, x: torch.Tensor) -> None:
+    def _check_buffers(self, x: torch.Tensor):
+        """(weight, scales, zeros, bias) as the kernels take them.  The caller passes and holds these tensors, read once: another
+        thread may replace the layer's."""
+        held = []
         for name in ("weight", "scales", "zeros"):
             t = getattr(self, name)
             if t.device != x.device:
                 raise RuntimeError(f"LinearQ.{name} is on {t.device} but the input is on {x.device}")
             if not t.is_contiguous():
-                setattr(self, name, t.contiguous())
-        if self.scales.dtype != torch.float16 or self.zeros.dtype != torch.float16:
+                t = t.contiguous()
+                setattr(self, name, t)
+            held.append(t)
+        weight, scales, zeros = held
+        bias = self.bias
+        if scales.dtype != torch.float16 or zeros.dtype != torch.float16:
             raise TypeError("LinearQ.scales and LinearQ.zeros must be float16")
-        if self.weight.dtype != torch.uint8:
+        if weight.dtype != torch.uint8:
             raise TypeError("LinearQ.weight must be uint8")
-        if self.bias is not None and (self.bias.dtype != torch.float16 or self.bias.device != x.device):
+        if bias is not None and (bias.dtype != torch.float16 or bias.device != x.device):
             raise TypeError("LinearQ.bias must be float16 on the input's device")
+        return weight, scales, zeros, bias
 
     def forward(self, input):
         if _native is not None and not _CHECK:
@@ -402,7 +410,7 @@ class LinearQ(nn.Module):
         dt = _require_cuda_16bit(input, "LinearQ.forward")
         if self.bits not in (2, 4):
             raise NotImplementedError("LinearQ.forward: bits must be 2 or 4")
-        self._check_buffers(input)
+        weight, scales, zeros, bias = self._check_buffers(input)
         n, k = self.out_features, self.in_features
         x2 = _as_2d(input, k)
         m = x2.shape[0]
@@ -411,7 +419,6 @@ class LinearQ(nn.Module):
             return y.reshape(*input.shape[:-1], n)
         ws = _workspace(input.device, _lib.workspace_bytes(_lib.WS_LINEARQ, m, n, k))
         stream = torch.cuda.current_stream(input.device).cuda_stream
-        bias = None if self.bias is None else self.bias.data_ptr()
         with _on_device(input.device):
             r2 = None
             if residual is not None:
@@ -421,7 +428,7 @@ class LinearQ(nn.Module):
                 r2 = r2 if r2.is_contiguous() else r2.contiguous()
             act = _lib.ACT_GELU if gelu else _lib.ACT_NONE
             w16 = _weights_scratch(_lib.load().asrq_linearq_a16_scratch_bytes(m, n, k, self.group_size, act, residual is not None), input.device)
-            args = (self.bits, x2.data_ptr(), self.weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(), bias)
+            args = (self.bits, x2.data_ptr(), weight.data_ptr(), scales.data_ptr(), zeros.data_ptr(), None if bias is None else bias.data_ptr())
             if w16 is not None:
                 _lib.call("asrq_linearq_a16_scratch", *args, None if r2 is None else r2.data_ptr(), y.data_ptr(), m, n, k, self.group_size, dt, act,
                           ws.data_ptr(), ws.numel(), w16.data_ptr(), w16.numel(), stream)
@@ -459,18 +466,20 @@ def linear_after(layer: LinearQ, pre: int, x: torch.Tensor, weight=None, bias=No
     k, n = layer.in_features, layer.out_features
     width = 2 * k if pre == PRE_SILU_MUL else k
     rows = x.numel() // width
-    if (rows > 2 or not x.is_cuda or x.shape[-1] != width or not x.is_contiguous() or x.dtype not in _DTYPES or
-            _lib.load().asrq_linearq_a16_pre_covers(layer.bits, pre, rows, n, k, layer.group_size, _DTYPES[x.dtype]) != 1):
+    if rows > 2 or not x.is_cuda or x.shape[-1] != width or not x.is_contiguous() or x.dtype not in _DTYPES:
         return None
-    layer._check_buffers(x)
+    with _on_device(x.device):
+        if _lib.load().asrq_linearq_a16_pre_covers(layer.bits, pre, rows, n, k, layer.group_size, _DTYPES[x.dtype]) != 1:
+            return None
+    packed, scales, zeros, layer_bias = layer._check_buffers(x)
     if residual is not None and not (residual.numel() == rows * n and residual.is_contiguous() and residual.dtype == x.dtype and residual.device == x.device):
         return None
-    if layer.bias is not None and not layer.bias.is_contiguous():
+    if layer_bias is not None and not layer_bias.is_contiguous():
         return None
     for t in (weight, bias):
         if t is not None and not (t.numel() == k and t.is_contiguous() and t.dtype == x.dtype and t.device == x.device):
             return None
-    if any(t is not None and t.data_ptr() % 16 for t in (x, layer.weight, layer.scales, layer.zeros, weight, bias)):
+    if any(t is not None and t.data_ptr() % 16 for t in (x, packed, scales, zeros, weight, bias)):
         return None
     y = torch.empty((*x.shape[:-1], n), dtype=x.dtype, device=x.device)
 
@@ -478,8 +487,8 @@ def linear_after(layer: LinearQ, pre: int, x: torch.Tensor, weight=None, bias=No
         return None if t is None else t.data_ptr()
 
     with _on_device(x.device):
-        _lib.call("asrq_linearq_a16_pre", layer.bits, pre, x.data_ptr(), ptr(weight), ptr(bias), float(eps), layer.weight.data_ptr(),
-                  layer.scales.data_ptr(), layer.zeros.data_ptr(), ptr(layer.bias), ptr(residual), y.data_ptr(), rows, n, k, layer.group_size,
+        _lib.call("asrq_linearq_a16_pre", layer.bits, pre, x.data_ptr(), ptr(weight), ptr(bias), float(eps), packed.data_ptr(),
+                  scales.data_ptr(), zeros.data_ptr(), ptr(layer_bias), ptr(residual), y.data_ptr(), rows, n, k, layer.group_size,
                   _DTYPES[x.dtype], _lib.ACT_GELU if gelu else _lib.ACT_NONE, torch.cuda.current_stream(x.device).cuda_stream)
     return y
 
@@ -594,20 +603,20 @@ class LinearQQ(LinearQ):
         """``two_call=True`` forces the packed-activation sequence (asrq_hadamard_quant_int4 then
         asrq_w4a4_gemm); the default for large M is the prologue writing 8-bit operands directly.
         Both produce the same bits."""
-        self._check_buffers(input)
+        weight, scales, _, bias = self._check_buffers(input)
         if input.numel() == 0:
             _require_cuda_16bit(input, "LinearQQ")
             return input.new_empty(*input.shape[:-1], self.out_features)
         n, k = self.out_features, self.in_features
-        bias = None if self.bias is None else self.bias.data_ptr()
+        bias_ptr = None if bias is None else bias.data_ptr()
         dump = None if acc_dump is None else acc_dump.data_ptr()
         if two_call or not self._tensor_core_ok(input.numel() // k):
             qa, sa, dt, stream = self._quantize(input)
             m = qa.shape[0]
             y = torch.empty((m, n), dtype=input.dtype, device=input.device)
             ws = _workspace(input.device, _lib.workspace_bytes(_lib.WS_W4A4_GEMM, m, n, k))
-            _lib.call("asrq_w4a4_gemm", qa.data_ptr(), sa.data_ptr(), self.weight.data_ptr(), self.scales.data_ptr(),
-                      bias, y.data_ptr(), dump, m, n, k, self.group_size, dt, ws.data_ptr(), ws.numel(), stream)
+            _lib.call("asrq_w4a4_gemm", qa.data_ptr(), sa.data_ptr(), weight.data_ptr(), scales.data_ptr(),
+                      bias_ptr, y.data_ptr(), dump, m, n, k, self.group_size, dt, ws.data_ptr(), ws.numel(), stream)
         else:
             dt = _require_cuda_16bit(input, "LinearQQ")
             x2 = _as_2d(input, k)
@@ -620,8 +629,8 @@ class LinearQQ(LinearQ):
             stream = torch.cuda.current_stream(input.device).cuda_stream
             _lib.call(self._entry("hadamard_quant"), x2.data_ptr(), a8.data_ptr(), sa.data_ptr(), m, k,
                       1 if self.hadamard else 0, dt, stream)
-            _lib.call(self._entry("w4a4_gemm"), a8.data_ptr(), sa.data_ptr(), w8.data_ptr(), self.scales.data_ptr(),
-                      bias, y.data_ptr(), dump, m, n, k, self.group_size, dt, ws.data_ptr(), ws.numel(), stream)
+            _lib.call(self._entry("w4a4_gemm"), a8.data_ptr(), sa.data_ptr(), w8.data_ptr(), scales.data_ptr(),
+                      bias_ptr, y.data_ptr(), dump, m, n, k, self.group_size, dt, ws.data_ptr(), ws.numel(), stream)
         if _CHECK:
             check_status(input.device)
         return y.reshape(*input.shape[:-1], n)

@@ -1,9 +1,11 @@
 """A layer with the step ahead of it in the same kernel (asrq_linearq_a16_pre): the norm of one or two rows, silu(gate) * up of one."""
+import weakref
+
 import pytest
 import torch
 
 import asrq_b200
-from asrq_b200 import _lib, packing, qwen3, whisper
+from asrq_b200 import _lib, linear, packing, qwen3, whisper
 from asrq_b200.linear import PRE_LAYERNORM, PRE_RMSNORM, PRE_SILU_MUL, linear_after
 from gpu_util import DEV
 from tests.qwen3_util import toy_models
@@ -100,3 +102,53 @@ def test_qwen_step_of_one_sequence_runs_the_hooks_of_its_layers(name):
     eng.layers[0][name].register_forward_hook(lambda m, i, o: calls.append(o.shape))
     assert torch.equal(eng.generate(emb, 3, use_graph=False), want)
     assert len(calls) == 3                                                                  # the prompt and two steps
+
+
+def test_the_query_is_asked_on_the_tensors_device(monkeypatch):
+    """asrq_linearq_a16_pre_covers answers for the current device, as asrq_linearq_a16_pre runs on it."""
+    layer, gen = _layer(1280, 1280, 4, 128)
+    x, g = torch.randn(1, 1280, generator=gen, device=DEV).half(), torch.ones(1280, device=DEV, dtype=torch.float16)
+    inside, asked = [], []
+
+    class OnDevice(linear._on_device):
+        def __enter__(self):
+            inside.append(self.idx)
+            return super().__enter__()
+
+        def __exit__(self, *exc):
+            inside.pop()
+            return super().__exit__(*exc)
+
+    class Lib:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+            return (lambda *a: asked.append(list(inside)) or fn(*a)) if name == "asrq_linearq_a16_pre_covers" else fn
+    lib = _lib.load()
+    monkeypatch.setattr(linear, "_on_device", OnDevice)
+    monkeypatch.setattr(_lib, "load", Lib)
+    assert linear_after(layer, PRE_LAYERNORM, x, g, g, 1e-5) is not None
+    assert asked == [[x.device.index]]
+
+
+@pytest.mark.parametrize("way", ["linear_after", "forward_fused"])
+def test_operands_are_held_while_the_library_is_called(way, monkeypatch):
+    """Another thread may replace a layer's buffers during the call: those whose addresses were passed stay."""
+    layer, gen = _layer(1280, 1280, 4, 128)
+    x, g = torch.randn(1, 1280, generator=gen, device=DEV).half(), torch.ones(1280, device=DEV, dtype=torch.float16)
+    names, gone, call = ("weight", "scales", "zeros", "bias"), [], _lib.call
+
+    def replacing(name, *args):
+        for n in names:
+            old = weakref.ref(getattr(layer, n))
+            setattr(layer, n, getattr(layer, n).clone())
+            if old() is None:
+                gone.append(n)
+        return call(name, *args)
+    layer(x)                                          # the stream's workspace exists
+    monkeypatch.setattr(linear, "_native", None)
+    monkeypatch.setattr(_lib, "call", replacing)
+    if way == "linear_after":
+        assert linear_after(layer, PRE_LAYERNORM, x, g, g, 1e-5) is not None
+    else:
+        layer.forward_fused(x, gelu=True)
+    assert not gone
