@@ -9,12 +9,12 @@
 // and are combined, scaled by the group's scale and offset by zero * sum(x) once per quantisation
 // group in fp32; sum(x) over the group comes from MMAs against a matrix of ones (half as many).
 //
-// bf16 activations take the same route without conversion: a code in the low bits of 128.0's mantissa is 128 + code in bf16, and the
-// 128 * sum(x) too much goes with the zero's term.  Turning the activations into fp16 instead cost a pack instruction of a
+// bf16 activations take the same route without conversion: bf16 has no room for a subnormal code, so one goes through the low bits of
+// 128.0's mantissa and a fused multiply-add (bf16_codes).  Turning the activations into fp16 instead cost a pack instruction of a
 // quarter of the issue rate or less per pair in every block, and their range.  Chains of launches, before (fp16 codes, converted
-// activations, twice the MMAs against ones) -> now, us: 6144 -> 2048, 2-bit, 16 tokens, bf16 9.8 -> 6.2, fp16 6.9 -> 6.0; 2048 -> 12288, 4-bit,
-// one token 9.2 -> 6.5 and 7.1 -> 6.0; 1280 -> 1280, 4-bit, one token 3.6 -> 3.0 and 3.0 -> 2.85; 2-bit at 8 tokens of 1280 -> 3840
-// in fp16 went from 3.6 to 4.0.
+// activations, twice the MMAs against ones) -> now, us: 6144 -> 2048, 2-bit, 16 tokens, bf16 9.6 -> 6.0, fp16 6.7 -> 5.7; 2048 -> 12288, 4-bit,
+// one token 9.1 -> 6.4 and 6.9 -> 5.9; 1280 -> 1280, 4-bit, one token 4.2 -> 3.2 and 3.2 -> 3.05; 2-bit at 8 tokens of 1280 -> 3840
+// in fp16 went from 3.35 to 3.94.
 //
 // Work split: a warp owns a strip of 16 weight rows (rows g and g+8 per lane, g = lane/4) over one
 // to four "steps" (a step = 64 bytes of a row per lane quad = 128 k for 4-bit, 256 k for 2-bit),
@@ -99,6 +99,25 @@ __device__ __forceinline__ void mma_new(float (&d)[4], uint32_t a0, uint32_t a1,
         "{%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// The codes of field ty of the low byte of either half of q, as bf16 numbers: in the mantissa of 128.0 they are 128 + 2^at * code, and one
+// fused multiply-add, whose pipe is idle here, leaves the code, exactly.  A field that the seven bits do not hold is moved down first.
+// (The products of 128 + code, with 128 * sum(x) taken off by the zero's term, spare that, but then every fp32 sum carries 128 * sum(x):
+// 6 to 60 times the error relative to the output before it is rounded.  That form measured, us, -> this one: 2-bit 6144 -> 2048
+// at 1 / 8 / 16 tokens 4.1 / 4.5 / 6.0 -> 4.0 / 4.9 / 6.0, 4-bit 1280 -> 3840 3.6 / 4.3 / 4.1 -> 3.7 / 4.55 / 4.0, 2048 -> 6144 4.0 / 4.3 / 7.0
+// -> 4.1 / 4.35 / 7.2.)
+template <int BITS>
+__device__ __forceinline__ uint32_t bf16_codes(uint32_t q, int ty) {  // ty is a compile-time value after unrolling
+  const int sh = BITS * ty;
+  const bool moved = sh + BITS > 7;
+  const int at = moved ? 0 : sh;
+  const uint32_t field = ((1u << BITS) - 1u) << at;
+  const uint32_t v = lop3_and_or(moved ? q >> sh : q, field | (field << 16), 0x43004300u);
+  const uint32_t mul = (0x3f80u - (uint32_t(at) << 7)) * 0x10001u;   // 2^-at
+  const uint32_t add = (0xc300u - (uint32_t(at) << 7)) * 0x10001u;   // -128 * 2^-at
+  uint32_t r;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(v), "r"(mul), "r"(add));
+  return r;
 }
 // two 16-bit activations as floats
 template <bool BF16>
@@ -430,12 +449,10 @@ gemv_a16_kernel(const GemvParams p) {
           for (int ty = 0; ty < NT; ++ty) {
             uint32_t a0, a1, a2, a3;
             if (BF16) {
-              // the code in the low bits of 128.0's mantissa: 128 + code
-              const int sh = BITS * ty;
-              a0 = lop3_and_or(q0 >> sh, MASK0, 0x43004300u);
-              a1 = lop3_and_or(q1 >> sh, MASK0, 0x43004300u);
-              a2 = lop3_and_or(q0 >> (8 + sh), MASK0, 0x43004300u);
-              a3 = lop3_and_or(q1 >> (8 + sh), MASK0, 0x43004300u);
+              a0 = bf16_codes<BITS>(q0, ty);
+              a1 = bf16_codes<BITS>(q1, ty);
+              a2 = bf16_codes<BITS>(q0h, ty);
+              a3 = bf16_codes<BITS>(q1h, ty);
             } else {
               const uint32_t mask = MASK0 << (BITS * ty);
               a0 = q0 & mask; a1 = q1 & mask; a2 = q0h & mask; a3 = q1h & mask;
@@ -492,11 +509,9 @@ gemv_a16_kernel(const GemvParams p) {
         // once per group: combine the types (a field at bit BITS*ty carries 2^(BITS*ty) times its code;
         // a code in the lowest field is code * 2^-24 as an fp16 number), scale, add zero * sum(x)
         const int gidx = i * GPS + j;
-        // (bf16: every code is 128 too large, so sum(x) takes zero - 128 * scale)
         constexpr float kUnit = BF16 ? 1.f : 16777216.f;
         const float s0 = table_entry(ts0, gidx) * kUnit, s1 = table_entry(ts1, gidx) * kUnit;
-        const float z0 = BF16 ? fmaf(-128.f, s0, table_entry(tz0, gidx)) : table_entry(tz0, gidx);
-        const float z1 = BF16 ? fmaf(-128.f, s1, table_entry(tz1, gidx)) : table_entry(tz1, gidx);
+        const float z0 = table_entry(tz0, gidx), z1 = table_entry(tz1, gidx);
         float xt[MH][2];  // sums of tokens 2c and 2c + 1
         if (!XC && PAIR) {  // from the lanes that hold tokens g and g + 8 (MH == 1: two parts of token g's)
           float lo = accx[0][0], hi = accx[0][2];
