@@ -13,8 +13,8 @@
 // 128.0's mantissa and a fused multiply-add (bf16_codes).  Turning the activations into fp16 instead cost a pack instruction of a
 // quarter of the issue rate or less per pair in every block, and their range.  Chains of launches, before (fp16 codes, converted
 // activations, twice the MMAs against ones) -> now, us: 6144 -> 2048, 2-bit, 16 tokens, bf16 9.6 -> 6.0, fp16 6.7 -> 5.7; 2048 -> 12288, 4-bit,
-// one token 9.1 -> 6.4 and 6.9 -> 5.9; 1280 -> 1280, 4-bit, one token 4.2 -> 3.2 and 3.2 -> 3.05; 2-bit at 8 tokens of 1280 -> 3840
-// in fp16 went from 3.35 to 3.94.
+// one token 9.1 -> 6.4 and 6.9 -> 5.9; 1280 -> 1280, 4-bit, one token 4.2 -> 3.2 and 3.2 -> 3.05.  fp16 calls that took less before: 2-bit
+// 1280 -> 5120 at 4 / 8 tokens 3.05 / 3.55 (now 3.2 / 3.8), 2048 -> 6144 in groups of 64 at 1 / 2 tokens 3.85 / 4.15 (4.05 / 4.4).
 //
 // Work split: a warp owns a strip of 16 weight rows (rows g and g+8 per lane, g = lane/4) over one
 // to four "steps" (a step = 64 bytes of a row per lane quad = 128 k for 4-bit, 256 k for 2-bit),
@@ -197,7 +197,8 @@ constexpr int gemv_registers(int bits, int mh, int cpw, bool loop, bool tight, b
 // 2.0-2.5 for one round per warp.  Requesting the next round's words before this round's arithmetic,
 // in registers or through a cp.async ring in shared memory, measured slower: the variant is bound by
 // per-warp latency with 12-16 warps per SM at 128 registers, not by bytes in flight.)
-template <int BITS, bool BF16, int MH, int GPS, int CPW, bool XC, bool TRACE, bool LOOP = false, bool TIGHT = false, bool PRE = false>
+// LATE: see gemv_starts_next_late.
+template <int BITS, bool BF16, int MH, int GPS, int CPW, bool XC, bool TRACE, bool LOOP = false, bool TIGHT = false, bool PRE = false, bool LATE = false>
 __global__ void __maxnreg__(gemv_registers(BITS, MH, CPW, LOOP, TIGHT, PRE))
 gemv_a16_kernel(const GemvParams p) {
   constexpr int CPWORD = 32 / BITS;   // codes per 32-bit word (8 / 16)
@@ -238,7 +239,7 @@ gemv_a16_kernel(const GemvParams p) {
   // Let the next kernel on the stream start, and start streaming weights before this kernel's
   // own predecessor has finished: weights, scales and zeros are constants; only the activations
   // and the output depend on earlier kernels.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!LATE) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int rounds = LOOP ? p.R : 1;
   // word (j, t) of step i sits at byte i*64 + j*(64/GPS) + c*(16/GPS) + 4*t of the warp's row span
   auto row_ptr = [&](int step0) { return p.w + size_t(r0) * row_bytes + size_t(step0) * 64 + c * (16 / GPS); };
@@ -284,6 +285,7 @@ gemv_a16_kernel(const GemvParams p) {
       }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (LATE) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (p.residual && p.KQ > 1 && warp < FR) {
       const int n = n_base + g + ((warp >> 1) & 1) * 8, m = 8 * (warp >> 2) + 2 * c + (warp & 1);
       if (m < p.M) res_first = p.residual[size_t(m) * p.N + n];
@@ -665,12 +667,49 @@ GemvKernel kernel_for(int bits, bool bf16, int mh, int gps, int cpw, bool xc, bo
 // share the row strip, KQ * CPW = steps.  The pair is chosen so that the whole grid is resident at
 // once if possible (fewest waves, from the occupancy of the kernel variant), then for the most
 // warps: all loads of the layer go out together and the per-warp instruction streams are short.
+// The form of a kernel that starts the next launch late, or none
+template <int BITS, bool BF16, int MH>
+GemvKernel late_kernel_for(int gps, int cpw) {
+  switch (gps * 8 + cpw) {
+    case 1 * 8 + 1: return gemv_a16_kernel<BITS, BF16, MH, 1, 1, false, false, false, false, false, true>;
+    case 1 * 8 + 2: return gemv_a16_kernel<BITS, BF16, MH, 1, 2, false, false, false, false, false, true>;
+    case 2 * 8 + 1: return gemv_a16_kernel<BITS, BF16, MH, 2, 1, false, false, false, false, false, true>;
+    case 2 * 8 + 2: return gemv_a16_kernel<BITS, BF16, MH, 2, 2, false, false, false, false, false, true>;
+    case 4 * 8 + 1: return gemv_a16_kernel<BITS, BF16, MH, 4, 1, false, false, false, false, false, true>;
+    case 4 * 8 + 2: return gemv_a16_kernel<BITS, BF16, MH, 4, 2, false, false, false, false, false, true>;
+    default: return nullptr;
+  }
+}
+template <int BITS, bool BF16>
+GemvKernel late_kernel_for(int mh, int gps, int cpw) {
+  return mh == 1 ? late_kernel_for<BITS, BF16, 1>(gps, cpw) : late_kernel_for<BITS, BF16, 2>(gps, cpw);
+}
+GemvKernel late_kernel_for(int bits, bool bf16, int mh, int gps, int cpw) {
+  if (bits == 4) return bf16 ? late_kernel_for<4, true>(mh, gps, cpw) : late_kernel_for<4, false>(mh, gps, cpw);
+  return bf16 ? late_kernel_for<2, true>(mh, gps, cpw) : late_kernel_for<2, false>(mh, gps, cpw);
+}
+
 struct GemvSplit {
   int KQ, CPW;
   GemvKernel kern;
   int R = 0;        // rounds per warp (LOOP variants)
   bool tight = false;
 };
+
+// Whether a launch of one wave lets the next one start only behind its own wait.  Where the chip has room for several launches, each early
+// start lets the one after it start too, and the blocks of a launch lie crowded on the few SMs that had room; behind the wait at most two
+// launches are under way.  The sooner start is worth more where a warp has many weights to fetch or the launch fills the chip.  From three
+// tokens on; a chain of one token's launches would gain as well (4-bit 1280 -> 1280 2.95 -> 2.0), but a decoding step has other kernels
+// between them, for which that has not been measured.
+// Chains of launches, fp16, us at 4 / 8 / 16 tokens, early -> late: 2-bit 1280 -> 1280 3.0 / 3.6 / 4.9 -> 1.85 / 2.1 / 2.9, 1280 -> 3840 3.25 / 3.9 /
+// 5.2 -> 2.3 / 2.6 / 4.9, 1280 -> 5120 (2.2 blocks an SM) 3.4 / 4.1 / 5.3 -> 3.2 / 3.8 / 5.0; 4-bit 2048 -> 2048 2.8 / 3.4 / 4.7 -> 2.1 / 2.2 / 3.0, 1280 ->
+// 3840 (16 warps an SM) 3.7 / 4.5 / 4.1 -> 3.5 / 3.1 / 3.8, 2048 -> 4096 2.95 / 3.25 / 4.4 -> 2.7 / 2.9 / 4.4 (bf16 3.6 / 3.8 / 5.0 -> 3.5 / 3.85 / 4.9).
+// Beyond the line: 2-bit 2048 -> 6144 (2.6 blocks an SM) 4.4 / 4.7 / 6.6 -> 4.6 / 5.0 / 6.9; 4-bit 1280 -> 5120 (22 warps) 3.65 / 4.35 -> 3.8 / 4.5, 2048 ->
+// 6144 (21) 4.1 / 4.3 / 6.8 -> 4.2 / 4.5 / 7.45; 5120 -> 1280 3.2 / 3.8 / 5.65 -> 3.3 / 4.1 / 5.85.
+bool gemv_starts_next_late(int kq, int64_t N, int64_t K, int sm_count) {
+  const int64_t blocks = N / 16, sms = sm_count;
+  return K <= 2048 && 2 * blocks <= 5 * sms && blocks * kq <= 18 * sms;
+}
 
 GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool trace, int64_t N, int64_t K, int sm_count) {
   const int stepk = bits == 4 ? 128 : 256;
@@ -714,6 +753,14 @@ GemvSplit gemv_pick_split(int bits, bool bf16, int mh, int gps, bool xc, bool tr
       best.tight = k_tight;
       best_waves = waves;
     }
+  }
+  if (best.kern && best_waves == 1 && !xc && !trace && !best.tight && gemv_starts_next_late(best.KQ, N, K, sm_count)) {
+    GemvKernel form = late_kernel_for(bits, bf16, mh, gps, best.CPW);
+    int per_sm = 0;
+    if (form && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form, 32 * best.KQ, 0) == cudaSuccess && N / 16 <= int64_t(per_sm) * sm_count)
+      best.kern = form;
+    else
+      cudaGetLastError();
   }
   // Layers that do not fit one resident wave (or whose K is longer than 16 warps x 4 steps): small
   // blocks that walk K in rounds, so that the blocks sharing an SM overlap loads and arithmetic.

@@ -53,13 +53,15 @@ def _consumers(dtype):
     after = {"split K": _layer(1024, 512, 256), "decode": _layer(1024, 512, 128)}
     for name, layer in after.items():
         out[name] = 4, 1024, layer
+    out["decode of 12 rows"] = 12, 1024, after["decode"]   # (from three rows on, a small layer starts the next launch behind its own wait)
     residual = rand(4, 512)
     out["residual pass"] = 4, 1024, lambda h: after["split K"].forward_fused(h, residual=residual, gelu=True)
     return out
 
 
 NAMES = ["layer norm 4x1280", "layer norm 400x1280", "layer norm 4x1008", "layer norm 400x1008", "rms norm 4x2048", "rms norm 400x2048",
-         "rms norm 400x1008", "silu", "norm and rotary embedding", "head", "argmax", "argmax of an odd width", "split K", "decode", "residual pass"]
+         "rms norm 400x1008", "silu", "norm and rotary embedding", "head", "argmax", "argmax of an odd width", "split K", "decode",
+         "decode of 12 rows", "residual pass"]
 
 
 @pytest.mark.parametrize("name", NAMES)
