@@ -228,7 +228,7 @@ quant_int4_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, floa
 // quotient is computed.
 __device__ __forceinline__ float2 sub2(float2 a, float2 c) { return __ffma2_rn(c, make_float2(-1.f, -1.f), a); }
 
-// The rare path of quant4_bytes, out of line so that its call sites do not swell the kernel: IEEE division and round-half-even,
+// The rare path of quant8_bytes, out of line so that its call sites do not swell the kernel: IEEE division and round-half-even,
 // as magic + code.
 __device__ __noinline__ float4 quant4_exact(float2 v01, float2 v23, float s) {
   return make_float4(__fadd_rn(rintf(__fdiv_rn(v01.x, s)), 12582912.f), __fadd_rn(rintf(__fdiv_rn(v01.y, s)), 12582912.f),
@@ -417,11 +417,11 @@ __device__ __forceinline__ bool wait_landed(uint32_t bar, uint32_t parity) {
 // place i holds unit i with the sign (-1)^popcount(i & r): over the o of phase B a Walsh function, under which the butterflies of
 // strides T, 2 T and 4 T exchange their results.  Place m after phase B is o = m ^ s, s = t / 8, and the codes are stored accordingly;
 // no sign is ever put back.
-// Bound: instruction issue (about 2 300 warp instructions a token, a third of them packed ones and conversions that issue at half rate
-// or less; ncu: 56% of the issue slots).  128 threads of 32 values with two transposes and 32 warps per SM: 24.9 us for 6 000
+// Bound: no single one.  About 2 300 warp instructions a token, a third of them packed ones and conversions that issue at half rate
+// or less (ncu: 56% of the issue slots), with three barriers a token between them; the bytes go at half the copy rate.  128 threads of 32 values with two transposes and 32 warps per SM: 24.9 us for 6 000
 // tokens; more warps of this code, at 80 registers: no change.  Chains of launches, loads in the chain and a branch per four codes -> this
-// form, us: one token 2.6 -> 2.3, 250 4.6 -> 4.0, 6 000 23.6 -> 22.6, 16 000 57.8 -> 53.9; the 1024-wide kernel with a branch per eight codes
-// 1.74 -> 1.57, 2.0 -> 1.87, 6.9 -> 6.8, 13.45 -> 13.7.
+// form, us: one token 2.6 -> 2.3, 250 4.95 -> 4.4, 6 000 22.2 -> 21.5, 16 000 57.6 -> 53.5; the 1024-wide kernel with a branch per eight codes
+// 1.70 -> 1.56, 2.0 -> 1.9, 6.2 -> 6.0, 12.85 -> 12.67.
 template <int OUT, bool BF16>
 __global__ void __launch_bounds__(64, 8)
 hadamard_4096_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ qa, float* __restrict__ sa, int M) {

@@ -142,7 +142,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t base = (tc::smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t boxes = base + kDnRingBytes;  // two per epilogue warp
+  const uint32_t boxes = base + kDnRingBytes;  // kBoxes per epilogue warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = tc::cluster_ctarank();
   const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
@@ -156,7 +156,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   {
     const int i = threadIdx.x;
     if (i < 2 * kDnMaxStages + 4 + kBoxes * kDnEpilogueWarps) {
-      // a drained accumulator: eight warps of each CTA
+      // a drained accumulator: the epilogue warps of both CTAs
       tc::mbar_init(bar0 + 8u * i, (i >= 2 * kDnMaxStages + 2 && i < 2 * kDnMaxStages + 4) ? 2 * kDnEpilogueWarps : 1);
       tc::fence_barrier_init();
       tc::fence_proxy_async_smem();

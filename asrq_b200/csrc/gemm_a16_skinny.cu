@@ -31,7 +31,7 @@
 // arithmetic left out).  Chains of launches, W4, unpacking through shared memory -> this form, us at 32 / 64 / 128 / 259 tokens:
 // 1280 -> 1280 4.3 / 4.6 / 5.9 / 6.6 -> 3.9 / 4.1 / 5.5 / 6.4; 1280 -> 5120 6.1 / 6.8 / 8.1 / 11.8 -> 5.0 / 6.0 / 8.0 / 11.0; 2048 -> 4096 6.7 / 7.5 /
 // 8.7 / 12.6 -> 5.3 / 6.6 / 8.7 / 11.3; 2048 -> 12288 15.3 / 16.1 / 17.9 -> 12.9 / 14.0 / 15.6; 6144 -> 2048 10.5 / 11.4 / 12.4 / 16.5 -> 8.5 / 10.0 / 12.1 /
-// 15.7; bf16 2048 -> 4096 at 80 to 128 tokens 0.2 us slower.  More slots than the MMAs' round trip needs changed nothing.
+// 15.7; bf16 2048 -> 4096 at 64 / 80 / 96 / 128 tokens 7.6 / 7.9 / 8.05 / 8.8 -> 6.6 / 7.85 / 8.0 / 8.7.  More slots than the MMAs' round trip needs changed nothing.
 //
 // Prompts of some hundred tokens: the persistent kernels give a tile the whole of K, and with few tiles most SMs idle (1280 x 5120
 // at 260 to 1500 tokens: 31 us on 20 to 60 of them).  Here K is cut so that one wave fills the chip.
